@@ -59,6 +59,15 @@ int ws_get(fknn_index *idx, int slot, size_t bytes, void **p) {
   return FKNN_OK;
 }
 
+void ws_drop(fknn_index *idx, int slot) {
+  DevBuf &b = idx->ws[slot];
+  if (!b.p) return;
+  cudaDeviceSynchronize();  // in-flight work may still read it
+  dev_free(idx, b.p, b.bytes);
+  b.p = nullptr;
+  b.bytes = 0;
+}
+
 int hs_get(fknn_index *idx, int slot, size_t bytes, void **p) {
   HostBuf &b = idx->hs[slot];
   if (b.bytes < bytes) {

@@ -67,13 +67,18 @@ __device__ __forceinline__ uint64_t global_ns() {
 }
 
 // Bounded wait: returns false (and raises ERR_WAIT_TIMEOUT) if the phase
-// has not completed within WAIT_NS.
+// has not completed within WAIT_NS.  The timer is first read after 64 polls:
+// reading it costs more than most waits last.
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity, int *err) {
   if (mbar_try_wait(bar, parity)) return true;
-  const uint64_t t0 = global_ns();
-  for (uint32_t it = 0; it < WAIT_LIMIT; ++it) {
+  uint64_t t0 = 0;
+  for (uint32_t it = 1; it < WAIT_LIMIT; ++it) {
     if (mbar_try_wait(bar, parity)) return true;
-    if ((it & 63u) == 63u && global_ns() - t0 > WAIT_NS) break;
+    if ((it & 63u) == 0u) {
+      const uint64_t t = global_ns();
+      if (t0 == 0) t0 = t;
+      else if (t - t0 > WAIT_NS) break;
+    }
   }
   atomicOr(err, ERR_WAIT_TIMEOUT);
   return false;

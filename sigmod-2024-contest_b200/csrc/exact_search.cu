@@ -4,18 +4,21 @@
 //   1. k_query_prep   predicate -> contiguous slab [s, e) of one row order
 //                     (binary search on the sorted attribute columns), ||q||^2
 //   2. host planner   slabs <= SMALL_SLAB -> row-by-row exact scan; others
-//                     sorted and grouped into 64-query tiles, split into
+//                     sorted and grouped into 256-query tiles, split into
 //                     (tile, row chunk) work items
-//   3. k_tile_stage   query tiles in the [101][64] layout of the base blocks
-//   4. k_screen       FP32 FFMA contraction q.x over 64-row blocks streamed by
-//                     the TMA bulk engine; ds = |x|^2+|q|^2-2q.x; rows whose
-//                     ds can still reach the running k-th bound are kept in a
-//                     per-(item, query) candidate list that a warp bitonic
-//                     sort compacts; the bound is shared across CTAs.
-//   5. k_merge        per query: union of its items' lists, k-th bound, then
+//   3. k_exact_screen tensor-core contraction q.x of float accuracy (two
+//                     fp16 pieces a side) over the 64-row blocks
+//                     (exact_screen.cu); ds = |x|^2+|q|^2-2q.x; rows whose ds
+//                     can still reach the running k-th bound are kept in a
+//                     per-(item, query) candidate list; the bound is shared
+//                     across CTAs.  A pilot pass over every pilot_stride-th
+//                     row block seeds the bounds (k_exact_seed).
+//   4. k_merge        per query: union of its items' lists, k-th bound, then
 //                     exact re-score of the survivors with the reference's
-//                     sequential arithmetic, (dist, id) sort, top-k out.
-//   6. k_exact_scan   small slabs and any query whose candidates overflowed:
+//                     sequential arithmetic, (dist, id) order, top-k out.  A
+//                     query whose seed lay below its k-th is found here and
+//                     screened and merged once more without one.
+//   5. k_exact_scan   small slabs and any query whose candidates overflowed:
 //                     exact distances row by row, block select on (dist, id).
 // Ids and distances equal the reference's bit for bit: every row that can
 // be in the top k (screening error bound in screen_eps) is re-scored with
@@ -141,408 +144,243 @@ __global__ void k_count(const float *__restrict__ meta, uint32_t nq, uint32_t n,
   counts[i] = e - s;
 }
 
-// Query tiles in the base-block layout: [101][64] (dims, then |q|^2).
-__global__ void k_tile_stage(const float *__restrict__ q, const QueryDesc *__restrict__ desc,
-                             const int32_t *__restrict__ lane_q, float *__restrict__ qtiles) {
-  const uint32_t t = blockIdx.x;
-  __shared__ float tile[TQ][DIM + 1];
-  for (int i = threadIdx.x; i < TQ * DIM; i += blockDim.x) {
-    int l = i / DIM, d = i % DIM;
-    int32_t qi = lane_q[t * TQ + l];
-    tile[l][d] = qi >= 0 ? q[(uint64_t)qi * DIM + d] : 0.f;
-  }
-  __syncthreads();
-  float *out = qtiles + (uint64_t)t * BLK_FLOATS;
-  for (int i = threadIdx.x; i < TQ * DIM; i += blockDim.x) {
-    int d = i / TQ, l = i % TQ;
-    out[d * TQ + l] = tile[l][d];
-  }
-  for (int l = threadIdx.x; l < TQ; l += blockDim.x) {
-    int32_t qi = lane_q[t * TQ + l];
-    out[DIM * TQ + l] = qi >= 0 ? desc[qi].qn : 0.f;
-  }
-}
-
-// -------------------------------------------------------------- screen --
-
-constexpr int SC_CONSUMERS = 4;                   // compute warps
-constexpr int SC_THREADS = (SC_CONSUMERS + 1) * 32;  // + one producer warp
-constexpr int SC_STAGES = 3;
-constexpr int SC_REFRESH = 16;  // sub-tiles between reads of the shared bound
-
-// Each consumer warp w owns the candidate lists of queries [16w, 16w+16) of
-// the tile: with the thread mapping below (rows ty*4.., queries tx*8..,
-// tx = tid/16) only warp w ever pushes into them, so lists are compacted by
-// their owner with no CTA-wide barrier.  Row blocks stream through a ring of
-// SC_STAGES buffers: the producer warp issues one bulk copy per 64-row block
-// after the four consumer warps released the slot (empty barrier).
-struct ScreenSmem {
-  float qs[BLK_FLOATS];
-  float xs[SC_STAGES][BLK_FLOATS];
-  float push[TQ];     // largest ds worth keeping
-  float thr[TQ];      // current upper bound T on the k-th distance
-  float qn[TQ];
-  int cnt[TQ];
-  uint32_t ls[TQ], le[TQ];
-  int32_t lq[TQ];
-  uint64_t full[SC_STAGES], empty[SC_STAGES], qbar;
-};
-
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
-// Sort, bound and trim one (item, query) candidate list.  Whole warp.
-__device__ __noinline__ void compact_list(Candidate *list, ScreenSmem &sm, int L, uint32_t k, uint32_t *T_global,
-                                          uint32_t *ovf) {
-  const int lane = threadIdx.x & 31;
-  const int n = sm.cnt[L];
-  float key[CAP / 32];
-  uint32_t val[CAP / 32];
-#pragma unroll
-  for (int j = 0; j < CAP / 32; ++j) {
-    int e = j * 32 + lane;
-    if (e < n) {
-      Candidate c = list[e];
-      key[j] = c.ds;
-      val[j] = c.pos;
-    } else {
-      key[j] = INFINITY;
-      val[j] = 0xffffffffu;
-    }
-  }
-  warp_bitonic_sort<CAP / 32>(key, val);
-  const float qn = sm.qn[L];
-  const int32_t qi = sm.lq[L];
-  float T = sm.thr[L];
-  if (n >= (int)k) {
-    const int e = (int)k - 1;
-    float mine = key[0];
-#pragma unroll
-    for (int j = 1; j < CAP / 32; ++j)
-      if (j == (e >> 5)) mine = key[j];
-    const float kth = __shfl_sync(0xffffffffu, mine, e & 31);
-    T = fminf(T, screen_hi(kth, qn));
-  }
-  const float Tg = sortable_f32(ld_volatile_u32(T_global + qi));
-  if (Tg < T) T = Tg;
-  if (lane == 0 && T < Tg) atomicMin(T_global + qi, f32_sortable(T));
-  int kept = 0;
-  const uint32_t lt = (1u << lane) - 1u;
-#pragma unroll
-  for (int j = 0; j < CAP / 32; ++j) {
-    const bool keep = (j * 32 + lane) < n && screen_lo(key[j], qn) <= T;
-    const uint32_t b = __ballot_sync(0xffffffffu, keep);
-    if (keep) {
-      Candidate c;
-      c.ds = key[j];
-      c.pos = val[j];
-      list[kept + __popc(b & lt)] = c;
-    }
-    kept += __popc(b);
-  }
-  __syncwarp();
-  if (lane == 0) {
-    if (kept > CAP - BLK) {
-      // More near-ties than the list can hold: hand the query to the exact scan.
-      ovf[qi] = 1u;
-      sm.cnt[L] = 0;
-      sm.thr[L] = -INFINITY;
-      sm.push[L] = -INFINITY;
-    } else {
-      sm.cnt[L] = kept;
-      sm.thr[L] = T;
-      sm.push[L] = (T == INFINITY) ? INFINITY : screen_push_limit(T, qn);
-    }
-  }
-  __syncwarp();
-}
-
-__global__ void __launch_bounds__(SC_THREADS, 2)
-    k_screen(const WorkItem *__restrict__ items, const Tile *__restrict__ tiles, const float *__restrict__ qtiles,
-             const int32_t *__restrict__ lane_q, const uint32_t *__restrict__ lane_s,
-             const uint32_t *__restrict__ lane_e, const float *__restrict__ blocks_t,
-             const float *__restrict__ blocks_c, uint32_t *__restrict__ T_global, uint32_t *__restrict__ ovf,
-             Candidate *__restrict__ out, uint32_t *__restrict__ out_cnt, uint32_t k, uint32_t stride, int *err) {
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  ScreenSmem &sm = *reinterpret_cast<ScreenSmem *>(smem_raw);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const uint32_t item_id = blockIdx.x;
-  const WorkItem it = items[item_id];
-  const Tile tl = tiles[it.tile];
-  const float *blocks = tl.order == ORDER_TIME ? blocks_t : blocks_c;
-  // every stride-th row block of the item (stride 1: all of them)
-  const uint32_t nsub = (it.blk1 - it.blk0 + stride - 1) / stride;
-  Candidate *out_item = out + (uint64_t)item_id * TQ * CAP;
-
-  if (tid == 0) {
-    for (int s = 0; s < SC_STAGES; ++s) {
-      mbar_init(&sm.full[s], 1);
-      mbar_init(&sm.empty[s], SC_CONSUMERS);
-    }
-    mbar_init(&sm.qbar, 1);
-    fence_mbar_init();
-  }
-  __syncthreads();  // the only CTA-wide barrier
-
-  if (warp == SC_CONSUMERS) {
-    // ---------------- producer: one lane issues every bulk copy
-    if (lane == 0) {
-      mbar_arrive_expect_tx(&sm.qbar, BLK_BYTES);
-      bulk_g2s(sm.qs, qtiles + (uint64_t)it.tile * BLK_FLOATS, BLK_BYTES, &sm.qbar);
-      uint32_t issued = 0;
-      for (uint32_t sub = 0; sub < nsub; ++sub) {
-        const int st = sub % SC_STAGES;
-        if (sub >= SC_STAGES && !mbar_wait_bounded(&sm.empty[st], ((sub / SC_STAGES) - 1) & 1, err)) break;
-        mbar_arrive_expect_tx(&sm.full[st], BLK_BYTES);
-        bulk_g2s(sm.xs[st], blocks + (uint64_t)(it.blk0 + sub * stride) * BLK_FLOATS, BLK_BYTES, &sm.full[st]);
-        ++issued;
-      }
-      // every issued copy must have landed before the CTA may exit
-      mbar_wait_bounded(&sm.qbar, 0, err);
-      for (uint32_t i = issued > SC_STAGES ? issued - SC_STAGES : 0; i < issued; ++i)
-        mbar_wait_bounded(&sm.full[i % SC_STAGES], (i / SC_STAGES) & 1, err);
-    }
-    return;
-  }
-
-  // ---------------- consumers
-  // waits are warp-uniform: the lanes' timers may disagree at the deadline
-  bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(&sm.qbar, 0, err));
-  if (lane < 16) {
-    const int L = 16 * warp + lane;
-    const int32_t qi = lane_q[it.tile * TQ + L];
-    sm.lq[L] = qi;
-    sm.cnt[L] = 0;
-    sm.qn[L] = sm.qs[DIM * TQ + L];
-    if (qi >= 0) {
-      sm.ls[L] = lane_s[it.tile * TQ + L];
-      sm.le[L] = lane_e[it.tile * TQ + L];
-      const float T = sortable_f32(ld_volatile_u32(T_global + qi));
-      sm.thr[L] = T;
-      sm.push[L] = (T == INFINITY) ? INFINITY : screen_push_limit(T, sm.qn[L]);
-      if (ld_volatile_u32(ovf + qi)) sm.push[L] = -INFINITY;
-    } else {
-      sm.ls[L] = sm.le[L] = 0;
-      sm.thr[L] = -INFINITY;
-      sm.push[L] = -INFINITY;
-    }
-  }
-  __syncwarp();
-
-  const int ty = tid & 15;  // rows ty*4 .. ty*4+3 of the 64-row block
-  const int tx = tid >> 4;  // queries tx*8 .. tx*8+7 of the tile (owned by this warp)
-  for (uint32_t sub = 0; sub < nsub && ok; ++sub) {
-    const int st = sub % SC_STAGES;
-    if (!__all_sync(0xffffffffu, mbar_wait_bounded(&sm.full[st], (sub / SC_STAGES) & 1, err))) {
-      ok = false;
-      break;
-    }
-    const float *xs = sm.xs[st];
-    float acc[4][8];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
-    const float4 *xr = reinterpret_cast<const float4 *>(xs) + ty;
-    const float4 *qr = reinterpret_cast<const float4 *>(sm.qs) + tx * 2;
-#pragma unroll 10
-    for (int d = 0; d < DIM; ++d) {
-      const float4 a = xr[d * (BLK / 4)];
-      const float4 b0 = qr[d * (TQ / 4)];
-      const float4 b1 = qr[d * (TQ / 4) + 1];
-      const float av[4] = {a.x, a.y, a.z, a.w};
-      const float bv[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
-    }
-    const float4 xn4 = reinterpret_cast<const float4 *>(xs + DIM * BLK)[ty];
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&sm.empty[st]);  // this warp is done with the slot
-    // epilogue: ds = (|x|^2 + |q|^2) - 2 q.x; keep rows that can reach the bound
-    const float xn[4] = {xn4.x, xn4.y, xn4.z, xn4.w};
-    const uint32_t row0 = (it.blk0 + sub * stride) * BLK + ty * 4;
-    uint32_t pass = 0;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int L = tx * 8 + j;
-      const float pl = sm.push[L];
-      const float qn = sm.qn[L];
-      const uint32_t s = sm.ls[L], e = sm.le[L];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float ds = fmaf(-2.f, acc[i][j], xn[i] + qn);
-        acc[i][j] = ds;
-        const uint32_t p = row0 + i;
-        pass |= (uint32_t)(ds <= pl && p >= s && p < e) << (j * 4 + i);
-      }
-    }
-    if (__any_sync(0xffffffffu, pass != 0)) {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          if (pass & (1u << (j * 4 + i))) {
-            const int L = tx * 8 + j;
-            const int idx = atomicAdd(&sm.cnt[L], 1);
-            Candidate c;
-            c.ds = acc[i][j];
-            c.pos = row0 + i;
-            out_item[(uint64_t)L * CAP + idx] = c;
-          }
-        }
-      }
-      __syncwarp();
-    }
-    // own lists near capacity are compacted; bounds refreshed from other CTAs
-    {
-      const int L = 16 * warp + (lane & 15);
-      const bool need = lane < 16 && sm.cnt[L] > CAP - BLK;
-      uint32_t m = __ballot_sync(0xffffffffu, need);
-      while (m) {
-        const int b = __ffs(m) - 1;
-        m &= m - 1;
-        compact_list(out_item + (uint64_t)(16 * warp + b) * CAP, sm, 16 * warp + b, k, T_global, ovf);
-      }
-      if ((sub % SC_REFRESH) == SC_REFRESH - 1 && lane < 16 && !need) {
-        const int32_t qi = sm.lq[L];
-        if (qi >= 0 && sm.push[L] != -INFINITY) {
-          const float Tg = sortable_f32(ld_volatile_u32(T_global + qi));
-          if (Tg < sm.thr[L]) {
-            sm.thr[L] = Tg;
-            sm.push[L] = screen_push_limit(Tg, sm.qn[L]);
-          }
-        }
-      }
-      __syncwarp();
-    }
-  }
-  if (!ok) {
-    // A bulk copy never landed (bounded wait gave up): this warp's queries
-    // are answered by the exact scan instead.
-    if (lane < 16) {
-      const int L = 16 * warp + lane;
-      if (sm.lq[L] >= 0) ovf[sm.lq[L]] = 1u;
-      out_cnt[(uint64_t)item_id * TQ + L] = 0;
-    }
-    return;
-  }
-  // final trim of this warp's non-empty lists
-  for (int b = 0; b < 16; ++b) {
-    const int L = 16 * warp + b;
-    if (sm.cnt[L] > 0) compact_list(out_item + (uint64_t)L * CAP, sm, L, k, T_global, ovf);
-  }
-  if (lane < 16) out_cnt[(uint64_t)item_id * TQ + 16 * warp + lane] = (uint32_t)sm.cnt[16 * warp + lane];
-}
-
 // --------------------------------------------------------------- merge --
 
-constexpr int MG_THREADS = 256;
+constexpr int MG_THREADS = 128;
 
+template <int MCAP>
 struct MergeSmem {
-  float key[MERGE_CAP];
-  uint32_t val[MERGE_CAP];
+  float key[MCAP];
+  uint32_t val[MCAP];
   uint64_t ekey[RESCORE_CAP];
   float qv[DIM];
-  uint32_t cnt_prefix[MG_THREADS + 1];
-  int total, surv, status;
+  uint32_t cnt_prefix[MAX_ITEMS_PER_TILE + 1];
+  uint32_t hist[256];
+  uint32_t red[4];
+  int total, surv;
 };
 
-__global__ void __launch_bounds__(MG_THREADS)
-    k_merge(const uint32_t *__restrict__ big_q, const uint32_t *__restrict__ big_tile,
-            const uint32_t *__restrict__ big_lane, const Tile *__restrict__ tiles, const uint32_t *__restrict__ item_slot,
-            const Candidate *__restrict__ out,
-            const uint32_t *__restrict__ out_cnt, const QueryDesc *__restrict__ desc, const float *__restrict__ q,
-            const float *__restrict__ vecs, const uint32_t *__restrict__ perm_t, const uint32_t *__restrict__ perm_c,
-            const uint32_t *__restrict__ T_global, const uint32_t *__restrict__ ovf, uint32_t *__restrict__ ovf_list,
-            uint32_t *__restrict__ ovf_count, uint32_t k, uint32_t *__restrict__ ids, float *__restrict__ dists) {
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  MergeSmem &sm = *reinterpret_cast<MergeSmem *>(smem_raw);
+struct ExactMergeArgs {
+  const uint32_t *big_q, *big_tile, *big_lane;
+  const Tile *tiles;
+  const uint32_t *item_slot;
+  const Candidate *out;
+  const uint32_t *out_cnt;
+  const QueryDesc *desc;
+  const float *q, *vecs;
+  const uint32_t *perm_t, *perm_c;
+  uint32_t *T_global;
+  const uint32_t *ovf;
+  uint32_t *ovf_list, *ovf_count;  // queries for the exact scan
+  // queries whose seeded bound may lie below their k-th (NULL: bounds are not seeded)
+  uint32_t *redo_list, *redo_count, *redo_skip;
+  uint32_t k;
+  uint32_t *ids;
+  float *dists;
+};
+
+// kth smallest (1-based, kth <= n) of key[0 .. n) in shared memory, as its
+// f32_sortable image: a radix select of the whole block that starts below
+// the bits all keys share.  red: 4 words of shared memory.
+__device__ uint32_t block_kth(const float *key, int n, uint32_t kth, uint32_t *hist, uint32_t *red) {
+  const int tid = threadIdx.x, lane = tid & 31;
+  if (tid == 0) {
+    red[0] = 0xffffffffu;
+    red[1] = 0;
+  }
+  __syncthreads();
+  uint32_t mn = 0xffffffffu, mx = 0;
+  for (int i = tid; i < n; i += MG_THREADS) {
+    const uint32_t u = f32_sortable(key[i]);
+    mn = min(mn, u);
+    mx = max(mx, u);
+  }
+  mn = __reduce_min_sync(0xffffffffu, mn);
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  if (lane == 0) {
+    atomicMin(&red[0], mn);
+    atomicMax(&red[1], mx);
+  }
+  __syncthreads();
+  mn = red[0];
+  mx = red[1];
+  int hi = mn == mx ? 0 : 32 - __clz(mn ^ mx);
+  uint32_t mask = hi == 32 ? 0u : ~((1u << hi) - 1u);
+  uint32_t prefix = mn & mask, remaining = kth;
+  while (hi > 0) {
+    const int w = min(8, hi), shift = hi - w;
+    for (int i = tid; i < 256; i += MG_THREADS) hist[i] = 0;
+    __syncthreads();
+    for (int i = tid; i < n; i += MG_THREADS) {
+      const uint32_t u = f32_sortable(key[i]);
+      if ((u & mask) == prefix) atomicAdd(&hist[(u >> shift) & ((1u << w) - 1)], 1u);
+    }
+    __syncthreads();
+    if (tid < 32) {
+      uint32_t local[8], sum = 0;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        local[j] = hist[lane * 8 + j];
+        sum += local[j];
+      }
+      uint32_t inc = sum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += v;
+      }
+      uint32_t c = inc - sum;
+      if (c < remaining && inc >= remaining) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          if (c < remaining && c + local[j] >= remaining) {
+            red[2] = lane * 8 + j;
+            red[3] = c;
+          }
+          c += local[j];
+        }
+      }
+    }
+    __syncthreads();
+    prefix |= red[2] << shift;
+    remaining -= red[3];
+    mask |= ((1u << w) - 1) << shift;
+    hi = shift;
+  }
+  __syncthreads();
+  return prefix;
+}
+
+// seq_l2_strided over a 16-byte aligned row, four dimensions per load
+__device__ __forceinline__ float seq_l2_row(const float *__restrict__ x, const float *q) {
+  const float4 *x4 = reinterpret_cast<const float4 *>(x);
+  float r = 0.f;
+#pragma unroll 5
+  for (int d = 0; d < DIM / 4; ++d) {
+    const float4 v = __ldg(x4 + d);
+    const float e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      float t = __fsub_rn(e[j], q[4 * d + j]);
+      t = __fmul_rn(t, t);
+      r = __fadd_rn(r, t);
+    }
+  }
+  return r;
+}
+
+// One big query b (index into the plan's big-query arrays): gather its
+// lists, bound the k-th distance over their union, re-score the survivors
+// with the reference's arithmetic, order them by (dist, id).  A query with
+// more than MCAP candidates goes to `spill` (the large merge) or, from the
+// large merge, to the exact scan.  Returns are block-uniform.
+template <int MCAP>
+__device__ void exact_merge_one(const ExactMergeArgs &A, uint32_t b, MergeSmem<MCAP> &sm, uint32_t *spill,
+                                uint32_t *spill_count) {
   const int tid = threadIdx.x;
-  const uint32_t qi = big_q[blockIdx.x];
-  if (ovf[qi]) {
-    if (tid == 0) ovf_list[atomicAdd(ovf_count, 1u)] = qi;
+  const uint32_t k = A.k;
+  const uint32_t qi = A.big_q[b];
+  if (A.ovf[qi]) {
+    if (tid == 0) A.ovf_list[atomicAdd(A.ovf_count, 1u)] = qi;
     return;
   }
-  const Tile tl = tiles[big_tile[blockIdx.x]];
-  const uint32_t L = big_lane[blockIdx.x];
+  const Tile tl = A.tiles[A.big_tile[b]];
+  const uint32_t L = A.big_lane[b];
   const uint32_t nitems = tl.item1 - tl.item0;
-  const QueryDesc dsc = desc[qi];
+  const QueryDesc dsc = A.desc[qi];
   const float qn = dsc.qn;
-  for (int d = tid; d < DIM; d += MG_THREADS) sm.qv[d] = q[(uint64_t)qi * DIM + d];
-  // 1. gather the lists: item offsets (a tile has at most a few dozen
-  // items), then the whole block copies each list
-  // more items than offset slots: the exact scan answers the query
-  list_offsets(item_slot, tl.item0, nitems, out_cnt, L, TQ, sm.cnt_prefix, &sm.total, MG_THREADS, MERGE_CAP + 1);
+  for (int d = tid; d < DIM; d += MG_THREADS) sm.qv[d] = A.q[(uint64_t)qi * DIM + d];
+  // 1. gather the lists: item offsets, then the whole block copies each list
+  list_offsets(A.item_slot, tl.item0, nitems, A.out_cnt, L, EXACT_TQ, sm.cnt_prefix, &sm.total, MAX_ITEMS_PER_TILE,
+               MERGE_CAP + 1);
+  if (tid == 0) sm.surv = 0;
   __syncthreads();
   const int M = sm.total;
-  if (M > MERGE_CAP) {
-    if (tid == 0) ovf_list[atomicAdd(ovf_count, 1u)] = qi;
+  if (M > MCAP) {
+    if (tid == 0) {
+      if (spill && M <= MERGE_CAP) spill[atomicAdd(spill_count, 1u)] = b;
+      else A.ovf_list[atomicAdd(A.ovf_count, 1u)] = qi;
+    }
     return;
   }
   for (uint32_t i = 0; i < nitems; ++i) {
-    const uint64_t item = item_slot[tl.item0 + i];
+    const uint64_t item = A.item_slot[tl.item0 + i];
     const uint32_t base = sm.cnt_prefix[i];
     const uint32_t c = (i + 1 < nitems ? sm.cnt_prefix[i + 1] : (uint32_t)M) - base;
-    const Candidate *src = out + (item * TQ + L) * CAP;
+    const Candidate *src = A.out + (item * EXACT_TQ + L) * EXACT_CAP;
     for (uint32_t j = tid; j < c; j += MG_THREADS) {
       const Candidate cd = src[j];
       sm.key[base + j] = cd.ds;
       sm.val[base + j] = cd.pos;
     }
   }
-  int np2 = 32;
-  while (np2 < M) np2 <<= 1;
-  for (int i = M + tid; i < np2; i += MG_THREADS) {
-    sm.key[i] = INFINITY;
-    sm.val[i] = 0xffffffffu;
+  __syncthreads();
+  // 2. k-th bound over the union.  A seeded bound admitted every row that
+  //    can be in the top k iff the union's k-th is proven to lie below it
+  const float Tg = sortable_f32(A.T_global[qi]);
+  float T = Tg;
+  bool proven = false;
+  if (M >= (int)k) {
+    const float h = screen_hi(sortable_f32(block_kth(sm.key, M, k, sm.hist, sm.red)), qn);
+    proven = h <= Tg + 5e-7f * fabsf(Tg);  // (screen_hi's own slack of 1e-6 covers the tolerance)
+    T = fminf(T, h);
   }
-  __syncthreads();
-  // 2. k-th bound over the union
-  block_bitonic_sort_kv(sm.key, sm.val, np2);
-  float T = sortable_f32(T_global[qi]);
-  if (M >= (int)k) T = fminf(T, screen_hi(sm.key[k - 1], qn));
-  // 3. survivors (a prefix of the sorted list up to rounding; scan anyway)
-  if (tid == 0) sm.surv = 0;
-  __syncthreads();
+  if (A.redo_list && !proven) {
+    if (tid == 0) {
+      A.redo_list[atomicAdd(A.redo_count, 1u)] = b;
+      A.redo_skip[qi] = 0u;
+      A.T_global[qi] = f32_sortable(INFINITY);
+    }
+    return;
+  }
+  // 3. survivors
   for (int i = tid; i < M; i += MG_THREADS) {
     if (screen_lo(sm.key[i], qn) <= T) {
-      int slot = atomicAdd(&sm.surv, 1);
-      if (slot < RESCORE_CAP) {
-        const uint32_t pos = sm.val[i];
-        const uint32_t id = (dsc.order == ORDER_TIME ? perm_t : perm_c)[pos];
-        sm.ekey[slot] = (uint64_t)id;  // re-scored below
-      }
+      const int slot = atomicAdd(&sm.surv, 1);
+      if (slot < RESCORE_CAP) sm.ekey[slot] = (dsc.order == ORDER_TIME ? A.perm_t : A.perm_c)[sm.val[i]];
     }
   }
   __syncthreads();
   const int S = sm.surv;
   if (S > RESCORE_CAP) {
-    if (tid == 0) ovf_list[atomicAdd(ovf_count, 1u)] = qi;
+    if (tid == 0) A.ovf_list[atomicAdd(A.ovf_count, 1u)] = qi;
     return;
   }
   // 4. exact re-score (distance.h:62-72 order of operations)
   for (int i = tid; i < S; i += MG_THREADS) {
     const uint32_t id = (uint32_t)sm.ekey[i];
-    const float d = seq_l2_strided(vecs + (uint64_t)id * DIM, 1, sm.qv);
-    sm.ekey[i] = exact_key(d, id);
+    sm.ekey[i] = exact_key(seq_l2_row(A.vecs + (uint64_t)id * DIM, sm.qv), id);
   }
-  int sp2 = 32;
-  while (sp2 < S) sp2 <<= 1;
-  for (int i = S + tid; i < sp2; i += MG_THREADS) sm.ekey[i] = ~0ull;
   __syncthreads();
-  block_bitonic_sort(sm.ekey, sp2);
-  for (uint32_t j = tid; j < k; j += MG_THREADS) {
-    uint32_t id = 0xffffffffu;
-    float d = INFINITY;
-    if ((int)j < S) {
-      id = (uint32_t)sm.ekey[j];
-      d = sortable_f32((uint32_t)(sm.ekey[j] >> 32));
+  // 5. each survivor's rank is the number of smaller keys (keys are distinct:
+  //    a row appears once), counted by its thread
+  for (int i = tid; i < S; i += MG_THREADS) {
+    const uint64_t e = sm.ekey[i];
+    uint32_t rank = 0;
+    for (int j = 0; j < S; ++j) rank += sm.ekey[j] < e ? 1u : 0u;
+    if (rank < k) {
+      A.ids[(uint64_t)qi * k + rank] = (uint32_t)e;
+      if (A.dists) A.dists[(uint64_t)qi * k + rank] = sortable_f32((uint32_t)(e >> 32));
     }
-    ids[(uint64_t)qi * k + j] = id;
-    if (dists) dists[(uint64_t)qi * k + j] = d;
+  }
+  for (uint32_t j = (uint32_t)S + tid; j < k; j += MG_THREADS) {
+    A.ids[(uint64_t)qi * k + j] = 0xffffffffu;
+    if (A.dists) A.dists[(uint64_t)qi * k + j] = INFINITY;
+  }
+}
+
+// work == nullptr: block b merges big query b (grid = number of big
+// queries); else the blocks stride over the *work_count entries of work.
+template <int MCAP>
+__global__ void __launch_bounds__(MG_THREADS)
+    k_merge(ExactMergeArgs A, uint32_t nbig, const uint32_t *__restrict__ work, const uint32_t *__restrict__ work_count,
+            uint32_t *__restrict__ spill, uint32_t *__restrict__ spill_count) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  MergeSmem<MCAP> &sm = *reinterpret_cast<MergeSmem<MCAP> *>(smem_raw);
+  const uint32_t nwork = work ? *work_count : nbig;
+  for (uint32_t w = blockIdx.x; w < nwork; w += gridDim.x) {
+    exact_merge_one<MCAP>(A, work ? work[w] : w, sm, spill, spill_count);
+    __syncthreads();  // shared memory is reused by the next query
   }
 }
 
@@ -1134,15 +972,44 @@ int search_exact(fknn_index *idx, const float *d_q, const float *d_meta, uint32_
   auto t0 = std::chrono::steady_clock::now();
   Plan &P = idx->plan;
   PlanShape shape;
-  shape.tq = TQ;
-  shape.blk_rows = BLK;
+  shape.tq = EXACT_TQ;
+  shape.blk_rows = EXACT_ROWS;
   shape.small_slab = SMALL_SLAB;
-  shape.max_items_per_tile = MAX_ITEMS_PER_TILE;
+  // without a pilot every item of a tile may fill its list, and the merge holds MERGE_CAP entries
+  const uint32_t pstride = idx->tuning[FKNN_MODE_EXACT_FP32].pilot_stride;
+  const bool pilot = pstride > 1;
+  shape.max_items_per_tile = pilot ? MAX_ITEMS_PER_TILE : MERGE_CAP / EXACT_CAP;
   shape.min_chunk_blocks = idx->tuning[FKNN_MODE_EXACT_FP32].min_chunk_blocks;
-  shape.target_items = idx->num_sms * idx->tuning[FKNN_MODE_EXACT_FP32].items_per_sm;
-  make_plan(h_desc, h_meta, nq, n, shape, P);
+  // Several items per SM even out tiles of unequal length; with few queries
+  // there are few tiles, cut alike, and every further item only adds its own
+  // start and end (16 queries over 1e6 rows: 0.82 ms at one item per SM, 1.29
+  // at four; 1e4 queries over 1e5 rows: 3.5 and 3.2 ms).
+  const uint32_t ips = nq < 1024 ? 1u : idx->tuning[FKNN_MODE_EXACT_FP32].items_per_sm;
+  Candidate *d_out = nullptr, *d_work = nullptr;
+  uint32_t *d_ocnt = nullptr, sgrid = 0, nitems = 0;
+  // Where the index's HBM budget (or the memory left) does not hold the lists
+  // of that many items and a working set for every SM, one item per tile and
+  // as many CTAs as fit.
+  for (int tight = 0;; ++tight) {
+    shape.target_items = tight ? 1u : (uint32_t)idx->num_sms * ips;
+    make_plan(h_desc, h_meta, nq, n, shape, P);
+    nitems = (uint32_t)P.items.size();
+    if (!nitems) break;
+    rc = ws_get(idx, 6, (size_t)nitems * EXACT_TQ * EXACT_CAP * sizeof(Candidate), (void **)&d_out);
+    if (!rc) rc = ws_get(idx, 7, (size_t)nitems * EXACT_TQ * 4, (void **)&d_ocnt);
+    if (!rc)
+      for (sgrid = std::min<uint32_t>(nitems, (uint32_t)idx->num_sms);; sgrid = (sgrid + 1) / 2) {
+        rc = ws_get(idx, 4, exact_work_bytes(sgrid), (void **)&d_work);
+        if (rc != FKNN_ENOMEM || !tight || sgrid == 1) break;
+        cudaGetLastError();
+      }
+    if (!rc) break;
+    if (rc != FKNN_ENOMEM || tight) return rc;
+    cudaGetLastError();  // (a refused allocation is not this call's error)
+    for (int slot : {4, 6, 7}) ws_drop(idx, slot);
+  }
   auto t1 = std::chrono::steady_clock::now();
-  const uint32_t ntile = (uint32_t)P.tiles.size(), nitems = (uint32_t)P.items.size();
+  const uint32_t ntile = (uint32_t)P.tiles.size();
   const uint32_t nbig = (uint32_t)P.big.size(), nsmall = (uint32_t)P.small.size();
 
   // item slots: the merge reads a tile's lists through tile.item0..item1 of
@@ -1165,8 +1032,8 @@ int search_exact(fknn_index *idx, const float *d_q, const float *d_meta, uint32_
   };
   const size_t o_small = take(nsmall * 4), o_big = take(nbig * 4), o_btile = take(nbig * 4),
                o_blane = take(nbig * 4), o_tiles = take(ntile * sizeof(Tile)), o_items = take(nitems * sizeof(WorkItem)),
-               o_lq = take((size_t)ntile * TQ * 4), o_ls = take((size_t)ntile * TQ * 4),
-               o_le = take((size_t)ntile * TQ * 4), o_slot = take(nitems * 4);
+               o_lq = take((size_t)ntile * EXACT_TQ * 4), o_ls = take((size_t)ntile * EXACT_TQ * 4),
+               o_le = take((size_t)ntile * EXACT_TQ * 4), o_slot = take(nitems * 4);
   const size_t blob = off;
   unsigned char *h_blob, *d_blob;
   if ((rc = hs_get(idx, 3, blob + 256, (void **)&h_blob))) return rc;
@@ -1180,68 +1047,129 @@ int search_exact(fknn_index *idx, const float *d_q, const float *d_meta, uint32_
   put(o_blane, P.big_lane.data(), nbig * 4);
   put(o_tiles, P.tiles.data(), ntile * sizeof(Tile));
   put(o_items, P.items.data(), nitems * sizeof(WorkItem));
-  put(o_lq, P.lane_q.data(), (size_t)ntile * TQ * 4);
-  put(o_ls, P.lane_s.data(), (size_t)ntile * TQ * 4);
-  put(o_le, P.lane_e.data(), (size_t)ntile * TQ * 4);
+  put(o_lq, P.lane_q.data(), (size_t)ntile * EXACT_TQ * 4);
+  put(o_ls, P.lane_s.data(), (size_t)ntile * EXACT_TQ * 4);
+  put(o_le, P.lane_e.data(), (size_t)ntile * EXACT_TQ * 4);
   put(o_slot, slot_of_tile_item.data(), nitems * 4);
   if (blob) FKNN_CUDA(cudaMemcpyAsync(d_blob, h_blob, blob, cudaMemcpyHostToDevice, st));
 
-  // per-query state: bound, overflow flag, overflow list + count
+  // per-query state: bound, not-screened flag, overflow list; pilot bound
+  // and flag; redo flag and list; spill lists of the two merges; then counts
   uint32_t *d_state;
-  if ((rc = ws_get(idx, 5, (size_t)nq * 12 + 64, (void **)&d_state))) return rc;
+  if ((rc = ws_get(idx, 5, (size_t)nq * 36 + 64, (void **)&d_state))) return rc;
   uint32_t *T_global = d_state, *ovf = d_state + nq, *ovf_list = d_state + 2 * (size_t)nq,
-           *ovf_count = d_state + 3 * (size_t)nq;
-  // bounds start at +inf (as an order-preserving integer image)
-  k_fill_u32<<<std::min<uint32_t>((nq + 255) / 256, 1024), 256, 0, st>>>(T_global, nq, f32_sortable(INFINITY));
-  g_launches += 1;
-  FKNN_CUDA(cudaMemsetAsync(ovf, 0, (size_t)nq * 4, st));
-  FKNN_CUDA(cudaMemsetAsync(ovf_count, 0, 4, st));
+           *T_pilot = d_state + 3 * (size_t)nq, *ovf_p = d_state + 4 * (size_t)nq,
+           *redo_skip = d_state + 5 * (size_t)nq, *redo_list = d_state + 6 * (size_t)nq,
+           *spill = d_state + 7 * (size_t)nq, *spill2 = d_state + 8 * (size_t)nq, *counts = d_state + 9 * (size_t)nq;
+  // counts: exact scans, redos, spills of the two merges, work queues of the three screens
+  uint32_t *ovf_count = counts, *redo_count = counts + 1, *spill_count = counts + 2, *spill2_count = counts + 3,
+           *queue = counts + 4;
 
   const OrderData &OT = idx->ord[ORDER_TIME], &OC = idx->ord[ORDER_CAT];
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
   if (stats) {
     for (auto &e : ev) FKNN_CUDA(cudaEventCreate(&e));
   }
+  FKNN_CUDA(cudaMemsetAsync(counts, 0, 32, st));
   if (nitems) {
-    float *d_qt;
-    Candidate *d_out;
-    uint32_t *d_ocnt;
-    if ((rc = ws_get(idx, 4, (size_t)ntile * BLK_BYTES, (void **)&d_qt))) return rc;
-    if ((rc = ws_get(idx, 6, (size_t)nitems * TQ * CAP * sizeof(Candidate), (void **)&d_out))) return rc;
-    if ((rc = ws_get(idx, 7, (size_t)nitems * TQ * 4, (void **)&d_ocnt))) return rc;
-    k_tile_stage<<<ntile, 256, 0, st>>>(d_q, d_desc, (const int32_t *)(d_blob + o_lq), d_qt);
-    const size_t smem = sizeof(ScreenSmem);
+    // bounds start at +inf (as an order-preserving integer image)
+    if ((rc = launch_fill_u32(T_global, nq, f32_sortable(INFINITY), st))) return rc;
+    FKNN_CUDA(cudaMemsetAsync(ovf, 0, (size_t)nq * 4, st));
     // per device context, so set on every call (cheap)
-    FKNN_CUDA(cudaFuncSetAttribute(k_screen, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    FKNN_CUDA(cudaFuncSetAttribute(k_merge, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MergeSmem)));
+    using SmallSmem = MergeSmem<MERGE_CAP_SMALL>;
+    using LargeSmem = MergeSmem<MERGE_CAP>;
+    FKNN_CUDA(cudaFuncSetAttribute(k_merge<MERGE_CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)sizeof(LargeSmem)));
     if (stats) FKNN_CUDA(cudaEventRecord(ev[0], st));
-    const uint32_t pstride = idx->tuning[FKNN_MODE_EXACT_FP32].pilot_stride;
-    if (pstride > 1) {
-      // Pilot: the same screen over every pstride-th row block.  Each list's
-      // k-th screening distance (widened by screen_hi) bounds the k-th
-      // reference distance of its query from above -- the k-th smallest of
-      // a subset is never below the k-th smallest of the whole slab -- so the
-      // bounds it leaves in T_global are valid seeds and the main pass keeps
-      // every row that can be in the top k.  Its overflow marks are its own.
-      uint32_t *ovf_p;
-      if ((rc = ws_get(idx, 13, (size_t)nq * 4, (void **)&ovf_p))) return rc;
+    ExactScreenArgs A;
+    A.items = (const WorkItem *)(d_blob + o_items);
+    A.tiles = (const Tile *)(d_blob + o_tiles);
+    A.lane_q = (const int32_t *)(d_blob + o_lq);
+    A.lane_s = (const uint32_t *)(d_blob + o_ls);
+    A.lane_e = (const uint32_t *)(d_blob + o_le);
+    A.q = d_q;
+    A.desc = d_desc;
+    A.blocks_t = OT.blocks;
+    A.blocks_c = OC.blocks;
+    A.nblk = idx->nblk;
+    A.work = d_work;
+    A.out = d_out;
+    A.out_cnt = d_ocnt;
+    A.nitems = nitems;
+    A.active = nullptr;
+    A.err = idx->d_flag;
+    const uint32_t *big_q = (const uint32_t *)(d_blob + o_big), *big_tile = (const uint32_t *)(d_blob + o_btile),
+                   *big_lane = (const uint32_t *)(d_blob + o_blane), *item_slot = (const uint32_t *)(d_blob + o_slot);
+    if (pilot) {
+      // Pilot: the same screen over every pstride-th row block.  The r-th
+      // distance of a query's sample seeds its bound: the k-th of all rows
+      // ranks about k / pstride in the sample, and r = 3 k / pstride + 8 lies
+      // above it but for a vanishing fraction of queries, which the merge
+      // finds and the redo pass below screens again without a seed.  The seed
+      // admits about 3 k + 8 pstride rows, a tenth of the pushes that
+      // tracking the k-th from nothing makes.
+      // (the sample of a short slab is up to twice its nominal share)
+      const uint32_t r = exact_seed_rank(k, 2, pstride);
+      if ((rc = launch_fill_u32(T_pilot, nq, f32_sortable(INFINITY), st))) return rc;
       FKNN_CUDA(cudaMemsetAsync(ovf_p, 0, (size_t)nq * 4, st));
-      k_screen<<<nitems, SC_THREADS, smem, st>>>(
-          (const WorkItem *)(d_blob + o_items), (const Tile *)(d_blob + o_tiles), d_qt,
-          (const int32_t *)(d_blob + o_lq), (const uint32_t *)(d_blob + o_ls), (const uint32_t *)(d_blob + o_le),
-          OT.blocks, OC.blocks, T_global, ovf_p, d_out, d_ocnt, k, pstride, idx->d_flag);
-      g_launches += 1;
+      FKNN_CUDA(cudaMemsetAsync(redo_skip, 0xff, (size_t)nq * 4, st));
+      A.T_global = T_pilot;
+      A.ovf = ovf_p;
+      A.stride = pstride;
+      A.k = r;
+      A.queue = queue;
+      if ((rc = launch_exact_screen(A, sgrid, st))) return rc;
+      if ((rc = launch_exact_seed(big_q, big_tile, big_lane, nbig, A, item_slot, k, T_global, st))) return rc;
     }
-    k_screen<<<nitems, SC_THREADS, smem, st>>>(
-        (const WorkItem *)(d_blob + o_items), (const Tile *)(d_blob + o_tiles), d_qt, (const int32_t *)(d_blob + o_lq),
-        (const uint32_t *)(d_blob + o_ls), (const uint32_t *)(d_blob + o_le), OT.blocks, OC.blocks, T_global, ovf,
-        d_out, d_ocnt, k, 1u, idx->d_flag);
+    A.T_global = T_global;
+    A.ovf = ovf;
+    A.stride = 1;
+    A.k = k;
+    A.queue = queue + 1;
+    if ((rc = launch_exact_screen(A, sgrid, st))) return rc;
     if (stats) FKNN_CUDA(cudaEventRecord(ev[1], st));
-    k_merge<<<nbig, MG_THREADS, sizeof(MergeSmem), st>>>(
-        (const uint32_t *)(d_blob + o_big), (const uint32_t *)(d_blob + o_btile), (const uint32_t *)(d_blob + o_blane),
-        (const Tile *)(d_blob + o_tiles), (const uint32_t *)(d_blob + o_slot), d_out, d_ocnt, d_desc, d_q, idx->vecs,
-        OT.perm, OC.perm, T_global, ovf, ovf_list, ovf_count, k, d_ids, d_dists);
-    g_launches += 3;
+    ExactMergeArgs G;
+    G.big_q = big_q;
+    G.big_tile = big_tile;
+    G.big_lane = big_lane;
+    G.tiles = A.tiles;
+    G.item_slot = item_slot;
+    G.out = d_out;
+    G.out_cnt = d_ocnt;
+    G.desc = d_desc;
+    G.q = d_q;
+    G.vecs = idx->vecs;
+    G.perm_t = OT.perm;
+    G.perm_c = OC.perm;
+    G.T_global = T_global;
+    G.ovf = ovf;
+    G.ovf_list = ovf_list;
+    G.ovf_count = ovf_count;
+    G.redo_list = pilot ? redo_list : nullptr;
+    G.redo_count = redo_count;
+    G.redo_skip = redo_skip;
+    G.k = k;
+    G.ids = d_ids;
+    G.dists = d_dists;
+    const unsigned lgrid = std::min<uint32_t>(nbig, (uint32_t)idx->num_sms * 2);
+    k_merge<MERGE_CAP_SMALL><<<nbig, MG_THREADS, sizeof(SmallSmem), st>>>(G, nbig, nullptr, nullptr, spill,
+                                                                          spill_count);
+    k_merge<MERGE_CAP><<<lgrid, MG_THREADS, sizeof(LargeSmem), st>>>(G, 0, spill, spill_count, nullptr, nullptr);
+    g_launches += 2;
+    if (pilot) {
+      // the same plan once more for the queries whose seed was too low, the
+      // others (and the items without any such query) skipped
+      A.ovf = redo_skip;
+      A.active = redo_count;
+      A.queue = queue + 2;
+      if ((rc = launch_exact_screen(A, sgrid, st))) return rc;
+      G.ovf = redo_skip;
+      G.redo_list = nullptr;
+      k_merge<MERGE_CAP_SMALL><<<lgrid, MG_THREADS, sizeof(SmallSmem), st>>>(G, 0, redo_list, redo_count, spill2,
+                                                                             spill2_count);
+      k_merge<MERGE_CAP><<<lgrid, MG_THREADS, sizeof(LargeSmem), st>>>(G, 0, spill2, spill2_count, nullptr, nullptr);
+      g_launches += 2;
+    }
   }
   if (stats) FKNN_CUDA(cudaEventRecord(ev[2], st));
   if (nbig) {

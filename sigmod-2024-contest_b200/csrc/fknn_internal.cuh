@@ -19,12 +19,14 @@ constexpr int BLK = 64;           // rows per layout block
 constexpr int BLK_ROWS_F = DIM + 1;            // 100 dims + the row norm
 constexpr int BLK_FLOATS = BLK_ROWS_F * BLK;   // one block: [101][64] float
 constexpr uint32_t BLK_BYTES = BLK_FLOATS * 4; // 25856, a multiple of 16
-constexpr int TQ = 64;            // queries per contraction tile
-constexpr int CAP = 256;          // candidate slots per (work item, query)
+constexpr int EXACT_TQ = 256;     // queries per contraction tile of the exact search
+constexpr int EXACT_ROWS = 128;   // rows of its sub-tiles (two layout blocks)
+constexpr int EXACT_CAP = 192;    // candidates a work item of it hands on per query
 constexpr int KMAX_TILE = 128;    // largest k the contraction path serves
 constexpr int SMALL_SLAB = 4096;  // slabs up to this size go to the row-by-row exact scan
-constexpr int MERGE_CAP = 8192;   // candidates one merge block can hold
-constexpr int MAX_ITEMS_PER_TILE = 32;  // so a tile's lists (<= 32 x 192) always fit one merge
+constexpr int MERGE_CAP = 8192;   // candidates the large exact merge can hold ...
+constexpr int MERGE_CAP_SMALL = 1024;  // ... and the common one
+constexpr int MAX_ITEMS_PER_TILE = 256;  // work items of one exact tile (the merge's offset slots)
 constexpr int RESCORE_CAP = 512;  // survivors one merge block can re-score
 
 enum Order : int { ORDER_TIME = 0, ORDER_CAT = 1 };
@@ -89,7 +91,7 @@ struct QueryDesc {
   float qn;       // ||q||^2 as a float FMA chain
 };
 
-// One contraction work item: rows [blk0*64, blk1*64) of the tile's order.
+// One contraction work item: row blocks [blk0, blk1) of 128 rows of the tile's order.
 struct WorkItem {
   uint32_t tile;
   uint32_t blk0, blk1;
@@ -273,7 +275,7 @@ struct fknn_index {
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   fknn::Plan plan;  // rebuilt by every search; capacity kept
   // per-mode plan / kernel parameters (fknn_index_set_tuning) and the SM count
-  fknn_tuning tuning[3] = {{0, 16, 16, 0, 0}, {256, 3, 8, 0, 16}, {256, 3, 8, 0, 16}};
+  fknn_tuning tuning[3] = {{0, 4, 16, 0, 32}, {256, 3, 8, 0, 16}, {256, 3, 8, 0, 16}};
   int num_sms = 148;
   uint32_t n_labels = 1;  // distinct category values (bounds a device plan's segments)
   // a view shares the device data of another index and owns only its
@@ -318,6 +320,7 @@ void destroy_index(fknn_index *idx);
 uint64_t scratch_bytes(const fknn_index *idx);
 void trim_scratch(fknn_index *idx);
 int ws_get(fknn_index *idx, int slot, size_t bytes, void **p);
+void ws_drop(fknn_index *idx, int slot);  // gives the slot's buffer back
 int hs_get(fknn_index *idx, int slot, size_t bytes, void **p);
 
 // index build (index_build.cu)
@@ -334,6 +337,41 @@ size_t device_plan_bytes(uint32_t nq, const DevPlanSizes &z);
 void device_plan_layout(DevPlan &P, void *mem, uint32_t nq, const DevPlanSizes &z);
 int device_plan_build(fknn_index *idx, const QueryDesc *d_desc, const float *d_meta, DevPlan &P,
                       const PlanShape &shape, cudaStream_t st);
+
+// tensor-core screen of the exact search (exact_screen.cu)
+struct ExactScreenArgs {
+  const WorkItem *items;
+  const Tile *tiles;
+  const int32_t *lane_q;
+  const uint32_t *lane_s, *lane_e;
+  const float *q;               // nq x 100
+  const QueryDesc *desc;
+  const float *blocks_t, *blocks_c;
+  uint32_t nblk;                // 64-row layout blocks of an order
+  uint32_t *T_global;           // per query: upper bound on its k-th distance (f32_sortable)
+  uint32_t *ovf;                // per query: non-zero = not screened (left to the exact scan, or answered)
+  Candidate *work;              // exact_work_bytes(grid): the CTAs' working lists
+  Candidate *out;               // [item][EXACT_TQ][EXACT_CAP]
+  uint32_t *out_cnt;            // [item][EXACT_TQ]
+  uint32_t nitems;
+  const uint32_t *active;       // NULL, or the count of queries to screen: 0 = nothing to do
+  uint32_t *queue;              // zero at the launch: next item past the grid's first ones
+  uint32_t k, stride;           // stride: every stride-th row block (1: all)
+  int *err;
+};
+size_t exact_work_bytes(uint32_t grid);
+int launch_exact_screen(const ExactScreenArgs &A, uint32_t grid, cudaStream_t st);
+// Rank, in a sample of `rows` rows of a slab of n, of the bound that seeds a
+// search of the slab's k nearest: about k rows / n of them are in the sample,
+// and 3 times that + 8 lies above all but 1e-8 of the (Poisson) cases.
+__host__ __device__ __forceinline__ uint32_t exact_seed_rank(uint32_t k, uint32_t rows, uint32_t n) {
+  const uint32_t r = (uint32_t)((3ull * k * rows + n - 1) / (n ? n : 1)) + 8;
+  return r < k ? r : k;
+}
+// T_global of the nbig queries set from their pilot lists (those that have enough entries)
+int launch_exact_seed(const uint32_t *big_q, const uint32_t *big_tile, const uint32_t *big_lane, uint32_t nbig,
+                      const ExactScreenArgs &A, const uint32_t *item_slot, uint32_t k, uint32_t *T_global,
+                      cudaStream_t st);
 
 // exact search (exact_search.cu)
 int search_exact(fknn_index *idx, const float *d_q, const float *d_meta, uint32_t nq, uint32_t k, uint32_t *d_ids,

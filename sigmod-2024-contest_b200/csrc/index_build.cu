@@ -169,8 +169,9 @@ __global__ void k_order_columns(const uint32_t *__restrict__ perm, const float *
 
 // One CTA per 64-row block: gather rows perm[b*64 .. b*64+63] (row-major,
 // coalesced per row), transpose through shared memory, write [101][64].
-__global__ void k_build_blocks(const float *__restrict__ vecs, const float *__restrict__ norms,
-                               const uint32_t *__restrict__ perm, uint64_t n, float *__restrict__ blocks) {
+// Row 100 is the norm, rounded once from a 64-bit sum.
+__global__ void k_build_blocks(const float *__restrict__ vecs, const uint32_t *__restrict__ perm, uint64_t n,
+                               float *__restrict__ blocks) {
   __shared__ float tile[BLK][DIM + 1];
   const uint64_t b = blockIdx.x;
   for (int i = threadIdx.x; i < BLK * DIM; i += blockDim.x) {
@@ -185,8 +186,13 @@ __global__ void k_build_blocks(const float *__restrict__ vecs, const float *__re
     out[d * BLK + r] = tile[r][d];
   }
   for (int r = threadIdx.x; r < BLK; r += blockDim.x) {
-    uint64_t p = b * BLK + r;
-    out[DIM * BLK + r] = p < n ? norms[perm[p]] : 0.f;
+    double s0 = 0.0, s1 = 0.0;  // rows past n are zero
+#pragma unroll 10
+    for (int d = 0; d < DIM; d += 2) {
+      s0 += (double)tile[r][d] * (double)tile[r][d];
+      s1 += (double)tile[r][d + 1] * (double)tile[r][d + 1];
+    }
+    out[DIM * BLK + r] = (float)(s0 + s1);
   }
 }
 
@@ -290,7 +296,7 @@ int build_index_from_columns(fknn_index *idx, cudaStream_t st) {
   for (int o = 0; o < 2; ++o) {
     OrderData &od = idx->ord[o];
     k_order_columns<<<grid_for(n, 256), 256, 0, st>>>(od.perm, idx->ts_f, idx->labels_f, n, od.ts, od.label);
-    k_build_blocks<<<idx->nblk, 256, 0, st>>>(idx->vecs, idx->norms, od.perm, n, od.blocks);
+    k_build_blocks<<<idx->nblk, 256, 0, st>>>(idx->vecs, od.perm, n, od.blocks);
     g_launches += 2;
   }
   FKNN_CUDA(cudaMemsetAsync(idx->d_flag, 0, sizeof(int), st));
