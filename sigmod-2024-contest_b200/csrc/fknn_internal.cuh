@@ -383,7 +383,7 @@ int count_matches(fknn_index *idx, const float *d_meta, uint32_t nq, uint32_t *d
 int graph_check_args(const fknn_graph *g, const float *queries, uint32_t nq, int mode, uint32_t k, uint32_t ef,
                      uint32_t refine, const float *bounds, const int32_t *id_bounds, const int32_t *out_ids,
                      uint32_t *cap);
-int graph_reserve(fknn_graph *g, uint32_t nq, uint32_t cap);
+int graph_reserve(fknn_graph *g, uint32_t nq, uint32_t cap, bool ranged, bool overflow_read);
 int graph_launch(fknn_graph *g, const float *d_q, uint32_t nq, int mode, uint32_t k, uint32_t cap, uint32_t refine,
                  const float *d_bounds, const int32_t *d_idb, int32_t *d_ids, float *d_dists, cudaStream_t st);
 int graph_flag_reset(fknn_graph *g, cudaStream_t st);

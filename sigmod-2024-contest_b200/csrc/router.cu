@@ -601,24 +601,23 @@ int fknn_router_search(fknn_router *r, const float *qvecs, const float *metas, u
         (rc2 = r->ldist.get(std::max<size_t>(no, 1))) || (rc2 = r->qcodes_b.get(nqs * CODE)) ||
         (rc2 = r->sel.get(std::max<size_t>(hsel.size(), 3))) || (rc2 = r->keys.get(std::max<size_t>(nk, 1))))
       return rc2;
-    // scratch of every graph at its largest search of the stage (nothing is
-    // allocated once searches are in flight)
+    // scratch of every graph for each of its searches of the stage (nothing
+    // is allocated once searches are in flight)
     std::vector<uint32_t> used;
     {
-      std::vector<uint32_t> mq(r->cats.size() + r->bks.size(), 0), mc(mq.size(), 0);
+      std::vector<uint8_t> searched(r->cats.size() + r->bks.size(), 0);
       for (GBatch &b : B) {
+        const uint32_t m = (uint32_t)b.list->size();
         uint32_t cap = 0;
-        if ((rc2 = graph_check_args(subs(b.sub).g, r->q.p, (uint32_t)b.list->size(), b.mode, b.K, 0, R, r->bounds.p,
-                                    r->idb.p, r->lids.p, &cap)))
+        if ((rc2 = graph_check_args(subs(b.sub).g, r->q.p, m, b.mode, b.K, 0, R, r->bounds.p, r->idb.p, r->lids.p,
+                                    &cap)))
           return rc2;
-        mq[b.sub] = std::max<uint32_t>(mq[b.sub], (uint32_t)b.list->size());
-        mc[b.sub] = std::max(mc[b.sub], cap);
+        if (!m) continue;
+        searched[b.sub] = 1;
+        if ((rc2 = graph_reserve(subs(b.sub).g, m, cap, b.mode >= FKNN_GRAPH_CATEGORY_RANGE, R > cap))) return rc2;
       }
-      for (uint32_t i = 0; i < mq.size(); ++i)
-        if (mq[i]) {
-          used.push_back(i);
-          if ((rc2 = graph_reserve(subs(i).g, mq[i], mc[i]))) return rc2;
-        }
+      for (uint32_t i = 0; i < searched.size(); ++i)
+        if (searched[i]) used.push_back(i);
     }
     FKNN_CUDA(cudaMemcpyAsync(r->rows.p, rows.data(), nqs * 4, cudaMemcpyHostToDevice, st));
     if (nb) {
