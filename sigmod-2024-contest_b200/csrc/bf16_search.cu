@@ -29,12 +29,21 @@ namespace fknn {
 
 namespace {
 
-constexpr int BQ = 128;                       // queries per tile = MMA M = TMEM lanes
-constexpr int BR = 128;                       // rows per sub-tile = MMA N
+constexpr int BQ = 256;                       // queries per tile: two halves of 128 = MMA M = TMEM lanes
+constexpr int BM = BQ / 2;
+constexpr int BR = 256;                       // rows per block = MMA N
+constexpr int BP = 128;                       // columns an epilogue warp screens
 constexpr int BS = 2;                         // shared-memory stages for row blocks
-constexpr int B_EPI_WARPS = 4;
-constexpr int B_THREADS = (2 + B_EPI_WARPS) * 32;  // producer, MMA issuer, 4 epilogue warps
-constexpr uint32_t TMEM_COLS = 2 * BR;        // double-buffered accumulator
+constexpr int B_ACCS = 2;                     // accumulators
+constexpr int B_EPI = 4 * (BR / BP);          // epilogue warps 0 .. 7: TMEM lanes 32 (w % 4) .., columns BP (w / 4) ..
+constexpr int B_LISTS = B_EPI * 32;           // working lists of a half: one per epilogue thread
+constexpr int B_LOAD_WARP = B_EPI;
+constexpr int B_MMA_WARP = B_EPI + 1;
+constexpr int B_THREADS = (B_EPI + 2) * 32;
+constexpr uint32_t TMEM_COLS = B_ACCS * BR;
+constexpr int B_SLOTS = 8;                    // 32-column chunks an epilogue warp stages at a time
+constexpr int B_ROW = 36;                     // words of a staged chunk: 32 columns, 4 of its query
+constexpr int B_SLACK = 24;                   // entries past the k'-th that a trim may keep
 
 // Operand formats of the tensor-core screen.  Both operands are K-major,
 // no swizzle, in core matrices of 8 rows x 16 bytes; every MMA consumes 32
@@ -45,25 +54,29 @@ struct FmtBF16 {
   static constexpr int K = 112;                 // 100 dims, 2 norm terms, zero padding
   static constexpr int ROW_BYTES = K * 2;
   static constexpr int MMAS = K / 16;           // kind::f16: K = 16 per MMA
-  // F32 accumulate, BF16 A and B, K-major, N = BR, M = BQ
+  // F32 accumulate, BF16 A and B, K-major, N = BR, M = BM
   static constexpr uint32_t IDESC =
-      (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BR >> 3) << 17) | ((uint32_t)(BQ >> 4) << 24);
+      (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BR >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
 };
 struct FmtFP8 {
   static constexpr bool kFP8 = true;
   static constexpr int K = 128;                 // 100 dims, 3 norm terms, zero padding
   static constexpr int ROW_BYTES = K;
   static constexpr int MMAS = K / 32;           // kind::f8f6f4: K = 32 per MMA
-  // F32 accumulate, E4M3 A and B, K-major, N = BR, M = BQ
+  // F32 accumulate, E4M3 A and B, K-major, N = BR, M = BM
   static constexpr uint32_t IDESC =
-      (1u << 4) | (0u << 7) | (0u << 10) | ((uint32_t)(BR >> 3) << 17) | ((uint32_t)(BQ >> 4) << 24);
+      (1u << 4) | (0u << 7) | (0u << 10) | ((uint32_t)(BR >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
 };
 template <class F>
 struct Tiles {
-  static constexpr uint32_t BYTES = (uint32_t)BQ * F::ROW_BYTES;  // one 128-row operand tile
+  static constexpr uint32_t A = (uint32_t)BM * F::ROW_BYTES;  // half a tile's queries
+  static constexpr uint32_t B = (uint32_t)BR * F::ROW_BYTES;  // a row block
 };
-constexpr uint32_t BF_TILE = Tiles<FmtBF16>::BYTES;  // 28672
-constexpr uint32_t F8_TILE = Tiles<FmtFP8>::BYTES;   // 16384
+
+// byte offset of (row r, byte b of the row) in a row block
+__device__ __forceinline__ uint32_t rb_byte(uint32_t r, uint32_t b) {
+  return ((b >> 4) * (BR / 8) + (r >> 3)) * 128 + (r & 7) * 16 + (b & 15);
+}
 
 template <class F>
 __device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t accumulate) {
@@ -86,7 +99,7 @@ __global__ void k_build_bf16_blocks(const float *__restrict__ vecs, const float 
                                     const uint32_t *__restrict__ perm, uint64_t n, __nv_bfloat16 *__restrict__ out) {
   const uint64_t b = blockIdx.x;
   constexpr int BK = FmtBF16::K;
-  __nv_bfloat16 *o = out + b * (BF_TILE / 2);
+  __nv_bfloat16 *o = out + b * (Tiles<FmtBF16>::B / 2);
   for (uint32_t i = threadIdx.x; i < (uint32_t)BR * BK; i += blockDim.x) {
     const uint32_t r = i / BK, k = i % BK;
     const uint64_t p = b * BR + r;
@@ -101,7 +114,7 @@ __global__ void k_build_bf16_blocks(const float *__restrict__ vecs, const float 
         v = (k == DIM) ? hi : h - hi;
       }
     }
-    o[cm_index(r, k)] = __float2bfloat16_rn(v);
+    o[rb_byte(r, 2 * k) / 2] = __float2bfloat16_rn(v);
   }
 }
 
@@ -142,7 +155,7 @@ __global__ void k_tile_stage_bf16(const float *__restrict__ q, LaneSrc ls, const
   __shared__ int32_t lq[BQ];
   for (uint32_t t = blockIdx.x; t < ntile; t += gridDim.x) {
     const Tile tl = tiles[t];
-    __nv_bfloat16 *o = out + (uint64_t)t * (BF_TILE / 2);
+    __nv_bfloat16 *o = out + (uint64_t)t * 2 * (Tiles<FmtBF16>::A / 2);
     for (uint32_t l = threadIdx.x; l < (uint32_t)BQ; l += blockDim.x) {
       uint32_t s_, e_;
       const int32_t qi = lane_query(ls, tl, t, (int)l, s_, e_);
@@ -158,7 +171,7 @@ __global__ void k_tile_stage_bf16(const float *__restrict__ q, LaneSrc ls, const
         if (k < (uint32_t)DIM) v = q[(uint64_t)qi * DIM + k];
         else if (k == DIM || k == DIM + 1) v = 1.f;
       }
-      o[cm_index(l, k)] = __float2bfloat16_rn(v);
+      o[(l / BM) * (Tiles<FmtBF16>::A / 2) + cm_index(l % BM, k)] = __float2bfloat16_rn(v);
     }
     __syncthreads();
   }
@@ -209,7 +222,7 @@ __global__ void k_build_fp8_blocks(const float *__restrict__ vecs, const uint32_
                                    const float *__restrict__ center, const float *__restrict__ scale,
                                    unsigned char *__restrict__ out) {
   const uint64_t b = blockIdx.x;
-  unsigned char *o = out + b * F8_TILE;
+  unsigned char *o = out + b * Tiles<FmtFP8>::B;
   __shared__ float cn[BR];
   // centred norms of the block's rows (float FMA chain)
   for (uint32_t r = threadIdx.x; r < (uint32_t)BR; r += blockDim.x) {
@@ -239,7 +252,7 @@ __global__ void k_build_fp8_blocks(const float *__restrict__ vecs, const uint32_
         v = (k == DIM) ? hi : (k == DIM + 1) ? mid : h - hi - mid;
       }
     }
-    o[cm_byte(r, k)] = __nv_fp8_e4m3(v).__x;
+    o[rb_byte(r, k)] = __nv_fp8_e4m3(v).__x;
   }
 }
 
@@ -251,7 +264,7 @@ __global__ void k_tile_stage_fp8(const float *__restrict__ q, LaneSrc ls, const 
   __shared__ int32_t lq[BQ];
   for (uint32_t t = blockIdx.x; t < ntile; t += gridDim.x) {
     const Tile tl = tiles[t];
-    unsigned char *o = out + (uint64_t)t * F8_TILE;
+    unsigned char *o = out + (uint64_t)t * 2 * Tiles<FmtFP8>::A;
     for (uint32_t l = threadIdx.x; l < (uint32_t)BQ; l += blockDim.x) {
       uint32_t s_, e_;
       const int32_t qi = lane_query(ls, tl, t, (int)l, s_, e_);
@@ -281,7 +294,7 @@ __global__ void k_tile_stage_fp8(const float *__restrict__ q, LaneSrc ls, const 
         if (k < (uint32_t)DIM) v = lam[l] * (q[(uint64_t)qi * DIM + k] - center[k]) * scale[k];
         else if (k <= DIM + 2) v = lam[l];
       }
-      o[cm_byte(l, k)] = __nv_fp8_e4m3(v).__x;
+      o[(l / BM) * Tiles<FmtFP8>::A + cm_byte(l % BM, k)] = __nv_fp8_e4m3(v).__x;
     }
     __syncthreads();
   }
@@ -291,48 +304,74 @@ __global__ void k_tile_stage_fp8(const float *__restrict__ q, LaneSrc ls, const 
 
 template <class F>
 struct BScreenSmem {
-  unsigned char a[Tiles<F>::BYTES];
-  unsigned char b[BS][Tiles<F>::BYTES];
-  float thr[BQ];  // current k'-th screening distance bound T
-  float qn[BQ];
-  int cnt[BQ];
+  unsigned char a[2][Tiles<F>::A];
+  unsigned char b[BS][Tiles<F>::B];
+  struct {
+    float row[B_SLOTS][B_ROW];  // staged chunks
+    uint32_t hist[256];         // the histogram of a trim
+  } w[B_EPI];
+  float4 q[BQ];      // per query: lowest accumulator value of a candidate, slab (bits), != 0: pilot takes the best of BP
+  float2 qs[BQ];     // |q|^2 (centred for FP8), -2 / lambda
+  float thr[BQ];     // current bound T on the k'-th screening distance
   int32_t lq[BQ];
-  uint32_t hist[B_EPI_WARPS][256];
-  // per epilogue lane, the 32 accumulator columns of a chunk that has
-  // candidates (rows padded to 36 floats: conflict-free 16-byte stores)
-  float stage[B_EPI_WARPS][32 * STAGE_ROW];
-  uint64_t full[BS], empty[BS], accfull[2], accempty[2], abar;
+  int cnt[2][B_LISTS];
+  uint64_t full[BS], empty[BS], accfull[B_ACCS], accempty[B_ACCS], afull;
   uint32_t tmem_base;
   uint32_t next[2];  // the next processing slot, by item parity (work queue)
 };
+static_assert(sizeof(BScreenSmem<FmtBF16>) <= 227 * 1024, "one screen CTA per SM");
 
-// two screening CTAs share an SM (228 KB of shared memory, 1 KB reserved per CTA)
-static_assert(sizeof(BScreenSmem<FmtBF16>) <= 113 * 1024 && sizeof(BScreenSmem<FmtFP8>) <= 113 * 1024,
-              "screen shared memory must leave room for two CTAs per SM");
+struct ScreenArgs {
+  const WorkItem *items;
+  const Tile *tiles;
+  const unsigned char *atiles;  // [tile][half], operand tiles of 128 queries
+  LaneSrc ls;
+  const float2 *lane_qs;        // per tile lane: |q|^2 (centred for FP8), 1 / lambda
+  const unsigned char *blocks_t, *blocks_c;
+  uint32_t *T_global;           // per query: upper bound on its k'-th screening distance (f32_sortable)
+  uint32_t *ovf;                // per query: non-zero = left to the exact scan
+  Candidate *work;              // [CTA][half][B_LISTS][capb]
+  Candidate *out;               // [item][BQ][capb]
+  uint32_t *out_cnt;            // [item][BQ]
+  uint32_t kprime, capb, refresh;
+  uint32_t kseed;               // pilot: k' of the search
+  uint32_t stride;              // > 1: a pilot pass over every stride-th row block
+  uint32_t withhold;
+  uint32_t nitems;
+  const uint32_t *nitems_d;     // device plan: the item count (NULL: nitems)
+  const uint32_t *order;        // processing slot -> item (NULL: the same)
+  uint32_t *queue;              // zero at the launch: next slot past the grid's first ones
+  int *err;
+};
 
-// Bound and trim list L to its k' smallest screening distances (ties kept):
-// the list (n <= 32 * NPL entries) is read once into registers, its k'-th
-// key selected there, the bound shared through T_global, and the kept
-// entries written back in order.
+// candidate iff qn - 2*sc*acc <= T  <=>  acc >= (qn - T) / (2 sc); with no
+// bound yet every column of the slab is one.  f2 = -2 sc, a power of two.
+__device__ __forceinline__ float acc_bound(float T, float2 qs) {
+  return T == INFINITY ? -FLT_MAX : (T - qs.x) / qs.y;
+}
+
+// Trim of one list (n entries) of query L: the k'-th screening distance, or
+// one a little above it, bounds what is kept; the bound is shared through
+// T_global and with the CTA's other lists of the query.  Whole warp; returns
+// the number kept (0 where ties do not fit: the exact scan answers the query).
 template <class F, int NPL>
-__device__ __noinline__ void bcompact(Candidate *list, BScreenSmem<F> &sm, int L, int wslot, uint32_t kprime,
+__device__ __noinline__ int b_trim(Candidate *list, int n, BScreenSmem<F> &sm, int L, uint32_t kprime,
                                       uint32_t capb, uint32_t *T_global, uint32_t *ovf) {
   const int lane = threadIdx.x & 31;
-  const int n = sm.cnt[L];
   const int32_t qi = sm.lq[L];
   float T = sm.thr[L];
+  const float Tg = sortable_f32(ld_volatile_u32(T_global + qi));
   uint32_t key[NPL], pos[NPL];
-  const uint2 *src = reinterpret_cast<const uint2 *>(list);
 #pragma unroll
   for (int j = 0; j < NPL; ++j) {
     const int i = j * 32 + lane;
     uint2 c = make_uint2(0xffffffffu, 0u);
-    if (i < n) c = src[i];
+    if (i < n) c = *reinterpret_cast<const uint2 *>(list + i);
     key[j] = i < n ? f32_sortable(__uint_as_float(c.x)) : 0xffffffffu;
     pos[j] = c.y;
   }
-  if (n >= (int)kprime) T = fminf(T, sortable_f32(warp_kth_regs<NPL>(key, n, (int)kprime, sm.hist[wslot])));
-  const float Tg = sortable_f32(ld_volatile_u32(T_global + qi));
+  if (n >= (int)kprime)
+    T = fminf(T, sortable_f32(warp_kth_upper<NPL>(key, n, (int)kprime, B_SLACK, sm.w[threadIdx.x >> 5].hist)));
   if (Tg < T) T = Tg;
   if (lane == 0 && T < Tg) atomicMin(T_global + qi, f32_sortable(T));
   const uint32_t tk = f32_sortable(T);
@@ -342,43 +381,130 @@ __device__ __noinline__ void bcompact(Candidate *list, BScreenSmem<F> &sm, int L
   __syncwarp();
 #pragma unroll
   for (int j = 0; j < NPL; ++j) {
+    if (j * 32 >= n) break;
     const bool keep = j * 32 + lane < n && key[j] <= tk;
     const uint32_t b = __ballot_sync(0xffffffffu, keep);
     if (keep) dst[kept + __popc(b & lt)] = make_uint2(__float_as_uint(sortable_f32(key[j])), pos[j]);
     kept += __popc(b);
   }
   __syncwarp();
+  if (kept > (int)capb - BP) {  // a tie flood
+    if (lane == 0) ovf[qi] = 1u;
+    T = -INFINITY;
+    kept = 0;
+  }
   if (lane == 0) {
-    if (kept > (int)capb - BR) {
-      ovf[qi] = 1u;  // a tie flood: the exact scan answers this query
-      sm.cnt[L] = 0;
-      sm.thr[L] = -INFINITY;
-    } else {
-      sm.cnt[L] = kept;
-      sm.thr[L] = T;
-    }
+    sm.thr[L] = T;
+    sm.q[L].x = acc_bound(T, sm.qs[L]);
   }
   __syncwarp();
+  return kept;
 }
 
-// One CTA per resident slot; it works through the items blockIdx.x,
-// blockIdx.x + gridDim.x, ... (a host plan launches one CTA per item, a
-// device plan a fixed grid over the device item count).  The barrier
-// phases run on across items: g counts the sub-tiles this CTA has issued.
+// The item's result for a query whose lists (one in every BM from work and cnt
+// on, more than capb entries in all) have to be bounded: their k'-th screening
+// distance by a radix select that reads them again for every digit (rare: a
+// seeded query has far fewer).  Whole warp; returns the entries written, more
+// than capb only where ties do not fit.
+template <class F>
+__device__ __noinline__ int b_select(const Candidate *work, const int *cnt, BScreenSmem<F> &sm, int L, uint32_t kprime,
+                                     uint32_t capb, uint32_t *T_global, Candidate *out) {
+  const int lane = threadIdx.x & 31;
+  uint32_t *hist = sm.w[threadIdx.x >> 5].hist;
+  auto each = [&](auto &&f) {  // every entry, the warp together
+#pragma unroll 1
+    for (int l = 0; l < B_LISTS; l += BM) {
+      const uint2 *list = reinterpret_cast<const uint2 *>(work + (uint64_t)l * capb);
+      const int n = cnt[l];
+#pragma unroll 1
+      for (int i = 0; i < n; i += 32) f(i + lane < n, i + lane < n ? list[i + lane] : make_uint2(0u, 0u));
+    }
+  };
+  uint32_t mask = 0, prefix = 0, want = kprime;
+#pragma unroll 1
+  for (int shift = 24; shift >= 0; shift -= 8) {
+    for (int i = lane; i < 256; i += 32) hist[i] = 0;
+    __syncwarp();
+    each([&](bool on, uint2 c) {
+      const uint32_t u = f32_sortable(__uint_as_float(c.x));
+      if (on && (u & mask) == prefix) atomicAdd(&hist[u >> shift & 255], 1u);
+    });
+    __syncwarp();
+    uint32_t before = 0, bin = 0;
+#pragma unroll 1
+    for (uint32_t b = 0; b < 256; b += 32) {  // the bin of the want-th key of the prefix
+      const uint32_t c = hist[b + lane];
+      uint32_t inc = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += v;
+      }
+      const uint32_t hit = __ballot_sync(0xffffffffu, before + inc >= want);
+      if (hit) {
+        const int w = __ffs(hit) - 1;
+        bin = b + w;
+        before += __shfl_sync(0xffffffffu, inc - c, w);
+        break;
+      }
+      before += __shfl_sync(0xffffffffu, inc, 31);
+    }
+    want -= before;
+    prefix |= bin << shift;
+    mask |= 255u << shift;
+    __syncwarp();
+  }
+  if (lane == 0) atomicMin(T_global + sm.lq[L], prefix);
+  int kept = 0;
+  each([&](bool on, uint2 c) {
+    const bool keep = on && f32_sortable(__uint_as_float(c.x)) <= prefix;
+    const uint32_t b = __ballot_sync(0xffffffffu, keep);
+    const uint32_t o = kept + __popc(b & ((1u << lane) - 1u));
+    if (keep && o < capb) *reinterpret_cast<uint2 *>(out + o) = c;
+    kept += __popc(b);
+  });
+  return kept;
+}
+
+// Stages one chunk of a lane's columns, and what an append needs of its
+// query: the bound, ds = qn + f2 v, and the slab's columns and lane packed.
+__device__ __forceinline__ void stage32(float *row, const uint32_t (&r)[32], float bound, float f2, float qn,
+                                        uint32_t pack) {
+#pragma unroll
+  for (int j = 0; j < 32; j += 4)
+    *reinterpret_cast<uint4 *>(row + j) = make_uint4(r[j], r[j + 1], r[j + 2], r[j + 3]);
+  *reinterpret_cast<uint4 *>(row + 32) = make_uint4(__float_as_uint(bound), __float_as_uint(f2), __float_as_uint(qn), pack);
+}
+// r0, r1 in [0, 256], lane
+__device__ __forceinline__ uint32_t pack_query(int r0, int r1, int lane, int col) {
+  return (uint32_t)r0 | (uint32_t)r1 << 9 | (uint32_t)lane << 18 | (uint32_t)col / 32 << 23;
+}
+
+// bit j set iff r0 <= j < r1
+__device__ __forceinline__ uint32_t range_mask(int r0, int r1) {
+  const int a = max(r0, 0), b = min(r1, 32);
+  return a >= b ? 0u : (0xffffffffu >> (32 - b)) & (0xffffffffu << a);
+}
+
+// Persistent, one CTA per SM, pulling work items (longest first) from a
+// queue: warp 16 copies row blocks in, warp 17 issues MMAs, warps 0-15 are the
+// epilogue.  A tile of more than 128 queries multiplies every row block with
+// both halves of its queries, so a block crosses from L2 once for 256 queries.
+// The products go to the two accumulators in turn, and every epilogue warp
+// takes its columns of each into registers and releases it at once: what a
+// warp does about candidates, which few blocks hold and then for a while, runs
+// while the next product is made (with an accumulator and half the warps for
+// each query half, every one of them waited for the slowest).
+// N = 256: an MMA of 128 columns takes 91 cycles here, one of 256 takes 128.
+// Barrier phases run on across items: g counts the row blocks of this CTA's
+// earlier items, u the products.
 template <class F, int NPL>
-__global__ void __launch_bounds__(B_THREADS, 2)
-    k_screen_tc(const WorkItem *__restrict__ items, const Tile *__restrict__ tiles,
-                const unsigned char *__restrict__ atiles, LaneSrc ls, const float2 *__restrict__ lane_qs,
-                const unsigned char *__restrict__ blocks_t, const unsigned char *__restrict__ blocks_c,
-                uint32_t *__restrict__ T_global, uint32_t *__restrict__ ovf, Candidate *__restrict__ out,
-                uint32_t *__restrict__ out_cnt, uint32_t kprime, uint32_t capb, uint32_t refresh, uint32_t stride,
-                uint32_t withhold, uint32_t nitems_h, const uint32_t *__restrict__ nitems_d,
-                const uint32_t *__restrict__ order, uint32_t *queue, int *err) {
+__global__ void __launch_bounds__(B_THREADS, 1) k_screen_tc(ScreenArgs A) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   BScreenSmem<F> &sm = *reinterpret_cast<BScreenSmem<F> *>(smem_raw);
-  constexpr uint32_t TB = Tiles<F>::BYTES;
+  constexpr uint32_t TA = Tiles<F>::A, TB = Tiles<F>::B;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const uint32_t nitems = nitems_d ? *nitems_d : nitems_h;
+  const uint32_t nitems = A.nitems_d ? *A.nitems_d : A.nitems;
   if (blockIdx.x >= nitems) return;  // (uniform: before any barrier or TMEM use)
 
   if (tid == 0) {
@@ -386,14 +512,14 @@ __global__ void __launch_bounds__(B_THREADS, 2)
       mbar_init(&sm.full[s], 1);
       mbar_init(&sm.empty[s], 1);
     }
-    for (int a = 0; a < 2; ++a) {
+    for (int a = 0; a < B_ACCS; ++a) {
       mbar_init(&sm.accfull[a], 1);
-      mbar_init(&sm.accempty[a], B_EPI_WARPS);
+      mbar_init(&sm.accempty[a], B_EPI);
     }
-    mbar_init(&sm.abar, 1);
+    mbar_init(&sm.afull, 1);
     fence_mbar_init();
   }
-  if (warp == 1) {
+  if (warp == B_MMA_WARP) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm.tmem_base)),
                  "r"(TMEM_COLS));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
@@ -403,210 +529,329 @@ __global__ void __launch_bounds__(B_THREADS, 2)
   tc_fence_after();
   const uint32_t tmem = sm.tmem_base;
 
-  uint32_t g = 0;  // sub-tiles of this CTA's earlier items
-  uint32_t iter = 0;
+  uint32_t g = 0, iter = 0, u = 0;
   // a bounded wait gave up: the CTA's later items only mark their queries
   // (combined over the block at each item's closing barrier, so uniform)
   bool aborted = false;
-  // processing slots: blockIdx.x first, then the next free slot of the work
-  // queue (queue != NULL) or blockIdx.x + k * gridDim.x; slot -> item
-  // through order (longest first) when given
   for (uint32_t slot = blockIdx.x; slot < nitems; ++iter) {
-    const uint32_t item_id = order ? order[slot] : slot;
-    const WorkItem it = items[item_id];
-    const Tile tl = tiles[it.tile];
-    const unsigned char *blocks = tl.order == ORDER_TIME ? blocks_t : blocks_c;
+    const uint32_t item_id = A.order ? A.order[slot] : slot;
+    const WorkItem it = A.items[item_id];
+    const Tile tl = A.tiles[it.tile];
+    const bool both = tl.nq > (uint32_t)BM;
     // every stride-th row block of the item (stride 1: all of them)
-    const uint32_t nsub = (it.blk1 - it.blk0 + stride - 1) / stride;
+    const uint32_t nsub = (it.blk1 - it.blk0 + A.stride - 1) / A.stride;
+    const uint32_t nprod = both ? 2 * nsub : nsub;
     bool gave_up = false;  // this thread saw a wait give up in this item
 
-    if (warp == 0) {
+    if (warp == B_LOAD_WARP) {
       // ------------------------------------------------ producer
       if (lane == 0 && !aborted) {
+        const unsigned char *blocks = tl.order == ORDER_TIME ? A.blocks_t : A.blocks_c;
         bool ok = true;
-        mbar_arrive_expect_tx(&sm.abar, TB);
-        bulk_g2s(sm.a, atiles + (uint64_t)it.tile * TB, TB, &sm.abar);
+        const uint32_t na = both ? 2 * TA : TA;
+        mbar_arrive_expect_tx(&sm.afull, na);
+        bulk_g2s(sm.a[0], A.atiles + (uint64_t)it.tile * 2 * TA, na, &sm.afull);
         uint32_t issued = 0;
         // test hook (fknn_index_test_withhold_copy): the first work item issues
         // no row-block copy, so its MMA issuer's and epilogue's waits run out
-        const uint32_t nsub_issue = (withhold && item_id == 0) ? 0u : nsub;
+        const uint32_t nsub_issue = (A.withhold && item_id == 0) ? 0u : nsub;
+#pragma unroll 1
         for (uint32_t sub = 0; sub < nsub_issue; ++sub) {
           const uint32_t gs = g + sub;
           const int st = gs % BS;
-          if (gs >= BS && !mbar_wait_bounded(&sm.empty[st], ((gs / BS) - 1) & 1, err)) {
+          if (gs >= BS && !mbar_wait_bounded(&sm.empty[st], ((gs / BS) - 1) & 1, A.err)) {
             ok = false;
             break;
           }
           mbar_arrive_expect_tx(&sm.full[st], TB);
-          bulk_g2s(sm.b[st], blocks + (uint64_t)(it.blk0 + sub * stride) * TB, TB, &sm.full[st]);
+          bulk_g2s(sm.b[st], blocks + (uint64_t)(it.blk0 + sub * A.stride) * TB, TB, &sm.full[st]);
           ++issued;
         }
         // every issued copy has landed before the item ends
-        ok = mbar_wait_bounded(&sm.abar, iter & 1, err) && ok;
+        ok = mbar_wait_bounded(&sm.afull, iter & 1, A.err) && ok;
+#pragma unroll 1
         for (uint32_t i = issued > BS ? issued - BS : 0; i < issued; ++i)
-          ok = mbar_wait_bounded(&sm.full[(g + i) % BS], ((g + i) / BS) & 1, err) && ok;
+          ok = mbar_wait_bounded(&sm.full[(g + i) % BS], ((g + i) / BS) & 1, A.err) && ok;
         if (!ok || issued != nsub) gave_up = true;
       }
-    } else if (warp == 1) {
+      __syncwarp();
+    } else if (warp == B_MMA_WARP) {
       // ------------------------------------------------ MMA issuer
       if (lane == 0 && !aborted) {
-        uint32_t done = 0;
-        if (mbar_wait_bounded(&sm.abar, iter & 1, err)) {
-          const uint32_t a0 = smem_u32(sm.a);
-          for (uint32_t sub = 0; sub < nsub; ++sub) {
-            const uint32_t gs = g + sub;
-            const int st = gs % BS, ab = gs & 1;
-            if (!mbar_wait_bounded(&sm.full[st], (gs / BS) & 1, err)) break;
-            if (gs >= 2 && !mbar_wait_bounded(&sm.accempty[ab], ((gs >> 1) - 1) & 1, err)) break;
+        uint32_t done = 0, v = u;
+        bool ok = mbar_wait_bounded(&sm.afull, iter & 1, A.err);
+        const uint32_t a0 = smem_u32(sm.a[0]);
+#pragma unroll 1
+        for (uint32_t sub = 0; sub < nsub && ok; ++sub) {
+          const uint32_t gs = g + sub;
+          const int st = gs % BS;
+          if (!mbar_wait_bounded(&sm.full[st], (gs / BS) & 1, A.err)) break;
+          const uint32_t b0 = smem_u32(sm.b[st]);
+#pragma unroll 1
+          for (int half = 0; half < (both ? 2 : 1); ++half, ++v) {
+            const uint32_t ab = v % B_ACCS;
+            if (v >= B_ACCS && !mbar_wait_bounded(&sm.accempty[ab], (v / B_ACCS - 1) & 1, A.err)) {
+              ok = false;
+              break;
+            }
             tc_fence_after();
-            const uint32_t b0 = smem_u32(sm.b[st]);
+            const uint32_t d = tmem + ab * BR, ah = a0 + half * TA;
 #pragma unroll
             for (int kk = 0; kk < F::MMAS; ++kk) {
-              const uint64_t da = umma_desc(a0 + kk * 2 * (BQ / 8) * 128, (BQ / 8) * 128, 128);
+              const uint64_t da = umma_desc(ah + kk * 2 * (BM / 8) * 128, (BM / 8) * 128, 128);
               const uint64_t db = umma_desc(b0 + kk * 2 * (BR / 8) * 128, (BR / 8) * 128, 128);
-              umma<F>(tmem + ab * BR, da, db, kk > 0);
+              umma<F>(d, da, db, kk > 0);
             }
-            umma_commit(&sm.empty[st]);     // the row block may be overwritten once these MMAs finish
-            umma_commit(&sm.accfull[ab]);   // the accumulator is ready for the epilogue
-            ++done;
+            umma_commit(&sm.accfull[ab]);  // the accumulator is ready for the epilogue
           }
+          if (!ok) break;
+          umma_commit(&sm.empty[st]);  // the row block may be overwritten once these MMAs finish
+          ++done;
         }
         // no MMA of this item is in flight when the next item (or the dealloc) comes
-        if (done) {
-          const uint32_t gl = g + done - 1;
-          mbar_wait_bounded(&sm.accfull[gl & 1], (gl >> 1) & 1, err);
-        }
+        if (v > u) mbar_wait_bounded(&sm.accfull[(v - 1) % B_ACCS], ((v - 1) / B_ACCS) & 1, A.err);
         if (done != nsub) gave_up = true;
       }
-    } else {
-      // ------------------------------------------------ epilogue: thread = query
-      const int wslot = warp - 2;
-      const int wg = warp & 3;  // TMEM lanes 32*wg .. 32*wg+31 are reachable from this warp
-      const int L = wg * 32 + lane;
-      uint32_t s = 0, e = 0;
-      const int32_t qi = lane_query(ls, tl, it.tile, L, s, e);
-      // per query: |q|^2 (centred for FP8) and the accumulator's scale 1/lambda
-      const float2 qsc = lane_qs[it.tile * BQ + L];
-      const float qn = qsc.x, sc = qsc.y;
-      float T = -INFINITY;
-      if (qi >= 0) {
-        T = sortable_f32(ld_volatile_u32(T_global + qi));
-        if (ld_volatile_u32(ovf + qi)) T = -INFINITY;
-      }
-      sm.lq[L] = qi;
-      sm.cnt[L] = 0;
-      sm.thr[L] = T;
       __syncwarp();
-      Candidate *list = out + ((uint64_t)item_id * BQ + L) * capb;
-      int cnt = 0;
+    } else {
+      // ------------------------------------------------ epilogue: lane = query = TMEM lane
+      const int c0 = warp / 4 * BP;  // its columns
+      const int row = tid & (BM - 1);
+      const bool pilot = A.stride > 1;
+      if (tid < (both ? BQ : BM)) {
+        uint32_t s = 0, e = 0;
+        const int32_t qi = lane_query(A.ls, tl, it.tile, tid, s, e);
+        float T = -INFINITY;
+        if (qi >= 0) {
+          T = sortable_f32(ld_volatile_u32(A.T_global + qi));
+          if (ld_volatile_u32(A.ovf + qi)) T = -INFINITY;
+        }
+        float2 qs = A.lane_qs[it.tile * BQ + tid];
+        qs.y *= -2.f;
+        sm.lq[tid] = qi;
+        sm.thr[tid] = T;
+        sm.qs[tid] = qs;
+        // in the pilot, a slab of many sampled blocks keeps the best of every
+        // BP rows, a shorter one the best of every 32
+        const bool coarse = (e - s) / (BP * A.stride) >= 4 * exact_seed_rank(A.kseed, 1, A.stride);
+        sm.q[tid] = make_float4(acc_bound(T, qs), __uint_as_float(s), __uint_as_float(e), coarse ? 1.f : 0.f);
+      }
+      asm volatile("bar.sync 1, %0;" ::"n"(B_EPI * 32) : "memory");
+      Candidate *const work = A.work + (uint64_t)blockIdx.x * 2 * B_LISTS * A.capb;
+      auto &wsm = sm.w[warp];
+      const uint32_t lt = (1u << lane) - 1u;
+      int cnt0 = 0, cnt1 = 0;  // entries of this thread's lists
       bool ok = !aborted;
-      // candidate iff qn - 2*sc*acc <= T  <=>  acc >= (qn - T) / (2 sc);
-      // with no bound yet every column of the slab is one (cq = -FLT_MAX),
-      // and columns outside the slab are -inf, which no cq admits.  cq is
-      // recomputed only when T changes.
-      auto acc_bound = [&](float t) { return (t == INFINITY) ? -FLT_MAX : 0.5f * (qn - t) / sc; };
-      float cq = acc_bound(T);
-      uint32_t until_refresh = refresh;  // sub-tiles until the next read of the shared bound
-      for (uint32_t sub = 0; sub < nsub && ok; ++sub) {
-        const uint32_t gs = g + sub;
-        const int ab = gs & 1;
+      uint32_t until_refresh = A.refresh;  // row blocks between reads of the shared bound
+      for (uint32_t v = 0; v < nprod && ok; ++v) {
+        const uint32_t ab = (u + v) % B_ACCS, sub = both ? v / 2 : v;
+        const int half = both ? (int)(v & 1) : 0, L = half * BM + row;
+        const float4 q = sm.q[L];
+        const uint32_t s = __float_as_uint(q.y), e = __float_as_uint(q.z);
+        const uint32_t p0 = (it.blk0 + sub * A.stride) * BR;
+        const int r0 = (int)min(max(s, p0), p0 + BR) - (int)p0;
+        const int r1 = (int)min(max(e, p0), p0 + BR) - (int)p0;
+        const float bound = r0 < r1 ? q.x : INFINITY;
         // warp-uniform: the lanes' timers may disagree at the deadline
-        if (!__all_sync(0xffffffffu, mbar_wait_bounded(&sm.accfull[ab], (gs >> 1) & 1, err))) {
+        if (!__all_sync(0xffffffffu, mbar_wait_bounded(&sm.accfull[ab], ((u + v) / B_ACCS) & 1, A.err))) {
           ok = false;
           break;
         }
         tc_fence_after();
-        const uint32_t p0 = (it.blk0 + sub * stride) * BR;
-        const int r0 = (int)min(max(s, p0), p0 + BR) - (int)p0;
-        const int r1 = (int)min(max(e, p0), p0 + BR) - (int)p0;
-        // four 32-column chunks; the TMEM load of the next chunk is in flight
-        // while this one is screened
-        const uint32_t tb = tmem + ((uint32_t)(wg * 32) << 16) + ab * BR;
-        uint32_t ra[32], rb[32];
-        tmem_ld32_issue(tb, ra);
-        tmem_wait_ld(ra);
-        tmem_ld32_issue(tb + 32, rb);
-        cnt = screen_chunk(ra, 0, r0, r1, cq, qn, sc, p0, &sm.stage[wslot][lane * STAGE_ROW], list, cnt);
-        __syncwarp();
-        tmem_wait_ld(rb);
-        tmem_ld32_issue(tb + 64, ra);
-        cnt = screen_chunk(rb, 32, r0, r1, cq, qn, sc, p0, &sm.stage[wslot][lane * STAGE_ROW], list, cnt);
-        __syncwarp();
-        tmem_wait_ld(ra);
-        tmem_ld32_issue(tb + 96, rb);
-        cnt = screen_chunk(ra, 64, r0, r1, cq, qn, sc, p0, &sm.stage[wslot][lane * STAGE_ROW], list, cnt);
-        __syncwarp();
-        tmem_wait_ld(rb);
-        cnt = screen_chunk(rb, 96, r0, r1, cq, qn, sc, p0, &sm.stage[wslot][lane * STAGE_ROW], list, cnt);
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive1(&sm.accempty[ab]);
-        // lists that could overflow in the next sub-tile are bounded and
-        // trimmed; counts and bounds pass through shared memory only then
-        uint32_t msk = __ballot_sync(0xffffffffu, cnt > (int)capb - BR);
-        if (msk) {
-          sm.cnt[L] = cnt;
-          __syncwarp();
-          while (msk) {
-            const int b = __ffs(msk) - 1;
-            msk &= msk - 1;
-            const int Lb = wg * 32 + b;
-            bcompact<F, NPL>(out + ((uint64_t)item_id * BQ + Lb) * capb, sm, Lb, wslot, kprime, capb, T_global, ovf);
+        const uint32_t tb = tmem + ((uint32_t)((warp & 3) * 32) << 16) + ab * BR + c0;
+        // A chunk of 32 columns whose maximum reaches the bound holds a
+        // candidate, or a row outside the slab that raises it (the appends look
+        // closer).  One chunk in registers at a time: 96 are all a thread has,
+        // and what spills from here comes back from L2 (shared memory takes
+        // the L1's room); the four warps of a scheduler hide the latencies.
+        int cnt = half ? cnt1 : cnt0;
+        const float2 qs = sm.qs[L];
+        bool any = pilot;
+        const bool fine = pilot && __any_sync(0xffffffffu, q.w == 0.f);
+        float best = -INFINITY;
+#pragma unroll 1
+        for (int c = 0; c < BP; c += 64) {
+          uint32_t ra[32], rb[32];
+          tmem_ld32_issue(tb + c, ra);
+          tmem_ld32_issue(tb + c + 32, rb);
+          tmem_wait_ld(ra);
+          tmem_wait_ld(rb);
+          if (c == BP - 64) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive1(&sm.accempty[ab]);
           }
-          cnt = sm.cnt[L];
-          T = sm.thr[L];
-          cq = acc_bound(T);
+          float ga[4], gb[4];
+          const float ma = max32(ra, ga), mb = max32(rb, gb);
+          best = fmax3(best, ma, mb);
+          if (pilot && !fine) continue;
+          uint32_t todo = (ma >= bound ? 1u : 0u) | (mb >= bound ? 2u : 0u);
+          if (!__any_sync(0xffffffffu, todo != 0)) continue;
+          any = true;
+          Candidate *const lists = work + (half * B_LISTS + warp * 32) * A.capb;
+          const int col0 = c0 + c;
+          if (pilot) {
+            if (q.w == 0.f) {
+              if ((todo & 1u) && col0 >= r0 && col0 + 32 <= r1)
+                lists[lane * A.capb + cnt++] = {fmaf(qs.y, ma, qs.x), p0 + col0};
+              if ((todo & 2u) && col0 + 32 >= r0 && col0 + 64 <= r1)
+                lists[lane * A.capb + cnt++] = {fmaf(qs.y, mb, qs.x), p0 + col0 + 32};
+            }
+            continue;
+          }
+          // One candidate in a chunk, as most have: it is the maximum, and its
+          // lane appends it by itself.  The rest are staged in shared memory
+          // and appended by the warp.
+          if (todo & 1u) {
+            const uint32_t in = ge_mask32(ra, ga, bound) & range_mask(r0 - col0, r1 - col0);
+            if ((in & (in - 1)) == 0) todo ^= 1u;
+            if (in && !(todo & 1u)) lists[lane * A.capb + cnt++] = {fmaf(qs.y, ma, qs.x), p0 + col0 + __ffs(in) - 1};
+          }
+          if (todo & 2u) {
+            const uint32_t in = ge_mask32(rb, gb, bound) & range_mask(r0 - col0 - 32, r1 - col0 - 32);
+            if ((in & (in - 1)) == 0) todo ^= 2u;
+            if (in && !(todo & 2u)) lists[lane * A.capb + cnt++] = {fmaf(qs.y, mb, qs.x), p0 + col0 + 31 + __ffs(in)};
+          }
+          while (__any_sync(0xffffffffu, todo != 0)) {
+            // staged in shared memory, in order of chunk, then lane
+            const uint32_t ba = __ballot_sync(0xffffffffu, todo & 1u), bb = __ballot_sync(0xffffffffu, todo & 2u);
+            const int ia = __popc(ba & lt), ib = __popc(ba) + __popc(bb & lt);
+            const uint32_t pack = pack_query(r0, r1, lane, col0);
+            if ((todo & 1u) && ia < B_SLOTS) stage32(wsm.row[ia], ra, bound, qs.y, qs.x, pack), todo ^= 1u;
+            if ((todo & 2u) && ib < B_SLOTS) stage32(wsm.row[ib], rb, bound, qs.y, qs.x, pack + (1u << 23)), todo ^= 2u;
+            const int ns = min(__popc(ba) + __popc(bb), B_SLOTS);
+            __syncwarp();
+            // and appended: a column per lane, two lanes' chunks at a time
+            constexpr int W = 2;
+#pragma unroll 1
+            for (int i = 0; i < ns; i += W) {
+              float ds[W];
+              uint32_t m[W], col[W];
+              int src[W];
+              bool pass[W];
+#pragma unroll
+              for (int j = 0; j < W; ++j) {
+                const float *x = wsm.row[min(i + j, ns - 1)];
+                const float val = x[lane];
+                const float4 t = *reinterpret_cast<const float4 *>(x + 32);
+                const uint32_t pk = __float_as_uint(t.w);
+                col[j] = (pk >> 23) * 32 + lane;
+                src[j] = (pk >> 18) & 31;
+                pass[j] = i + j < ns && val >= t.x && col[j] >= (pk & 511) && col[j] < (pk >> 9 & 511);
+                ds[j] = fmaf(t.y, val, t.z);
+              }
+#pragma unroll
+              for (int j = 0; j < W; ++j) m[j] = __ballot_sync(0xffffffffu, pass[j]);
+#pragma unroll
+              for (int j = 0; j < W; ++j) {
+                const int n = __shfl_sync(0xffffffffu, cnt, src[j]);
+                if (pass[j]) lists[src[j] * A.capb + n + __popc(m[j] & lt)] = {ds[j], p0 + col[j]};
+                if (lane == src[j]) cnt += __popc(m[j]);
+              }
+            }
+            __syncwarp();  // the rows are free again
+          }
+        }
+        if (any) {
+          if (pilot && q.w != 0.f && best >= bound && c0 >= r0 && c0 + BP <= r1)
+            work[(half * B_LISTS + tid) * A.capb + cnt++] = {fmaf(qs.y, best, qs.x), p0 + c0};
+          Candidate *const lists = work + (half * B_LISTS + warp * 32) * A.capb;
+          // lists that could overflow next are trimmed (a product adds at most BP)
+          uint32_t msk = __ballot_sync(0xffffffffu, cnt > (int)A.capb - BP);
+#pragma unroll 1
+          for (; msk; msk &= msk - 1) {
+            const int b = __ffs(msk) - 1;
+            const int n = b_trim<F, NPL>(lists + (uint64_t)b * A.capb, __shfl_sync(0xffffffffu, cnt, b), sm,
+                                         half * BM + (warp & 3) * 32 + b, A.kprime, A.capb, A.T_global, A.ovf);
+            if (lane == b) cnt = n;
+          }
+          if (half) cnt1 = cnt;
+          else cnt0 = cnt;
         }
         // other items of the same query tighten the shared bound meanwhile
-        // (every refresh-th sub-tile of the item)
-        if (refresh && --until_refresh == 0) {
-          until_refresh = refresh;
-          if (qi >= 0) {
-            const float Tg = sortable_f32(ld_volatile_u32(T_global + qi));
-            if (Tg < T) {
-              T = Tg;
-              sm.thr[L] = T;
-              cq = acc_bound(T);
+        // (every refresh-th row block of the item)
+        if (A.refresh && half == (both ? 1 : 0) && --until_refresh == 0) {
+          until_refresh = A.refresh;
+#pragma unroll 1
+          for (int i = tid; i < (both ? BQ : BM); i += B_EPI * 32) {
+            const int32_t qi = sm.lq[i];
+            if (qi < 0) continue;
+            const float Tg = sortable_f32(ld_volatile_u32(A.T_global + qi));
+            if (Tg < sm.thr[i]) {
+              sm.thr[i] = Tg;
+              sm.q[i].x = acc_bound(Tg, sm.qs[i]);
             }
           }
         }
       }
       if (!ok) {
         // this item's queries are answered by the exact scan
-        if (qi >= 0) ovf[qi] = 1u;
-        out_cnt[(uint64_t)item_id * BQ + L] = 0;
+#pragma unroll 1
+        for (int i = row; i < (both ? BQ : BM); i += BM)
+          if (sm.lq[i] >= 0) A.ovf[sm.lq[i]] = 1u;
+        cnt0 = cnt1 = 0;
         gave_up = true;
-      } else {
-        sm.cnt[L] = cnt;
-        __syncwarp();
-        for (int b = 0; b < 32; ++b) {
-          const int Lb = wg * 32 + b;
-          if (sm.cnt[Lb] > 0 && sm.lq[Lb] >= 0)
-            bcompact<F, NPL>(out + ((uint64_t)item_id * BQ + Lb) * capb, sm, Lb, wslot, kprime, capb, T_global,
-                             ovf);
-        }
-        out_cnt[(uint64_t)item_id * BQ + L] = (uint32_t)sm.cnt[L];
       }
+      sm.cnt[0][tid] = cnt0;
+      sm.cnt[1][tid] = cnt1;
+      // every list of the item is complete (and visible)
+      asm volatile("bar.sync 1, %0;" ::"n"(B_EPI * 32) : "memory");
+      // a query's lists become the item's result
+      const int per = (both ? BQ : BM) / B_EPI;
+      const int q0 = warp * per, l0 = q0 % BM, hf = q0 / BM;  // its first query
+      int n = 0;
+      if (lane < per && sm.thr[q0 + lane] != -INFINITY)  // (marked: the exact scan answers it)
+#pragma unroll 1
+        for (int l = 0; l < B_LISTS; l += BM) n += sm.cnt[hf][l0 + lane + l];
+      const uint64_t o0 = (uint64_t)item_id * BQ + q0;
+#pragma unroll 1
+      for (int b = 0; b < per; ++b) {
+        const int nb = __shfl_sync(0xffffffffu, n, b);
+        if (nb == 0) continue;
+        Candidate *src = work + (uint64_t)(hf * B_LISTS + l0 + b) * A.capb, *dst = A.out + (o0 + b) * A.capb;
+        int *c = &sm.cnt[hf][l0 + b];
+        if (nb > (int)A.capb) {
+          const int kept = b_select<F>(src, c, sm, q0 + b, A.kprime, A.capb, A.T_global, dst);
+          if (lane == b) n = kept;
+          continue;
+        }
+        int at = 0;
+#pragma unroll 1
+        for (int l = 0; l < B_LISTS; l += BM) {
+          const uint2 *x = reinterpret_cast<const uint2 *>(src + (uint64_t)l * A.capb);
+#pragma unroll 1
+          for (int i = lane; i < c[l]; i += 32) reinterpret_cast<uint2 *>(dst)[at + i] = x[i];
+          at += c[l];
+        }
+      }
+      if (n > (int)A.capb) {  // more ties than fit
+        A.ovf[sm.lq[q0 + lane]] = 1u;
+        n = 0;
+      }
+      if (lane < per) A.out_cnt[o0 + lane] = (uint32_t)n;
     }
     g += nsub;
+    u += nprod;
     // double-buffered by item parity: a slow thread may still read the slot
     // of this barrier while thread 0 writes the one after
-    if (queue && tid == 0) sm.next[(iter + 1) & 1] = atomicAdd(queue, 1u) + gridDim.x;
+    if (tid == 0) sm.next[iter & 1] = atomicAdd(A.queue, 1u) + gridDim.x;
     tc_fence_before();
-    // the item's shared state (A tile, lists' counts, bounds) is reused by the next
+    // the item's shared state (queries, counts, bounds) is reused by the next
     aborted = __syncthreads_or(aborted || gave_up) != 0;
     tc_fence_after();
-    slot = queue ? sm.next[(iter + 1) & 1] : slot + gridDim.x;
+    slot = sm.next[iter & 1];
   }
-  if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
+  if (warp == B_MMA_WARP)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
 }
 
 // ------------------------------------------------------------ re-rank --
 
-constexpr int RR_THREADS = 256;
+constexpr int RR_THREADS = 128;
 constexpr int RR_CAP = 8192;        // screening candidates the large merge holds
-constexpr int RR_CAP_SMALL = 2048;  // ... and the common one (8 blocks per SM)
+constexpr int RR_CAP_SMALL = 1024;  // ... and the common one (12 blocks per SM)
 constexpr int RR_KMAX = 1024;       // largest k'
+constexpr int RR_ITEMS = 256;       // work items of a tile (the lists' offsets)
 
 template <int CAP>
 struct RerankSmem {
@@ -614,8 +859,9 @@ struct RerankSmem {
   uint32_t val[CAP];
   uint64_t ekey[RR_KMAX];
   float qv[DIM];
-  uint32_t cnt_prefix[RR_THREADS + 1];
-  int total;
+  uint32_t cnt_prefix[RR_ITEMS + 1];
+  uint32_t hist[256], red[4];
+  int total, kept;
 };
 
 struct MergeArgs {
@@ -665,7 +911,8 @@ __device__ void merge_one(const MergeArgs &A, uint32_t b, RerankSmem<CAP> &sm, u
   for (int d = tid; d < DIM; d += RR_THREADS) sm.qv[d] = q[(uint64_t)qi * DIM + d];
   // candidate counts of the query's items (a tile has at most a few dozen)
   // more items than prefix slots: the exact scan answers the query
-  list_offsets(item_slot, tl.item0, nitems, out_cnt, L, BQ, sm.cnt_prefix, &sm.total, RR_THREADS, RR_CAP + 1);
+  list_offsets(item_slot, tl.item0, nitems, out_cnt, L, BQ, sm.cnt_prefix, &sm.total, RR_ITEMS, RR_CAP + 1);
+  if (tid == 0) sm.kept = 0;
   __syncthreads();
   const int M = sm.total;
   if (M > CAP && spill && M <= RR_CAP) {  // the large merge takes it
@@ -678,39 +925,69 @@ __device__ void merge_one(const MergeArgs &A, uint32_t b, RerankSmem<CAP> &sm, u
     if (tid == 0) ovf_list[atomicAdd(ovf_count, 1u)] = qi;
     return;
   }
-  // the whole block copies each item's list
-  for (uint32_t i = 0; i < nitems; ++i) {
+  // a warp copies a list at a time
+  for (uint32_t i = tid / 32; i < nitems; i += RR_THREADS / 32) {
     const uint64_t item = item_slot ? item_slot[tl.item0 + i] : tl.item0 + i;
     const uint32_t base = sm.cnt_prefix[i];
     const uint32_t c = (i + 1 < nitems ? sm.cnt_prefix[i + 1] : (uint32_t)M) - base;
     const Candidate *src = out + (item * BQ + L) * capb;
-    for (uint32_t j = tid; j < c; j += RR_THREADS) {
+    for (uint32_t j = tid & 31; j < c; j += 32) {
       const Candidate cd = src[j];
       sm.key[base + j] = cd.ds;
       sm.val[base + j] = cd.pos;
     }
   }
-  int np2 = 32;
-  while (np2 < M) np2 <<= 1;
-  for (int i = M + tid; i < np2; i += RR_THREADS) {
-    sm.key[i] = INFINITY;
-    sm.val[i] = 0xffffffffu;
-  }
   __syncthreads();
-  block_bitonic_sort_kv(sm.key, sm.val, np2);
   // FP32 re-rank of the k' best screened rows with the reference's arithmetic
+  // (of those at the k'-th screening distance itself, the first ones of the order)
   const int C = min(M, (int)kprime);
   const uint32_t *perm = dsc.order == ORDER_TIME ? perm_t : perm_c;
-  for (int i = tid; i < C; i += RR_THREADS) {
-    const uint32_t id = perm[sm.val[i]];
-    const float d = seq_l2_strided(vecs + (uint64_t)id * DIM, 1, sm.qv);
-    sm.ekey[i] = exact_key(d, id);
+  uint32_t kth = 0xffffffffu;
+  if (M > C) kth = block_kth<RR_THREADS>(sm.key, M, (uint32_t)C, sm.hist, sm.red);
+  for (int i = tid; i < M; i += RR_THREADS) {
+    const uint32_t u = f32_sortable(sm.key[i]);
+    if (u < kth || M == C) sm.ekey[atomicAdd(&sm.kept, 1)] = sm.val[i];
   }
-  int cp2 = 32;
-  while (cp2 < C) cp2 <<= 1;
-  for (int i = C + tid; i < cp2; i += RR_THREADS) sm.ekey[i] = ~0ull;
   __syncthreads();
-  block_bitonic_sort(sm.ekey, cp2);
+  if (M > C) {
+    const int below = sm.kept;
+    const float tie = sortable_f32(kth);
+    for (int i = tid; i < M; i += RR_THREADS)
+      if (f32_sortable(sm.key[i]) == kth) {
+        int at = below;
+        for (int j = 0; j < M; ++j) at += sm.key[j] == tie && sm.val[j] < sm.val[i] ? 1 : 0;
+        if (at < C) sm.ekey[at] = sm.val[i];
+      }
+    __syncthreads();
+  }
+  for (int i = tid; i < C; i += RR_THREADS) {
+    const uint32_t id = perm[(uint32_t)sm.ekey[i]];
+    sm.ekey[i] = exact_key(seq_l2_row(vecs + (uint64_t)id * DIM, sm.qv), id);
+  }
+  // order: a key's place is the number of smaller ones (they are distinct),
+  // counted by its thread; above 2 keys a thread the sort is faster
+  if (C <= 2 * RR_THREADS) {
+    uint64_t e[2];
+    int rank[2] = {0, 0};
+    __syncthreads();
+    e[0] = tid < C ? sm.ekey[tid] : ~0ull;
+    e[1] = tid + RR_THREADS < C ? sm.ekey[tid + RR_THREADS] : ~0ull;
+    for (int j = 0; j < C; ++j) {
+      const uint64_t x = sm.ekey[j];
+      rank[0] += x < e[0] ? 1 : 0;
+      rank[1] += x < e[1] ? 1 : 0;
+    }
+    __syncthreads();
+    if (tid < C) sm.ekey[rank[0]] = e[0];
+    if (tid + RR_THREADS < C) sm.ekey[rank[1]] = e[1];
+    __syncthreads();
+  } else {
+    int cp2 = 32;
+    while (cp2 < C) cp2 <<= 1;
+    for (int i = C + tid; i < cp2; i += RR_THREADS) sm.ekey[i] = ~0ull;
+    __syncthreads();
+    block_bitonic_sort(sm.ekey, cp2);
+  }
   // FP64 at the k-th boundary: candidates within 1e-6 relative of the k-th
   // FP32 distance are ordered by their exact double distance
   if (tid == 0 && C > 0) {
@@ -777,22 +1054,52 @@ __global__ void __launch_bounds__(RR_THREADS)
   }
 }
 
-// Seeds the shared bound of every long query from the pilot pass: T_A is
-// the r-th smallest screening distance over every stride-th row block, an
-// estimate of the k'-th over all rows (r is chosen so that it lies above it
-// with high probability; the merge catches the rest).
-__global__ void k_seed_bounds(const uint32_t *__restrict__ big_q, uint32_t nbig_h, const uint32_t *__restrict__ nbig_d,
-                              const QueryDesc *__restrict__ desc, const uint32_t *__restrict__ T_A,
-                              const uint32_t *__restrict__ ovf_A, uint32_t min_rows, uint32_t *__restrict__ T_global,
-                              uint32_t *__restrict__ seeded) {
-  const uint32_t nbig = nbig_d ? *nbig_d : nbig_h;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nbig; i += gridDim.x * blockDim.x) {
-    const uint32_t qi = big_q[i];
-    const uint32_t inf = f32_sortable(INFINITY);
-    const bool s = desc[qi].e - desc[qi].s >= min_rows && T_A[qi] < inf && !ovf_A[qi];
-    T_global[qi] = s ? T_A[qi] : inf;
-    seeded[qi] = s ? 1u : 0u;
+struct SeedBound {
+  __device__ float operator()(float ds, const QueryDesc &) const { return ds; }
+};
+
+// A search's per-query state and counters, in one buffer of words: the bounds
+// (filled with +inf), what starts at zero, and the lists.
+struct TcState {
+  uint32_t *T_global, *T_pilot;                    // nq each, adjacent
+  uint32_t *ovf, *ovf_pilot, *seeded;              // nq each, adjacent, before the counters
+  uint32_t *ovf_count, *n_f64, *spill_count, *queue;  // queue: pilot, main
+  uint32_t *ovf_list, *spill;                      // nq each
+  static size_t bytes(uint32_t nq) { return ((size_t)nq * 7 + 16) * 4; }
+  TcState(uint32_t *d, uint32_t nq) {
+    T_global = d;
+    T_pilot = T_global + nq;
+    ovf = T_pilot + nq;
+    ovf_pilot = ovf + nq;
+    seeded = ovf_pilot + nq;
+    ovf_count = seeded + nq;
+    n_f64 = ovf_count + 1;
+    spill_count = ovf_count + 2;
+    queue = ovf_count + 4;
+    ovf_list = ovf_count + 16;
+    spill = ovf_list + nq;
   }
+  int reset(uint32_t nq, cudaStream_t st) const {
+    int rc;
+    if ((rc = launch_fill_u32(T_global, nq * 2, f32_sortable(INFINITY), st))) return rc;
+    FKNN_CUDA(cudaMemsetAsync(ovf, 0, ((size_t)nq * 3 + 16) * 4, st));
+    return FKNN_OK;
+  }
+};
+
+// Work items a tile may have: what the merge holds of their lists, and the
+// scratch (8 GB).  Behind a seeded bound all of a query's lists together hold
+// 3 k' entries or so, and a query too short to be seeded meets few items.
+inline uint32_t max_items(uint32_t capb, uint32_t pilot_stride, uint64_t per_item, uint64_t tiles) {
+  const uint64_t lists = pilot_stride > 1 ? RR_ITEMS : std::min<uint64_t>(RR_ITEMS, RR_CAP / capb);
+  return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(lists, (8ull << 30) / (per_item * tiles)));
+}
+
+// the trim holds a whole list in registers: 32 x NPL >= capb
+template <class F>
+static void (*screen_kernel(uint32_t capb))(ScreenArgs) {
+  return capb <= 384 ? k_screen_tc<F, 12> : capb <= 512 ? k_screen_tc<F, 16> : capb <= 768 ? k_screen_tc<F, 24>
+       : capb <= 1024 ? k_screen_tc<F, 32> : k_screen_tc<F, 40>;
 }
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
@@ -802,7 +1109,7 @@ inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 int build_bf16(fknn_index *idx, cudaStream_t st) {
   const uint64_t nblk = (idx->n + BR - 1) / BR;
   for (int o = 0; o < 2; ++o) {
-    int rc = dev_alloc(idx, &idx->bf16_blocks[o], nblk * BF_TILE);
+    int rc = dev_alloc(idx, &idx->bf16_blocks[o], nblk * Tiles<FmtBF16>::B);
     if (rc) return rc;
     k_build_bf16_blocks<<<(unsigned)nblk, 256, 0, st>>>(idx->vecs, idx->norms, idx->ord[o].perm, idx->n,
                                                         (__nv_bfloat16 *)idx->bf16_blocks[o]);
@@ -824,7 +1131,7 @@ int build_fp8(fknn_index *idx, cudaStream_t st) {
   k_fp8_params<<<1, 128, 0, st>>>(mm, mm + DIM, idx->fp8_scale, idx->fp8_scale + DIM);
   g_launches += 2;
   for (int o = 0; o < 2; ++o) {
-    if ((rc = dev_alloc(idx, &idx->fp8_blocks[o], nblk * F8_TILE))) return rc;
+    if ((rc = dev_alloc(idx, &idx->fp8_blocks[o], nblk * Tiles<FmtFP8>::B))) return rc;
     k_build_fp8_blocks<<<(unsigned)nblk, 256, 0, st>>>(idx->vecs, idx->ord[o].perm, idx->n, idx->fp8_scale,
                                                        idx->fp8_scale + DIM, (unsigned char *)idx->fp8_blocks[o]);
     g_launches += 1;
@@ -833,11 +1140,55 @@ int build_fp8(fknn_index *idx, cudaStream_t st) {
   return FKNN_OK;
 }
 
+// The pilot, its seeds and the screen proper.  The pilot keeps the best of
+// every 32 rows of every stride-th row block: as the few rows that matter lie
+// in different groups as a rule, the r-th best of these is little above the
+// r-th of the sample's rows (and never below it), at a 32nd of the entries.
+template <class K>
+static void launch_screens(K screen, ScreenArgs X, SeedArgs Z, const TcState &S, uint32_t kprime, uint32_t stride,
+                           uint32_t refresh, bool withhold, uint32_t grid, uint32_t nbig_max, size_t smem,
+                           cudaStream_t st) {
+  if (stride > 1) {
+    X.T_global = S.T_pilot;
+    X.ovf = S.ovf_pilot;
+    // (the sample of a short slab is up to twice its nominal share)
+    X.kprime = exact_seed_rank(kprime, 2, stride);
+    X.kseed = kprime;
+    X.refresh = 0;
+    X.stride = stride;
+    X.withhold = 0;
+    X.queue = S.queue;
+    screen<<<grid, B_THREADS, smem, st>>>(X);
+    Z.tiles = X.tiles;
+    Z.items = X.items;
+    Z.out = X.out;
+    Z.out_cnt = X.out_cnt;
+    Z.tq = BQ;
+    Z.list_cap = X.capb;
+    Z.blk_rows = BR;
+    Z.stride = stride;
+    Z.k = kprime;
+    Z.T_global = S.T_global;
+    Z.seeded = S.seeded;
+    launch_screen_seed(Z, nbig_max, SeedBound(), st);
+    g_launches += 1;
+  }
+  X.T_global = S.T_global;
+  X.ovf = S.ovf;
+  X.kprime = kprime;
+  X.refresh = refresh;
+  X.stride = 1;
+  X.withhold = withhold ? 1u : 0u;
+  X.queue = S.queue + 1;
+  screen<<<grid, B_THREADS, smem, st>>>(X);
+  g_launches += 1;
+}
+
 template <class F>
 static int search_tc(fknn_index *idx, const float *d_q, const float *d_meta, uint32_t nq, uint32_t k, uint32_t kprime,
                      uint32_t *d_ids, float *d_dists, cudaStream_t st, fknn_search_stats *stats) {
   const uint64_t n = idx->n;
-  constexpr uint32_t TB = Tiles<F>::BYTES;
+  constexpr uint32_t TA = Tiles<F>::A;
   int rc;
   QueryDesc *d_desc, *h_desc;
   float *h_meta;
@@ -848,7 +1199,7 @@ static int search_tc(fknn_index *idx, const float *d_q, const float *d_meta, uin
   // candidate slots per (item, query): k' plus the pushes between trims; a
   // list holds at most 1280 (32 lanes x 40 registers in the trim)
   const uint32_t capb =
-      (uint32_t)std::min<size_t>(1280, align_up(kprime + std::max<uint32_t>(tune.list_slack, 2 * BR), 128));
+      (uint32_t)std::min<size_t>(1280, align_up(kprime + std::max<uint32_t>(tune.list_slack, 2 * BP), 128));
   auto t0 = std::chrono::steady_clock::now();
   Plan &P = idx->plan;
   PlanShape shape;
@@ -858,9 +1209,8 @@ static int search_tc(fknn_index *idx, const float *d_q, const float *d_meta, uin
   // candidate scratch (items x 128 x capb x 8 B) stays within ~8 GB
   const uint64_t per_item = (uint64_t)BQ * capb * sizeof(Candidate);
   const uint64_t tiles_est = std::max<uint64_t>(1, (nq + BQ - 1) / BQ);
-  shape.max_items_per_tile = (uint32_t)std::max<uint64_t>(
-      1, std::min<uint64_t>(RR_CAP / capb, (8ull << 30) / (per_item * tiles_est)));
-  shape.min_chunk_blocks = tune.min_chunk_blocks;
+  shape.max_items_per_tile = max_items(capb, tune.pilot_stride, per_item, tiles_est);
+  shape.min_chunk_blocks = (tune.min_chunk_blocks + 1) / 2;  // (given in 128-row blocks)
   shape.target_items = idx->num_sms * tune.items_per_sm;
   make_plan(h_desc, h_meta, nq, n, shape, P);
   auto t1 = std::chrono::steady_clock::now();
@@ -903,32 +1253,23 @@ static int search_tc(fknn_index *idx, const float *d_q, const float *d_meta, uin
   put(o_slot, slot.data(), nitems * 4);
   if (blob) FKNN_CUDA(cudaMemcpyAsync(d_blob, h_blob, blob, cudaMemcpyHostToDevice, st));
   uint32_t *d_state;
-  if ((rc = ws_get(idx, 5, (size_t)nq * 16 + 64, (void **)&d_state))) return rc;
-  uint32_t *T_global = d_state, *ovf = d_state + nq, *ovf_list = d_state + 2 * (size_t)nq,
-           *ovf_count = d_state + 3 * (size_t)nq, *n_f64 = ovf_count + 1, *spill_count = ovf_count + 2;
-  // spill list (big-query indices for the large merge): spill_count + 1 .. + nq
-  if ((rc = launch_fill_u32(T_global, nq, f32_sortable(INFINITY), st))) return rc;
-  FKNN_CUDA(cudaMemsetAsync(ovf, 0, (size_t)nq * 4, st));
-  FKNN_CUDA(cudaMemsetAsync(ovf_count, 0, 12, st));
-  // pilot state: bound estimate, seeded flag, pilot overflow per query
-  uint32_t *d_pilot = nullptr, *seeded = nullptr;
-  if (tune.pilot_stride > 1) {
-    if ((rc = ws_get(idx, 11, (size_t)nq * 12, (void **)&d_pilot))) return rc;
-    seeded = d_pilot + nq;
-    FKNN_CUDA(cudaMemsetAsync(seeded, 0, (size_t)nq * 4, st));
-  }
+  if ((rc = ws_get(idx, 5, TcState::bytes(nq), (void **)&d_state))) return rc;
+  const TcState S(d_state, nq);
+  if ((rc = S.reset(nq, st))) return rc;
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
   if (stats)
     for (auto &e : ev) FKNN_CUDA(cudaEventCreate(&e));
   const OrderData &OT = idx->ord[ORDER_TIME], &OC = idx->ord[ORDER_CAT];
   if (nitems) {
     unsigned char *d_at;
-    Candidate *d_out;
+    Candidate *d_out, *d_work;
     uint32_t *d_ocnt;
     float2 *d_lqs;
-    if ((rc = ws_get(idx, 4, (size_t)ntile * TB, (void **)&d_at))) return rc;
+    if ((rc = ws_get(idx, 4, (size_t)ntile * 2 * TA, (void **)&d_at))) return rc;
     if ((rc = ws_get(idx, 10, (size_t)ntile * BQ * sizeof(float2), (void **)&d_lqs))) return rc;
-    if ((rc = ws_get(idx, 6, (size_t)nitems * BQ * capb * sizeof(Candidate), (void **)&d_out))) return rc;
+    if ((rc = ws_get(idx, 6, (size_t)nitems * per_item, (void **)&d_out))) return rc;
+    const uint32_t sgrid = std::min<uint32_t>(nitems, (uint32_t)idx->num_sms);
+    if ((rc = ws_get(idx, 11, (size_t)sgrid * 2 * B_LISTS * capb * sizeof(Candidate), (void **)&d_work))) return rc;
     if ((rc = ws_get(idx, 7, (size_t)nitems * BQ * 4, (void **)&d_ocnt))) return rc;
     LaneSrc ls;
     ls.lane_q = (const int32_t *)(d_blob + o_lq);
@@ -941,9 +1282,7 @@ static int search_tc(fknn_index *idx, const float *d_q, const float *d_meta, uin
       k_tile_stage_bf16<<<ntile, 256, 0, st>>>(d_q, ls, (const Tile *)(d_blob + o_tiles), ntile, d_desc,
                                                (__nv_bfloat16 *)d_at, d_lqs);
     // per device context, so set on every call (cheap)
-    // the compaction holds a whole list in registers: 32 x NPL >= capb
-    auto screen = capb <= 512 ? k_screen_tc<F, 16> : capb <= 768 ? k_screen_tc<F, 24>
-                : capb <= 1024 ? k_screen_tc<F, 32> : k_screen_tc<F, 40>;
+    auto screen = screen_kernel<F>(capb);
     FKNN_CUDA(cudaFuncSetAttribute(screen, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)sizeof(BScreenSmem<F>)));
     FKNN_CUDA(cudaFuncSetAttribute(k_merge_rerank<RR_CAP_SMALL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -953,28 +1292,32 @@ static int search_tc(fknn_index *idx, const float *d_q, const float *d_meta, uin
     if (stats) FKNN_CUDA(cudaEventRecord(ev[0], st));
     void *const *blocks = F::kFP8 ? idx->fp8_blocks : idx->bf16_blocks;
     const uint32_t stride = tune.pilot_stride;
-    if (stride > 1) {
-      // pilot: every stride-th row block with a short list; its r-th
-      // distance seeds the bound of queries with long slabs
-      // the k'-th of all rows ranks about k'/stride in the sample; r = 3 k'/stride
-      // + 8 lies above it but for a vanishing fraction of queries
-      const uint32_t r = std::min<uint32_t>(kprime, (3 * kprime + stride - 1) / stride + 8);
-      uint32_t *T_A = d_pilot, *ovf_A = d_pilot + 2 * (size_t)nq;
-      if ((rc = launch_fill_u32(T_A, nq, f32_sortable(INFINITY), st))) return rc;
-      FKNN_CUDA(cudaMemsetAsync(ovf_A, 0, (size_t)nq * 4, st));
-      screen<<<nitems, B_THREADS, sizeof(BScreenSmem<F>), st>>>(
-          (const WorkItem *)(d_blob + o_items), (const Tile *)(d_blob + o_tiles), d_at, ls, d_lqs,
-          (const unsigned char *)blocks[ORDER_TIME], (const unsigned char *)blocks[ORDER_CAT], T_A, ovf_A, d_out,
-          d_ocnt, r, capb, 0, stride, 0u, nitems, nullptr, nullptr, nullptr, idx->d_flag);
-      k_seed_bounds<<<std::max<uint32_t>(1, std::min<uint32_t>((nbig + 255) / 256, 1184)), 256, 0, st>>>(
-          (const uint32_t *)(d_blob + o_big), nbig, nullptr, d_desc, T_A, ovf_A, 16 * stride * BR, T_global, seeded);
-      g_launches += 3;
-    }
-    screen<<<nitems, B_THREADS, sizeof(BScreenSmem<F>), st>>>(
-        (const WorkItem *)(d_blob + o_items), (const Tile *)(d_blob + o_tiles), d_at, ls, d_lqs,
-        (const unsigned char *)blocks[ORDER_TIME], (const unsigned char *)blocks[ORDER_CAT], T_global, ovf, d_out,
-        d_ocnt, kprime, capb, tune.bound_refresh, 1, idx->test_withhold ? 1u : 0u, nitems, nullptr, nullptr, nullptr,
-        idx->d_flag);
+    ScreenArgs X;
+    X.items = (const WorkItem *)(d_blob + o_items);
+    X.tiles = (const Tile *)(d_blob + o_tiles);
+    X.atiles = d_at;
+    X.ls = ls;
+    X.lane_qs = d_lqs;
+    X.blocks_t = (const unsigned char *)blocks[ORDER_TIME];
+    X.blocks_c = (const unsigned char *)blocks[ORDER_CAT];
+    X.out = d_out;
+    X.out_cnt = d_ocnt;
+    X.work = d_work;
+    X.capb = capb;
+    X.nitems = nitems;
+    X.nitems_d = nullptr;
+    X.order = nullptr;
+    X.err = idx->d_flag;
+    SeedArgs Z;
+    Z.big_q = (const uint32_t *)(d_blob + o_big);
+    Z.big_tile = (const uint32_t *)(d_blob + o_btile);
+    Z.big_lane = (const uint32_t *)(d_blob + o_blane);
+    Z.nbig = nbig;
+    Z.nbig_d = nullptr;
+    Z.item_slot = (const uint32_t *)(d_blob + o_slot);
+    Z.desc = d_desc;
+    launch_screens(screen, X, Z, S, kprime, stride, tune.bound_refresh, idx->test_withhold, sgrid, nbig,
+                   sizeof(BScreenSmem<F>), st);
     idx->test_withhold = false;
     if (stats) FKNN_CUDA(cudaEventRecord(ev[1], st));
     MergeArgs A;
@@ -990,28 +1333,27 @@ static int search_tc(fknn_index *idx, const float *d_q, const float *d_meta, uin
     A.vecs = idx->vecs;
     A.perm_t = OT.perm;
     A.perm_c = OC.perm;
-    A.ovf = ovf;
-    A.ovf_list = ovf_list;
-    A.ovf_count = ovf_count;
+    A.ovf = S.ovf;
+    A.ovf_list = S.ovf_list;
+    A.ovf_count = S.ovf_count;
     A.k = k;
     A.kprime = kprime;
     A.capb = capb;
-    A.seeded = stride > 1 ? seeded : nullptr;
+    A.seeded = stride > 1 ? S.seeded : nullptr;
     A.ids = d_ids;
     A.dists = d_dists;
-    A.n_f64 = n_f64;
+    A.n_f64 = S.n_f64;
     A.nbig_d = nullptr;
     // queries with more candidates than the common merge holds go to the large one
-    uint32_t *spill = spill_count + 1;
     k_merge_rerank<RR_CAP_SMALL><<<nbig, RR_THREADS, sizeof(RerankSmem<RR_CAP_SMALL>), st>>>(
-        A, nbig, nullptr, nullptr, spill, spill_count);
-    k_merge_rerank<RR_CAP><<<148 * 2, RR_THREADS, sizeof(RerankSmem<RR_CAP>), st>>>(A, 0, spill, spill_count,
+        A, nbig, nullptr, nullptr, S.spill, S.spill_count);
+    k_merge_rerank<RR_CAP><<<148 * 2, RR_THREADS, sizeof(RerankSmem<RR_CAP>), st>>>(A, 0, S.spill, S.spill_count,
                                                                                      nullptr, nullptr);
-    g_launches += 4;
+    g_launches += 3;
   }
   if (stats) FKNN_CUDA(cudaEventRecord(ev[2], st));
   if (nbig)
-    if ((rc = launch_exact_scan(idx, ovf_list, ovf_count, 0, 148 * 2, d_desc, d_q, k, d_ids, d_dists, st))) return rc;
+    if ((rc = launch_exact_scan(idx, S.ovf_list, S.ovf_count, 0, 148 * 2, d_desc, d_q, k, d_ids, d_dists, st))) return rc;
   if (nsmall_early && (rc = join_small_scans(idx, st))) return rc;
   FKNN_CUDA(cudaGetLastError());
   if (stats) {
@@ -1035,7 +1377,7 @@ static int search_tc(fknn_index *idx, const float *d_q, const float *d_meta, uin
     stats->n_small = nsmall;
     stats->ms_plan = std::chrono::duration<float, std::milli>(t1 - t0).count();
     uint32_t h2[2] = {0, 0};
-    FKNN_CUDA(cudaMemcpyAsync(h2, ovf_count, 8, cudaMemcpyDeviceToHost, st));
+    FKNN_CUDA(cudaMemcpyAsync(h2, S.ovf_count, 8, cudaMemcpyDeviceToHost, st));
     FKNN_CUDA(cudaStreamSynchronize(st));
     stats->n_overflow = h2[0];
     stats->n_boundary_f64 = h2[1];
@@ -1052,37 +1394,38 @@ template <class F>
 static int search_tc_graph(fknn_index *idx, const float *d_q, const float *d_meta, uint32_t nq, uint32_t k,
                            uint32_t kprime, uint32_t *d_ids, float *d_dists, cudaStream_t st,
                            fknn_search_stats *stats) {
-  constexpr uint32_t TB = Tiles<F>::BYTES;
+  constexpr uint32_t TA = Tiles<F>::A;
   int rc;
   const fknn_tuning tune = idx->tuning[F::kFP8 ? FKNN_MODE_FP8_RERANK : FKNN_MODE_BF16_RERANK];
   const uint32_t capb =
-      (uint32_t)std::min<size_t>(1280, align_up(kprime + std::max<uint32_t>(tune.list_slack, 2 * BR), 128));
+      (uint32_t)std::min<size_t>(1280, align_up(kprime + std::max<uint32_t>(tune.list_slack, 2 * BP), 128));
   PlanShape shape;
   shape.tq = BQ;
   shape.blk_rows = BR;
   shape.small_slab = SMALL_SLAB;
-  shape.min_chunk_blocks = tune.min_chunk_blocks;
+  shape.min_chunk_blocks = (tune.min_chunk_blocks + 1) / 2;  // (given in 128-row blocks)
   shape.target_items = idx->num_sms * tune.items_per_sm;
   DevPlanSizes z = device_plan_sizes(idx, nq, shape);
   const uint64_t per_item = (uint64_t)BQ * capb * sizeof(Candidate);
-  shape.max_items_per_tile = (uint32_t)std::max<uint64_t>(
-      1, std::min<uint64_t>(RR_CAP / capb, (8ull << 30) / (per_item * z.ntile_max)));
+  shape.max_items_per_tile = max_items(capb, tune.pilot_stride, per_item, z.ntile_max);
   // all buffers exist before the capture (a capture may not allocate)
   QueryDesc *d_desc;
   void *d_plan;
   unsigned char *d_at;
   float2 *d_lqs;
-  Candidate *d_out;
-  uint32_t *d_ocnt, *d_state, *d_pilot = nullptr;
+  Candidate *d_out, *d_work;
+  uint32_t *d_ocnt, *d_state;
   if ((rc = ws_get(idx, 2, (size_t)nq * sizeof(QueryDesc), (void **)&d_desc))) return rc;
   if ((rc = ws_get(idx, 19, device_plan_bytes(nq, z), &d_plan))) return rc;
-  if ((rc = ws_get(idx, 4, (size_t)z.ntile_max * TB, (void **)&d_at))) return rc;
+  if ((rc = ws_get(idx, 4, (size_t)z.ntile_max * 2 * TA, (void **)&d_at))) return rc;
   if ((rc = ws_get(idx, 10, (size_t)z.ntile_max * BQ * sizeof(float2), (void **)&d_lqs))) return rc;
   if ((rc = ws_get(idx, 6, (size_t)z.nitems_max * per_item, (void **)&d_out))) return rc;
+  const unsigned sgrid = std::min<uint32_t>(z.nitems_max, (uint32_t)idx->num_sms);
+  if ((rc = ws_get(idx, 11, (size_t)sgrid * 2 * B_LISTS * capb * sizeof(Candidate), (void **)&d_work))) return rc;
   if ((rc = ws_get(idx, 7, (size_t)z.nitems_max * BQ * 4, (void **)&d_ocnt))) return rc;
-  if ((rc = ws_get(idx, 5, (size_t)nq * 16 + 64, (void **)&d_state))) return rc;
+  if ((rc = ws_get(idx, 5, TcState::bytes(nq), (void **)&d_state))) return rc;
+  const TcState S(d_state, nq);
   const uint32_t stride = tune.pilot_stride;
-  if (stride > 1 && (rc = ws_get(idx, 11, (size_t)nq * 12, (void **)&d_pilot))) return rc;
   {  // the radix sort's histogram slot at its largest (the plan sorts nq keys)
     void *h;
     const size_t keys = std::max<size_t>(nq, z.nitems_max);  // ... and the work items
@@ -1090,8 +1433,7 @@ static int search_tc_graph(fknn_index *idx, const float *d_q, const float *d_met
   }
   DevPlan P;
   device_plan_layout(P, d_plan, nq, z);
-  auto screen = capb <= 512 ? k_screen_tc<F, 16> : capb <= 768 ? k_screen_tc<F, 24>
-              : capb <= 1024 ? k_screen_tc<F, 32> : k_screen_tc<F, 40>;
+  auto screen = screen_kernel<F>(capb);
   FKNN_CUDA(cudaFuncSetAttribute(screen, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BScreenSmem<F>)));
   FKNN_CUDA(cudaFuncSetAttribute(k_merge_rerank<RR_CAP_SMALL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)sizeof(RerankSmem<RR_CAP_SMALL>)));
@@ -1105,7 +1447,8 @@ static int search_tc_graph(fknn_index *idx, const float *d_q, const float *d_met
       tune.bound_refresh, tune.pilot_stride, (uint64_t)withhold, (uint64_t)(uintptr_t)d_q, (uint64_t)(uintptr_t)d_meta,
       (uint64_t)(uintptr_t)d_ids, (uint64_t)(uintptr_t)d_dists, (uint64_t)(uintptr_t)d_desc,
       (uint64_t)(uintptr_t)d_plan, (uint64_t)(uintptr_t)d_at, (uint64_t)(uintptr_t)d_lqs, (uint64_t)(uintptr_t)d_out,
-      (uint64_t)(uintptr_t)d_ocnt, (uint64_t)(uintptr_t)d_state, (uint64_t)(uintptr_t)d_pilot,
+      (uint64_t)(uintptr_t)d_work,
+      (uint64_t)(uintptr_t)d_ocnt, (uint64_t)(uintptr_t)d_state,
       (uint64_t)(uintptr_t)idx->ws[15].p};
   if (!G.exec || G.key != key) {
     G.release();
@@ -1132,11 +1475,7 @@ static int search_tc_graph(fknn_index *idx, const float *d_q, const float *d_met
                                  G.side)))
         return r;
       FKNN_CUDA(cudaEventRecord(G.join, G.side));
-      uint32_t *T_global = d_state, *ovf = d_state + nq, *ovf_list = d_state + 2 * (size_t)nq,
-               *ovf_count = d_state + 3 * (size_t)nq, *n_f64 = ovf_count + 1, *spill_count = ovf_count + 2;
-      if ((r = launch_fill_u32(T_global, nq, f32_sortable(INFINITY), st))) return r;
-      FKNN_CUDA(cudaMemsetAsync(ovf, 0, (size_t)nq * 4, st));
-      FKNN_CUDA(cudaMemsetAsync(ovf_count, 0, 12, st));
+      if ((r = S.reset(nq, st))) return r;
       const OrderData &OT = idx->ord[ORDER_TIME], &OC = idx->ord[ORDER_CAT];
       LaneSrc ls;
       ls.tile_first = P.tile_first;
@@ -1152,28 +1491,32 @@ static int search_tc_graph(fknn_index *idx, const float *d_q, const float *d_met
       g_launches += 1;
       FKNN_CUDA(cudaEventRecordWithFlags(G.ev[0], st, cudaEventRecordExternal));  // an event node of the graph
       void *const *blocks = F::kFP8 ? idx->fp8_blocks : idx->bf16_blocks;
-      const unsigned sgrid = std::min<uint32_t>(z.nitems_max, (uint32_t)idx->num_sms * 2);
-      uint32_t *seeded = nullptr;
-      if (stride > 1) {
-        const uint32_t rr = std::min<uint32_t>(kprime, (3 * kprime + stride - 1) / stride + 8);
-        uint32_t *T_A = d_pilot, *ovf_A = d_pilot + 2 * (size_t)nq;
-        seeded = d_pilot + nq;
-        FKNN_CUDA(cudaMemsetAsync(seeded, 0, (size_t)nq * 4, st));
-        if ((r = launch_fill_u32(T_A, nq, f32_sortable(INFINITY), st))) return r;
-        FKNN_CUDA(cudaMemsetAsync(ovf_A, 0, (size_t)nq * 4, st));
-        screen<<<sgrid, B_THREADS, sizeof(BScreenSmem<F>), st>>>(
-            P.items, P.tiles, d_at, ls, d_lqs, (const unsigned char *)blocks[ORDER_TIME],
-            (const unsigned char *)blocks[ORDER_CAT], T_A, ovf_A, d_out, d_ocnt, rr, capb, 0, stride, 0u, 0,
-            P.cnt + DP_NITEMS, P.ord_val, P.queue, idx->d_flag);
-        k_seed_bounds<<<1184, 256, 0, st>>>(P.big_q, 0, P.cnt + DP_NBIG, d_desc, T_A, ovf_A, 16 * stride * BR,
-                                            T_global, seeded);
-        g_launches += 2;
-      }
-      screen<<<sgrid, B_THREADS, sizeof(BScreenSmem<F>), st>>>(
-          P.items, P.tiles, d_at, ls, d_lqs, (const unsigned char *)blocks[ORDER_TIME],
-          (const unsigned char *)blocks[ORDER_CAT], T_global, ovf, d_out, d_ocnt, kprime, capb, tune.bound_refresh, 1,
-          withhold ? 1u : 0u, 0, P.cnt + DP_NITEMS, P.ord_val, P.queue + 1, idx->d_flag);
-      g_launches += 1;
+      ScreenArgs X;
+      X.items = P.items;
+      X.tiles = P.tiles;
+      X.atiles = d_at;
+      X.ls = ls;
+      X.lane_qs = d_lqs;
+      X.blocks_t = (const unsigned char *)blocks[ORDER_TIME];
+      X.blocks_c = (const unsigned char *)blocks[ORDER_CAT];
+      X.out = d_out;
+      X.out_cnt = d_ocnt;
+      X.work = d_work;
+      X.capb = capb;
+        X.nitems = 0;
+      X.nitems_d = P.cnt + DP_NITEMS;
+      X.order = P.ord_val;
+      X.err = idx->d_flag;
+      SeedArgs Z;
+      Z.big_q = P.big_q;
+      Z.big_tile = P.big_tile;
+      Z.big_lane = P.big_lane;
+      Z.nbig = 0;
+      Z.nbig_d = P.cnt + DP_NBIG;
+      Z.item_slot = nullptr;  // a tile's items are consecutive
+      Z.desc = d_desc;
+      launch_screens(screen, X, Z, S, kprime, stride, tune.bound_refresh, withhold, sgrid, nq, sizeof(BScreenSmem<F>),
+                     st);
       FKNN_CUDA(cudaEventRecordWithFlags(G.ev[1], st, cudaEventRecordExternal));  // an event node of the graph
       MergeArgs A;
       A.big_q = P.big_q;
@@ -1188,26 +1531,24 @@ static int search_tc_graph(fknn_index *idx, const float *d_q, const float *d_met
       A.vecs = idx->vecs;
       A.perm_t = OT.perm;
       A.perm_c = OC.perm;
-      A.ovf = ovf;
-      A.ovf_list = ovf_list;
-      A.ovf_count = ovf_count;
+      A.ovf = S.ovf;
+      A.ovf_list = S.ovf_list;
+      A.ovf_count = S.ovf_count;
       A.k = k;
       A.kprime = kprime;
       A.capb = capb;
-      A.seeded = seeded;
+      A.seeded = stride > 1 ? S.seeded : nullptr;
       A.ids = d_ids;
       A.dists = d_dists;
-      A.n_f64 = n_f64;
+      A.n_f64 = S.n_f64;
       A.nbig_d = P.cnt + DP_NBIG;
-      uint32_t *spill = spill_count + 1;
-      k_merge_rerank<RR_CAP_SMALL><<<std::min<uint32_t>(nq, (uint32_t)idx->num_sms * 32), RR_THREADS,
-                                     sizeof(RerankSmem<RR_CAP_SMALL>), st>>>(A, 0, nullptr, nullptr, spill,
-                                                                             spill_count);
-      k_merge_rerank<RR_CAP><<<148 * 2, RR_THREADS, sizeof(RerankSmem<RR_CAP>), st>>>(A, 0, spill, spill_count,
+        k_merge_rerank<RR_CAP_SMALL><<<std::min<uint32_t>(nq, (uint32_t)idx->num_sms * 32), RR_THREADS,
+                                     sizeof(RerankSmem<RR_CAP_SMALL>), st>>>(A, 0, nullptr, nullptr, S.spill, S.spill_count);
+      k_merge_rerank<RR_CAP><<<148 * 2, RR_THREADS, sizeof(RerankSmem<RR_CAP>), st>>>(A, 0, S.spill, S.spill_count,
                                                                                        nullptr, nullptr);
       g_launches += 2;
       FKNN_CUDA(cudaEventRecordWithFlags(G.ev[2], st, cudaEventRecordExternal));  // an event node of the graph
-      if ((r = launch_exact_scan(idx, ovf_list, ovf_count, 0, 148 * 2, d_desc, d_q, k, d_ids, d_dists, st))) return r;
+      if ((r = launch_exact_scan(idx, S.ovf_list, S.ovf_count, 0, 148 * 2, d_desc, d_q, k, d_ids, d_dists, st))) return r;
       FKNN_CUDA(cudaStreamWaitEvent(st, G.join, 0));
       FKNN_CUDA(cudaEventRecordWithFlags(G.ev[3], st, cudaEventRecordExternal));  // an event node of the graph
       FKNN_CUDA(cudaGetLastError());
@@ -1251,7 +1592,7 @@ static int search_tc_graph(fknn_index *idx, const float *d_q, const float *d_met
     uint32_t c[16];
     FKNN_CUDA(cudaMemcpy(c, P.cnt, sizeof(c), cudaMemcpyDeviceToHost));
     uint32_t h2[2] = {0, 0};
-    FKNN_CUDA(cudaMemcpy(h2, d_state + 3 * (size_t)nq, 8, cudaMemcpyDeviceToHost));
+    FKNN_CUDA(cudaMemcpy(h2, S.ovf_count, 8, cudaMemcpyDeviceToHost));
     auto u64 = [&](int i) { return (uint64_t)c[i] | ((uint64_t)c[i + 1] << 32); };
     stats->pairs_screened = u64(10);
     stats->pairs_passing = u64(12);

@@ -72,6 +72,7 @@ __device__ __forceinline__ uint64_t global_ns() {
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity, int *err) {
   if (mbar_try_wait(bar, parity)) return true;
   uint64_t t0 = 0;
+#pragma unroll 1
   for (uint32_t it = 1; it < WAIT_LIMIT; ++it) {
     if (mbar_try_wait(bar, parity)) return true;
     if ((it & 63u) == 0u) {
@@ -243,6 +244,97 @@ __device__ __forceinline__ void list_offsets(const uint32_t *__restrict__ item_s
     carry += __shfl_sync(0xffffffffu, inc, 31);
   }
   if (lane == 0) *total = (int)carry;
+}
+
+// kth smallest (1-based, kth <= n) of key[0 .. n) in shared memory, as its
+// f32_sortable image: a radix select of the whole block that starts below
+// the bits all keys share.  red: 4 words of shared memory.
+template <int THREADS>
+__device__ uint32_t block_kth(const float *key, int n, uint32_t kth, uint32_t *hist, uint32_t *red) {
+  const int tid = threadIdx.x, lane = tid & 31;
+  if (tid == 0) {
+    red[0] = 0xffffffffu;
+    red[1] = 0;
+  }
+  __syncthreads();
+  uint32_t mn = 0xffffffffu, mx = 0;
+  for (int i = tid; i < n; i += THREADS) {
+    const uint32_t u = f32_sortable(key[i]);
+    mn = min(mn, u);
+    mx = max(mx, u);
+  }
+  mn = __reduce_min_sync(0xffffffffu, mn);
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  if (lane == 0) {
+    atomicMin(&red[0], mn);
+    atomicMax(&red[1], mx);
+  }
+  __syncthreads();
+  mn = red[0];
+  mx = red[1];
+  int hi = mn == mx ? 0 : 32 - __clz(mn ^ mx);
+  uint32_t mask = hi == 32 ? 0u : ~((1u << hi) - 1u);
+  uint32_t prefix = mn & mask, remaining = kth;
+  while (hi > 0) {
+    const int w = min(8, hi), shift = hi - w;
+    for (int i = tid; i < 256; i += THREADS) hist[i] = 0;
+    __syncthreads();
+    for (int i = tid; i < n; i += THREADS) {
+      const uint32_t u = f32_sortable(key[i]);
+      if ((u & mask) == prefix) atomicAdd(&hist[(u >> shift) & ((1u << w) - 1)], 1u);
+    }
+    __syncthreads();
+    if (tid < 32) {
+      uint32_t local[8], sum = 0;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        local[j] = hist[lane * 8 + j];
+        sum += local[j];
+      }
+      uint32_t inc = sum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += v;
+      }
+      uint32_t c = inc - sum;
+      if (c < remaining && inc >= remaining) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          if (c < remaining && c + local[j] >= remaining) {
+            red[2] = lane * 8 + j;
+            red[3] = c;
+          }
+          c += local[j];
+        }
+      }
+    }
+    __syncthreads();
+    prefix |= red[2] << shift;
+    remaining -= red[3];
+    mask |= ((1u << w) - 1) << shift;
+    hi = shift;
+  }
+  __syncthreads();
+  return prefix;
+}
+
+// seq_l2_strided over a 16-byte aligned row, four dimensions per load
+__device__ __forceinline__ float seq_l2_row(const float *__restrict__ x, const float *q) {
+  const float4 *x4 = reinterpret_cast<const float4 *>(x);
+  float r = 0.f;
+#pragma unroll 5
+  for (int d = 0; d < DIM / 4; ++d) {
+    const float4 v = __ldg(x4 + d);
+    const float e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      float t = __fsub_rn(e[j], q[4 * d + j]);
+      t = __fmul_rn(t, t);
+      r = __fadd_rn(r, t);
+    }
+  }
+  return r;
 }
 
 }  // namespace fknn

@@ -57,15 +57,7 @@ constexpr uint32_t X_REFRESH = 16;            // sub-tiles between reads of the 
 // F32 accumulate, FP16 A and B, K-major, N = XR, M = XM
 constexpr uint32_t X_IDESC = (1u << 4) | ((uint32_t)(XR >> 3) << 17) | ((uint32_t)(XM >> 4) << 24);
 
-// one epilogue warp's scratch: staged candidate chunks, or the histogram of a trim
-struct XWarp {
-  union {
-    float row[X_SLOTS][STAGE_ROW];
-    uint32_t hist[256];
-  };
-  float4 q[32];
-  int info[X_SLOTS];  // first column | lane
-};
+using XWarp = ScreenWarp<X_SLOTS>;
 
 struct XSmem {
   unsigned char b[X_ST][2][X_PIECE];  // split row sub-tiles
@@ -95,12 +87,6 @@ __device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64
       "r"(tmem_a), "l"(db), "r"(X_IDESC), "r"(accumulate));
 }
 
-__device__ __forceinline__ void tmem_st8(uint32_t addr, const uint32_t (&r)[8]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(addr), "r"(r[0]),
-               "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-               : "memory");
-}
-
 // Exponent of the scale of a vector with squared norm n2: |x_i| 2^e < 2^14
 // (1 + 1e-5).  Any float n2 >= 0, a zero or subnormal one included.
 __device__ __forceinline__ int scale_exp(float n2) {
@@ -124,72 +110,6 @@ __device__ __forceinline__ void split2(float a, float b, uint32_t &h, uint32_t &
 __device__ __forceinline__ int fold_exp(const XSmem &sm, uint32_t par) {
   const int lo = sm.hmin[par], hi = sm.hmax[par];
   return lo <= hi && hi - lo <= X_FOLD_SPAN ? lo + 1 : X_NO_FOLD;
-}
-
-// An upper bound on the kth smallest (1-based, kth <= n) of the n keys held
-// NPL per lane (element j * 32 + lane in key[j]), at most `slack` keys above
-// it: a warp radix select from the highest differing bit that stops as soon
-// as the digit it is in ends near enough (one pass of three, as a rule).
-template <int NPL>
-__device__ __forceinline__ uint32_t warp_kth_upper(const uint32_t (&key)[NPL], int n, int kth, int slack,
-                                                   uint32_t *hist) {
-  const int lane = threadIdx.x & 31;
-  uint32_t mn = 0xffffffffu, mx = 0u;
-#pragma unroll
-  for (int j = 0; j < NPL; ++j)
-    if (j * 32 + lane < n) {
-      mn = min(mn, key[j]);
-      mx = max(mx, key[j]);
-    }
-  mn = __reduce_min_sync(0xffffffffu, mn);
-  mx = __reduce_max_sync(0xffffffffu, mx);
-  int hi = mn == mx ? 0 : 32 - __clz(mn ^ mx);  // bits [hi-1, 0] still differ
-  uint32_t mask = hi == 32 ? 0u : ~((1u << hi) - 1u);
-  uint32_t prefix = mn & mask;
-  int below = 0;  // keys smaller than the prefix's range
-  while (hi > 0) {
-    const int w = min(8, hi), shift = hi - w;
-    for (int i = lane; i < 256; i += 32) hist[i] = 0;
-    __syncwarp();
-#pragma unroll
-    for (int j = 0; j < NPL; ++j)
-      if (j * 32 + lane < n && (key[j] & mask) == prefix) atomicAdd(&hist[(key[j] >> shift) & ((1u << w) - 1)], 1u);
-    __syncwarp();
-    const uint4 a = reinterpret_cast<const uint4 *>(hist)[lane * 2], b = reinterpret_cast<const uint4 *>(hist)[lane * 2 + 1];
-    const uint32_t local[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-    int sum = 0;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) sum += (int)local[j];
-    int inc = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, inc, o);
-      if (lane >= o) inc += v;
-    }
-    const int want = kth - below;
-    int c = inc - sum, bin = -1, upto = 0;
-    if (c < want && inc >= want) {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        if (bin < 0 && c + (int)local[j] >= want) {
-          bin = lane * 8 + j;
-          upto = c;  // keys before the bin
-        }
-        if (bin < 0) c += (int)local[j];
-      }
-      upto = upto << 16 | (int)local[bin & 7];
-    }
-    const int owner = __ffs(__ballot_sync(0xffffffffu, bin >= 0)) - 1;
-    bin = __shfl_sync(0xffffffffu, bin, owner);
-    upto = __shfl_sync(0xffffffffu, upto, owner);
-    __syncwarp();
-    prefix |= (uint32_t)bin << shift;
-    mask |= ((1u << w) - 1) << shift;
-    hi = shift;
-    if (below + (upto >> 16) + (upto & 0xffff) <= kth + slack) break;
-    below += upto >> 16;
-  }
-  return prefix | ~mask;
 }
 
 // The entries of up to two lists (32 NPL entries at most, n in all, element i
@@ -365,70 +285,6 @@ __device__ __forceinline__ void x_values(uint32_t (&r)[32], const XSmem &sm, uin
     r[4 * j + 2] = __float_as_uint(fmaf(__uint_as_float(r[4 * j + 2]) * s.z, iq, v.z));
     r[4 * j + 3] = __float_as_uint(fmaf(__uint_as_float(r[4 * j + 3]) * s.w, iq, v.w));
   }
-}
-
-// Candidates: the lanes (queries) whose 32-column chunk holds some stage its
-// values in slots of their warp (x_stage); once the accumulator is released
-// the warp takes a slot at a time, a column per lane, and appends the passing
-// ones with one ballot (x_flush).  Each lane walking its own registers instead
-// diverges, and measured slower.  Both are out of line and reload the chunk:
-// they run for a few chunks of a sub-tile at most, and a copy per chunk pushes
-// the other roles' code out of the instruction caches.
-//   pass: column in [r0, r1) and v >= bound;  ds = qn + f2 v
-struct XQuery {
-  float bound, f2, qn;
-  int range;  // r0 << 16 | r1
-};
-__device__ __noinline__ int x_flush(XWarp &w, int ns, uint32_t p0, Candidate *lists, int cnt) {
-  const int lane = threadIdx.x & 31;
-  const uint32_t lt = (1u << lane) - 1u;
-  __syncwarp();
-#pragma unroll 1
-  for (int i = 0; i < ns; ++i) {
-    const int inf = w.info[i], src = inf & 31, c = (inf & ~31) + lane;
-    const float v = w.row[i][lane];
-    const float4 t = w.q[src];
-    const int n = __shfl_sync(0xffffffffu, cnt, src), rg = __float_as_int(t.w);
-    const bool pass = v >= t.x && c >= (rg >> 16) && c < (rg & 0xffff);
-    const uint32_t m = __ballot_sync(0xffffffffu, pass);
-    if (pass) {
-      Candidate cd;
-      cd.ds = fmaf(t.y, v, t.z);
-      cd.pos = p0 + c;
-      lists[src * X_LIST + n + __popc(m & lt)] = cd;
-    }
-    if (lane == src) cnt += __popc(m);
-  }
-  __syncwarp();  // the slots are free again, the list entries visible to the warp
-  return cnt;
-}
-// chunk of columns c .. c + 31, lanes fm; returns cnt << 8 | the slots in use
-// (cnt changes when the slots run out)
-__device__ __noinline__ int x_stage(uint32_t taddr, int c, uint32_t fm, XQuery q, uint32_t p0, XWarp &w, int ns,
-                                    Candidate *lists, int cnt) {
-  const int lane = threadIdx.x & 31;
-  uint32_t r[32];
-  tmem_ld32_issue(taddr + c, r);
-  w.q[lane] = make_float4(q.bound, q.f2, q.qn, __int_as_float(q.range));
-  tmem_wait_ld(r);
-  while (fm) {  // warp-uniform
-    if (ns == X_SLOTS) {
-      cnt = x_flush(w, ns, p0, lists, cnt);
-      ns = 0;
-    }
-    const int at = ns + __popc(fm & ((1u << lane) - 1u));
-    const bool mine = ((fm >> lane) & 1u) && at < X_SLOTS;
-    if (mine) {
-#pragma unroll
-      for (int j = 0; j < 32; j += 4)
-        *reinterpret_cast<uint4 *>(&w.row[at][j]) = make_uint4(r[j], r[j + 1], r[j + 2], r[j + 3]);
-      w.info[at] = c | lane;
-    }
-    const uint32_t took = __ballot_sync(0xffffffffu, mine);
-    ns += __popc(took);
-    fm &= ~took;
-  }
-  return cnt << 8 | ns;
 }
 
 // A sub-tile in which some norms are not in the accumulator (rows whose
@@ -693,7 +549,7 @@ __global__ void __launch_bounds__(X_THREADS, 1) k_exact_screen(ExactScreenArgs A
           const float4 cr4 = *reinterpret_cast<const float4 *>(sm.crs[slot]);
           if (cr4.x > 0.f && cr4.x == cr4.y && cr4.x == cr4.z && cr4.x == cr4.w) {  // (block-uniform)
             // the rows' scale 2^ex = 1 / cr: v >= cq iff acc >= cs 2^ex (-inf would admit masked columns)
-            XQuery q;
+            ScreenQuery q;
             q.bound = r0 < r1 ? fmaxf(cs * pow2f(127 - (int)(__float_as_uint(cr4.x) >> 23)), -FLT_MAX) : INFINITY;
             q.f2 = -2.f * (cr4.x * iq);
             q.qn = qd;
@@ -716,7 +572,7 @@ __global__ void __launch_bounds__(X_THREADS, 1) k_exact_screen(ExactScreenArgs A
               for (int c = 0; c < XR / 32; ++c) {
                 const uint32_t fm = __ballot_sync(0xffffffffu, (hits >> c) & 1u);
                 if (fm) {
-                  const int cn = x_stage(tb, 32 * c, fm, q, p0, wsm, ns, lists, cnt);
+                  const int cn = x_stage(tb, 32 * c, fm, q, p0, wsm, ns, lists, X_LIST, cnt);
                   ns = cn & 0xff;
                   cnt = cn >> 8;
                 }
@@ -725,7 +581,7 @@ __global__ void __launch_bounds__(X_THREADS, 1) k_exact_screen(ExactScreenArgs A
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive1(&sm.accempty[grp]);
-            if (ns) cnt = x_flush(wsm, ns, p0, lists, cnt);
+            if (ns) cnt = x_flush(wsm, ns, p0, lists, X_LIST, cnt);
           } else {
             tmem_wait_ld(ra);
 #pragma unroll 1
@@ -805,126 +661,6 @@ __global__ void __launch_bounds__(X_THREADS, 1) k_exact_screen(ExactScreenArgs A
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(X_TMEM_COLS));
 }
 
-// Bounds from the pilot pass: the r-th smallest screening distance over the
-// union of a query's pilot lists (a sample of its rows), widened by screen_hi:
-// an estimate from above of the k-th of all its rows, which the merge checks.
-// r follows from the share of the query's own slab that was sampled.  NT
-// threads per query.
-template <int NT>
-__global__ void __launch_bounds__(256)
-    k_exact_seed(const uint32_t *__restrict__ big_q, const uint32_t *__restrict__ big_tile,
-                 const uint32_t *__restrict__ big_lane, uint32_t nbig, const Tile *__restrict__ tiles,
-                 const uint32_t *__restrict__ item_slot, const Candidate *__restrict__ out,
-                 const uint32_t *__restrict__ out_cnt, const QueryDesc *__restrict__ desc, const WorkItem *__restrict__ items, uint32_t stride,
-                 uint32_t k, uint32_t *__restrict__ T_global) {
-  __shared__ uint32_t hist[256 / NT][256];
-  __shared__ uint32_t red[256 / NT][4];  // total, min, max of the keys; digit found
-  const int grp = threadIdx.x / NT, t = threadIdx.x % NT, lane = threadIdx.x & 31;
-  const uint32_t b = blockIdx.x * (256 / NT) + grp;
-  const bool on = b < nbig;
-  auto sync = [&]() {
-    if (NT == 32) __syncwarp();
-    else __syncthreads();
-  };
-  if (NT == 32 && !on) return;  // (NT == 256: the grid is nbig blocks, every group is on)
-  const uint32_t qi = big_q[b], L = big_lane[b];
-  const Tile tl = tiles[big_tile[b]];
-  uint32_t *h = hist[grp], *rd = red[grp];
-  // the sampled rows of the query's slab, and the rank of the seed among them
-  const QueryDesc dq = desc[qi];
-  uint32_t rows = 0;
-  for (uint32_t i = tl.item0; i < tl.item1; ++i) {
-    const WorkItem it = items[item_slot[i]];
-    for (uint64_t p = it.blk0 + (uint64_t)t * stride; p < it.blk1; p += (uint64_t)NT * stride) {
-      const uint64_t lo = max((uint64_t)dq.s, p * XR), hi = min((uint64_t)dq.e, (p + 1) * XR);
-      if (hi > lo) rows += (uint32_t)(hi - lo);
-    }
-  }
-  // every list of the query, NT entries at a time
-  auto each = [&](auto &&f) {
-    for (uint32_t i = tl.item0; i < tl.item1; ++i) {
-      const uint64_t item = item_slot[i];
-      const uint32_t c = out_cnt[item * XQ + L];
-      const Candidate *src = out + (item * XQ + L) * EXACT_CAP;
-      for (uint32_t j = t; j < c; j += NT) f(f32_sortable(src[j].ds));
-    }
-  };
-  if (t == 0) {
-    rd[0] = 0;
-    rd[1] = 0xffffffffu;
-    rd[2] = 0;
-    rd[3] = 0;
-  }
-  sync();
-  uint32_t n = 0, mn = 0xffffffffu, mx = 0;
-  each([&](uint32_t u) {
-    ++n;
-    mn = min(mn, u);
-    mx = max(mx, u);
-  });
-  n = __reduce_add_sync(0xffffffffu, n);
-  mn = __reduce_min_sync(0xffffffffu, mn);
-  mx = __reduce_max_sync(0xffffffffu, mx);
-  rows = __reduce_add_sync(0xffffffffu, rows);
-  if (lane == 0) {
-    atomicAdd(&rd[3], rows);
-    atomicAdd(&rd[0], n);
-    atomicMin(&rd[1], mn);
-    atomicMax(&rd[2], mx);
-  }
-  sync();
-  n = rd[0];
-  mn = rd[1];
-  mx = rd[2];
-  const uint32_t r = exact_seed_rank(k, rd[3], dq.e - dq.s);
-  if (n < r) return;  // group-uniform
-  // radix select from the highest bit in which the keys differ
-  int hi = mn == mx ? 0 : 32 - __clz(mn ^ mx);
-  uint32_t mask = hi == 32 ? 0u : ~((1u << hi) - 1u);
-  uint32_t prefix = mn & mask, remaining = r;
-  while (hi > 0) {
-    const int w = min(8, hi), shift = hi - w;
-    for (int i = t; i < 256; i += NT) h[i] = 0;
-    sync();
-    each([&](uint32_t u) {
-      if ((u & mask) == prefix) atomicAdd(&h[(u >> shift) & ((1u << w) - 1)], 1u);
-    });
-    sync();
-    if (t < 32) {
-      uint32_t local[8], sum = 0;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        local[j] = h[lane * 8 + j];
-        sum += local[j];
-      }
-      uint32_t inc = sum;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += v;
-      }
-      uint32_t c = inc - sum;
-      if (c < remaining && inc >= remaining) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          if (c < remaining && c + local[j] >= remaining) {
-            rd[2] = lane * 8 + j;
-            rd[3] = c;
-          }
-          c += local[j];
-        }
-      }
-    }
-    sync();
-    prefix |= rd[2] << shift;
-    remaining -= rd[3];
-    mask |= ((1u << w) - 1) << shift;
-    hi = shift;
-    sync();
-  }
-  if (t == 0) T_global[qi] = f32_sortable(screen_hi(sortable_f32(prefix), dq.qn));
-}
-
 }  // namespace
 
 size_t exact_work_bytes(uint32_t grid) { return (size_t)grid * XQ * X_LIST * sizeof(Candidate); }
@@ -938,18 +674,35 @@ int launch_exact_screen(const ExactScreenArgs &A, uint32_t grid, cudaStream_t st
   return FKNN_OK;
 }
 
+namespace {
+struct ExactSeedBound {
+  __device__ float operator()(float ds, const QueryDesc &dq) const { return screen_hi(ds, dq.qn); }
+};
+}  // namespace
+
 int launch_exact_seed(const uint32_t *big_q, const uint32_t *big_tile, const uint32_t *big_lane, uint32_t nbig,
                       const ExactScreenArgs &A, const uint32_t *item_slot, uint32_t k, uint32_t *T_global,
                       cudaStream_t st) {
-  // a warp per query where there are enough queries to fill the GPU that
-  // way (their lists are then few), else a block per query
-  if (nbig >= 4096)
-    k_exact_seed<32><<<(nbig + 7) / 8, 256, 0, st>>>(big_q, big_tile, big_lane, nbig, A.tiles, item_slot, A.out,
-                                                     A.out_cnt, A.desc, A.items, A.stride, k, T_global);
-  else
-    k_exact_seed<256><<<nbig, 256, 0, st>>>(big_q, big_tile, big_lane, nbig, A.tiles, item_slot, A.out, A.out_cnt,
-                                            A.desc, A.items, A.stride, k, T_global);
-  g_launches += 1;
+  SeedArgs S;
+  S.big_q = big_q;
+  S.big_tile = big_tile;
+  S.big_lane = big_lane;
+  S.nbig = nbig;
+  S.nbig_d = nullptr;
+  S.tiles = A.tiles;
+  S.items = A.items;
+  S.item_slot = item_slot;
+  S.out = A.out;
+  S.out_cnt = A.out_cnt;
+  S.tq = XQ;
+  S.list_cap = EXACT_CAP;
+  S.blk_rows = XR;
+  S.desc = A.desc;
+  S.stride = A.stride;
+  S.k = k;
+  S.T_global = T_global;
+  S.seeded = nullptr;
+  launch_screen_seed(S, nbig, ExactSeedBound(), st);
   FKNN_CUDA(cudaGetLastError());
   return FKNN_OK;
 }

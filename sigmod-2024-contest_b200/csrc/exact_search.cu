@@ -179,96 +179,6 @@ struct ExactMergeArgs {
   float *dists;
 };
 
-// kth smallest (1-based, kth <= n) of key[0 .. n) in shared memory, as its
-// f32_sortable image: a radix select of the whole block that starts below
-// the bits all keys share.  red: 4 words of shared memory.
-__device__ uint32_t block_kth(const float *key, int n, uint32_t kth, uint32_t *hist, uint32_t *red) {
-  const int tid = threadIdx.x, lane = tid & 31;
-  if (tid == 0) {
-    red[0] = 0xffffffffu;
-    red[1] = 0;
-  }
-  __syncthreads();
-  uint32_t mn = 0xffffffffu, mx = 0;
-  for (int i = tid; i < n; i += MG_THREADS) {
-    const uint32_t u = f32_sortable(key[i]);
-    mn = min(mn, u);
-    mx = max(mx, u);
-  }
-  mn = __reduce_min_sync(0xffffffffu, mn);
-  mx = __reduce_max_sync(0xffffffffu, mx);
-  if (lane == 0) {
-    atomicMin(&red[0], mn);
-    atomicMax(&red[1], mx);
-  }
-  __syncthreads();
-  mn = red[0];
-  mx = red[1];
-  int hi = mn == mx ? 0 : 32 - __clz(mn ^ mx);
-  uint32_t mask = hi == 32 ? 0u : ~((1u << hi) - 1u);
-  uint32_t prefix = mn & mask, remaining = kth;
-  while (hi > 0) {
-    const int w = min(8, hi), shift = hi - w;
-    for (int i = tid; i < 256; i += MG_THREADS) hist[i] = 0;
-    __syncthreads();
-    for (int i = tid; i < n; i += MG_THREADS) {
-      const uint32_t u = f32_sortable(key[i]);
-      if ((u & mask) == prefix) atomicAdd(&hist[(u >> shift) & ((1u << w) - 1)], 1u);
-    }
-    __syncthreads();
-    if (tid < 32) {
-      uint32_t local[8], sum = 0;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        local[j] = hist[lane * 8 + j];
-        sum += local[j];
-      }
-      uint32_t inc = sum;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += v;
-      }
-      uint32_t c = inc - sum;
-      if (c < remaining && inc >= remaining) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          if (c < remaining && c + local[j] >= remaining) {
-            red[2] = lane * 8 + j;
-            red[3] = c;
-          }
-          c += local[j];
-        }
-      }
-    }
-    __syncthreads();
-    prefix |= red[2] << shift;
-    remaining -= red[3];
-    mask |= ((1u << w) - 1) << shift;
-    hi = shift;
-  }
-  __syncthreads();
-  return prefix;
-}
-
-// seq_l2_strided over a 16-byte aligned row, four dimensions per load
-__device__ __forceinline__ float seq_l2_row(const float *__restrict__ x, const float *q) {
-  const float4 *x4 = reinterpret_cast<const float4 *>(x);
-  float r = 0.f;
-#pragma unroll 5
-  for (int d = 0; d < DIM / 4; ++d) {
-    const float4 v = __ldg(x4 + d);
-    const float e[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      float t = __fsub_rn(e[j], q[4 * d + j]);
-      t = __fmul_rn(t, t);
-      r = __fadd_rn(r, t);
-    }
-  }
-  return r;
-}
-
 // One big query b (index into the plan's big-query arrays): gather its
 // lists, bound the k-th distance over their union, re-score the survivors
 // with the reference's arithmetic, order them by (dist, id).  A query with
@@ -290,7 +200,7 @@ __device__ void exact_merge_one(const ExactMergeArgs &A, uint32_t b, MergeSmem<M
   const QueryDesc dsc = A.desc[qi];
   const float qn = dsc.qn;
   for (int d = tid; d < DIM; d += MG_THREADS) sm.qv[d] = A.q[(uint64_t)qi * DIM + d];
-  // 1. gather the lists: item offsets, then the whole block copies each list
+  // 1. gather the lists: item offsets, then a warp copies a list at a time
   list_offsets(A.item_slot, tl.item0, nitems, A.out_cnt, L, EXACT_TQ, sm.cnt_prefix, &sm.total, MAX_ITEMS_PER_TILE,
                MERGE_CAP + 1);
   if (tid == 0) sm.surv = 0;
@@ -303,12 +213,12 @@ __device__ void exact_merge_one(const ExactMergeArgs &A, uint32_t b, MergeSmem<M
     }
     return;
   }
-  for (uint32_t i = 0; i < nitems; ++i) {
+  for (uint32_t i = tid / 32; i < nitems; i += MG_THREADS / 32) {
     const uint64_t item = A.item_slot[tl.item0 + i];
     const uint32_t base = sm.cnt_prefix[i];
     const uint32_t c = (i + 1 < nitems ? sm.cnt_prefix[i + 1] : (uint32_t)M) - base;
     const Candidate *src = A.out + (item * EXACT_TQ + L) * EXACT_CAP;
-    for (uint32_t j = tid; j < c; j += MG_THREADS) {
+    for (uint32_t j = tid & 31; j < c; j += 32) {
       const Candidate cd = src[j];
       sm.key[base + j] = cd.ds;
       sm.val[base + j] = cd.pos;
@@ -321,7 +231,7 @@ __device__ void exact_merge_one(const ExactMergeArgs &A, uint32_t b, MergeSmem<M
   float T = Tg;
   bool proven = false;
   if (M >= (int)k) {
-    const float h = screen_hi(sortable_f32(block_kth(sm.key, M, k, sm.hist, sm.red)), qn);
+    const float h = screen_hi(sortable_f32(block_kth<MG_THREADS>(sm.key, M, k, sm.hist, sm.red)), qn);
     proven = h <= Tg + 5e-7f * fabsf(Tg);  // (screen_hi's own slack of 1e-6 covers the tolerance)
     T = fminf(T, h);
   }

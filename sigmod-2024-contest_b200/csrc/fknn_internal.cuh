@@ -275,7 +275,7 @@ struct fknn_index {
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   fknn::Plan plan;  // rebuilt by every search; capacity kept
   // per-mode plan / kernel parameters (fknn_index_set_tuning) and the SM count
-  fknn_tuning tuning[3] = {{0, 4, 16, 0, 32}, {256, 3, 8, 0, 16}, {256, 3, 8, 0, 16}};
+  fknn_tuning tuning[3] = {{0, 4, 16, 0, 32}, {256, 3, 8, 0, 8}, {256, 3, 8, 0, 8}};
   int num_sms = 148;
   uint32_t n_labels = 1;  // distinct category values (bounds a device plan's segments)
   // a view shares the device data of another index and owns only its
@@ -362,11 +362,13 @@ struct ExactScreenArgs {
 size_t exact_work_bytes(uint32_t grid);
 int launch_exact_screen(const ExactScreenArgs &A, uint32_t grid, cudaStream_t st);
 // Rank, in a sample of `rows` rows of a slab of n, of the bound that seeds a
-// search of the slab's k nearest: about k rows / n of them are in the sample,
-// and 3 times that + 8 lies above all but 1e-8 of the (Poisson) cases.
+// search of the slab's k nearest: about m = k rows / n of them are in the
+// sample, and the smaller of 3 m + 8 and m + 6.2 sqrt(m) + 5 lies above all but
+// 1e-8 of the (Poisson) cases.
 __host__ __device__ __forceinline__ uint32_t exact_seed_rank(uint32_t k, uint32_t rows, uint32_t n) {
-  const uint32_t r = (uint32_t)((3ull * k * rows + n - 1) / (n ? n : 1)) + 8;
-  return r < k ? r : k;
+  const float m = (float)k * ((float)rows / (float)(n ? n : 1));
+  const float r = fminf(3.f * m + 8.f, m + 6.2f * sqrtf(m) + 5.f);
+  return r < (float)k ? (uint32_t)r + 1 : k;
 }
 // T_global of the nbig queries set from their pilot lists (those that have enough entries)
 int launch_exact_seed(const uint32_t *big_q, const uint32_t *big_tile, const uint32_t *big_lane, uint32_t nbig,

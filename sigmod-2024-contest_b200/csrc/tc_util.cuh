@@ -85,6 +85,13 @@ __device__ __forceinline__ void tmem_wait_ld(uint32_t (&r)[32]) {
                : "memory");
 }
 
+// 8 columns of this warp's 32 TMEM lanes
+__device__ __forceinline__ void tmem_st8(uint32_t addr, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(addr), "r"(r[0]),
+               "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
+
 // max of three floats in one instruction (NaN operands ignored)
 __device__ __forceinline__ float fmax3(float a, float b, float c) {
   float r;
