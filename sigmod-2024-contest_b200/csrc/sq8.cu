@@ -50,30 +50,38 @@ struct HeapNode {
 };
 
 // ------------------------------------------------------------------------
-// The slab brute force as three steps per batch of queries:
+// The slab brute force per batch of queries, over parts of the slab that grow
+// by SQ_GROW:
 //
-//  1. k_sq8_prefix (one warp per query): the first SQ_PREFIX codes replayed
-//     exactly -- emplace of the first k, then must_pop_emplace -- with a
-//     warp-wide filter in front of the serial heap steps.  The heap root
-//     afterwards, T_q, bounds every later root (the root only falls), so a
-//     later code can enter only if its distance is below T_q.
+//  1. k_sq8_dist and k_sq8_prefix (one warp per query): the distances of the
+//     first SQ_PREFIX codes, then their replay -- emplace of the first k, then
+//     must_pop_emplace -- with a warp-wide filter in front of the heap steps.
+//     The heap root afterwards, T_q, bounds every later root (the root only
+//     falls), so a later code can enter only if its distance is below T_q.
 //  2. k_sq8_screen (tcgen05, kind::i8): the int32 inner products of a tile of
-//     128 queries with the code tiles of one slab segment, exact in the
+//     128 queries with the code tiles of one segment of the part, exact in the
 //     accumulator; an epilogue thread per query writes every code of the
 //     segment with d = |q|^2 + |c|^2 - 2 q.c < T_q, in slab order, to the
 //     query's list for that segment.  A list that fills up marks the query.
-//  3. k_sq8_tail (one warp per query): the heap from step 1, the segment lists
-//     in order through the same filter and serial steps, the heap array out.
-//     A marked query scans the codes itself instead, with the step-1 code.
+//  3. k_sq8_tail (one warp per query): the heap so far, the segment lists in
+//     order through the same filter and heap steps; then the next part with a
+//     lower T_q, or the heap array out.  A marked query scans the part's codes
+//     itself instead.
 //
 // Every distance is the exact int32 L2SqrSQ8_sym value and every code that
-// can enter the heap reaches the serial steps in slab order, so the heap
-// array is the reference's.
+// can enter the heap reaches the heap steps in slab order, so the heap array
+// is the reference's.
+//
+// About k (SQ_GROW - 1) codes of a part are below its T_q: 1,800 in all for
+// k = 140 and 450,000 codes, where one part after the prefix had 7,700.
 constexpr uint32_t SQ_PREFIX = 8192;    // codes replayed before the screen (multiple of 128)
+constexpr uint64_t SQ_GROW = 8;         // a part ends at this multiple of its first code
+constexpr int SQ_DQ = 32;               // queries of a block of k_sq8_dist
 constexpr int SQ_WARPS = 4;             // queries per block of the replay kernels
 constexpr int SQ_SCAN = 128;            // codes per warp step of the replay kernels
 constexpr uint32_t SQ_TILE = TC_ROWS * 128;  // 128 rows x 128 bytes (112 code bytes, 16 zero)
 constexpr int SQ_BS = 4;                // shared-memory stages of code tiles
+constexpr int SQ_NB = 2 * SQ_BS;        // ... of their norms, which the epilogue reads up to two tiles later
 constexpr int SQ_EPI_WARPS = 4;
 constexpr int SQ_THREADS = (2 + SQ_EPI_WARPS) * 32;  // producer, MMA issuer, epilogue
 constexpr uint32_t SQ_TMEM_COLS = 2 * TC_ROWS;       // double-buffered accumulator
@@ -118,49 +126,139 @@ __device__ __forceinline__ void heap_emplace(HeapNode *h, int now, HeapNode nd) 
   h[now] = nd;
 }
 
-// must_pop_emplace (bruteforce.h:99-105) behind the root test
-// bruteforce.h:258-260 makes; push_down (bruteforce.h:78-87) reads both
-// children of a level with one 16-byte load (h is 16-byte aligned and the
-// pair h[2x], h[2x+1] lies inside the heap's region even when 2x = cnt).
-__device__ __forceinline__ void heap_offer(HeapNode *h, int cnt, HeapNode nd) {
-  if (h[1].d <= nd.d) return;
-  int x = 1;
-  while ((x << 1) <= cnt) {
-    const int t0 = x << 1;
-    const int4 pr = *reinterpret_cast<const int4 *>(h + t0);
-    const bool r = t0 < cnt && pr.z > pr.x;
-    HeapNode c;
-    c.d = r ? pr.z : pr.x;
-    c.id = r ? pr.w : pr.y;
-    if (c.d <= nd.d) break;
-    h[x] = c;
-    x = t0 + (r ? 1 : 0);
-  }
-  h[x] = nd;
+// The way down from the root always takes the larger child (push_down,
+// bruteforce.h:78-87) and does not depend on the new node, only its end does.
+// So next[x] keeps every node's larger child (low half) and that child's (high
+// half; 0: none), as byte offsets into next: the warp follows two levels per
+// load, without a branch, and lane l then moves level l's node.
+struct WarpHeap {
+  HeapNode *h;      // 1-based, cnt nodes
+  uint32_t *next;   // 0 .. cnt (next[0]: none)
+  HeapNode *stage;
+  int cnt, root;    // root: h[1].d
+  int steps;        // loads from the root to any leaf's level
+};
+
+// shared memory of one warp's heap, in nodes: the heap (k + 1 nodes), next, the stage
+__host__ __device__ __forceinline__ uint32_t sq_heap_nodes(uint32_t k) { return (k + 2u) & ~1u; }
+__host__ __device__ __forceinline__ uint32_t sq_next_nodes(uint32_t k) { return (k + 2u) / 2u; }
+__host__ __device__ __forceinline__ uint32_t sq_region(uint32_t k) {
+  return (sq_heap_nodes(k) + sq_next_nodes(k) + SQ_SCAN + 1u) & ~1u;
 }
 
-// nodes of one warp's shared-memory region: the heap (1-based, k + 1 nodes,
-// rounded up to an even count past k + 1 for the pair loads), then the stage
-__host__ __device__ __forceinline__ uint32_t sq_region(uint32_t k) { return ((k + 2u + 1u) & ~1u) + SQ_SCAN; }
+__device__ __forceinline__ WarpHeap warp_heap(unsigned char *smem, int warp, uint32_t k) {
+  WarpHeap w;
+  w.h = reinterpret_cast<HeapNode *>(smem) + (size_t)warp * sq_region(k);
+  w.next = reinterpret_cast<uint32_t *>(w.h + sq_heap_nodes(k));
+  w.stage = w.h + sq_heap_nodes(k) + sq_next_nodes(k);
+  w.cnt = (int)k;
+  w.steps = (32 - __clz(k)) / 2;  // levels 0 .. floor(log2(k))
+  return w;
+}
 
-// list[0..n) (shared memory) offered in order by lane 0
-__device__ __forceinline__ void offer_list(HeapNode *h, int cnt, const HeapNode *list, int n, int lane) {
-  if (lane == 0)
-    for (int j = 0; j < n; ++j) heap_offer(h, cnt, list[j]);
+// next and root of a full heap; the whole warp
+__device__ __forceinline__ void heap_ready(WarpHeap &w, int lane) {
+  __syncwarp();
+  for (int x = lane; x <= w.cnt; x += 32) {
+    const int c = 2 * x;
+    const bool r = x && c < w.cnt && w.h[c + 1].d > w.h[c].d;
+    w.next[x] = x && c <= w.cnt ? 4 * (c + (r ? 1 : 0)) : 0;
+  }
+  __syncwarp();
+  for (int x = lane; x <= w.cnt; x += 32) {  // (the low halves stay as they are)
+    const uint32_t c = w.next[x] & 0xffffu;
+    w.next[x] = c | (w.next[c / 4] & 0xffffu) << 16;
+  }
+  w.root = w.h[1].d;
   __syncwarp();
 }
 
-// Codes [p0, p1) of the slab through one query's heap, in order: positions
-// below k are emplaced, the rest offered.  The warp scores SQ_SCAN codes per
-// step; lane 0 runs the heap steps for the ones that can enter: all of a step
-// that starts before the heap holds k nodes, else those below the root at the
-// start of the step (the root only falls).  cc[p] = |c_p|^2 = -ncc[p].
-__device__ void scan_codes(HeapNode *heap, HeapNode *stage, const int4 (&qv)[7], int qq,
-                           const int8_t *__restrict__ codes, const int *__restrict__ ncc, uint64_t p0, uint64_t p1,
-                           uint32_t k, int lane) {
+// must_pop_emplace (bruteforce.h:99-105) behind the root test
+// bruteforce.h:258-260 makes, by the whole warp.  (Lane 0 alone, a level at a
+// time with its branch and store, took 1,080 cycles a node at k = 140.)
+__device__ __forceinline__ void heap_offer(WarpHeap &w, HeapNode nd, int lane) {
+  if (w.root <= nd.d) return;
+  const char *const nb = reinterpret_cast<const char *>(w.next);
+  // lane l: the node of level l and the one below (offsets; 0 past the leaf)
+  uint32_t x = 4, px = lane == 0 ? 4u : 0u, nx = 0;
+#pragma unroll 1
+  for (int i = 0; i < 2 * w.steps; i += 2) {
+    const uint32_t j = *reinterpret_cast<const uint32_t *>(nb + x), j0 = j & 0xffffu;
+    x = j >> 16;
+    if (lane == i) nx = j0;
+    if (lane == i + 1) px = j0, nx = x;
+    if (lane == i + 2) px = x;
+  }
+  // its larger child, and the other one, if there is one, with that one's larger child
+  HeapNode c;
+  c.d = INT_MIN;
+  c.id = 0;
+  int sd = INT_MIN;
+  uint32_t sn = 0;
+  const uint32_t sx = nx ^ 4u;
+  if (nx) {
+    c = *reinterpret_cast<const HeapNode *>(reinterpret_cast<const char *>(w.h) + 2 * nx);
+    if (sx <= 4u * w.cnt) {
+      sd = *reinterpret_cast<const int *>(reinterpret_cast<const char *>(w.h) + 2 * sx);
+      sn = *reinterpret_cast<const uint32_t *>(nb + sx) & 0xffffu;
+    }
+  }
+  const int cd1 = __shfl_down_sync(0xffffffffu, c.d, 1);
+  // the new node's level: the first whose larger child is not larger, or the leaf's
+  const int t = __ffs(__ballot_sync(0xffffffffu, px && c.d <= nd.d)) - 1;
+  w.root = __shfl_sync(0xffffffffu, t == 0 ? nd.d : c.d, 0);
+  // lanes < t: their larger child now (of two equal ones the left)
+  const int below = lane + 1 < t ? cd1 : nd.d;
+  uint32_t big = nx;
+  if (lane < t && ((nx & 4u) ? below <= sd : sd > below)) big = sx;
+  const uint32_t big1 = __shfl_down_sync(0xffffffffu, big, 1);
+  if (lane <= t) {
+    HeapNode v = nd;
+    if (lane < t) {
+      v = c;
+      *reinterpret_cast<uint32_t *>(reinterpret_cast<char *>(w.next) + px) = big | (big == nx ? big1 : sn) << 16;
+    }
+    *reinterpret_cast<HeapNode *>(reinterpret_cast<char *>(w.h) + 2 * px) = v;
+  }
+  __syncwarp();
+}
+
+// A step of at most SQ_SCAN nodes, (d[i], id[i]) in lane order for i = 0 ..,
+// those at the largest distance absent: the ones that can enter are staged in
+// order and offered.
+__device__ __forceinline__ void offer_step(WarpHeap &w, const int (&d)[SQ_SCAN / 32], const int (&id)[SQ_SCAN / 32],
+                                           int lane) {
   const uint32_t below = (1u << lane) - 1u;
+  int off = 0;
+#pragma unroll
+  for (int i = 0; i < SQ_SCAN / 32; ++i) {
+    const uint32_t m = __ballot_sync(0xffffffffu, d[i] < w.root);
+    if ((m >> lane) & 1u) {
+      HeapNode nd;
+      nd.d = d[i];
+      nd.id = id[i];
+      w.stage[off + __popc(m & below)] = nd;
+    }
+    off += __popc(m);
+  }
+  if (off == 0) return;
+  __syncwarp();
+  HeapNode nd = w.stage[0];
+#pragma unroll 1
+  for (int j = 1; j <= off; ++j) {
+    const HeapNode nn = w.stage[min(j, off - 1)];
+    heap_offer(w, nd, lane);
+    nd = nn;
+  }
+  __syncwarp();
+}
+
+// Codes [p0, p1) of the slab (heap full) through one query's heap, in order;
+// the warp scores SQ_SCAN codes per step.  |c_p|^2 = -ncc[p].
+__device__ __forceinline__ void scan_codes(WarpHeap &w, const int4 (&qv)[7], int qq, const int8_t *__restrict__ codes,
+                                           const int *__restrict__ ncc, uint64_t p0, uint64_t p1, int lane) {
   for (uint64_t base = p0; base < p1; base += SQ_SCAN) {
-    int d[SQ_SCAN / 32];
+    int d[SQ_SCAN / 32], id[SQ_SCAN / 32];
     int4 c[SQ_SCAN / 32][7];
 #pragma unroll
     for (int i = 0; i < SQ_SCAN / 32; ++i) load_code(codes, base + 32 * i + lane, p1, c[i]);
@@ -168,34 +266,9 @@ __device__ void scan_codes(HeapNode *heap, HeapNode *stage, const int4 (&qv)[7],
     for (int i = 0; i < SQ_SCAN / 32; ++i) {
       const uint64_t p = base + 32 * i + lane;
       d[i] = p < p1 ? qq - ncc[p] - 2 * dot112(c[i], qv) : INT_MAX;
+      id[i] = (int)p;
     }
-    const bool full = base >= k;  // the heap holds k nodes from here on
-    const int root = heap[1].d;
-    int off = 0;
-#pragma unroll
-    for (int i = 0; i < SQ_SCAN / 32; ++i) {
-      const uint64_t p = base + 32 * i + lane;
-      const uint32_t m = __ballot_sync(0xffffffffu, p < p1 && (!full || d[i] < root));
-      if ((m >> lane) & 1u) {
-        HeapNode nd;
-        nd.d = d[i];
-        nd.id = (int)p;
-        stage[off + __popc(m & below)] = nd;
-      }
-      off += __popc(m);
-    }
-    __syncwarp();
-    if (full) {
-      offer_list(heap, (int)k, stage, off, lane);
-    } else {
-      if (lane == 0)
-        for (int j = 0; j < off; ++j) {
-          const HeapNode nd = stage[j];
-          if ((uint32_t)nd.id < k) heap_emplace(heap, nd.id + 1, nd);
-          else heap_offer(heap, (int)k, nd);
-        }
-      __syncwarp();
-    }
+    offer_step(w, d, id, lane);
   }
 }
 
@@ -269,27 +342,82 @@ __global__ void __launch_bounds__(256) k_sq8_tiles(const int8_t *__restrict__ ro
   }
 }
 
+// Distances of the first n codes (rows of stride n padded to SQ_SCAN in dist):
+// a thread per code, SQ_DQ queries of a block from shared memory.
+__global__ void __launch_bounds__(SQ_SCAN)
+    k_sq8_dist(const int8_t *__restrict__ codes, const int *__restrict__ ncc, uint64_t n, uint64_t stride,
+               const int8_t *__restrict__ queries, uint32_t nq, int *__restrict__ dist) {
+  __shared__ int4 qs[SQ_DQ][7];
+  const uint32_t q0 = blockIdx.y * SQ_DQ, m = min((uint32_t)SQ_DQ, nq - q0);
+  for (uint32_t i = threadIdx.x; i < m * 7; i += SQ_SCAN)
+    qs[i / 7][i % 7] = __ldg(reinterpret_cast<const int4 *>(queries + (uint64_t)q0 * SQ8_CODE) + i);
+  const uint64_t p = (uint64_t)blockIdx.x * SQ_SCAN + threadIdx.x;
+  int4 c[7];
+  load_code(codes, p, n, c);
+  const int cc = p < n ? -ncc[p] : 0;
+  __syncthreads();
+  for (uint32_t j = 0; j < m; ++j) {
+    int4 qv[7];
+#pragma unroll
+    for (int w = 0; w < 7; ++w) qv[w] = qs[j][w];
+    dist[(uint64_t)(q0 + j) * stride + p] = p < n ? dot112(qv, qv) + cc - 2 * dot112(c, qv) : INT_MAX;
+  }
+}
+
 // Step 1.  With final set (the whole slab is the prefix) it writes the
-// answer; else the heap and its root T_q.
+// answer; else the heap and its root T_q.  dist: the prefix's distances.
 __global__ void __launch_bounds__(SQ_WARPS * 32, 4)
-    k_sq8_prefix(const int8_t *__restrict__ codes, const int *__restrict__ ncc, uint64_t prefix,
-                 const int8_t *__restrict__ queries, uint32_t nq, uint32_t k, int final, HeapNode *__restrict__ heaps,
-                 int *__restrict__ T, int *__restrict__ closest, float *__restrict__ dists, float alpha) {
+    k_sq8_prefix(const int *__restrict__ dist, uint64_t prefix, uint64_t stride, uint32_t nq, uint32_t k, int final,
+                 HeapNode *__restrict__ heaps, int *__restrict__ T, int *__restrict__ closest,
+                 float *__restrict__ dists, float alpha) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t q = blockIdx.x * SQ_WARPS + warp;
   if (q >= nq) return;  // warp-uniform; the kernel has no block barrier
-  HeapNode *heap = reinterpret_cast<HeapNode *>(smem_raw) + (size_t)warp * sq_region(k);
-  HeapNode *stage = heap + (sq_region(k) - SQ_SCAN);
-  int4 qv[7];
-  int qq;
-  load_query(queries, q, qv, qq);
-  scan_codes(heap, stage, qv, qq, codes, ncc, 0, prefix, k, lane);
+  WarpHeap w = warp_heap(smem_raw, warp, k);
+  const int *row = dist + (uint64_t)q * stride;
+  // emplace of the first k
+  for (uint64_t base = 0; base < k; base += SQ_SCAN) {
+    const int n = (int)min((uint64_t)SQ_SCAN, k - base);
+    for (int i = lane; i < n; i += 32) {
+      HeapNode nd;
+      nd.d = row[base + i];
+      nd.id = (int)(base + i);
+      w.stage[i] = nd;
+    }
+    __syncwarp();
+    if (lane == 0)
+      for (int j = 0; j < n; ++j) heap_emplace(w.h, (int)base + j + 1, w.stage[j]);
+    __syncwarp();
+  }
+  heap_ready(w, lane);
+  // the rest, a step's distances loaded while the one before is offered
+  const uint64_t b0 = k / SQ_SCAN * SQ_SCAN;
+  int nx[SQ_SCAN / 32];
+  auto fetch = [&](uint64_t base) {
+#pragma unroll
+    for (int i = 0; i < SQ_SCAN / 32; ++i) {
+      const uint64_t p = base + 32 * i + lane;
+      nx[i] = base < prefix && p >= k ? row[p] : INT_MAX;
+    }
+  };
+  fetch(b0);
+#pragma unroll 1
+  for (uint64_t base = b0; base < prefix; base += SQ_SCAN) {
+    int d[SQ_SCAN / 32], id[SQ_SCAN / 32];
+#pragma unroll
+    for (int i = 0; i < SQ_SCAN / 32; ++i) {
+      d[i] = nx[i];
+      id[i] = (int)(base + 32 * i + lane);
+    }
+    fetch(base + SQ_SCAN);
+    offer_step(w, d, id, lane);
+  }
   if (final) {
-    write_heap(heap, k, q, closest, dists, alpha, lane);
+    write_heap(w.h, k, q, closest, dists, alpha, lane);
   } else {
-    for (uint32_t l = lane; l <= k; l += 32) heaps[(uint64_t)q * (k + 1) + l] = heap[l];
-    if (lane == 0) T[q] = heap[1].d;
+    for (uint32_t l = lane; l <= k; l += 32) heaps[(uint64_t)q * (k + 1) + l] = w.h[l];
+    if (lane == 0) T[q] = w.root;
   }
 }
 
@@ -301,6 +429,7 @@ struct SqScreenSmem {
   // per epilogue lane, the 32 values y of a chunk that holds candidates
   // (rows padded to 36 ints: conflict-free 16-byte stores)
   int stage[SQ_EPI_WARPS][32 * SQ_STAGE_ROW];
+  int ncc[SQ_NB][TC_ROWS];  // -|c|^2 of the tiles' rows
   uint64_t full[SQ_BS], empty[SQ_BS], accfull[2], accempty[2], abar;
   uint32_t tmem_base;
 };
@@ -314,7 +443,7 @@ __device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t da, uint64_t d
 }
 
 // Step 2.  Block (query tile, segment); the segment is code tiles
-// [seg * tps, min(nct, (seg + 1) * tps)) of the screened part, whose tile t
+// [seg * tps, min(nct, (seg + 1) * tps)) of the part, whose tile t
 // holds slab rows row0 + 128 t ...  The list of query q for segment seg is
 // cand[(q * nseg + seg) * cap ...], its length counts[q * nseg + seg].
 __global__ void __launch_bounds__(SQ_THREADS, 2)
@@ -360,8 +489,11 @@ __global__ void __launch_bounds__(SQ_THREADS, 2)
       for (uint32_t sub = 0; sub < ntile; ++sub) {
         const int st = sub % SQ_BS;
         if (sub >= SQ_BS && !mbar_wait_bounded(&sm.empty[st], ((sub / SQ_BS) - 1) & 1, err)) break;
-        mbar_arrive_expect_tx(&sm.full[st], SQ_TILE);
+        mbar_arrive_expect_tx(&sm.full[st], SQ_TILE + TC_ROWS * 4);
         bulk_g2s(sm.b[st], ctiles + (uint64_t)(t0 + sub) * SQ_TILE, SQ_TILE, &sm.full[st]);
+        // (tile sub - SQ_NB's are done with: its accumulator was released
+        // before the MMAs of tile sub - SQ_BS were issued)
+        bulk_g2s(sm.ncc[sub % SQ_NB], cncc + (uint64_t)(t0 + sub) * TC_ROWS, TC_ROWS * 4, &sm.full[st]);
         ++issued;
       }
       // no copy may still be landing when the block exits
@@ -419,7 +551,7 @@ __global__ void __launch_bounds__(SQ_THREADS, 2)
       }
       tc_fence_after();
       const uint32_t tile = t0 + sub;
-      const int *nc = cncc + (uint64_t)tile * TC_ROWS;
+      const int *nc = sm.ncc[sub % SQ_NB];
       const int id0 = (int)(row0 + tile * TC_ROWS);
       const int ncols = (int)min((uint64_t)TC_ROWS, npoints - (uint64_t)id0);  // the slab's last tile is short
 #pragma unroll 1
@@ -446,7 +578,7 @@ __global__ void __launch_bounds__(SQ_THREADS, 2)
             do {
               const int j = __ffs(mask) - 1;
               mask &= mask - 1;
-              const int cc = -__ldg(nc + c2 + h + j);
+              const int cc = -nc[c2 + h + j];
               if (cnt < cap) list[cnt] = make_int2(qq + cc - 2 * (row[j] + sq_fold(cc)), id0 + c2 + h + j);
               ++cnt;
             } while (mask);
@@ -470,57 +602,77 @@ __global__ void __launch_bounds__(SQ_THREADS, 2)
   }
 }
 
-// Step 3.
+// Step 3, the part [r0, r1); last: the answer, else the heap and T_q go on.
+// The lists of 32 segments are read as one: a lane finds its entry's segment
+// among their running counts, and the next step's entries load while one is
+// offered.  (A segment at a time cost a query on its own, whose part has 592
+// of them, two memory latencies each.)
 __global__ void __launch_bounds__(SQ_WARPS * 32, 4)
-    k_sq8_tail(const int8_t *__restrict__ codes, const int *__restrict__ ncc, uint64_t prefix, uint64_t npoints,
-               const int8_t *__restrict__ queries, uint32_t nq, uint32_t k, const HeapNode *__restrict__ heaps,
-               const int2 *__restrict__ cand, uint32_t cap, const uint32_t *__restrict__ counts, uint32_t nseg,
-               const uint32_t *__restrict__ mark, int *__restrict__ closest, float *__restrict__ dists, float alpha) {
+    k_sq8_tail(const int8_t *__restrict__ codes, const int *__restrict__ ncc, uint64_t r0, uint64_t r1, int last,
+               const int8_t *__restrict__ queries, uint32_t nq, uint32_t k, HeapNode *__restrict__ heaps,
+               int *__restrict__ T, const int2 *__restrict__ cand, uint32_t cap, const uint32_t *__restrict__ counts,
+               uint32_t nseg, const uint32_t *__restrict__ mark, int *__restrict__ closest, float *__restrict__ dists,
+               float alpha) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t q = blockIdx.x * SQ_WARPS + warp;
   if (q >= nq) return;  // warp-uniform; the kernel has no block barrier
-  HeapNode *heap = reinterpret_cast<HeapNode *>(smem_raw) + (size_t)warp * sq_region(k);
-  HeapNode *stage = heap + (sq_region(k) - SQ_SCAN);
-  for (uint32_t l = lane; l <= k; l += 32) heap[l] = heaps[(uint64_t)q * (k + 1) + l];
-  __syncwarp();
+  WarpHeap w = warp_heap(smem_raw, warp, k);
+  for (uint32_t l = lane; l <= k; l += 32) w.h[l] = heaps[(uint64_t)q * (k + 1) + l];
+  heap_ready(w, lane);
   if (mark[q]) {
     int4 qv[7];
     int qq;
     load_query(queries, q, qv, qq);
-    scan_codes(heap, stage, qv, qq, codes, ncc, prefix, npoints, k, lane);
+    scan_codes(w, qv, qq, codes, ncc, r0, r1, lane);
   } else {
-    const uint32_t below = (1u << lane) - 1u;
-    for (uint32_t s = 0; s < nseg; ++s) {
-      const uint32_t cnt = counts[(uint64_t)q * nseg + s];
-      const int2 *list = cand + ((uint64_t)q * nseg + s) * cap;
-      for (uint32_t j0 = 0; j0 < cnt; j0 += SQ_SCAN) {
-        int2 cd[SQ_SCAN / 32];
+    const uint32_t *cn = counts + (uint64_t)q * nseg;
+    uint32_t c = lane < nseg ? cn[lane] : 0u;
+#pragma unroll 1
+    for (uint32_t s0 = 0; s0 < nseg; s0 += 32) {
+      uint32_t inc = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += v;
+      }
+      const uint32_t total = __shfl_sync(0xffffffffu, inc, 31), first = inc - c;
+      c = s0 + 32 + lane < nseg ? cn[s0 + 32 + lane] : 0u;
+      const int2 *lists = cand + ((uint64_t)q * nseg + s0) * cap;
+      int2 nx[SQ_SCAN / 32];
+      auto fetch = [&](uint32_t j0) {
 #pragma unroll
         for (int i = 0; i < SQ_SCAN / 32; ++i) {
           const uint32_t j = j0 + 32 * i + lane;
-          cd[i] = j < cnt ? list[j] : make_int2(INT_MAX, 0);
+          int seg = 0;  // the lists that end at or before j
+#pragma unroll
+          for (int o = 16; o; o >>= 1)
+            if (__shfl_sync(0xffffffffu, inc, seg + o - 1) <= j) seg += o;
+          const uint32_t f = __shfl_sync(0xffffffffu, first, seg & 31);
+          nx[i] = j < total ? lists[(uint64_t)seg * cap + (j - f)] : make_int2(INT_MAX, 0);
         }
-        const int root = heap[1].d;
-        int off = 0;
+      };
+      if (total) fetch(0);
+#pragma unroll 1
+      for (uint32_t j0 = 0; j0 < total; j0 += SQ_SCAN) {
+        int d[SQ_SCAN / 32], id[SQ_SCAN / 32];
 #pragma unroll
         for (int i = 0; i < SQ_SCAN / 32; ++i) {
-          const uint32_t m = __ballot_sync(0xffffffffu, cd[i].x < root);
-          if ((m >> lane) & 1u) {
-            HeapNode nd;
-            nd.d = cd[i].x;
-            nd.id = cd[i].y;
-            stage[off + __popc(m & below)] = nd;
-          }
-          off += __popc(m);
+          d[i] = nx[i].x;
+          id[i] = nx[i].y;
         }
-        __syncwarp();
-        offer_list(heap, (int)k, stage, off, lane);
+        if (j0 + SQ_SCAN < total) fetch(j0 + SQ_SCAN);
+        offer_step(w, d, id, lane);
       }
     }
   }
   __syncwarp();
-  write_heap(heap, k, q, closest, dists, alpha, lane);
+  if (last) {
+    write_heap(w.h, k, q, closest, dists, alpha, lane);
+  } else {
+    for (uint32_t l = lane; l <= k; l += 32) heaps[(uint64_t)q * (k + 1) + l] = w.h[l];
+    if (lane == 0) T[q] = w.root;
+  }
 }
 
 // Device memory of the current device (or managed memory).
@@ -645,28 +797,49 @@ Sq8Scratch &sq8_scratch() {
 
 size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
 
-// segments and list capacity for a pass of nqb queries over nct code tiles
-struct Sq8Pass {
-  uint32_t nqt, tps, nseg, cap;
-  size_t bytes;  // query tiles, norms, heaps, bounds, lists, counts, marks
+// Segments and list capacity of one part [r0, r1) for a pass of nqb queries.
+struct Sq8Part {
+  uint64_t r0, r1;
+  uint32_t nct, tps, nseg, cap;
 };
 
-Sq8Pass sq8_pass(uint32_t nqb, uint32_t nct, size_t k, int num_sms) {
+Sq8Part sq8_part(uint64_t r0, uint64_t npoints, uint32_t nqt, size_t k, int num_sms) {
+  Sq8Part p{};
+  p.r0 = r0;
+  p.r1 = std::min(npoints, r0 * SQ_GROW);
+  p.nct = (uint32_t)((p.r1 - p.r0 + TC_ROWS - 1) / TC_ROWS);
+  // about four screen CTAs per SM (two resident, two waves)
+  const uint32_t nseg = std::max(1u, std::min(p.nct, (uint32_t)((4u * num_sms + nqt - 1) / nqt)));
+  p.tps = (p.nct + nseg - 1) / nseg;
+  p.nseg = (p.nct + p.tps - 1) / p.tps;
+  // a code of the part is a candidate iff it is below the k-th smallest of
+  // the r0 before it: about k / r0 of them; the lists hold twice that, and a
+  // query whose list fills up takes the exact scan
+  const double expect = (double)p.tps * TC_ROWS * (double)k / (double)r0;
+  p.cap = (uint32_t)std::min<double>((double)p.tps * TC_ROWS, ((uint32_t)(2.0 * expect) + 64 + 31) & ~31u);
+  return p;
+}
+
+// Scratch of a pass of nqb queries: query tiles, norms, heaps, bounds, the
+// prefix's distances (over before the lists begin) or the lists, counts, marks.
+struct Sq8Pass {
+  uint32_t nqt;
+  size_t lists, counts, bytes;
+};
+
+Sq8Pass sq8_pass(uint32_t nqb, uint64_t npoints, uint64_t prefix, size_t k, int num_sms) {
   Sq8Pass p{};
   p.nqt = (nqb + TC_ROWS - 1) / TC_ROWS;
-  // about four screen CTAs per SM (two resident, two waves)
-  uint32_t nseg = std::max(1u, std::min(nct, (uint32_t)((4u * num_sms + p.nqt - 1) / p.nqt)));
-  p.tps = (nct + nseg - 1) / nseg;
-  p.nseg = (nct + p.tps - 1) / p.tps;
-  // a code of the screened part is a candidate iff it is below the k-th
-  // smallest of the prefix: about k / SQ_PREFIX of them; the lists hold twice
-  // that, and a query whose list fills up takes the exact scan
-  const double expect = (double)p.tps * TC_ROWS * (double)k / SQ_PREFIX;
-  p.cap = (uint32_t)std::min<double>((double)p.tps * TC_ROWS, ((uint32_t)(2.0 * expect) + 64 + 31) & ~31u);
+  p.lists = (size_t)nqb * ((prefix + SQ_SCAN - 1) / SQ_SCAN * SQ_SCAN) * 4;
+  for (uint64_t r0 = prefix; r0 < npoints;) {
+    const Sq8Part a = sq8_part(r0, npoints, p.nqt, k, num_sms);
+    p.lists = std::max(p.lists, (size_t)nqb * a.nseg * a.cap * sizeof(int2));
+    p.counts = std::max(p.counts, (size_t)nqb * a.nseg * 4);
+    r0 = a.r1;
+  }
   p.bytes = al256((size_t)p.nqt * SQ_TILE) + al256((size_t)p.nqt * TC_ROWS * 4) +
-            al256((size_t)nqb * (k + 1) * sizeof(HeapNode)) + al256((size_t)nqb * 4) +
-            al256((size_t)nqb * p.nseg * p.cap * sizeof(int2)) + al256((size_t)nqb * p.nseg * 4) +
-            al256((size_t)nqb * 4) + 256;
+            al256((size_t)nqb * (k + 1) * sizeof(HeapNode)) + al256((size_t)nqb * 4) + al256(p.lists) +
+            al256(p.counts) + al256((size_t)nqb * 4) + 256;
   return p;
 }
 
@@ -702,11 +875,10 @@ int sq8_bf_impl(size_t k, int *closest, float *dists, size_t npoints, const char
   const bool screened = npoints > SQ_PREFIX;
   const uint64_t prefix = screened ? SQ_PREFIX : npoints;
   const uint32_t nct_all = (uint32_t)((npoints + TC_ROWS - 1) / TC_ROWS);
-  const uint32_t nct = screened ? nct_all - SQ_PREFIX / TC_ROWS : 0;
   const uint32_t qbatch = std::min(nq, SQ_QBATCH);
   const uint32_t qlast = nq - (nq - 1) / qbatch * qbatch;
-  const Sq8Pass pa = sq8_pass(qbatch, std::max(nct, 1u), k, num_sms);
-  const Sq8Pass pb = sq8_pass(qlast, std::max(nct, 1u), k, num_sms);
+  const Sq8Pass pa = sq8_pass(qbatch, npoints, prefix, k, num_sms);
+  const Sq8Pass pb = sq8_pass(qlast, npoints, prefix, k, num_sms);
 
   // inputs already on the device (16-byte aligned) are used in place, the
   // rest staged through the scratch, as are outputs that live on the host
@@ -758,7 +930,7 @@ int sq8_bf_impl(size_t k, int *closest, float *dists, size_t npoints, const char
   g_launches += 2;
   for (uint32_t q0 = 0; q0 < nq; q0 += qbatch) {
     const uint32_t nqb = std::min(qbatch, nq - q0);
-    const Sq8Pass ps = sq8_pass(nqb, std::max(nct, 1u), k, num_sms);
+    const Sq8Pass ps = sq8_pass(nqb, npoints, prefix, k, num_sms);
     size_t off = 0;
     auto take = [&](size_t b) {
       unsigned char *p = pass_base + off;
@@ -769,25 +941,34 @@ int sq8_bf_impl(size_t k, int *closest, float *dists, size_t npoints, const char
     int *qncc = reinterpret_cast<int *>(take((size_t)ps.nqt * TC_ROWS * 4));
     HeapNode *heaps = reinterpret_cast<HeapNode *>(take((size_t)nqb * (k + 1) * sizeof(HeapNode)));
     int *T = reinterpret_cast<int *>(take((size_t)nqb * 4));
-    int2 *cand = reinterpret_cast<int2 *>(take((size_t)nqb * ps.nseg * ps.cap * sizeof(int2)));
-    uint32_t *counts = reinterpret_cast<uint32_t *>(take((size_t)nqb * ps.nseg * 4));
+    void *lists = take(ps.lists);
+    int2 *cand = static_cast<int2 *>(lists);
+    uint32_t *counts = reinterpret_cast<uint32_t *>(take(ps.counts));
     uint32_t *mark = reinterpret_cast<uint32_t *>(take((size_t)nqb * 4));
     const int8_t *qs = d_q + (uint64_t)q0 * SQ8_CODE;
     int *ids = d_ids + (uint64_t)q0 * k;
     float *dd = d_d ? d_d + (uint64_t)q0 * k : nullptr;
     const unsigned rblocks = (nqb + SQ_WARPS - 1) / SQ_WARPS;
-    k_sq8_prefix<<<rblocks, SQ_WARPS * 32, rsmem, st>>>(d_codes, cncc, prefix, qs, nqb, K, screened ? 0 : 1, heaps,
-                                                        T, ids, dd, alpha);
-    g_launches += 1;
+    const uint64_t steps = (prefix + SQ_SCAN - 1) / SQ_SCAN;
+    k_sq8_dist<<<dim3((unsigned)steps, (nqb + SQ_DQ - 1) / SQ_DQ), SQ_SCAN, 0, st>>>(
+        d_codes, cncc, prefix, steps * SQ_SCAN, qs, nqb, static_cast<int *>(lists));
+    k_sq8_prefix<<<rblocks, SQ_WARPS * 32, rsmem, st>>>(static_cast<int *>(lists), prefix, steps * SQ_SCAN, nqb, K,
+                                                        screened ? 0 : 1, heaps, T, ids, dd, alpha);
+    g_launches += 2;
     if (screened) {
-      FKNN_CUDA(cudaMemsetAsync(mark, 0, (size_t)nqb * 4, st));
       k_sq8_tiles<<<ps.nqt, 256, 0, st>>>(qs, nqb, 0, 1, qtiles, qncc);
-      k_sq8_screen<<<dim3(ps.nqt, ps.nseg), SQ_THREADS, sizeof(SqScreenSmem), st>>>(
-          qtiles, qncc, nqb, ctiles + (size_t)(SQ_PREFIX / TC_ROWS) * SQ_TILE, cncc + SQ_PREFIX, nct, ps.tps, ps.nseg,
-          SQ_PREFIX, npoints, T, cand, ps.cap, counts, mark, d_err);
-      k_sq8_tail<<<rblocks, SQ_WARPS * 32, rsmem, st>>>(d_codes, cncc, SQ_PREFIX, npoints, qs, nqb, K, heaps, cand,
-                                                        ps.cap, counts, ps.nseg, mark, ids, dd, alpha);
-      g_launches += 3;
+      g_launches += 1;
+    }
+    for (uint64_t r0 = prefix; r0 < npoints;) {
+      const Sq8Part a = sq8_part(r0, npoints, ps.nqt, k, num_sms);
+      FKNN_CUDA(cudaMemsetAsync(mark, 0, (size_t)nqb * 4, st));
+      k_sq8_screen<<<dim3(ps.nqt, a.nseg), SQ_THREADS, sizeof(SqScreenSmem), st>>>(
+          qtiles, qncc, nqb, ctiles + (size_t)(r0 / TC_ROWS) * SQ_TILE, cncc + r0, a.nct, a.tps, a.nseg, (uint32_t)r0,
+          a.r1, T, cand, a.cap, counts, mark, d_err);
+      k_sq8_tail<<<rblocks, SQ_WARPS * 32, rsmem, st>>>(d_codes, cncc, r0, a.r1, a.r1 == npoints, qs, nqb, K, heaps, T,
+                                                        cand, a.cap, counts, a.nseg, mark, ids, dd, alpha);
+      g_launches += 2;
+      r0 = a.r1;
     }
     FKNN_CUDA(cudaGetLastError());
   }
