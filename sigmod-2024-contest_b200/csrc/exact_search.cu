@@ -40,37 +40,6 @@ namespace {
 
 // ---------------------------------------------------------------- prep --
 
-__device__ __forceinline__ uint32_t lower_bound_i32(const int32_t *a, uint32_t lo, uint32_t hi, int32_t v) {
-  while (lo < hi) {
-    uint32_t m = lo + ((hi - lo) >> 1);
-    if (a[m] < v) lo = m + 1; else hi = m;
-  }
-  return lo;
-}
-__device__ __forceinline__ uint32_t upper_bound_i32(const int32_t *a, uint32_t lo, uint32_t hi, int32_t v) {
-  while (lo < hi) {
-    uint32_t m = lo + ((hi - lo) >> 1);
-    if (a[m] <= v) lo = m + 1; else hi = m;
-  }
-  return lo;
-}
-// first position with ts >= v
-__device__ __forceinline__ uint32_t lower_bound_f32(const float *a, uint32_t lo, uint32_t hi, float v) {
-  while (lo < hi) {
-    uint32_t m = lo + ((hi - lo) >> 1);
-    if (a[m] < v) lo = m + 1; else hi = m;
-  }
-  return lo;
-}
-// first position with ts > v
-__device__ __forceinline__ uint32_t upper_bound_f32(const float *a, uint32_t lo, uint32_t hi, float v) {
-  while (lo < hi) {
-    uint32_t m = lo + ((hi - lo) >> 1);
-    if (a[m] <= v) lo = m + 1; else hi = m;
-  }
-  return lo;
-}
-
 // Query checks: type in {0,1,2,3} (searcher.hpp:39-42 rejects the rest),
 // v inside int32 for types 1/3 (read as int32, utils.h:99), window bounds
 // not NaN for types 2/3, vector values finite and <= 1e15.
@@ -92,56 +61,82 @@ __global__ void k_validate_queries(const float *__restrict__ q, const float *__r
   if (bad) atomicOr(flag, bad);
 }
 
+// The first position in [lo, hi) that is not below (pred: monotone, true
+// first), by the whole warp: 32 probes a step, so a million positions take
+// four memory latencies where halving takes twenty.
+template <class Pred>
+__device__ __forceinline__ uint32_t warp_partition(uint32_t lo, uint32_t hi, Pred pred) {
+  const uint32_t lane = threadIdx.x & 31;
+  while (hi > lo) {
+    const uint32_t chunk = (hi - lo + 31) / 32;
+    const uint64_t p = (uint64_t)lo + (lane + 1ull) * chunk - 1;
+    const uint32_t c = __popc(__ballot_sync(0xffffffffu, p < hi && pred((uint32_t)p)));
+    const uint64_t end = (uint64_t)lo + (c + 1ull) * chunk - 1;
+    lo += c * chunk;  // the probe after is not below, or past the end
+    if (lo > hi) lo = hi;
+    hi = (uint32_t)min((uint64_t)hi, end);
+  }
+  return lo;
+}
+
 // Predicate -> slab.  type 0: all rows (time order); 1: label == v (category
 // order); 2: l <= ts <= r (time order); 3: both (category order, the window
-// inside the label's slab).  The semantics are utils.h:110-137's.
+// inside the label's slab).  The semantics are utils.h:110-137's.  Whole warp.
 __device__ __forceinline__ void resolve_slab(const float *m, uint32_t n, const float *ts_t, const int32_t *lab_c,
                                              const float *ts_c, int32_t &order, uint32_t &s, uint32_t &e) {
   const uint32_t type = (uint32_t)m[0];
+  auto window = [&](const float *ts, uint32_t lo, uint32_t hi) {
+    const float l = m[2], r = m[3];
+    s = warp_partition(lo, hi, [&](uint32_t p) { return ts[p] < l; });
+    e = warp_partition(lo, hi, [&](uint32_t p) { return ts[p] <= r; });
+  };
+  order = type == 0 || type == 2 ? ORDER_TIME : ORDER_CAT;
   if (type == 0) {
-    order = ORDER_TIME; s = 0; e = n;
+    s = 0;
+    e = n;
   } else if (type == 2) {
-    order = ORDER_TIME;
-    s = lower_bound_f32(ts_t, 0, n, m[2]);
-    e = upper_bound_f32(ts_t, 0, n, m[3]);
+    window(ts_t, 0, n);
   } else {
-    order = ORDER_CAT;
     const int32_t v = (int32_t)m[1];
-    s = lower_bound_i32(lab_c, 0, n, v);
-    e = upper_bound_i32(lab_c, s, n, v);
-    if (type == 3) {
-      uint32_t cs = s, ce = e;
-      s = lower_bound_f32(ts_c, cs, ce, m[2]);
-      e = upper_bound_f32(ts_c, cs, ce, m[3]);
-    }
+    s = warp_partition(0, n, [&](uint32_t p) { return lab_c[p] < v; });
+    e = warp_partition(s, n, [&](uint32_t p) { return lab_c[p] <= v; });
+    if (type == 3) window(ts_c, s, e);
   }
   if (e < s) e = s;
 }
 
+// A warp per query.  (50 queries over 1e6 rows: 54 us with a thread each.)
 __global__ void k_query_prep(const float *__restrict__ q, const float *__restrict__ meta, uint32_t nq, uint32_t n,
                              const float *__restrict__ ts_t, const int32_t *__restrict__ lab_c,
                              const float *__restrict__ ts_c, QueryDesc *__restrict__ desc) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) / 32, lane = threadIdx.x & 31;
   if (i >= nq) return;
+  const float *x = q + (uint64_t)i * DIM;
+  float v[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) v[j] = 32 * j + lane < DIM ? x[32 * j + lane] : 0.f;
   QueryDesc dsc;
   resolve_slab(meta + (uint64_t)i * 4, n, ts_t, lab_c, ts_c, dsc.order, dsc.s, dsc.e);
-  const float *v = q + (uint64_t)i * DIM;
+  // |q|^2 in dimension order (every lane the same chain)
   float s = 0.f;
-#pragma unroll 10
-  for (int d = 0; d < DIM; ++d) s = fmaf(v[d], v[d], s);
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) {
+    const float t = __shfl_sync(0xffffffffu, v[d / 32], d % 32);
+    s = fmaf(t, t, s);
+  }
   dsc.qn = s;
-  desc[i] = dsc;
+  if (lane == 0) desc[i] = dsc;
 }
 
 __global__ void k_count(const float *__restrict__ meta, uint32_t nq, uint32_t n, const float *__restrict__ ts_t,
                         const int32_t *__restrict__ lab_c, const float *__restrict__ ts_c,
                         uint32_t *__restrict__ counts) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) / 32;  // a warp per query
   if (i >= nq) return;
   int32_t o;
   uint32_t s, e;
   resolve_slab(meta + (uint64_t)i * 4, n, ts_t, lab_c, ts_c, o, s, e);
-  counts[i] = e - s;
+  if ((threadIdx.x & 31) == 0) counts[i] = e - s;
 }
 
 // --------------------------------------------------------------- merge --
@@ -296,8 +291,98 @@ __global__ void __launch_bounds__(MG_THREADS)
 
 // ----------------------------------------------------------- exact scan --
 
-constexpr int ES_THREADS = 256;
-constexpr int ES_CAP = 1024;
+// Bound by latency: a slab of 4,096 rows is 1.6 MB, and one block reads it.  So
+// a thread has 25 loads of a row in flight, eight rows cover the longest slab
+// that is planned for here, and its keys stay in shared memory until the k
+// smallest are selected (a radix select, then every survivor counts its place);
+// longer slabs (queries whose candidates overflowed) select whenever the buffer
+// fills.  16 queries over 1e6 rows, 3 of them here: 226 us before, with 256
+// threads, ten loads and sorts of 1,024 keys.
+constexpr int ES_THREADS = 512;
+constexpr int ES_CAP = 4096;   // keys in shared memory
+constexpr int ES_KEEP = 1024;  // largest k
+
+struct ScanSmem {
+  uint64_t buf[ES_CAP];
+  uint64_t sel[ES_KEEP];
+  float qv[DIM];
+  uint32_t hist[256];
+  unsigned long long mn, mx;
+  uint32_t bin, before, count;
+  int cnt, kept;
+  uint64_t thr;
+};
+
+// The k smallest of the cnt > k distinct keys in buf to sel, in no order.
+__device__ void scan_select(ScanSmem &sm, int cnt, uint32_t k) {
+  const int tid = threadIdx.x, lane = tid & 31;
+  if (tid == 0) {
+    sm.mn = ~0ull;
+    sm.mx = 0;
+    sm.kept = 0;
+  }
+  __syncthreads();
+  uint64_t mn = ~0ull, mx = 0;
+  for (int i = tid; i < cnt; i += ES_THREADS) {
+    mn = min(mn, sm.buf[i]);
+    mx = max(mx, sm.buf[i]);
+  }
+  atomicMin(&sm.mn, (unsigned long long)mn);
+  atomicMax(&sm.mx, (unsigned long long)mx);
+  __syncthreads();
+  // radix select from the highest bit in which the keys differ, until the
+  // digit it is in holds one key
+  int hi = 64 - __clzll((long long)(sm.mn ^ sm.mx));
+  uint64_t mask = hi == 64 ? 0ull : ~((1ull << hi) - 1ull), prefix = sm.mn & mask;
+  uint32_t want = k;
+  while (hi > 0) {
+    const int w = min(8, hi), shift = hi - w;
+    for (int i = tid; i < 256; i += ES_THREADS) sm.hist[i] = 0;
+    __syncthreads();
+    for (int i = tid; i < cnt; i += ES_THREADS) {
+      const uint64_t u = sm.buf[i];
+      if ((u & mask) == prefix) atomicAdd(&sm.hist[(u >> shift) & ((1u << w) - 1)], 1u);
+    }
+    __syncthreads();
+    if (tid < 32) {
+      uint32_t local[8], sum = 0;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        local[j] = sm.hist[lane * 8 + j];
+        sum += local[j];
+      }
+      uint32_t inc = sum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += v;
+      }
+      uint32_t c = inc - sum;
+      if (c < want && inc >= want) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          if (c < want && c + local[j] >= want) {
+            sm.bin = lane * 8 + j;
+            sm.before = c;
+            sm.count = local[j];
+          }
+          c += local[j];
+        }
+      }
+    }
+    __syncthreads();
+    prefix |= (uint64_t)sm.bin << shift;
+    mask |= ((1ull << w) - 1ull) << shift;
+    want -= sm.before;
+    hi = shift;
+    if (sm.count == 1) break;
+  }
+  for (int i = tid; i < cnt; i += ES_THREADS) {
+    const uint64_t u = sm.buf[i];
+    if ((u & mask) <= prefix) sm.sel[atomicAdd(&sm.kept, 1)] = u;
+  }
+  __syncthreads();
+}
 
 __global__ void __launch_bounds__(ES_THREADS)
     k_exact_scan(const uint32_t *__restrict__ list, const uint32_t *__restrict__ d_count, uint32_t h_count,
@@ -305,10 +390,7 @@ __global__ void __launch_bounds__(ES_THREADS)
                  const float *__restrict__ blocks_c, const uint32_t *__restrict__ perm_t,
                  const uint32_t *__restrict__ perm_c, uint32_t k, uint32_t *__restrict__ ids,
                  float *__restrict__ dists) {
-  __shared__ uint64_t buf[ES_CAP];
-  __shared__ float qv[DIM];
-  __shared__ int cnt;
-  __shared__ uint64_t thr;
+  __shared__ ScanSmem sm;
   const uint32_t count = d_count ? *d_count : h_count;
   const int tid = threadIdx.x;
   for (uint32_t li = blockIdx.x; li < count; li += gridDim.x) {
@@ -316,47 +398,70 @@ __global__ void __launch_bounds__(ES_THREADS)
     const QueryDesc dsc = desc[qi];
     const float *blocks = dsc.order == ORDER_TIME ? blocks_t : blocks_c;
     const uint32_t *perm = dsc.order == ORDER_TIME ? perm_t : perm_c;
-    for (int d = tid; d < DIM; d += ES_THREADS) qv[d] = q[(uint64_t)qi * DIM + d];
+    for (int d = tid; d < DIM; d += ES_THREADS) sm.qv[d] = q[(uint64_t)qi * DIM + d];
     if (tid == 0) {
-      cnt = 0;
-      thr = ~0ull;
+      sm.cnt = 0;
+      sm.thr = ~0ull;
     }
     __syncthreads();
     for (uint64_t base = dsc.s; base < dsc.e; base += ES_THREADS) {
       const uint64_t p = base + tid;
       if (p < dsc.e) {
         const float *x = blocks + (p / BLK) * BLK_FLOATS + (p % BLK);
-        const float d = seq_l2_strided(x, BLK, qv);
-        const uint64_t key = exact_key(d, perm[p]);
-        if (key < thr) buf[atomicAdd(&cnt, 1)] = key;
+        const uint32_t id = perm[p];
+        float r = 0.f;
+#pragma unroll 1
+        for (int d0 = 0; d0 < DIM; d0 += 25) {
+          float v[25];
+#pragma unroll
+          for (int d = 0; d < 25; ++d) v[d] = __ldg(x + (d0 + d) * BLK);
+#pragma unroll
+          for (int d = 0; d < 25; ++d) {  // seq_l2_strided's operations
+            float t = __fsub_rn(v[d], sm.qv[d0 + d]);
+            t = __fmul_rn(t, t);
+            r = __fadd_rn(r, t);
+          }
+        }
+        const uint64_t key = exact_key(r, id);
+        if (key < sm.thr) sm.buf[atomicAdd(&sm.cnt, 1)] = key;
       }
       __syncthreads();
-      if (cnt > ES_CAP - ES_THREADS) {
-        for (int i = cnt + tid; i < ES_CAP; i += ES_THREADS) buf[i] = ~0ull;
-        __syncthreads();
-        block_bitonic_sort(buf, ES_CAP);
-        if (tid == 0) {
-          cnt = (int)k;
-          thr = buf[k - 1];
+      if (sm.cnt > ES_CAP - ES_THREADS && base + ES_THREADS < dsc.e) {
+        scan_select(sm, sm.cnt, k);
+        uint64_t mx = 0;
+        for (uint32_t i = tid; i < k; i += ES_THREADS) {
+          sm.buf[i] = sm.sel[i];
+          mx = max(mx, sm.sel[i]);
         }
+        if (tid == 0) {
+          sm.cnt = (int)k;
+          sm.mx = 0;
+        }
+        __syncthreads();
+        atomicMax(&sm.mx, (unsigned long long)mx);
+        __syncthreads();
+        if (tid == 0) sm.thr = sm.mx;
         __syncthreads();
       }
     }
-    int c = cnt;
-    int np2 = 32;
-    while (np2 < c) np2 <<= 1;
-    for (int i = c + tid; i < np2; i += ES_THREADS) buf[i] = ~0ull;
-    __syncthreads();
-    block_bitonic_sort(buf, np2);
-    for (uint32_t j = tid; j < k; j += ES_THREADS) {
-      uint32_t id = 0xffffffffu;
-      float d = INFINITY;
-      if ((int)j < c) {
-        id = (uint32_t)buf[j];
-        d = sortable_f32((uint32_t)(buf[j] >> 32));
-      }
-      ids[(uint64_t)qi * k + j] = id;
-      if (dists) dists[(uint64_t)qi * k + j] = d;
+    int c = sm.cnt;
+    const uint64_t *keys = sm.buf;
+    if (c > (int)k) {
+      scan_select(sm, c, k);
+      keys = sm.sel;
+      c = (int)k;
+    }
+    // a key's place is the number of smaller ones (they are distinct)
+    for (int i = tid; i < c; i += ES_THREADS) {
+      const uint64_t e = keys[i];
+      uint32_t rank = 0;
+      for (int j = 0; j < c; ++j) rank += keys[j] < e ? 1u : 0u;
+      ids[(uint64_t)qi * k + rank] = (uint32_t)e;
+      if (dists) dists[(uint64_t)qi * k + rank] = sortable_f32((uint32_t)(e >> 32));
+    }
+    for (uint32_t j = (uint32_t)c + tid; j < k; j += ES_THREADS) {
+      ids[(uint64_t)qi * k + j] = 0xffffffffu;
+      if (dists) dists[(uint64_t)qi * k + j] = INFINITY;
     }
     __syncthreads();
   }
@@ -535,7 +640,7 @@ static int check_query_flag(int flag) {
 
 int count_matches(fknn_index *idx, const float *d_meta, uint32_t nq, uint32_t *d_counts, cudaStream_t st) {
   if (nq == 0) return FKNN_OK;
-  k_count<<<(nq + 255) / 256, 256, 0, st>>>(d_meta, nq, (uint32_t)idx->n, idx->ord[ORDER_TIME].ts,
+  k_count<<<(nq + 7) / 8, 256, 0, st>>>(d_meta, nq, (uint32_t)idx->n, idx->ord[ORDER_TIME].ts,
                                            idx->ord[ORDER_CAT].label, idx->ord[ORDER_CAT].ts, d_counts);
   g_launches += 1;
   FKNN_CUDA(cudaGetLastError());
@@ -778,7 +883,7 @@ int enqueue_query_prep(fknn_index *idx, const float *d_q, const float *d_meta, u
                        cudaStream_t st) {
   int rc;
   if ((rc = validate_queries(idx, d_q, d_meta, nq, st))) return rc;
-  k_query_prep<<<(nq + 255) / 256, 256, 0, st>>>(d_q, d_meta, nq, (uint32_t)idx->n, idx->ord[ORDER_TIME].ts,
+  k_query_prep<<<(nq + 7) / 8, 256, 0, st>>>(d_q, d_meta, nq, (uint32_t)idx->n, idx->ord[ORDER_TIME].ts,
                                                  idx->ord[ORDER_CAT].label, idx->ord[ORDER_CAT].ts, d_desc);
   g_launches += 1;
   FKNN_CUDA(cudaGetLastError());
@@ -794,7 +899,7 @@ int prepare_queries(fknn_index *idx, const float *d_q, const float *d_meta, uint
   QueryDesc *d_desc;
   if ((rc = ws_get(idx, 2, (size_t)nq * sizeof(QueryDesc), (void **)&d_desc))) return rc;
   if ((rc = validate_queries(idx, d_q, d_meta, nq, st))) return rc;
-  k_query_prep<<<(nq + 255) / 256, 256, 0, st>>>(d_q, d_meta, nq, (uint32_t)n, idx->ord[ORDER_TIME].ts,
+  k_query_prep<<<(nq + 7) / 8, 256, 0, st>>>(d_q, d_meta, nq, (uint32_t)n, idx->ord[ORDER_TIME].ts,
                                                  idx->ord[ORDER_CAT].label, idx->ord[ORDER_CAT].ts, d_desc);
   g_launches += 1;
   QueryDesc *h_desc;

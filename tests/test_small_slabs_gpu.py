@@ -1,0 +1,65 @@
+"""Queries answered row by row: slabs of a block's threads, its key buffer and
+the longest planned for here, one row more and less; floods of equal distances
+across the k-th place; and the search for a slab's ends (labels and times with
+many repeats, windows that miss, touch and cross).  Ids, distances and counts
+equal the oracle's."""
+import numpy as np
+import pytest
+
+import fknn
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [1, 2, 31, 32, 33, 99, 100, 101, 128, 129, 511, 512, 513, 1025, 3583, 3584, 3585, 4095, 4096, 4097]
+
+
+def dataset(seed, distinct):
+    """Category c holds SIZES[c] rows, each of `distinct` vectors many times."""
+    rng = np.random.default_rng(seed)
+    labels = np.repeat(np.arange(len(SIZES)), SIZES).astype(np.float32)
+    n = labels.shape[0]
+    vecs = rng.standard_normal((distinct, 100), dtype=np.float32)[rng.integers(0, distinct, n)]
+    perm = rng.permutation(n)
+    ts = np.round(rng.random(n) * 50).astype(np.float32) / 50  # 51 times
+    return vecs[perm], labels[perm], ts[perm], rng
+
+
+@pytest.mark.parametrize("distinct", [3, 40_000])
+@pytest.mark.parametrize("k", [1, 100, 128])
+def test_slabs_of_every_size(distinct, k):
+    vecs, labels, ts, rng = dataset(k, distinct)
+    c = len(SIZES)
+    q = rng.standard_normal((2 * c, 100), dtype=np.float32)
+    metas = np.zeros((2 * c, 4), np.float32)
+    metas[:, 0] = np.repeat([1, 3], c)
+    metas[:, 1] = np.tile(np.arange(c), 2)
+    metas[:, 2:] = [0.2, 0.8]
+    with fknn.Index(vecs, labels, ts) as idx:
+        ids, dists = idx.search(q, metas, k=k)
+        oids, odists = oracle.exact_knn(vecs, labels, ts, q, metas, k=k)
+        np.testing.assert_array_equal(ids, oids)
+        np.testing.assert_array_equal(dists, odists)
+
+
+def test_ends_of_a_slab():
+    vecs, labels, ts, rng = dataset(7, 40_000)
+    edges = np.array([-1, 0, 0.01, 0.02, 0.5, 0.51, 0.98, 1, 1.5, np.inf, -np.inf], np.float32)
+    metas = [[t, v, l, r] for t in (0, 1, 2, 3) for v in (-1, 0, 5, 19, 20, 7) for l in edges for r in edges]
+    metas = np.array(metas, np.float32)
+    with fknn.Index(vecs, labels, ts) as idx:
+        np.testing.assert_array_equal(idx.count_matches(metas), oracle.count_matches(labels, ts, metas))
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 1023, 1025, 33_000])
+def test_ends_in_tables_of_any_length(n):
+    rng = np.random.default_rng(n)
+    vecs = rng.standard_normal((n, 100), dtype=np.float32)
+    labels = rng.integers(0, 3, n).astype(np.float32)
+    ts = rng.random(n, dtype=np.float32)
+    metas = np.zeros((200, 4), np.float32)
+    metas[:, 0] = rng.integers(0, 4, 200)
+    metas[:, 1] = rng.integers(-1, 4, 200)
+    metas[:, 2:] = np.sort(ts[rng.integers(0, n, (200, 2))], axis=1)
+    with fknn.Index(vecs, labels, ts) as idx:
+        np.testing.assert_array_equal(idx.count_matches(metas), oracle.count_matches(labels, ts, metas))
