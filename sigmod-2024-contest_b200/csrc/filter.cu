@@ -6,8 +6,8 @@
 // One cooperative launch per group of up to FP_MAXP predicates reads the
 // columns once (k_filter_coop).  Every CTA owns a contiguous run of rows
 // per round:
-//   1. it streams its labels and timestamps (float4 loads, a few steps in
-//      flight per warp), evaluates every predicate and keeps, per 128-row
+//   1. it streams its labels and timestamps (bulk copies through a ring of
+//      shared memory), evaluates every predicate and keeps, per 128-row
 //      warp segment and predicate, four ballot words of pass bits and their
 //      count in shared memory;
 //   2. it scans the segment counts into offsets inside the CTA and
@@ -57,37 +57,11 @@ struct FilterPreds {
   float4 b[FP_MAXP];
 };
 
-// 4 pass bits (rows 4 * lane + c) of one predicate
-__device__ __forceinline__ uint32_t pred_bits4(const float4 &b, const float4 &lab, const float4 &t) {
-  auto one = [&](float l, float ts) -> uint32_t {
-    return (l >= b.x && l <= b.y && ts >= b.z && ts <= b.w) ? 1u : 0u;
-  };
-  return one(lab.x, t.x) | (one(lab.y, t.y) << 1) | (one(lab.z, t.z) << 2) | (one(lab.w, t.w) << 3);
+__device__ __forceinline__ bool row_in(const float4 &b, float l, float ts) {
+  return l >= b.x && l <= b.y && ts >= b.z && ts <= b.w;
 }
 
 __device__ __forceinline__ uint64_t ld_volatile_u64(const uint64_t *p) { return *(const volatile uint64_t *)p; }
-
-// Loads one step's float4 of each column for this thread (rows r .. r + 3;
-// past n: zeros and valid bits cleared).
-__device__ __forceinline__ void load_step(const float *__restrict__ labels, const float *__restrict__ ts, uint32_t n,
-                                          uint32_t r, float4 &a, float4 &b, uint32_t &valid) {
-  if (r + 4 <= n) {
-    a = __ldcs(reinterpret_cast<const float4 *>(labels + r));
-    b = __ldcs(reinterpret_cast<const float4 *>(ts + r));
-    valid = 0xfu;
-  } else {
-    float la[4] = {0.f, 0.f, 0.f, 0.f}, tb[4] = {0.f, 0.f, 0.f, 0.f};
-    valid = 0;
-    for (int c = 0; c < 4; ++c)
-      if (r + c < n) {
-        la[c] = labels[r + c];
-        tb[c] = ts[r + c];
-        valid |= 1u << c;
-      }
-    a = make_float4(la[0], la[1], la[2], la[3]);
-    b = make_float4(tb[0], tb[1], tb[2], tb[3]);
-  }
-}
 
 // Grid: G CTAs, all resident.  Rows per CTA per round: R (a multiple of
 // FC_STEP).  Dynamic shared memory: S ring stages of FC_STEP rows of both
@@ -108,7 +82,7 @@ __global__ void __launch_bounds__(FC_THREADS, 2)
   uint32_t *segoff = reinterpret_cast<uint32_t *>(bits + (size_t)np * nseg);      // [np][nseg]
   __shared__ uint64_t full[FC_SMAX];
   __shared__ float4 pb[FP_MAXP];
-  __shared__ uint32_t wtot[FP_MAXP][FC_WARPS], wsum[FP_MAXP][FC_WARPS];
+  __shared__ uint32_t tot[FP_MAXP];
   __shared__ uint64_t s_off[FP_MAXP], s_base[FP_MAXP];
   __shared__ int s_fail;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
@@ -140,36 +114,49 @@ __global__ void __launch_bounds__(FC_THREADS, 2)
     };
     if (tid == 0)
       for (uint32_t c = 0; c < S && c < nfull; ++c) issue(c, c);
-    for (uint32_t p = tid; p < np * FC_WARPS; p += FC_THREADS) wsum[p / FC_WARPS][p % FC_WARPS] = 0;
+    if (tid < (int)FP_MAXP) tot[tid] = 0;
     __syncthreads();
-    // ---- 1. pass bits per warp segment (segment c * FC_WARPS + w: rows
-    //         cbase + c * FC_STEP + w * FC_SEG + 4 * lane + 0..3)
+    // ---- 1. pass bits per warp segment (segment c * FC_WARPS + w: word j
+    //         holds rows cbase + c * FC_STEP + w * FC_SEG + 32 j + 0..31, so
+    //         that a word's passing rows are written by neighbouring lanes).
+    //         The instructions per row and predicate bound this phase and the
+    //         writes: four compares, a vote, a count.
     bool gave_up = false;
     uint32_t c = 0, st = 0;  // chunk, its ring stage (c mod S)
-    const float *mine = ring + w * FC_SEG + 4 * lane;
+    uint32_t mytot = 0;      // lane p: the warp's rows that pass predicate p
+    const float *mine = ring + w * FC_SEG + lane;
     for (; c < nchunk; ++c) {
       const uint32_t seg = c * FC_WARPS + w;
-      float4 la, tb;
-      uint32_t vb = 0xfu;
+      float la[4], tb[4];
       if (c < nfull) {
         // warp-uniform: the lanes' timers may disagree at the deadline
         if (!__all_sync(0xffffffffu, mbar_wait_bounded(&full[st], (phase >> st) & 1u, err))) gave_up = true;
         phase ^= 1u << st;
-        la = *reinterpret_cast<const float4 *>(mine + st * (2 * FC_STEP));
-        tb = *reinterpret_cast<const float4 *>(mine + st * (2 * FC_STEP) + FC_STEP);
-      } else {
-        load_step(labels, ts, n, cbase + c * FC_STEP + w * FC_SEG + 4 * lane, la, tb, vb);
-      }
-      for (uint32_t p = 0; p < np; ++p) {
-        const uint32_t b4 = pred_bits4(pb[p], la, tb) & vb;
-        const uint32_t m0 = __ballot_sync(0xffffffffu, b4 & 1u), m1 = __ballot_sync(0xffffffffu, b4 & 2u);
-        const uint32_t m2 = __ballot_sync(0xffffffffu, b4 & 4u), m3 = __ballot_sync(0xffffffffu, b4 & 8u);
-        if (lane == 0) {
-          const uint32_t cnt = __popc(m0) + __popc(m1) + __popc(m2) + __popc(m3);
-          bits[p * nseg + seg] = make_uint4(m0, m1, m2, m3);
-          segoff[p * nseg + seg] = cnt;
-          wsum[p][w] += cnt;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          la[j] = mine[st * (2 * FC_STEP) + 32 * j];
+          tb[j] = mine[st * (2 * FC_STEP) + FC_STEP + 32 * j];
         }
+      } else {
+        const uint64_t r = (uint64_t)cbase + c * FC_STEP + w * FC_SEG + lane;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {  // (past the end: a NaN passes no predicate)
+          la[j] = r + 32 * j < n ? labels[r + 32 * j] : __int_as_float(0x7fc00000);
+          tb[j] = r + 32 * j < n ? ts[r + 32 * j] : __int_as_float(0x7fc00000);
+        }
+      }
+#pragma unroll 2
+      for (uint32_t p = 0; p < np; ++p) {
+        const float4 b = pb[p];
+        uint32_t m[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) m[j] = __ballot_sync(0xffffffffu, row_in(b, la[j], tb[j]));
+        const uint32_t cnt = __popc(m[0]) + __popc(m[1]) + __popc(m[2]) + __popc(m[3]);
+        if (lane == 0) {
+          bits[p * nseg + seg] = make_uint4(m[0], m[1], m[2], m[3]);
+          segoff[p * nseg + seg] = cnt;
+        }
+        if (lane == (int)p) mytot += cnt;
       }
       // the stage is free once every warp has read it; refill it
       if (__syncthreads_or(gave_up)) {
@@ -197,43 +184,28 @@ __global__ void __launch_bounds__(FC_THREADS, 2)
       return;
     }
     // ---- 2. the CTA's totals, published; the barrier arrival (release)
-    if (tid == 0) {
-      uint64_t *mypart = part + ((size_t)(rd & 1) * G + cta) * FP_MAXP;
-      for (uint32_t p = 0; p < np; ++p) {
-        uint32_t t = 0;
-        for (int j = 0; j < FC_WARPS; ++j) t += wsum[p][j];
-        mypart[p] = t;
-      }
-      asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(bar), "l"(1ull) : "memory");
+    if (lane < (int)np) atomicAdd(&tot[lane], mytot);
+    __syncthreads();
+    if (w == 0) {
+      if (lane < (int)np) part[((size_t)(rd & 1) * G + cta) * FP_MAXP + lane] = tot[lane];
+      __syncwarp();
+      if (lane == 0) asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(bar), "l"(1ull) : "memory");
     }
-    // ---- 3. segment offsets inside the CTA, while the other CTAs finish
-    for (uint32_t i0 = 0; i0 < nseg; i0 += FC_THREADS) {
-      const uint32_t i = i0 + tid;
-      for (uint32_t p = 0; p < np; ++p) {
-        const uint32_t v = i < nseg ? segoff[p * nseg + i] : 0u;
+    // ---- 3. segment offsets inside the CTA, a warp to a predicate, while
+    //         the other CTAs finish
+    for (uint32_t p = w; p < np; p += FC_WARPS) {
+      uint32_t run = 0;
+      for (uint32_t i0 = 0; i0 < nseg; i0 += 32) {
+        const uint32_t v = i0 + lane < nseg ? segoff[p * nseg + i0 + lane] : 0u;
         uint32_t inc = v;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
           const uint32_t x = __shfl_up_sync(0xffffffffu, inc, o);
           if (lane >= o) inc += x;
         }
-        if (i < nseg) segoff[p * nseg + i] = inc - v;  // exclusive within the warp's 32 segments
-        if (lane == 31) wtot[p][w] = inc;
+        if (i0 + lane < nseg) segoff[p * nseg + i0 + lane] = run + inc - v;
+        run += __shfl_sync(0xffffffffu, inc, 31);
       }
-      __syncthreads();
-      if (tid < (int)np) {  // the warps' totals -> exclusive prefixes, carried across chunks of segments
-        uint32_t acc = i0 ? (uint32_t)s_off[tid] : 0u;  // the running total of the earlier chunks
-        for (int j = 0; j < FC_WARPS; ++j) {
-          const uint32_t x = wtot[tid][j];
-          wtot[tid][j] = acc;
-          acc += x;
-        }
-        s_off[tid] = acc;
-      }
-      __syncthreads();
-      if (i < nseg)
-        for (uint32_t p = 0; p < np; ++p) segoff[p * nseg + i] += wtot[p][w];
-      __syncthreads();
     }
     // ---- 4. the grid barrier's wait (bounded, acquire)
     if (tid == 0) {
@@ -293,35 +265,26 @@ __global__ void __launch_bounds__(FC_THREADS, 2)
       }
     }
     __syncthreads();
-    // ---- 5. ids of the passing rows: per segment staged in this warp's
-    //         slice of the (now idle) ring, then stored contiguously
-    uint32_t *stage = reinterpret_cast<uint32_t *>(ring) + w * FC_SEG;
+    // ---- 5. ids of the passing rows, a word of 32 at a time
     for (uint32_t p = 0; p < np; ++p) {
-      uint32_t *op = out + p * out_stride;
-      const uint32_t base = (uint32_t)s_off[p];
+      uint32_t *op = out + p * out_stride + (uint32_t)s_off[p];
       const uint4 *bp = bits + p * nseg + w;
       const uint32_t *sp = segoff + p * nseg + w;
+#pragma unroll 2
       for (uint32_t cc = 0; cc < nchunk; ++cc) {
         const uint4 m = bp[cc * FC_WARPS];  // the same for the whole warp: the skip is uniform
-        const uint32_t cnt = __popc(m.x) + __popc(m.y) + __popc(m.z) + __popc(m.w);
-        if (cnt == 0) continue;
-        const uint32_t b4 = ((m.x >> lane) & 1u) | (((m.y >> lane) & 1u) << 1) | (((m.z >> lane) & 1u) << 2) |
-                            (((m.w >> lane) & 1u) << 3);
-        uint32_t k = __popc(m.x & lanemask_lt) + __popc(m.y & lanemask_lt) + __popc(m.z & lanemask_lt) +
-                     __popc(m.w & lanemask_lt);
-        const uint32_t r = cbase + cc * FC_STEP + w * FC_SEG + 4 * lane;
+        if ((m.x | m.y | m.z | m.w) == 0) continue;
+        uint32_t *dst = op + sp[cc * FC_WARPS];
+        const uint32_t r = cbase + cc * FC_STEP + w * FC_SEG + lane;
+        const uint32_t ms[4] = {m.x, m.y, m.z, m.w};
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
-          if ((b4 >> q) & 1u) stage[k++] = r + q;
-        __syncwarp();
-        uint32_t *dst = op + base + sp[cc * FC_WARPS];
-        for (uint32_t j = lane; j < cnt; j += 32) dst[j] = stage[j];
-        __syncwarp();  // the slice is rewritten by the next segment
+        for (int j = 0; j < 4; ++j) {
+          if ((ms[j] >> lane) & 1u) dst[__popc(ms[j] & lanemask_lt)] = r + 32 * j;
+          dst += __popc(ms[j]);
+        }
       }
     }
-    // the ring's generic writes before the next round's bulk copies into it
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncthreads();  // bits, offsets and the ring are rewritten by the next round
+    __syncthreads();  // bits and offsets are rewritten by the next round
   }
   if (cta == 0 && tid < (int)np) {
     const bool failed = ld_volatile_u64(flag) == ep;
