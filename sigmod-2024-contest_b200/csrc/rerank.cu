@@ -12,6 +12,12 @@ namespace {
 constexpr int RK_THREADS = 256;
 constexpr int RK_MAXC = 2048;  // candidates per query
 
+// Up to a candidate per thread, a thread counts its key's place among the
+// others (two passes over shared memory: repeats first); above that the keys
+// are sorted and a prefix sum drops the repeats.  Rows are read 16 bytes at a
+// time.  10,000 queries of 150 candidates: 365 us with the sort and thread 0
+// adding up 256 counts.
+
 __global__ void __launch_bounds__(RK_THREADS)
     k_rerank(const float *__restrict__ vecs, uint64_t n, const float *__restrict__ q, uint32_t nq,
              const uint32_t *__restrict__ cand, uint32_t nc, uint32_t k, uint32_t *__restrict__ ids,
@@ -29,10 +35,36 @@ __global__ void __launch_bounds__(RK_THREADS)
     uint64_t kk = ~0ull;
     if (i < (int)nc) {
       const uint32_t id = cand[(uint64_t)qi * nc + i];
-      if (id < n) kk = exact_key(seq_l2_strided(vecs + (uint64_t)id * DIM, 1, qv), id);
+      if (id < n) kk = exact_key(seq_l2_row(vecs + (uint64_t)id * DIM, qv), id);
       else if (id != 0xffffffffu) atomicOr(err, ERR_BAD_QUERY_VALUE);
     }
     key[i] = kk;
+  }
+  if (nc <= RK_THREADS) {
+    __shared__ uint32_t total;
+    if (tid == 0) total = 0;
+    __syncthreads();
+    const uint64_t e = tid < (int)nc ? key[tid] : ~0ull;
+    bool first = e != ~0ull;  // not a repeat of an earlier candidate
+    for (int j = 0; j < tid && j < (int)nc; ++j) first &= key[j] != e;
+    __syncthreads();
+    if (tid < (int)nc && !first) key[tid] = ~0ull;
+    const uint32_t m = __ballot_sync(0xffffffffu, first);
+    if ((tid & 31) == 0) atomicAdd(&total, (uint32_t)__popc(m));
+    __syncthreads();
+    if (first) {
+      uint32_t w = 0;
+      for (int j = 0; j < (int)nc; ++j) w += key[j] < e ? 1u : 0u;
+      if (w < k) {
+        ids[(uint64_t)qi * k + w] = (uint32_t)e;
+        if (dists) dists[(uint64_t)qi * k + w] = sortable_f32((uint32_t)(e >> 32));
+      }
+    }
+    for (uint32_t j = total + tid; j < k; j += RK_THREADS) {
+      ids[(uint64_t)qi * k + j] = 0xffffffffu;
+      if (dists) dists[(uint64_t)qi * k + j] = INFINITY;
+    }
+    return;  // (block-uniform)
   }
   __syncthreads();
   block_bitonic_sort(key, np2);
@@ -44,8 +76,18 @@ __global__ void __launch_bounds__(RK_THREADS)
   keep[tid + 1] = c;
   if (tid == 0) keep[0] = 0;
   __syncthreads();
-  if (tid == 0)
-    for (int t = 0; t < RK_THREADS; ++t) keep[t + 1] += keep[t];
+  if (tid < 32) {  // running sums, RK_THREADS / 32 to a lane
+    constexpr int PER = RK_THREADS / 32;
+    uint32_t sum = 0;
+    for (int j = 1; j <= PER; ++j) sum += keep[tid * PER + j];
+    uint32_t inc = sum;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
+      if (tid >= o) inc += v;
+    }
+    uint32_t run = inc - sum;
+    for (int j = 1; j <= PER; ++j) keep[tid * PER + j] = run += keep[tid * PER + j];
+  }
   __syncthreads();
   uint32_t w = keep[tid];
   for (int i = i0; i < i1 && w < k; ++i)
