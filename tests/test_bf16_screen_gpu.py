@@ -1,0 +1,57 @@
+"""The BF16 screen at the edges of its tiles: one and two query halves, row
+blocks of 256 and a short last one, lists of every register class, with and
+without a pilot, host and device plans.  The vectors are multiples of 1/8 up to
+2, so BF16 operands, products, norms and sums are exact, the screening order is
+the exact one, and ids and distances equal the oracle's (k' exceeds k by more
+rows than share a distance)."""
+import numpy as np
+import pytest
+
+import fknn
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def grid(rng, shape):
+    return (np.clip(np.round(rng.standard_normal(shape) * 5), -16, 16) / 8).astype(np.float32)
+
+
+@pytest.fixture(scope="module")
+def data():
+    rng = np.random.default_rng(5)
+    n = 30_011
+    vecs = grid(rng, (n, 100))
+    labels = (np.arange(n) % 5 == 0).astype(np.float32)  # 6,003 and 24,008 rows
+    ts = rng.random(n, dtype=np.float32)
+    q = grid(rng, (600, 100))
+    metas = np.zeros((600, 4), np.float32)
+    metas[:, 0] = rng.choice([0, 0, 0, 1, 2, 3], 600)
+    metas[:, 1] = rng.integers(0, 2, 600)
+    metas[:, 2] = rng.random(600) * 0.4
+    metas[:, 3] = metas[:, 2] + 0.6
+    want = oracle.exact_knn(vecs, labels, ts, q, metas, k=100)
+    with fknn.Index(vecs, labels, ts, build_bf16=True) as idx:
+        yield idx, q, metas, want
+
+
+@pytest.mark.parametrize("nq", [1, 127, 128, 129, 255, 256, 257, 600])
+@pytest.mark.parametrize("pilot", [0, 2, 8])
+def test_tiles(data, nq, pilot):
+    idx, q, metas, (ids, dists) = data
+    idx.set_tuning(fknn.MODE_BF16_RERANK, 256, 3, 8, 0, pilot)
+    for graph in (False, True):
+        got, d = idx.search(q[:nq], metas[:nq], k=100, mode=fknn.MODE_BF16_RERANK, kprime=128, graph=graph)
+        np.testing.assert_array_equal(got, ids[:nq])
+        np.testing.assert_array_equal(d, dists[:nq])
+
+
+@pytest.mark.parametrize("kprime", [128, 256, 257, 512, 513, 768, 769, 1024])
+@pytest.mark.parametrize("slack", [256, 512])
+def test_list_classes(data, kprime, slack):
+    idx, q, metas, (ids, dists) = data
+    for pilot in (0, 4):
+        idx.set_tuning(fknn.MODE_BF16_RERANK, slack, 2, 4, 4, pilot)
+        got, d = idx.search(q, metas, k=100, mode=fknn.MODE_BF16_RERANK, kprime=kprime)
+        np.testing.assert_array_equal(got, ids)
+        np.testing.assert_array_equal(d, dists)
