@@ -480,12 +480,6 @@ __device__ __forceinline__ uint32_t pack_query(int r0, int r1, int lane, int col
   return (uint32_t)r0 | (uint32_t)r1 << 9 | (uint32_t)lane << 18 | (uint32_t)col / 32 << 23;
 }
 
-// bit j set iff r0 <= j < r1
-__device__ __forceinline__ uint32_t range_mask(int r0, int r1) {
-  const int a = max(r0, 0), b = min(r1, 32);
-  return a >= b ? 0u : (0xffffffffu >> (32 - b)) & (0xffffffffu << a);
-}
-
 // Persistent, one CTA per SM, pulling work items (longest first) from a
 // queue: warp 16 copies row blocks in, warp 17 issues MMAs, warps 0-15 are the
 // epilogue.  A tile of more than 128 queries multiplies every row block with
@@ -699,17 +693,17 @@ __global__ void __launch_bounds__(B_THREADS, 1) k_screen_tc(ScreenArgs A) {
             }
             continue;
           }
-          // One candidate in a chunk, as most have: it is the maximum, and its
-          // lane appends it by itself.  The rest are staged in shared memory
-          // and appended by the warp.
+          // One that passes on its own, as in most chunks: it is the maximum,
+          // and its lane appends it by itself if it is inside the slab.  The
+          // rest are staged in shared memory and appended by the warp.
           if (todo & 1u) {
-            const uint32_t in = ge_mask32(ra, ga, bound) & range_mask(r0 - col0, r1 - col0);
-            if ((in & (in - 1)) == 0) todo ^= 1u;
+            const uint32_t all = ge_mask32(ra, ga, bound), in = all & range_mask(r0 - col0, r1 - col0);
+            if (in == 0 || (all & (all - 1)) == 0) todo ^= 1u;
             if (in && !(todo & 1u)) lists[lane * A.capb + cnt++] = {fmaf(qs.y, ma, qs.x), p0 + col0 + __ffs(in) - 1};
           }
           if (todo & 2u) {
-            const uint32_t in = ge_mask32(rb, gb, bound) & range_mask(r0 - col0 - 32, r1 - col0 - 32);
-            if ((in & (in - 1)) == 0) todo ^= 2u;
+            const uint32_t all = ge_mask32(rb, gb, bound), in = all & range_mask(r0 - col0 - 32, r1 - col0 - 32);
+            if (in == 0 || (all & (all - 1)) == 0) todo ^= 2u;
             if (in && !(todo & 2u)) lists[lane * A.capb + cnt++] = {fmaf(qs.y, mb, qs.x), p0 + col0 + 31 + __ffs(in)};
           }
           while (__any_sync(0xffffffffu, todo != 0)) {

@@ -52,6 +52,12 @@ __device__ __forceinline__ uint32_t ge_mask32(const uint32_t (&r)[32], const flo
   return in;
 }
 
+// bit j set iff r0 <= j < r1
+__device__ __forceinline__ uint32_t range_mask(int r0, int r1) {
+  const int a = max(r0, 0), b = min(r1, 32);
+  return a >= b ? 0u : (0xffffffffu >> (32 - b)) & (0xffffffffu << a);
+}
+
 // one epilogue warp's scratch: staged candidate chunks, or the histogram of a trim
 template <int SLOTS>
 struct ScreenWarp {

@@ -55,3 +55,36 @@ def test_list_classes(data, kprime, slack):
         got, d = idx.search(q, metas, k=100, mode=fknn.MODE_BF16_RERANK, kprime=kprime)
         np.testing.assert_array_equal(got, ids)
         np.testing.assert_array_equal(d, dists)
+
+
+@pytest.mark.parametrize("mode", ["bf16", "exact"])
+def test_nearer_row_beyond_the_slab(mode):
+    """The last row of a slab passes the bound but is not among the k best,
+    and the row after it, outside, is the query itself: the two share a chunk
+    of the screen, and the one inside must keep its own distance."""
+    rng = np.random.default_rng(11)
+    n, nq, k = 30_000, 96, 100
+    vecs, q = grid(rng, (n, 100)), grid(rng, (nq, 100))
+    ts = np.arange(n, dtype=np.float32)
+    metas = np.zeros((nq, 4), np.float32)
+    metas[:, 0] = 2
+    end = 9000 + 211 * np.arange(nq)  # the last row inside
+    metas[:, 3] = end
+    for i in range(nq):
+        d = ((vecs[: end[i]] - q[i]) ** 2).sum(1)
+        r = np.argsort(d, kind="stable")[int(rng.integers(k + 2, 2 * k))]
+        vecs[end[i]] = vecs[r]
+        vecs[end[i], 0] += np.float32(0.125) * np.sign(vecs[r, 0] - q[i, 0] + np.float32(0.01))
+        vecs[end[i] + 1] = q[i]
+    with fknn.Index(vecs, np.zeros(n, np.float32), ts, build_bf16=True) as idx:
+        ids, dists = oracle.exact_knn(vecs, np.zeros(n, np.float32), ts, q, metas, k=k)
+        for pilot in (2, 4, 8):
+            if mode == "bf16":
+                idx.set_tuning(fknn.MODE_BF16_RERANK, 256, 3, 8, 0, pilot)
+                got, gd = idx.search(q, metas, k=k, mode=fknn.MODE_BF16_RERANK, kprime=k)
+            else:
+                idx.set_tuning(fknn.MODE_EXACT_FP32, 0, 4, 16, 0, pilot)
+                got, gd = idx.search(q, metas, k=k)
+            np.testing.assert_array_equal(gd, dists)  # (rows at the same distance as the k-th may differ in bf16)
+            if mode == "exact":
+                np.testing.assert_array_equal(got, ids)
