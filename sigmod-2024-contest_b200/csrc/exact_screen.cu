@@ -217,6 +217,7 @@ __device__ __noinline__ void x_finish(const Candidate *work, XSmem &sm, int L, i
 __device__ __forceinline__ bool convert_rows(XSmem &sm, uint32_t nblk, uint32_t blk0, uint32_t stride, uint32_t nsub,
                                              uint32_t g0, int cw, int fold, int *err) {
   const int lane = threadIdx.x & 31;
+#pragma unroll 1
   for (uint32_t sub = 0; sub < nsub; ++sub) {
     const uint32_t gs = g0 + sub;
     const uint32_t st = gs % X_ST, rd = gs / X_ST;
@@ -391,6 +392,7 @@ __global__ void __launch_bounds__(X_THREADS, 1) k_exact_screen(ExactScreenArgs A
       if (lane == 0 && !aborted) {
         const uint32_t f0 = g * (XR / BLK), nf = nsub * (XR / BLK);
         uint32_t done = 0;
+#pragma unroll 1
         for (; done < nf; ++done) {
           const uint32_t fi = f0 + done, fs = fi % X_FB, fr = fi / X_FB;
           if (fr > 0 && !mbar_wait_bounded(&sm.fempty[fs], (fr - 1) & 1, A.err)) break;
@@ -404,6 +406,7 @@ __global__ void __launch_bounds__(X_THREADS, 1) k_exact_screen(ExactScreenArgs A
         }
         // every issued copy has landed before the item ends
         bool ok = done == nf;
+#pragma unroll 1
         for (uint32_t i = done > X_FB ? done - X_FB : 0; i < done; ++i)
           ok = mbar_wait_bounded(&sm.ffull[(f0 + i) % X_FB], ((f0 + i) / X_FB) & 1, A.err) && ok;
         if (!ok) gave_up = true;
@@ -415,10 +418,12 @@ __global__ void __launch_bounds__(X_THREADS, 1) k_exact_screen(ExactScreenArgs A
       if (lane == 0 && !aborted && nsub) {
         uint32_t done = 0, ua[X_GROUPS] = {u0, u1};
         bool ok = mbar_wait_bounded(&sm.afull, nrun & 1, A.err);
+#pragma unroll 1
         for (uint32_t sub = 0; sub < nsub && ok; ++sub) {
           const uint32_t st = (g + sub) % X_ST, rd = (g + sub) / X_ST;
           if (!mbar_wait_bounded(&sm.bfull[st], rd & 1, A.err)) break;
           const uint32_t b0 = smem_u32(sm.b[st][0]);
+#pragma unroll 1
           for (int half = 0; half < (both ? X_GROUPS : 1); ++half) {
             const int a = both ? half : (int)(sub & 1);  // the accumulator
             const uint32_t u = a ? ua[1] : ua[0];
@@ -520,6 +525,11 @@ __global__ void __launch_bounds__(X_THREADS, 1) k_exact_screen(ExactScreenArgs A
         Candidate *work = A.work + (uint64_t)blockIdx.x * XQ * X_LIST;
         Candidate *lists = work + (uint64_t)(warp * 32) * X_LIST, *list = lists + lane * X_LIST;
         XWarp &wsm = sm.w[warp];
+        // a pilot over a slab of many sampled rows keeps the best of every XR
+        // or 32 of them: the few that matter lie apart as a rule, so the seed's
+        // rank in these is little above its rank in all (and never below it)
+        const uint32_t sampled = (e - s) / A.stride;
+        const int sample = A.stride == 1 ? 0 : sampled / XR >= 2 * A.k ? XR : sampled / 32 >= 2 * A.k ? 32 : 0;
         int cnt = 0;
         bool ok = !aborted;
         // keep iff qn - 2 v <= push limit, as one compare on v = q.x - |x|^2/2
@@ -530,6 +540,7 @@ __global__ void __launch_bounds__(X_THREADS, 1) k_exact_screen(ExactScreenArgs A
         float cq = acc_bound(T);
         float cs = cq * qs;
         uint32_t until_refresh = X_REFRESH, u = grp ? u1 : u0;
+#pragma unroll 1
         for (uint32_t sub = both ? 0u : (uint32_t)grp; sub < nsub && ok; sub += both ? 1u : X_GROUPS, ++u) {
           const uint32_t slot = (g + sub) % X_NORMS;
           if (!__all_sync(0xffffffffu, mbar_wait_bounded(&sm.accfull[grp], u & 1, A.err))) {
@@ -540,12 +551,7 @@ __global__ void __launch_bounds__(X_THREADS, 1) k_exact_screen(ExactScreenArgs A
           const uint32_t p0 = (it.blk0 + sub * A.stride) * XR;
           const int r0 = (int)min(max(s, p0), p0 + XR) - (int)p0;
           const int r1 = (int)min(max(e, p0), p0 + XR) - (int)p0;
-          // four 32-column chunks: the ones whose maximum reaches the bound are
-          // staged (rows outside the slab may raise it; x_flush looks closer).
-          // The next chunk's TMEM load is in flight meanwhile.
           const uint32_t tb = tq + X_ACC + grp * XR;
-          uint32_t ra[32], rb[32];
-          tmem_ld32_issue(tb, ra);
           const float4 cr4 = *reinterpret_cast<const float4 *>(sm.crs[slot]);
           if (cr4.x > 0.f && cr4.x == cr4.y && cr4.x == cr4.z && cr4.x == cr4.w) {  // (block-uniform)
             // the rows' scale 2^ex = 1 / cr: v >= cq iff acc >= cs 2^ex (-inf would admit masked columns)
@@ -554,18 +560,46 @@ __global__ void __launch_bounds__(X_THREADS, 1) k_exact_screen(ExactScreenArgs A
             q.f2 = -2.f * (cr4.x * iq);
             q.qn = qd;
             q.range = (r0 << 16) | r1;
+            // 32-column chunks, two at a time: one whose maximum reaches the
+            // bound holds a candidate, or a row outside the slab that raises it.
+            // One that passes on its own, as in most chunks, is the maximum, and
+            // its lane appends it; the rest are staged (x_flush looks closer).  A
+            // pilot over a long slab keeps the maxima themselves.
             uint32_t hits = 0;
-            tmem_wait_ld(ra);
-            tmem_ld32_issue(tb + 32, rb);
-            hits |= max32(ra) >= q.bound ? 1u : 0u;
-            tmem_wait_ld(rb);
-            tmem_ld32_issue(tb + 64, ra);
-            hits |= max32(rb) >= q.bound ? 2u : 0u;
-            tmem_wait_ld(ra);
-            tmem_ld32_issue(tb + 96, rb);
-            hits |= max32(ra) >= q.bound ? 4u : 0u;
-            tmem_wait_ld(rb);
-            hits |= max32(rb) >= q.bound ? 8u : 0u;
+            float best = -INFINITY;
+#pragma unroll 1
+            for (int c = 0; c < XR; c += 64) {
+              uint32_t ra[32], rb[32];
+              float ga[4], gb[4];
+              tmem_ld32_issue(tb + c, ra);
+              tmem_ld32_issue(tb + c + 32, rb);
+              tmem_wait_ld(ra);
+              tmem_wait_ld(rb);
+              const float ma = max32(ra, ga), mb = max32(rb, gb);
+              best = fmax3(best, ma, mb);
+              uint32_t h = (ma >= q.bound ? 1u : 0u) | (mb >= q.bound ? 2u : 0u);
+              if (!__any_sync(0xffffffffu, h != 0)) continue;
+              if (sample) {
+                if (sample == 32) {
+                  if ((h & 1u) && c >= r0 && c + 32 <= r1) list[cnt++] = {fmaf(q.f2, ma, qd), p0 + c};
+                  if ((h & 2u) && c + 32 >= r0 && c + 64 <= r1) list[cnt++] = {fmaf(q.f2, mb, qd), p0 + c + 32};
+                }
+                h = 0;
+              }
+              if (h & 1u) {
+                const uint32_t all = ge_mask32(ra, ga, q.bound), in = all & range_mask(r0 - c, r1 - c);
+                if (in == 0 || (all & (all - 1)) == 0) h ^= 1u;
+                if (in && !(h & 1u)) list[cnt++] = {fmaf(q.f2, ma, qd), p0 + c + __ffs(in) - 1};
+              }
+              if (h & 2u) {
+                const uint32_t all = ge_mask32(rb, gb, q.bound), in = all & range_mask(r0 - c - 32, r1 - c - 32);
+                if (in == 0 || (all & (all - 1)) == 0) h ^= 2u;
+                if (in && !(h & 2u)) list[cnt++] = {fmaf(q.f2, mb, qd), p0 + c + 31 + __ffs(in)};
+              }
+              hits |= h << (c / 32);
+              __syncwarp();  // (the next TMEM loads are the whole warp's)
+            }
+            if (sample == XR && best >= q.bound && r1 - r0 == XR) list[cnt++] = {fmaf(q.f2, best, qd), p0};
             int ns = 0;
             if (__any_sync(0xffffffffu, hits != 0)) {
 #pragma unroll 1
@@ -583,7 +617,6 @@ __global__ void __launch_bounds__(X_THREADS, 1) k_exact_screen(ExactScreenArgs A
             if (lane == 0) mbar_arrive1(&sm.accempty[grp]);
             if (ns) cnt = x_flush(wsm, ns, p0, lists, X_LIST, cnt);
           } else {
-            tmem_wait_ld(ra);
 #pragma unroll 1
             for (int o = 0; o < XR; o += 32)
               cnt = x_push_norms(tb + o, sm, slot, o, iq, cq, qd, r0 - o, r1 - o, p0 + o, list, cnt);
@@ -630,6 +663,7 @@ __global__ void __launch_bounds__(X_THREADS, 1) k_exact_screen(ExactScreenArgs A
         // every list of the item is complete (and visible)
         asm volatile("bar.sync 1, %0;" ::"n"(X_EPI * 32) : "memory");
         const int per = both ? XQ / X_EPI : XM / X_EPI;
+#pragma unroll 1
         for (int b = 0; b < per; ++b) {
           const int Lb = warp * per + b;
           const uint64_t o = (uint64_t)item_id * XQ + Lb;
