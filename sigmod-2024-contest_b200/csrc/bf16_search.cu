@@ -5,9 +5,10 @@
 // distance so the boundary order follows exact arithmetic.
 //
 // Layouts (both operands K-major, no swizzle, core matrices of 8 rows x 16 B):
-//   query tile A: 128 queries x 112 bf16, element (q, k) at
+//   query half A: 128 queries x 112 bf16, element (q, k) at
 //                 ((k/8)*16 + q/8)*64 + (q%8)*8 + k%8
-//   row block  B: 128 rows x 112 bf16, same formula with the row index
+//   row block  B: 256 rows x 112 bf16, element (r, k) at
+//                 ((k/8)*32 + r/8)*64 + (r%8)*8 + k%8
 // Dims 0..99 carry the vector; on the row side dims 100/101 carry
 // -|x|^2/2 split into a bf16 high part and a bf16 remainder, on the query
 // side dims 100/101 are 1.0.  The MMA therefore produces
@@ -490,6 +491,12 @@ __device__ __forceinline__ uint32_t pack_query(int r0, int r1, int lane, int col
 // while the next product is made (with an accumulator and half the warps for
 // each query half, every one of them waited for the slowest).
 // N = 256: an MMA of 128 columns takes 91 cycles here, one of 256 takes 128.
+// Bound by the epilogue's latency: a warp needs about 1,200 cycles a product
+// (the MMAs 896) and 640 more when one of its queries has a candidate; sixteen
+// warps of 64 columns each measured the same.  Screens of a call, pilot
+// included, before (tiles of 128 x 128, two CTAs per SM) and now: 50 queries
+// over 1e6 rows 0.92 and 0.17 ms, 4,096 over 2e6 4.35 and 2.04 ms, 100,000 over
+// 4e6 41.1 and 36 to 38 ms.
 // Barrier phases run on across items: g counts the row blocks of this CTA's
 // earlier items, u the products.
 template <class F, int NPL>
@@ -877,7 +884,9 @@ struct MergeArgs {
 };
 
 // One big query b (index into the plan's big-query arrays): gather its
-// lists, keep the k' best screening distances, re-rank them in FP32.  A
+// lists, keep the k' best screening distances, re-rank them in FP32.  Bound by
+// latency: barriers and the gather of k' rows of 400 B (4,096 queries over 2e6
+// rows, k' = 200: 0.70 ms with sorts of up to 8,192 candidates, 0.31 ms now).  A
 // query with more than CAP candidates goes to `spill` (the large merge) or,
 // from the large merge, to the exact scan.  Returns are block-uniform.
 template <int CAP>

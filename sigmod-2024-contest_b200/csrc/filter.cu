@@ -120,7 +120,9 @@ __global__ void __launch_bounds__(FC_THREADS, 2)
     //         holds rows cbase + c * FC_STEP + w * FC_SEG + 32 j + 0..31, so
     //         that a word's passing rows are written by neighbouring lanes).
     //         The instructions per row and predicate bound this phase and the
-    //         writes: four compares, a vote, a count.
+    //         writes: four compares, a vote, a count.  (8 predicates over 4e6
+    //         rows: 77 us with four neighbouring rows a lane, packed, voted on
+    //         and staged; 48 us now.)
     bool gave_up = false;
     uint32_t c = 0, st = 0;  // chunk, its ring stage (c mod S)
     uint32_t mytot = 0;      // lane p: the warp's rows that pass predicate p

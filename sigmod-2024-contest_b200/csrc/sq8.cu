@@ -174,8 +174,9 @@ __device__ __forceinline__ void heap_ready(WarpHeap &w, int lane) {
 }
 
 // must_pop_emplace (bruteforce.h:99-105) behind the root test
-// bruteforce.h:258-260 makes, by the whole warp.  (Lane 0 alone, a level at a
-// time with its branch and store, took 1,080 cycles a node at k = 140.)
+// bruteforce.h:258-260 makes, by the whole warp.  A chain of loads and shuffles,
+// so bound by latency: 500 cycles a node at k = 140, where lane 0 alone, a level
+// at a time with its branch and store, took 1,080.
 __device__ __forceinline__ void heap_offer(WarpHeap &w, HeapNode nd, int lane) {
   if (w.root <= nd.d) return;
   const char *const nb = reinterpret_cast<const char *>(w.next);
