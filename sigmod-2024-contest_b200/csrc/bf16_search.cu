@@ -332,9 +332,10 @@ struct ScreenArgs {
   uint32_t *T_global;           // per query: upper bound on its k'-th screening distance (f32_sortable)
   uint32_t *ovf;                // per query: non-zero = left to the exact scan
   Candidate *work;              // [CTA][half][B_LISTS][capb]
-  Candidate *out;               // [item][BQ][capb]
+  Candidate *out;               // [item][BQ][ocap]
   uint32_t *out_cnt;            // [item][BQ]
-  uint32_t kprime, capb, refresh;
+  uint32_t kprime, capb, ocap, refresh;
+  uint32_t halves;              // working lists per CTA: 1 where no tile has more than BM queries
   uint32_t kseed;               // pilot: k' of the search
   uint32_t stride;              // > 1: a pilot pass over every stride-th row block
   uint32_t withhold;
@@ -403,13 +404,13 @@ __device__ __noinline__ int b_trim(Candidate *list, int n, BScreenSmem<F> &sm, i
 }
 
 // The item's result for a query whose lists (one in every BM from work and cnt
-// on, more than capb entries in all) have to be bounded: their k'-th screening
+// on, more than ocap entries in all) have to be bounded: their k'-th screening
 // distance by a radix select that reads them again for every digit (rare: a
 // seeded query has far fewer).  Whole warp; returns the entries written, more
-// than capb only where ties do not fit.
+// than ocap only where ties do not fit.
 template <class F>
 __device__ __noinline__ int b_select(const Candidate *work, const int *cnt, BScreenSmem<F> &sm, int L, uint32_t kprime,
-                                     uint32_t capb, uint32_t *T_global, Candidate *out) {
+                                     uint32_t capb, uint32_t ocap, uint32_t *T_global, Candidate *out) {
   const int lane = threadIdx.x & 31;
   uint32_t *hist = sm.w[threadIdx.x >> 5].hist;
   auto each = [&](auto &&f) {  // every entry, the warp together
@@ -461,7 +462,7 @@ __device__ __noinline__ int b_select(const Candidate *work, const int *cnt, BScr
     const bool keep = on && f32_sortable(__uint_as_float(c.x)) <= prefix;
     const uint32_t b = __ballot_sync(0xffffffffu, keep);
     const uint32_t o = kept + __popc(b & ((1u << lane) - 1u));
-    if (keep && o < capb) *reinterpret_cast<uint2 *>(out + o) = c;
+    if (keep && o < ocap) *reinterpret_cast<uint2 *>(out + o) = c;
     kept += __popc(b);
   });
   return kept;
@@ -638,7 +639,7 @@ __global__ void __launch_bounds__(B_THREADS, 1) k_screen_tc(ScreenArgs A) {
         sm.q[tid] = make_float4(acc_bound(T, qs), __uint_as_float(s), __uint_as_float(e), coarse ? 1.f : 0.f);
       }
       asm volatile("bar.sync 1, %0;" ::"n"(B_EPI * 32) : "memory");
-      Candidate *const work = A.work + (uint64_t)blockIdx.x * 2 * B_LISTS * A.capb;
+      Candidate *const work = A.work + (uint64_t)blockIdx.x * A.halves * B_LISTS * A.capb;
       auto &wsm = sm.w[warp];
       const uint32_t lt = (1u << lane) - 1u;
       int cnt0 = 0, cnt1 = 0;  // entries of this thread's lists
@@ -809,10 +810,10 @@ __global__ void __launch_bounds__(B_THREADS, 1) k_screen_tc(ScreenArgs A) {
       for (int b = 0; b < per; ++b) {
         const int nb = __shfl_sync(0xffffffffu, n, b);
         if (nb == 0) continue;
-        Candidate *src = work + (uint64_t)(hf * B_LISTS + l0 + b) * A.capb, *dst = A.out + (o0 + b) * A.capb;
+        Candidate *src = work + (uint64_t)(hf * B_LISTS + l0 + b) * A.capb, *dst = A.out + (o0 + b) * A.ocap;
         int *c = &sm.cnt[hf][l0 + b];
-        if (nb > (int)A.capb) {
-          const int kept = b_select<F>(src, c, sm, q0 + b, A.kprime, A.capb, A.T_global, dst);
+        if (nb > (int)A.ocap) {
+          const int kept = b_select<F>(src, c, sm, q0 + b, A.kprime, A.capb, A.ocap, A.T_global, dst);
           if (lane == b) n = kept;
           continue;
         }
@@ -825,7 +826,7 @@ __global__ void __launch_bounds__(B_THREADS, 1) k_screen_tc(ScreenArgs A) {
           at += c[l];
         }
       }
-      if (n > (int)A.capb) {  // more ties than fit
+      if (n > (int)A.ocap) {  // more ties than fit
         A.ovf[sm.lq[q0 + lane]] = 1u;
         n = 0;
       }
@@ -1106,6 +1107,33 @@ inline uint32_t max_items(uint32_t capb, uint32_t pilot_stride, uint64_t per_ite
   return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(lists, (8ull << 30) / (per_item * tiles)));
 }
 
+// Entries of a query in an item's result when memory is short: k' and a few
+// ties, which a select makes of the working lists.
+inline uint32_t tight_cap(uint32_t kprime, uint32_t capb) { return std::min(capb, (kprime + 64 + 31) / 32 * 32); }
+
+// Scratch of the lists: nitems results of BQ queries, and working lists for
+// every CTA.  Where the index's HBM budget or the memory left does not hold
+// that, the caller plans again with one item per tile, and here as many CTAs
+// as fit (tight).
+inline int list_scratch(fknn_index *idx, uint32_t nitems, uint32_t halves, uint32_t capb, uint32_t ocap, bool tight,
+                        Candidate **out, uint32_t **cnt, Candidate **work, uint32_t *grid) {
+  int rc = ws_get(idx, 6, (size_t)nitems * BQ * ocap * sizeof(Candidate), (void **)out);
+  if (!rc) rc = ws_get(idx, 7, (size_t)nitems * BQ * 4, (void **)cnt);
+  if (!rc)
+    for (*grid = std::min<uint32_t>(nitems, (uint32_t)idx->num_sms);; *grid = (*grid + 1) / 2) {
+      rc = ws_get(idx, 11, (size_t)*grid * halves * B_LISTS * capb * sizeof(Candidate), (void **)work);
+      if (rc != FKNN_ENOMEM || !tight || *grid == 1) break;
+      cudaGetLastError();
+    }
+  return rc;
+}
+
+// What a tight plan does without is given back (slot 4: the exact path's lists).
+inline void drop_lists(fknn_index *idx) {
+  cudaGetLastError();  // (a refused allocation is not this call's error)
+  for (int slot : {4, 6, 7, 11}) ws_drop(idx, slot);
+}
+
 // the trim holds a whole list in registers: 32 x NPL >= capb
 template <class F>
 static void (*screen_kernel(uint32_t capb))(ScreenArgs) {
@@ -1175,7 +1203,7 @@ static void launch_screens(K screen, ScreenArgs X, SeedArgs Z, const TcState &S,
     Z.out = X.out;
     Z.out_cnt = X.out_cnt;
     Z.tq = BQ;
-    Z.list_cap = X.capb;
+    Z.list_cap = X.ocap;
     Z.blk_rows = BR;
     Z.stride = stride;
     Z.k = kprime;
@@ -1217,15 +1245,35 @@ static int search_tc(fknn_index *idx, const float *d_q, const float *d_meta, uin
   shape.tq = BQ;
   shape.blk_rows = BR;
   shape.small_slab = SMALL_SLAB;
-  // candidate scratch (items x 128 x capb x 8 B) stays within ~8 GB
-  const uint64_t per_item = (uint64_t)BQ * capb * sizeof(Candidate);
-  const uint64_t tiles_est = std::max<uint64_t>(1, (nq + BQ - 1) / BQ);
-  shape.max_items_per_tile = max_items(capb, tune.pilot_stride, per_item, tiles_est);
   shape.min_chunk_blocks = (tune.min_chunk_blocks + 1) / 2;  // (given in 128-row blocks)
-  shape.target_items = target_items(idx, tune, nq);
-  make_plan(h_desc, h_meta, nq, n, shape, P);
+  const uint64_t tiles_est = std::max<uint64_t>(1, (nq + BQ - 1) / BQ);
+  Candidate *d_out = nullptr, *d_work = nullptr;
+  uint32_t *d_ocnt = nullptr, *d_state, nitems = 0, sgrid = 0, ocap = capb, halves = 1;
+  unsigned char *d_at = nullptr, *d_blob;
+  float2 *d_lqs = nullptr;
+  if ((rc = ws_get(idx, 5, TcState::bytes(nq), (void **)&d_state))) return rc;
+  for (int tight = 0;; ++tight) {
+    // results (items x 256 x ocap x 8 B) stay within ~8 GB
+    ocap = tight ? tight_cap(kprime, capb) : capb;
+    const uint64_t per_item = (uint64_t)BQ * ocap * sizeof(Candidate);
+    shape.max_items_per_tile = tight ? 1u : max_items(capb, tune.pilot_stride, per_item, tiles_est);
+    shape.target_items = tight ? 1u : target_items(idx, tune, nq);
+    make_plan(h_desc, h_meta, nq, n, shape, P);
+    nitems = (uint32_t)P.items.size();
+    for (const Tile &t : P.tiles)
+      if (t.nq > (uint32_t)BM) halves = 2;
+    if (!nitems) break;
+    // (the lists last: when tight, they take what is left)
+    rc = ws_get(idx, 3, plan_blob_bytes(P), (void **)&d_blob);
+    if (!rc) rc = ws_get(idx, 4, P.tiles.size() * 2 * TA, (void **)&d_at);
+    if (!rc) rc = ws_get(idx, 10, P.tiles.size() * BQ * sizeof(float2), (void **)&d_lqs);
+    if (!rc) rc = list_scratch(idx, nitems, halves, capb, ocap, tight, &d_out, &d_ocnt, &d_work, &sgrid);
+    if (!rc) break;
+    if (rc != FKNN_ENOMEM || tight) return rc;
+    drop_lists(idx);
+  }
   auto t1 = std::chrono::steady_clock::now();
-  const uint32_t ntile = (uint32_t)P.tiles.size(), nitems = (uint32_t)P.items.size();
+  const uint32_t ntile = (uint32_t)P.tiles.size();
   const uint32_t nbig = (uint32_t)P.big.size(), nsmall = (uint32_t)P.small.size();
   std::vector<uint32_t> &slot = P.w_slot;
   slot.resize(nitems);
@@ -1246,7 +1294,7 @@ static int search_tc(fknn_index *idx, const float *d_q, const float *d_meta, uin
                o_items = take(nitems * sizeof(WorkItem)), o_lq = take((size_t)ntile * BQ * 4),
                o_ls = take((size_t)ntile * BQ * 4), o_le = take((size_t)ntile * BQ * 4), o_slot = take(nitems * 4);
   const size_t blob = off;
-  unsigned char *h_blob, *d_blob;
+  unsigned char *h_blob;
   if ((rc = hs_get(idx, 3, blob + 256, (void **)&h_blob))) return rc;
   if ((rc = ws_get(idx, 3, blob + 256, (void **)&d_blob))) return rc;
   auto put = [&](size_t o, const void *src, size_t bytes) {
@@ -1263,8 +1311,6 @@ static int search_tc(fknn_index *idx, const float *d_q, const float *d_meta, uin
   put(o_le, P.lane_e.data(), (size_t)ntile * BQ * 4);
   put(o_slot, slot.data(), nitems * 4);
   if (blob) FKNN_CUDA(cudaMemcpyAsync(d_blob, h_blob, blob, cudaMemcpyHostToDevice, st));
-  uint32_t *d_state;
-  if ((rc = ws_get(idx, 5, TcState::bytes(nq), (void **)&d_state))) return rc;
   const TcState S(d_state, nq);
   if ((rc = S.reset(nq, st))) return rc;
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -1272,16 +1318,6 @@ static int search_tc(fknn_index *idx, const float *d_q, const float *d_meta, uin
     for (auto &e : ev) FKNN_CUDA(cudaEventCreate(&e));
   const OrderData &OT = idx->ord[ORDER_TIME], &OC = idx->ord[ORDER_CAT];
   if (nitems) {
-    unsigned char *d_at;
-    Candidate *d_out, *d_work;
-    uint32_t *d_ocnt;
-    float2 *d_lqs;
-    if ((rc = ws_get(idx, 4, (size_t)ntile * 2 * TA, (void **)&d_at))) return rc;
-    if ((rc = ws_get(idx, 10, (size_t)ntile * BQ * sizeof(float2), (void **)&d_lqs))) return rc;
-    if ((rc = ws_get(idx, 6, (size_t)nitems * per_item, (void **)&d_out))) return rc;
-    const uint32_t sgrid = std::min<uint32_t>(nitems, (uint32_t)idx->num_sms);
-    if ((rc = ws_get(idx, 11, (size_t)sgrid * 2 * B_LISTS * capb * sizeof(Candidate), (void **)&d_work))) return rc;
-    if ((rc = ws_get(idx, 7, (size_t)nitems * BQ * 4, (void **)&d_ocnt))) return rc;
     LaneSrc ls;
     ls.lane_q = (const int32_t *)(d_blob + o_lq);
     ls.lane_s = (const uint32_t *)(d_blob + o_ls);
@@ -1315,6 +1351,8 @@ static int search_tc(fknn_index *idx, const float *d_q, const float *d_meta, uin
     X.out_cnt = d_ocnt;
     X.work = d_work;
     X.capb = capb;
+    X.ocap = ocap;
+    X.halves = halves;
     X.nitems = nitems;
     X.nitems_d = nullptr;
     X.order = nullptr;
@@ -1349,7 +1387,7 @@ static int search_tc(fknn_index *idx, const float *d_q, const float *d_meta, uin
     A.ovf_count = S.ovf_count;
     A.k = k;
     A.kprime = kprime;
-    A.capb = capb;
+    A.capb = ocap;
     A.seeded = stride > 1 ? S.seeded : nullptr;
     A.ids = d_ids;
     A.dists = d_dists;
@@ -1415,33 +1453,36 @@ static int search_tc_graph(fknn_index *idx, const float *d_q, const float *d_met
   shape.blk_rows = BR;
   shape.small_slab = SMALL_SLAB;
   shape.min_chunk_blocks = (tune.min_chunk_blocks + 1) / 2;  // (given in 128-row blocks)
-  shape.target_items = target_items(idx, tune, nq);
-  DevPlanSizes z = device_plan_sizes(idx, nq, shape);
-  const uint64_t per_item = (uint64_t)BQ * capb * sizeof(Candidate);
-  shape.max_items_per_tile = max_items(capb, tune.pilot_stride, per_item, z.ntile_max);
   // all buffers exist before the capture (a capture may not allocate)
   QueryDesc *d_desc;
   void *d_plan;
   unsigned char *d_at;
   float2 *d_lqs;
   Candidate *d_out, *d_work;
-  uint32_t *d_ocnt, *d_state;
+  uint32_t *d_ocnt, *d_state, sgrid, ocap;
+  DevPlanSizes z;
   if ((rc = ws_get(idx, 2, (size_t)nq * sizeof(QueryDesc), (void **)&d_desc))) return rc;
-  if ((rc = ws_get(idx, 19, device_plan_bytes(nq, z), &d_plan))) return rc;
-  if ((rc = ws_get(idx, 4, (size_t)z.ntile_max * 2 * TA, (void **)&d_at))) return rc;
-  if ((rc = ws_get(idx, 10, (size_t)z.ntile_max * BQ * sizeof(float2), (void **)&d_lqs))) return rc;
-  if ((rc = ws_get(idx, 6, (size_t)z.nitems_max * per_item, (void **)&d_out))) return rc;
-  const unsigned sgrid = std::min<uint32_t>(z.nitems_max, (uint32_t)idx->num_sms);
-  if ((rc = ws_get(idx, 11, (size_t)sgrid * 2 * B_LISTS * capb * sizeof(Candidate), (void **)&d_work))) return rc;
-  if ((rc = ws_get(idx, 7, (size_t)z.nitems_max * BQ * 4, (void **)&d_ocnt))) return rc;
   if ((rc = ws_get(idx, 5, TcState::bytes(nq), (void **)&d_state))) return rc;
+  for (int tight = 0;; ++tight) {
+    ocap = tight ? tight_cap(kprime, capb) : capb;
+    shape.target_items = tight ? 1u : target_items(idx, tune, nq);
+    z = device_plan_sizes(idx, nq, shape);
+    shape.max_items_per_tile =
+        tight ? 1u : max_items(capb, tune.pilot_stride, (uint64_t)BQ * ocap * sizeof(Candidate), z.ntile_max);
+    void *h;  // the radix sort's histogram slot at its largest: the plan sorts the queries and the work items
+    const size_t keys = std::max<size_t>(nq, z.nitems_max);
+    rc = ws_get(idx, 15, ((keys + 4095) / 4096) * 256 * sizeof(uint32_t) + 256, &h);
+    if (!rc) rc = ws_get(idx, 19, device_plan_bytes(nq, z), &d_plan);
+    if (!rc) rc = ws_get(idx, 4, (size_t)z.ntile_max * 2 * TA, (void **)&d_at);
+    if (!rc) rc = ws_get(idx, 10, (size_t)z.ntile_max * BQ * sizeof(float2), (void **)&d_lqs);
+    // (the lists last: when tight, they take what is left)
+    if (!rc) rc = list_scratch(idx, z.nitems_max, 2, capb, ocap, tight, &d_out, &d_ocnt, &d_work, &sgrid);
+    if (!rc) break;
+    if (rc != FKNN_ENOMEM || tight) return rc;
+    drop_lists(idx);
+  }
   const TcState S(d_state, nq);
   const uint32_t stride = tune.pilot_stride;
-  {  // the radix sort's histogram slot at its largest (the plan sorts nq keys)
-    void *h;
-    const size_t keys = std::max<size_t>(nq, z.nitems_max);  // ... and the work items
-    if ((rc = ws_get(idx, 15, ((keys + 4095) / 4096) * 256 * sizeof(uint32_t) + 256, &h))) return rc;
-  }
   DevPlan P;
   device_plan_layout(P, d_plan, nq, z);
   auto screen = screen_kernel<F>(capb);
@@ -1454,8 +1495,8 @@ static int search_tc_graph(fknn_index *idx, const float *d_q, const float *d_met
   const bool withhold = idx->test_withhold;
   idx->test_withhold = false;
   const std::vector<uint64_t> key = {
-      (uint64_t)F::kFP8, nq, k, kprime, capb, tune.list_slack, tune.items_per_sm, tune.min_chunk_blocks,
-      tune.bound_refresh, tune.pilot_stride, (uint64_t)withhold, (uint64_t)(uintptr_t)d_q, (uint64_t)(uintptr_t)d_meta,
+      (uint64_t)F::kFP8, nq, k, kprime, capb, ocap, sgrid, shape.target_items, tune.list_slack,
+      tune.items_per_sm, tune.min_chunk_blocks, tune.bound_refresh, tune.pilot_stride, (uint64_t)withhold, (uint64_t)(uintptr_t)d_q, (uint64_t)(uintptr_t)d_meta,
       (uint64_t)(uintptr_t)d_ids, (uint64_t)(uintptr_t)d_dists, (uint64_t)(uintptr_t)d_desc,
       (uint64_t)(uintptr_t)d_plan, (uint64_t)(uintptr_t)d_at, (uint64_t)(uintptr_t)d_lqs, (uint64_t)(uintptr_t)d_out,
       (uint64_t)(uintptr_t)d_work,
@@ -1514,7 +1555,9 @@ static int search_tc_graph(fknn_index *idx, const float *d_q, const float *d_met
       X.out_cnt = d_ocnt;
       X.work = d_work;
       X.capb = capb;
-        X.nitems = 0;
+      X.ocap = ocap;
+      X.halves = 2;
+      X.nitems = 0;
       X.nitems_d = P.cnt + DP_NITEMS;
       X.order = P.ord_val;
       X.err = idx->d_flag;
@@ -1547,7 +1590,7 @@ static int search_tc_graph(fknn_index *idx, const float *d_q, const float *d_met
       A.ovf_count = S.ovf_count;
       A.k = k;
       A.kprime = kprime;
-      A.capb = capb;
+      A.capb = ocap;
       A.seeded = stride > 1 ? S.seeded : nullptr;
       A.ids = d_ids;
       A.dists = d_dists;

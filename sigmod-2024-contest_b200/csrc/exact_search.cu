@@ -1002,7 +1002,9 @@ int search_exact(fknn_index *idx, const float *d_q, const float *d_meta, uint32_
   // at four; 1e4 queries over 1e5 rows: 3.5 and 3.2 ms).
   const uint32_t ips = nq < 1024 ? 1u : idx->tuning[FKNN_MODE_EXACT_FP32].items_per_sm;
   Candidate *d_out = nullptr, *d_work = nullptr;
-  uint32_t *d_ocnt = nullptr, sgrid = 0, nitems = 0;
+  uint32_t *d_ocnt = nullptr, *d_state, sgrid = 0, nitems = 0;
+  unsigned char *d_blob;
+  if ((rc = ws_get(idx, 5, (size_t)nq * 36 + 64, (void **)&d_state))) return rc;
   // Where the index's HBM budget (or the memory left) does not hold the lists
   // of that many items and a working set for every SM, one item per tile and
   // as many CTAs as fit.
@@ -1011,7 +1013,9 @@ int search_exact(fknn_index *idx, const float *d_q, const float *d_meta, uint32_
     make_plan(h_desc, h_meta, nq, n, shape, P);
     nitems = (uint32_t)P.items.size();
     if (!nitems) break;
-    rc = ws_get(idx, 6, (size_t)nitems * EXACT_TQ * EXACT_CAP * sizeof(Candidate), (void **)&d_out);
+    // (the lists last: when tight, they take what is left)
+    rc = ws_get(idx, 3, plan_blob_bytes(P), (void **)&d_blob);
+    if (!rc) rc = ws_get(idx, 6, (size_t)nitems * EXACT_TQ * EXACT_CAP * sizeof(Candidate), (void **)&d_out);
     if (!rc) rc = ws_get(idx, 7, (size_t)nitems * EXACT_TQ * 4, (void **)&d_ocnt);
     if (!rc)
       for (sgrid = std::min<uint32_t>(nitems, (uint32_t)idx->num_sms);; sgrid = (sgrid + 1) / 2) {
@@ -1022,7 +1026,7 @@ int search_exact(fknn_index *idx, const float *d_q, const float *d_meta, uint32_
     if (!rc) break;
     if (rc != FKNN_ENOMEM || tight) return rc;
     cudaGetLastError();  // (a refused allocation is not this call's error)
-    for (int slot : {4, 6, 7}) ws_drop(idx, slot);
+    for (int slot : {4, 6, 7, 11}) ws_drop(idx, slot);
   }
   auto t1 = std::chrono::steady_clock::now();
   const uint32_t ntile = (uint32_t)P.tiles.size();
@@ -1051,7 +1055,7 @@ int search_exact(fknn_index *idx, const float *d_q, const float *d_meta, uint32_
                o_lq = take((size_t)ntile * EXACT_TQ * 4), o_ls = take((size_t)ntile * EXACT_TQ * 4),
                o_le = take((size_t)ntile * EXACT_TQ * 4), o_slot = take(nitems * 4);
   const size_t blob = off;
-  unsigned char *h_blob, *d_blob;
+  unsigned char *h_blob;
   if ((rc = hs_get(idx, 3, blob + 256, (void **)&h_blob))) return rc;
   if ((rc = ws_get(idx, 3, blob + 256, (void **)&d_blob))) return rc;
   auto put = [&](size_t o, const void *src, size_t bytes) {
@@ -1071,8 +1075,6 @@ int search_exact(fknn_index *idx, const float *d_q, const float *d_meta, uint32_
 
   // per-query state: bound, not-screened flag, overflow list; pilot bound
   // and flag; redo flag and list; spill lists of the two merges; then counts
-  uint32_t *d_state;
-  if ((rc = ws_get(idx, 5, (size_t)nq * 36 + 64, (void **)&d_state))) return rc;
   uint32_t *T_global = d_state, *ovf = d_state + nq, *ovf_list = d_state + 2 * (size_t)nq,
            *T_pilot = d_state + 3 * (size_t)nq, *ovf_p = d_state + 4 * (size_t)nq,
            *redo_skip = d_state + 5 * (size_t)nq, *redo_list = d_state + 6 * (size_t)nq,

@@ -158,6 +158,11 @@ struct Plan {
     pairs_screened = pairs_passing = pairs_contraction = 0;
   }
 };
+// At least what the plan's arrays, uploaded as one blob, take (every array on a 256-byte boundary).
+inline size_t plan_blob_bytes(const Plan &P) {
+  return P.small.size() * 4 + P.big.size() * 12 + P.tiles.size() * sizeof(Tile) +
+         P.items.size() * (sizeof(WorkItem) + 4) + P.lane_q.size() * 12 + 11 * 256;
+}
 
 struct PlanShape {
   int tq;                   // queries per tile

@@ -88,3 +88,26 @@ def test_nearer_row_beyond_the_slab(mode):
             np.testing.assert_array_equal(gd, dists)  # (rows at the same distance as the k-th may differ in bf16)
             if mode == "exact":
                 np.testing.assert_array_equal(got, ids)
+
+
+@pytest.mark.parametrize("room_mb", [16, 64])
+@pytest.mark.parametrize("mode", [fknn.MODE_BF16_RERANK, fknn.MODE_FP8_RERANK])
+def test_small_hbm_budget(room_mb, mode):
+    """With little scratch a tile is one item, its results hold k' entries and
+    a few ties, and fewer CTAs run; the answers are the same."""
+    rng = np.random.default_rng(11)
+    n, nq = 30_011, 600
+    vecs, q = grid(rng, (n, 100)), grid(rng, (nq, 100))
+    labels, ts = np.zeros(n, np.float32), rng.random(n, dtype=np.float32)
+    metas = np.full((nq, 4), -1, np.float32)
+    metas[:, 0] = 0
+    form = {"build_bf16": True} if mode == fknn.MODE_BF16_RERANK else {"build_fp8": True}
+    with fknn.Index(vecs, labels, ts, **form) as idx:
+        size = idx.device_bytes
+        want, want_d = idx.search(q, metas, k=100, mode=mode, kprime=128)
+    with fknn.Index(vecs, labels, ts, hbm_budget=size + (room_mb << 20), **form) as idx:
+        for graph in (False, True):
+            for m in (1, nq):
+                got, d = idx.search(q[:m], metas[:m], k=100, mode=mode, kprime=128, graph=graph)
+                np.testing.assert_array_equal(got, want[:m])
+                np.testing.assert_array_equal(d, want_d[:m])
