@@ -39,6 +39,7 @@ constexpr int X_NORMS = 8;                    // sub-tiles whose norms are kept 
 constexpr int X_GROUPS = 2;                   // accumulators, each with a group of epilogue warps
 constexpr int X_EPI_WARPS = 4;                // warps of a group: TMEM lanes 32 w ..
 constexpr int X_EPI = X_GROUPS * X_EPI_WARPS; // warps 0 .. 7
+static_assert(X_EPI * 32 == XQ, "an epilogue thread per query of a tile");
 constexpr int X_CONV_WARPS = 6;               // warps 8 .. 13
 constexpr int X_UNITS = (BLK / 32) * 13;      // converter units of a block: 32 rows x 8 dims
 constexpr int X_LOAD_WARP = X_EPI + X_CONV_WARPS;
@@ -677,6 +678,8 @@ __global__ void __launch_bounds__(X_THREADS, 1) k_exact_screen(ExactScreenArgs A
             x_finish<X_GROUPS * X_NPL>(work, sm, Lb, XM + Lb, A.k, A.T_global, A.ovf, A.out + o * EXACT_CAP,
                                        A.out_cnt + o);
         }
+      } else {
+        A.out_cnt[(uint64_t)item_id * XQ + tid] = 0;  // read all the same: by the seeds, which know no marks
       }
     }
     g += nsub;

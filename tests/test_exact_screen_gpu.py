@@ -96,3 +96,29 @@ def test_low_seeds_are_screened_again():
 def test_small_hbm_budget(room_mb):
     vecs, labels, ts, q, metas = datagen.make_workload(1, n=60000, nq=64)
     check(vecs, labels, ts, q, metas, budget_room=room_mb << 20)
+
+
+def test_items_of_marked_queries():
+    """A category of equal rows: the first items' pilot lists overflow and mark
+    their queries, and the later items of those tiles (more items than the GPU
+    takes at once) are skipped; the seeds still read every item's counts, which
+    an earlier search of the other kind left behind."""
+    rng = np.random.default_rng(11)
+    n, same, nq = 20000, 12000, 10000
+    vecs = rng.standard_normal((n, 100), dtype=np.float32)
+    vecs[:same] = vecs[0]
+    labels = np.where(np.arange(n) < same, 3, 4).astype(np.float32)
+    ts = rng.random(n, dtype=np.float32)
+    q = rng.standard_normal((nq, 100), dtype=np.float32)
+    metas = np.tile(np.array([1, 3, -1, -1], np.float32), (nq, 1))
+    with fknn.Index(vecs, labels, ts, build_bf16=True) as idx:
+        idx.set_tuning(fknn.MODE_EXACT_FP32, items_per_sm=4, min_chunk_blocks=16, pilot_stride=2)
+        other = metas[:2000].copy()
+        other[:, :2] = (0, -1)
+        idx.search(q[:2000], other, mode=fknn.MODE_BF16_RERANK, kprime=200)
+        ids, dists, st = idx.search(q, metas, return_stats=True)
+    assert st["n_work_items"] > 148 and st["n_overflow"] == nq
+    # equal distances: the order is the ids'
+    np.testing.assert_array_equal(ids, np.tile(np.arange(100, dtype=np.uint32), (nq, 1)))
+    _, odists = oracle.exact_knn(vecs, labels, ts, q[:50], metas[:50])
+    np.testing.assert_array_equal(dists[:50], odists)
