@@ -405,8 +405,10 @@ __global__ void __launch_bounds__(ES_THREADS)
       sm.thr = ~0ull;
     }
     __syncthreads();
+    int held = 0;  // keys in buf: counted at the step's barrier, for sm.cnt grows again as soon as a warp has passed it
     for (uint64_t base = dsc.s; base < dsc.e; base += ES_THREADS) {
       const uint64_t p = base + tid;
+      bool push = false;
       if (p < dsc.e) {
         const float *x = blocks + (p / BLK) * BLK_FLOATS + (p % BLK);
         const uint32_t id = perm[p];
@@ -424,11 +426,12 @@ __global__ void __launch_bounds__(ES_THREADS)
           }
         }
         const uint64_t key = exact_key(r, id);
-        if (key < sm.thr) sm.buf[atomicAdd(&sm.cnt, 1)] = key;
+        push = key < sm.thr;
+        if (push) sm.buf[atomicAdd(&sm.cnt, 1)] = key;
       }
-      __syncthreads();
-      if (sm.cnt > ES_CAP - ES_THREADS && base + ES_THREADS < dsc.e) {
-        scan_select(sm, sm.cnt, k);
+      held += __syncthreads_count(push);
+      if (held > ES_CAP - ES_THREADS && base + ES_THREADS < dsc.e) {  // (block-uniform)
+        scan_select(sm, held, k);
         uint64_t mx = 0;
         for (uint32_t i = tid; i < k; i += ES_THREADS) {
           sm.buf[i] = sm.sel[i];
@@ -442,10 +445,11 @@ __global__ void __launch_bounds__(ES_THREADS)
         atomicMax(&sm.mx, (unsigned long long)mx);
         __syncthreads();
         if (tid == 0) sm.thr = sm.mx;
+        held = (int)k;
         __syncthreads();
       }
     }
-    int c = sm.cnt;
+    int c = held;
     const uint64_t *keys = sm.buf;
     if (c > (int)k) {
       scan_select(sm, c, k);

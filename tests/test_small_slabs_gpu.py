@@ -63,3 +63,40 @@ def test_ends_in_tables_of_any_length(n):
     metas[:, 2:] = np.sort(ts[rng.integers(0, n, (200, 2))], axis=1)
     with fknn.Index(vecs, labels, ts) as idx:
         np.testing.assert_array_equal(idx.count_matches(metas), oracle.count_matches(labels, ts, metas))
+
+
+@pytest.mark.parametrize("rows", [3584, 3585, 4096])
+def test_many_scans_at_the_edge_of_the_key_buffer(rows):
+    """Slabs whose last step may or may not be the one before a selection, in
+    every block several times over: all warps of a block decide alike."""
+    rng = np.random.default_rng(rows)
+    vecs = rng.standard_normal((rows + 500, 100), dtype=np.float32)
+    labels = (np.arange(rows + 500) >= rows).astype(np.float32)
+    ts = rng.random(rows + 500, dtype=np.float32)
+    q = rng.standard_normal((3000, 100), dtype=np.float32)
+    metas = np.tile(np.array([1, 0, -1, -1], np.float32), (3000, 1))
+    with fknn.Index(vecs, labels, ts) as idx:
+        ids, dists = idx.search(q, metas, k=100)
+        oids, odists = oracle.exact_knn(vecs, labels, ts, q, metas, k=100)
+        np.testing.assert_array_equal(ids, oids)
+        np.testing.assert_array_equal(dists, odists)
+
+
+def test_scans_that_select_many_times():
+    """Near-ties that no candidate list holds: slabs of several buffers are
+    scanned, with a bound that falls from one selection to the next."""
+    rng = np.random.default_rng(3)
+    n = 30_000
+    vecs = np.repeat(rng.standard_normal((1, 100), dtype=np.float32), n, axis=0)
+    vecs *= (1 + np.linspace(1e-5, 0, n, dtype=np.float32))[:, None]
+    labels = (np.arange(n) >= 9000).astype(np.float32)
+    ts = np.linspace(0, 1, n, dtype=np.float32)
+    q = rng.standard_normal((400, 100), dtype=np.float32)
+    metas = np.zeros((400, 4), np.float32)
+    metas[:, 0] = np.arange(400) % 2
+    with fknn.Index(vecs, labels, ts) as idx:
+        ids, dists, st = idx.search(q, metas, k=100, return_stats=True)
+        assert st["n_overflow"] == 400
+        oids, odists = oracle.exact_knn(vecs, labels, ts, q, metas, k=100)
+        np.testing.assert_array_equal(ids, oids)
+        np.testing.assert_array_equal(dists, odists)
