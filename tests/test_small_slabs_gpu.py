@@ -100,3 +100,22 @@ def test_scans_that_select_many_times():
         oids, odists = oracle.exact_knn(vecs, labels, ts, q, metas, k=100)
         np.testing.assert_array_equal(ids, oids)
         np.testing.assert_array_equal(dists, odists)
+
+
+def test_more_queries_than_32_bit_threads_number():
+    """2^27 queries of a warp each have 2^32 threads: the ones past that are
+    counted too."""
+    import torch
+    rng = np.random.default_rng(5)
+    vecs = rng.standard_normal((300, 100), dtype=np.float32)
+    labels = (np.arange(300) % 3).astype(np.float32)
+    nq = (1 << 27) + 9
+    metas = torch.zeros((nq, 4), device="cuda")
+    metas[-9:, 0] = 1
+    metas[-9:, 1] = torch.arange(9, device="cuda") % 4
+    counts = torch.full((nq,), -1, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    with fknn.Index(vecs, labels, rng.random(300, dtype=np.float32)) as idx:
+        assert fknn._lib.load().fknn_count_matches(idx._h, metas.data_ptr(), nq, counts.data_ptr(), None) == 0
+    assert bool((counts[:-9] == 300).all())
+    assert counts[-9:].tolist() == [100, 100, 100, 0] * 2 + [100]
