@@ -253,7 +253,7 @@ int make_index_view(fknn_index *base, fknn_index **out) {
   v->fp8_scale = base->fp8_scale;
   for (int m = 0; m < 3; ++m) v->tuning[m] = base->tuning[m];
   v->num_sms = base->num_sms;
-  v->n_labels = base->n_labels;
+  v->n_large_labels = base->n_large_labels;
   v->is_view = true;
   cudaError_t e = cudaSetDevice(v->device);
   if (e == cudaSuccess) e = cudaMalloc(&v->d_flag, 64);

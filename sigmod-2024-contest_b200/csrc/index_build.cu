@@ -196,11 +196,11 @@ __global__ void k_build_blocks(const float *__restrict__ vecs, const uint32_t *_
   }
 }
 
-// distinct labels: starts of the label runs of the category order
-__global__ void k_label_runs(const int32_t *__restrict__ lab, uint64_t n, uint32_t *__restrict__ count) {
+// labels of more than SMALL_SLAB rows: starts of the long label runs of the category order
+__global__ void k_large_labels(const int32_t *__restrict__ lab, uint64_t n, uint32_t *__restrict__ count) {
   uint32_t c = 0;
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-    c += (i == 0 || lab[i] != lab[i - 1]) ? 1u : 0u;
+    c += (i == 0 || lab[i] != lab[i - 1]) && i + SMALL_SLAB < n && lab[i + SMALL_SLAB] == lab[i] ? 1u : 0u;
   if (c) atomicAdd(count, c);
 }
 
@@ -300,14 +300,12 @@ int build_index_from_columns(fknn_index *idx, cudaStream_t st) {
     g_launches += 2;
   }
   FKNN_CUDA(cudaMemsetAsync(idx->d_flag, 0, sizeof(int), st));
-  k_label_runs<<<148 * 4, 256, 0, st>>>(idx->ord[ORDER_CAT].label, n, reinterpret_cast<uint32_t *>(idx->d_flag));
+  k_large_labels<<<148 * 4, 256, 0, st>>>(idx->ord[ORDER_CAT].label, n, reinterpret_cast<uint32_t *>(idx->d_flag));
   g_launches += 1;
   FKNN_CUDA(cudaGetLastError());
-  uint32_t runs = 0;
-  FKNN_CUDA(cudaMemcpyAsync(&runs, idx->d_flag, 4, cudaMemcpyDeviceToHost, st));
+  FKNN_CUDA(cudaMemcpyAsync(&idx->n_large_labels, idx->d_flag, 4, cudaMemcpyDeviceToHost, st));
   FKNN_CUDA(cudaMemsetAsync(idx->d_flag, 0, sizeof(int), st));
   FKNN_CUDA(cudaStreamSynchronize(st));
-  idx->n_labels = runs ? runs : 1;
   return FKNN_OK;
 }
 

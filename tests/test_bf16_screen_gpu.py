@@ -111,3 +111,28 @@ def test_small_hbm_budget(room_mb, mode):
                 got, d = idx.search(q[:m], metas[:m], k=100, mode=mode, kprime=128, graph=graph)
                 np.testing.assert_array_equal(got, want[:m])
                 np.testing.assert_array_equal(d, want_d[:m])
+
+
+def test_captured_plan_of_many_short_categories():
+    """Categories too short for the contraction are no tiles of a captured
+    search: neither its scratch nor the cutting of its tiles depends on them."""
+    rng = np.random.default_rng(17)
+    n, nq, k = 60_000, 3000, 20
+    vecs, q = grid(rng, (n, 100)), grid(rng, (nq, 100))
+    labels = np.where(np.arange(n) < 20_000, 0, np.arange(n)).astype(np.float32)  # one long category, 40,000 of one row
+    ts = rng.random(n, dtype=np.float32)
+    metas = np.zeros((nq, 4), np.float32)
+    metas[:, 0] = np.arange(nq) % 4
+    metas[1::8, 1] = n - 1
+    metas[:, 3] = 0.9
+    with fknn.Index(vecs, labels, ts, build_bf16=True) as idx:
+        before = idx.device_bytes
+        ids, dists, st = idx.search(q, metas, k=k, mode=fknn.MODE_BF16_RERANK, kprime=1024, graph=True, return_stats=True)
+        assert st["n_work_items"] > 2 * st["n_tiles"]
+        assert idx.device_bytes - before < 3 << 30
+        want, want_d = idx.search(q, metas, k=k, mode=fknn.MODE_BF16_RERANK, kprime=1024)
+    np.testing.assert_array_equal(ids, want)
+    np.testing.assert_array_equal(dists, want_d)
+    got, got_d = oracle.exact_knn(vecs, labels, ts, q, metas, k=k)
+    np.testing.assert_array_equal(ids, got)
+    np.testing.assert_array_equal(dists, got_d)
