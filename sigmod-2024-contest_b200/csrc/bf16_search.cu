@@ -849,9 +849,9 @@ __global__ void __launch_bounds__(B_THREADS, 1) k_screen_tc(ScreenArgs A) {
 
 // ------------------------------------------------------------ re-rank --
 
-constexpr int RR_THREADS = 128;
+constexpr int RR_THREADS = 256;
 constexpr int RR_CAP = 8192;        // screening candidates the large merge holds
-constexpr int RR_CAP_SMALL = 1024;  // ... and the common one (12 blocks per SM)
+constexpr int RR_CAP_SMALL = 1024;  // ... and the common one (8 blocks per SM)
 constexpr int RR_KMAX = 1024;       // largest k'
 constexpr int RR_ITEMS = 256;       // work items of a tile (the lists' offsets)
 
