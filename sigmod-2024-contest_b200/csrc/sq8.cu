@@ -77,6 +77,8 @@ struct HeapNode {
 constexpr uint32_t SQ_PREFIX = 8192;    // codes replayed before the screen (multiple of 128)
 constexpr uint64_t SQ_GROW = 8;         // a part ends at this multiple of its first code
 constexpr int SQ_DQ = 32;               // queries of a block of k_sq8_dist
+constexpr uint64_t SQ_DIST_BYTES = 192ull << 20;  // prefix distances of a call made all at once, else ...
+constexpr uint32_t SQ_REPLAY_WARPS = 32;          // ... for as many queries per SM as k_sq8_prefix has resident
 constexpr int SQ_WARPS = 4;             // queries per block of the replay kernels
 constexpr int SQ_SCAN = 128;            // codes per warp step of the replay kernels
 constexpr uint32_t SQ_TILE = TC_ROWS * 128;  // 128 rows x 128 bytes (112 code bytes, 16 zero)
@@ -344,24 +346,30 @@ __global__ void __launch_bounds__(256) k_sq8_tiles(const int8_t *__restrict__ ro
 }
 
 // Distances of the first n codes (rows of stride n padded to SQ_SCAN in dist):
-// a thread per code, SQ_DQ queries of a block from shared memory.
+// a thread per code, SQ_DQ queries of a block from shared memory.  Bound by the
+// dot products: 28 per pair, |q|^2 and |c|^2 taken once a block (2,048 queries
+// over 8,192 codes, k = 140, whole call: 407 us with |q|^2 for every pair, 389
+// us now).
 __global__ void __launch_bounds__(SQ_SCAN)
-    k_sq8_dist(const int8_t *__restrict__ codes, const int *__restrict__ ncc, uint64_t n, uint64_t stride,
-               const int8_t *__restrict__ queries, uint32_t nq, int *__restrict__ dist) {
+    k_sq8_dist(const int8_t *__restrict__ codes, uint64_t n, uint64_t stride, const int8_t *__restrict__ queries,
+               uint32_t nq, int *__restrict__ dist) {
   __shared__ int4 qs[SQ_DQ][7];
+  __shared__ int qq[SQ_DQ];
   const uint32_t q0 = blockIdx.y * SQ_DQ, m = min((uint32_t)SQ_DQ, nq - q0);
   for (uint32_t i = threadIdx.x; i < m * 7; i += SQ_SCAN)
     qs[i / 7][i % 7] = __ldg(reinterpret_cast<const int4 *>(queries + (uint64_t)q0 * SQ8_CODE) + i);
   const uint64_t p = (uint64_t)blockIdx.x * SQ_SCAN + threadIdx.x;
   int4 c[7];
   load_code(codes, p, n, c);
-  const int cc = p < n ? -ncc[p] : 0;
+  const int cc = dot112(c, c);
+  __syncthreads();
+  if (threadIdx.x < m) qq[threadIdx.x] = dot112(qs[threadIdx.x], qs[threadIdx.x]);
   __syncthreads();
   for (uint32_t j = 0; j < m; ++j) {
     int4 qv[7];
 #pragma unroll
     for (int w = 0; w < 7; ++w) qv[w] = qs[j][w];
-    dist[(uint64_t)(q0 + j) * stride + p] = p < n ? dot112(qv, qv) + cc - 2 * dot112(c, qv) : INT_MAX;
+    dist[(uint64_t)(q0 + j) * stride + p] = p < n ? qq[j] + cc - 2 * dot112(c, qv) : INT_MAX;
   }
 }
 
@@ -828,10 +836,19 @@ struct Sq8Pass {
   size_t lists, counts, bytes;
 };
 
+// The prefix's distances: entries of a query, and the queries at a time.  A
+// call of many queries makes them for as many as are replayed together, which
+// bounds the scratch: 155 MB in place of 268 for 8,192 queries and codes, at
+// 1,187 us as before (k = 140).
+size_t sq8_dist_stride(uint64_t prefix) { return (size_t)((prefix + SQ_SCAN - 1) / SQ_SCAN * SQ_SCAN); }
+uint32_t sq8_dist_queries(uint32_t nqb, uint64_t prefix, int num_sms) {
+  return nqb * sq8_dist_stride(prefix) * 4 <= SQ_DIST_BYTES ? nqb : std::min(nqb, (uint32_t)num_sms * SQ_REPLAY_WARPS);
+}
+
 Sq8Pass sq8_pass(uint32_t nqb, uint64_t npoints, uint64_t prefix, size_t k, int num_sms) {
   Sq8Pass p{};
   p.nqt = (nqb + TC_ROWS - 1) / TC_ROWS;
-  p.lists = (size_t)nqb * ((prefix + SQ_SCAN - 1) / SQ_SCAN * SQ_SCAN) * 4;
+  p.lists = sq8_dist_queries(nqb, prefix, num_sms) * sq8_dist_stride(prefix) * 4;
   for (uint64_t r0 = prefix; r0 < npoints;) {
     const Sq8Part a = sq8_part(r0, npoints, p.nqt, k, num_sms);
     p.lists = std::max(p.lists, (size_t)nqb * a.nseg * a.cap * sizeof(int2));
@@ -891,7 +908,7 @@ int sq8_bf_impl(size_t k, int *closest, float *dists, size_t npoints, const char
   const size_t b_q = q_dev ? 0 : al256(nqueries * SQ8_CODE);
   const size_t b_ids = ids_dev ? 0 : al256(nqueries * k * 4);
   const size_t b_d = (!dists || d_dev) ? 0 : al256(nqueries * k * 4);
-  const size_t codes_bytes = al256((size_t)nct_all * SQ_TILE) + al256((size_t)nct_all * TC_ROWS * 4);
+  const size_t codes_bytes = screened ? al256((size_t)nct_all * SQ_TILE) + al256((size_t)nct_all * TC_ROWS * 4) : 0;
   const size_t need = b_codes + b_q + b_ids + b_d + codes_bytes + std::max(pa.bytes, pb.bytes) + 256;
 
   if (scr.bytes < need) {
@@ -925,10 +942,14 @@ int sq8_bf_impl(size_t k, int *closest, float *dists, size_t npoints, const char
   int *d_err = reinterpret_cast<int *>(base + codes_bytes + std::max(pa.bytes, pb.bytes));
 
   const size_t rsmem = (size_t)SQ_WARPS * sq_region(K) * sizeof(HeapNode);
-  FKNN_CUDA(cudaMemsetAsync(d_err, 0, sizeof(int), st));
-  // |c|^2 of every code (the replay kernels use it too) and the tiles
-  k_sq8_tiles<<<nct_all, 256, 0, st>>>(d_codes, npoints, 0, 0, ctiles, cncc);
-  g_launches += 2;
+  if (screened) {
+    FKNN_CUDA(cudaMemsetAsync(d_err, 0, sizeof(int), st));
+    // |c|^2 of every code (the tail uses it too) and the tiles.  A slab that is
+    // replayed whole needs neither, nor an error flag (2,048 queries over 2,000
+    // codes, k = 140: 256 us with them, 240 without)
+    k_sq8_tiles<<<nct_all, 256, 0, st>>>(d_codes, npoints, 0, 0, ctiles, cncc);
+    g_launches += 1;
+  }
   for (uint32_t q0 = 0; q0 < nq; q0 += qbatch) {
     const uint32_t nqb = std::min(qbatch, nq - q0);
     const Sq8Pass ps = sq8_pass(nqb, npoints, prefix, k, num_sms);
@@ -950,12 +971,18 @@ int sq8_bf_impl(size_t k, int *closest, float *dists, size_t npoints, const char
     int *ids = d_ids + (uint64_t)q0 * k;
     float *dd = d_d ? d_d + (uint64_t)q0 * k : nullptr;
     const unsigned rblocks = (nqb + SQ_WARPS - 1) / SQ_WARPS;
-    const uint64_t steps = (prefix + SQ_SCAN - 1) / SQ_SCAN;
-    k_sq8_dist<<<dim3((unsigned)steps, (nqb + SQ_DQ - 1) / SQ_DQ), SQ_SCAN, 0, st>>>(
-        d_codes, cncc, prefix, steps * SQ_SCAN, qs, nqb, static_cast<int *>(lists));
-    k_sq8_prefix<<<rblocks, SQ_WARPS * 32, rsmem, st>>>(static_cast<int *>(lists), prefix, steps * SQ_SCAN, nqb, K,
-                                                        screened ? 0 : 1, heaps, T, ids, dd, alpha);
-    g_launches += 2;
+    int *dist = static_cast<int *>(lists);
+    const size_t stride = sq8_dist_stride(prefix);
+    const uint32_t dq = sq8_dist_queries(nqb, prefix, num_sms);
+    for (uint32_t c0 = 0; c0 < nqb; c0 += dq) {
+      const uint32_t m = std::min(nqb - c0, dq);
+      k_sq8_dist<<<dim3((unsigned)(stride / SQ_SCAN), (m + SQ_DQ - 1) / SQ_DQ), SQ_SCAN, 0, st>>>(
+          d_codes, prefix, stride, qs + (uint64_t)c0 * SQ8_CODE, m, dist);
+      k_sq8_prefix<<<(m + SQ_WARPS - 1) / SQ_WARPS, SQ_WARPS * 32, rsmem, st>>>(
+          dist, prefix, stride, m, K, screened ? 0 : 1, heaps + (uint64_t)c0 * (k + 1), T + c0, ids + (uint64_t)c0 * k,
+          dd ? dd + (uint64_t)c0 * k : nullptr, alpha);
+      g_launches += 2;
+    }
     if (screened) {
       k_sq8_tiles<<<ps.nqt, 256, 0, st>>>(qs, nqb, 0, 1, qtiles, qncc);
       g_launches += 1;
@@ -980,7 +1007,7 @@ int sq8_bf_impl(size_t k, int *closest, float *dists, size_t npoints, const char
   if (!ids_dev) FKNN_CUDA(cudaMemcpyAsync(closest, d_ids, nqueries * k * 4, cudaMemcpyDeviceToHost, st));
   if (dists && !d_dev) FKNN_CUDA(cudaMemcpyAsync(dists, d_d, nqueries * k * 4, cudaMemcpyDeviceToHost, st));
   int err = 0;
-  FKNN_CUDA(cudaMemcpyAsync(&err, d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
+  if (screened) FKNN_CUDA(cudaMemcpyAsync(&err, d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
   FKNN_CUDA(cudaStreamSynchronize(st));
   if (err & ERR_WAIT_TIMEOUT) {
     // outputs are complete (the affected queries took the exact scan)

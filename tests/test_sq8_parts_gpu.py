@@ -52,3 +52,48 @@ def test_rows_that_come_nearer_fill_the_lists(npoints):
     vecs = q[:1] + far * rng.standard_normal((npoints, 100), dtype=np.float32)
     alpha, codes = oracle.sq8_sym_train(vecs)
     check(codes, alpha, oracle.sq8_sym_encode(q, alpha), 140)
+
+
+@pytest.mark.parametrize("npoints", [300, 9000])
+def test_more_queries_than_are_replayed_at_once(npoints):
+    rng = np.random.default_rng(npoints)
+    alpha, codes = oracle.sq8_sym_train(rng.standard_normal((npoints, 100), dtype=np.float32))
+    nq, k = 6200, 10  # 4,736 and 1,464 where the slab is long enough
+    qv = oracle.sq8_sym_encode(rng.standard_normal((nq, 100), dtype=np.float32), alpha)
+    ids = np.empty((nq, k), dtype=np.int32)
+    d = np.empty((nq, k), dtype=np.float32)
+    fknn.bruteforce_subgraph(100, k, ids, d, npoints, codes, alpha, nq, qv)
+    for i in [0, 1, 4735, 4736, 4737, *range(nq - 10, nq)]:
+        oi, od = oracle.sq8_bruteforce(k, codes, alpha, qv[i], with_dists=True)
+        np.testing.assert_array_equal(ids[i], oi, err_msg=f"query {i}")
+        np.testing.assert_array_equal(d[i], od)
+
+
+def test_scratch_of_a_short_slab_is_bounded():
+    """The prefix's distances are made for as many queries as are replayed at
+    once, however many the call has."""
+    import threading
+
+    import torch
+    n, nq, k = 8192, 8192, 10
+    g = torch.Generator(device="cuda")
+    g.manual_seed(1)
+    codes = torch.randint(-127, 128, (n, 112), generator=g, device="cuda", dtype=torch.int8)
+    q = torch.randint(-127, 128, (nq, 112), generator=g, device="cuda", dtype=torch.int8)
+    codes[:, 100:] = 0
+    q[:, 100:] = 0
+    out = torch.empty((nq, k), dtype=torch.int32, device="cuda")
+    d = torch.empty((nq, k), device="cuda")
+    torch.cuda.synchronize()
+    used = []
+
+    def call():  # a thread has a scratch of its own
+        before = torch.cuda.mem_get_info()[0]
+        fknn.bruteforce_subgraph(100, k, out, d, n, codes, 1.0, nq, q)
+        used.append(before - torch.cuda.mem_get_info()[0])
+        fknn._lib.load().fknn_sq8_release_thread_scratch()
+
+    t = threading.Thread(target=call)
+    t.start()
+    t.join()
+    assert used and used[0] < 180 << 20, used
