@@ -1215,7 +1215,7 @@ static void launch_screens(K screen, ScreenArgs X, SeedArgs Z, const TcState &S,
   X.T_global = S.T_global;
   X.ovf = S.ovf;
   X.kprime = kprime;
-  X.refresh = refresh;
+  X.refresh = (refresh + 1) / 2;  // (given in sub-tiles of 128 rows)
   X.stride = 1;
   X.withhold = withhold ? 1u : 0u;
   X.queue = S.queue + 1;

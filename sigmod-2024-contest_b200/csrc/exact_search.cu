@@ -1006,7 +1006,7 @@ int search_exact(fknn_index *idx, const float *d_q, const float *d_meta, uint32_
   const uint32_t pstride = idx->tuning[FKNN_MODE_EXACT_FP32].pilot_stride;
   const bool pilot = pstride > 1;
   shape.max_items_per_tile = pilot ? MAX_ITEMS_PER_TILE : MERGE_CAP / EXACT_CAP;
-  shape.min_chunk_blocks = idx->tuning[FKNN_MODE_EXACT_FP32].min_chunk_blocks;
+  shape.min_chunk_blocks = (idx->tuning[FKNN_MODE_EXACT_FP32].min_chunk_blocks + 1) / 2;  // (given in 64-row blocks)
   // Several items per SM even out tiles of unequal length; with few queries
   // there are few tiles, cut alike, and every further item only adds its own
   // start and end (16 queries over 1e6 rows: 0.82 ms at one item per SM, 1.29

@@ -280,7 +280,7 @@ struct fknn_index {
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   fknn::Plan plan;  // rebuilt by every search; capacity kept
   // per-mode plan / kernel parameters (fknn_index_set_tuning) and the SM count
-  fknn_tuning tuning[3] = {{0, 4, 16, 0, 32}, {256, 3, 8, 0, 8}, {256, 3, 8, 0, 8}};
+  fknn_tuning tuning[3] = {{0, 4, 32, 0, 32}, {256, 3, 8, 0, 8}, {256, 3, 8, 0, 8}};
   int num_sms = 148;
   uint32_t n_large_labels = 0;  // categories of more than SMALL_SLAB rows (bounds a device plan's segments)
   // a view shares the device data of another index and owns only its

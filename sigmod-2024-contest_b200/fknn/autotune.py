@@ -33,7 +33,7 @@ SPACE = {
     "min_chunk_blocks": [4, 8, 16],
     "bound_refresh": [0, 2, 8, 32],
 }
-EXACT_SPACE = {"items_per_sm": [2, 4, 8], "min_chunk_blocks": [8, 16, 32], "pilot_stride": [16, 32, 64]}
+EXACT_SPACE = {"items_per_sm": [2, 4, 8], "min_chunk_blocks": [16, 32, 64], "pilot_stride": [16, 32, 64]}
 KPRIMES = [100, 112, 128, 160, 200, 256, 320, 400, 512, 640, 800, 1024]
 
 
