@@ -1095,8 +1095,8 @@ struct TcState {
 // few queries there are few tiles, cut alike, and every further item only adds
 // its own start, end and lists (50 queries over 1e6 rows: 0.50 ms at one item
 // per SM, 0.60 at three; 4,096 over 2e6: 3.17 and 2.73 ms).
-inline uint32_t target_items(const fknn_index *idx, const fknn_tuning &tune, uint32_t nq) {
-  return (uint32_t)idx->num_sms * (nq < 1024 ? 1u : tune.items_per_sm);
+inline uint32_t target_items(const fknn_index *idx, const fknn_tuning &tune, const fknn_tuning &dflt, uint32_t nq) {
+  return (uint32_t)idx->num_sms * items_per_sm(tune, dflt, nq);
 }
 
 // Work items a tile may have: what the merge holds of their lists, and the
@@ -1234,7 +1234,8 @@ static int search_tc(fknn_index *idx, const float *d_q, const float *d_meta, uin
   if ((rc = prepare_queries(idx, d_q, d_meta, nq, st, &d_desc, &h_desc, &h_meta))) return rc;
   uint32_t nsmall_early = 0;
   if ((rc = launch_small_scans(idx, h_desc, d_desc, nq, d_q, k, d_ids, d_dists, st, &nsmall_early))) return rc;
-  const fknn_tuning tune = idx->tuning[F::kFP8 ? FKNN_MODE_FP8_RERANK : FKNN_MODE_BF16_RERANK];
+  constexpr int mode = F::kFP8 ? FKNN_MODE_FP8_RERANK : FKNN_MODE_BF16_RERANK;
+  const fknn_tuning tune = idx->tuning[mode];
   // candidate slots per (item, query): k' plus the pushes between trims; a
   // list holds at most 1280 (32 lanes x 40 registers in the trim)
   const uint32_t capb =
@@ -1257,7 +1258,7 @@ static int search_tc(fknn_index *idx, const float *d_q, const float *d_meta, uin
     ocap = tight ? tight_cap(kprime, capb) : capb;
     const uint64_t per_item = (uint64_t)BQ * ocap * sizeof(Candidate);
     shape.max_items_per_tile = tight ? 1u : max_items(capb, tune.pilot_stride, per_item, tiles_est);
-    shape.target_items = tight ? 1u : target_items(idx, tune, nq);
+    shape.target_items = tight ? 1u : target_items(idx, tune, DEFAULT_TUNING[mode], nq);
     make_plan(h_desc, h_meta, nq, n, shape, P);
     nitems = (uint32_t)P.items.size();
     for (const Tile &t : P.tiles)
@@ -1445,7 +1446,8 @@ static int search_tc_graph(fknn_index *idx, const float *d_q, const float *d_met
                            fknn_search_stats *stats) {
   constexpr uint32_t TA = Tiles<F>::A;
   int rc;
-  const fknn_tuning tune = idx->tuning[F::kFP8 ? FKNN_MODE_FP8_RERANK : FKNN_MODE_BF16_RERANK];
+  constexpr int mode = F::kFP8 ? FKNN_MODE_FP8_RERANK : FKNN_MODE_BF16_RERANK;
+  const fknn_tuning tune = idx->tuning[mode];
   const uint32_t capb =
       (uint32_t)std::min<size_t>(1280, align_up(kprime + std::max<uint32_t>(tune.list_slack, 2 * BP), 128));
   PlanShape shape;
@@ -1465,7 +1467,7 @@ static int search_tc_graph(fknn_index *idx, const float *d_q, const float *d_met
   if ((rc = ws_get(idx, 5, TcState::bytes(nq), (void **)&d_state))) return rc;
   for (int tight = 0;; ++tight) {
     ocap = tight ? tight_cap(kprime, capb) : capb;
-    shape.target_items = tight ? 1u : target_items(idx, tune, nq);
+    shape.target_items = tight ? 1u : target_items(idx, tune, DEFAULT_TUNING[mode], nq);
     z = device_plan_sizes(idx, nq, shape);
     shape.max_items_per_tile =
         tight ? 1u : max_items(capb, tune.pilot_stride, (uint64_t)BQ * ocap * sizeof(Candidate), z.ntile_max);

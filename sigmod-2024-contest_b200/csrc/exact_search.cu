@@ -1011,7 +1011,7 @@ int search_exact(fknn_index *idx, const float *d_q, const float *d_meta, uint32_
   // there are few tiles, cut alike, and every further item only adds its own
   // start and end (16 queries over 1e6 rows: 0.82 ms at one item per SM, 1.29
   // at four; 1e4 queries over 1e5 rows: 3.5 and 3.2 ms).
-  const uint32_t ips = nq < 1024 ? 1u : idx->tuning[FKNN_MODE_EXACT_FP32].items_per_sm;
+  const uint32_t ips = items_per_sm(idx->tuning[FKNN_MODE_EXACT_FP32], DEFAULT_TUNING[FKNN_MODE_EXACT_FP32], nq);
   Candidate *d_out = nullptr, *d_work = nullptr;
   uint32_t *d_ocnt = nullptr, *d_state, sgrid = 0, nitems = 0;
   unsigned char *d_blob;

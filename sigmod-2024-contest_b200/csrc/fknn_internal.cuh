@@ -252,6 +252,20 @@ struct HostBuf {
   size_t bytes = 0;
 };
 
+// The tuning an index starts with, by mode (exact, BF16, FP8), and the work
+// items per SM of a call: below ITEMS_MIN_QUERIES queries the default is one
+// (another value is the caller's and holds for every call).  Both sides of the
+// line, one item per SM and several: exact over 1e6 rows 1.49 and 1.48 ms
+// (1,000 queries), 1.74 and 1.82 (1,600), 3.14 and 3.12 (5,000); BF16 1.05 and
+// 1.10, 1.41 and 1.49, 2.71 and 2.84.  Over 1e5 rows exact 0.69 and 0.70, 0.74
+// and 0.75, 1.48 and 1.36; BF16 would take several from 600 queries on (0.69
+// and 0.65 ms, 0.93 and 0.75 at 1,000).
+constexpr fknn_tuning DEFAULT_TUNING[3] = {{0, 4, 32, 0, 32}, {256, 3, 8, 0, 8}, {256, 3, 8, 0, 8}};
+constexpr uint32_t ITEMS_MIN_QUERIES = 1024;
+inline uint32_t items_per_sm(const fknn_tuning &t, const fknn_tuning &dflt, uint32_t nq) {
+  return nq < ITEMS_MIN_QUERIES && t.items_per_sm == dflt.items_per_sm ? 1u : t.items_per_sm;
+}
+
 }  // namespace fknn
 
 struct fknn_index {
@@ -280,7 +294,7 @@ struct fknn_index {
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   fknn::Plan plan;  // rebuilt by every search; capacity kept
   // per-mode plan / kernel parameters (fknn_index_set_tuning) and the SM count
-  fknn_tuning tuning[3] = {{0, 4, 32, 0, 32}, {256, 3, 8, 0, 8}, {256, 3, 8, 0, 8}};
+  fknn_tuning tuning[3] = {fknn::DEFAULT_TUNING[0], fknn::DEFAULT_TUNING[1], fknn::DEFAULT_TUNING[2]};
   int num_sms = 148;
   uint32_t n_large_labels = 0;  // categories of more than SMALL_SLAB rows (bounds a device plan's segments)
   // a view shares the device data of another index and owns only its

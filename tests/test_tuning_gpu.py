@@ -1,5 +1,6 @@
-"""A tuning holds as it was given: row blocks in their unit.  Results do not
-depend on it."""
+"""A tuning holds as it was given: row blocks in their unit, and work items per
+SM also in small calls, where only the default counts as one.  Results do not
+depend on either."""
 import numpy as np
 import pytest
 
@@ -34,3 +35,16 @@ def test_shortest_chunk(data, mode, rows, slack, default):
     got = idx.search(q, metas, mode=mode, kprime=200)
     np.testing.assert_array_equal(got[0], want[0])
     np.testing.assert_array_equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("mode,rows,slack,default", MODES)
+def test_items_per_sm_of_a_small_call(data, mode, rows, slack, default):
+    idx, q, metas = data
+    out = {}
+    for items in (1, 2, default):
+        idx.set_tuning(mode, slack, items, 2, 0, 8)
+        out[items] = idx.search(q[:300], metas[:300], mode=mode, kprime=200, return_stats=True)
+        np.testing.assert_array_equal(out[items][0], out[1][0])
+        np.testing.assert_array_equal(out[items][1], out[1][1])
+    n = {items: o[2]["n_work_items"] for items, o in out.items()}
+    assert n[2] > 1.5 * n[1] and n[default] == n[1]
