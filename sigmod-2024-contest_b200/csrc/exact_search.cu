@@ -79,16 +79,32 @@ __device__ __forceinline__ uint32_t warp_partition(uint32_t lo, uint32_t hi, Pre
   return lo;
 }
 
+// The same by one thread, halving.
+template <class Pred>
+__device__ __forceinline__ uint32_t thread_partition(uint32_t lo, uint32_t hi, Pred pred) {
+  while (lo < hi) {
+    const uint32_t m = lo + ((hi - lo) >> 1);
+    if (pred(m)) lo = m + 1;
+    else hi = m;
+  }
+  return lo;
+}
+
 // Predicate -> slab.  type 0: all rows (time order); 1: label == v (category
 // order); 2: l <= ts <= r (time order); 3: both (category order, the window
-// inside the label's slab).  The semantics are utils.h:110-137's.  Whole warp.
+// inside the label's slab).  The semantics are utils.h:110-137's.  WARP: by the
+// whole warp, else by each thread.
+template <bool WARP>
 __device__ __forceinline__ void resolve_slab(const float *m, uint32_t n, const float *ts_t, const int32_t *lab_c,
                                              const float *ts_c, int32_t &order, uint32_t &s, uint32_t &e) {
   const uint32_t type = (uint32_t)m[0];
+  auto partition = [](uint32_t lo, uint32_t hi, auto pred) {
+    return WARP ? warp_partition(lo, hi, pred) : thread_partition(lo, hi, pred);
+  };
   auto window = [&](const float *ts, uint32_t lo, uint32_t hi) {
     const float l = m[2], r = m[3];
-    s = warp_partition(lo, hi, [&](uint32_t p) { return ts[p] < l; });
-    e = warp_partition(lo, hi, [&](uint32_t p) { return ts[p] <= r; });
+    s = partition(lo, hi, [&](uint32_t p) { return ts[p] < l; });
+    e = partition(lo, hi, [&](uint32_t p) { return ts[p] <= r; });
   };
   order = type == 0 || type == 2 ? ORDER_TIME : ORDER_CAT;
   if (type == 0) {
@@ -98,53 +114,71 @@ __device__ __forceinline__ void resolve_slab(const float *m, uint32_t n, const f
     window(ts_t, 0, n);
   } else {
     const int32_t v = (int32_t)m[1];
-    s = warp_partition(0, n, [&](uint32_t p) { return lab_c[p] < v; });
-    e = warp_partition(s, n, [&](uint32_t p) { return lab_c[p] <= v; });
+    s = partition(0, n, [&](uint32_t p) { return lab_c[p] < v; });
+    e = partition(s, n, [&](uint32_t p) { return lab_c[p] <= v; });
     if (type == 3) window(ts_c, s, e);
   }
   if (e < s) e = s;
 }
 
-// The query of a warp, eight to a block.  64 bits: nq warps have up to 2^37 threads.
+// A warp per query (WARP) below QP_MANY queries, else a thread: the one has the
+// shorter chain of memory latencies, the other a fifth of the loads.  Counts
+// over 1e6 rows, whole calls, by warps and by threads: 25 and 40 us (4,000
+// queries), 32 and 41 (16,000), 37 and 42 (32,000), 67 and 40 (100,000), 1,253
+// and 240 (3e6).  64 bits: nq warps have up to 2^37 threads.
 constexpr int QP_THREADS = 256;
-constexpr uint32_t QP_WARPS = QP_THREADS / 32;
-__device__ __forceinline__ uint64_t query_of_warp() { return (uint64_t)blockIdx.x * QP_WARPS + threadIdx.x / 32; }
-inline unsigned query_blocks(uint32_t nq) { return (unsigned)(((uint64_t)nq + QP_WARPS - 1) / QP_WARPS); }
-
-// A warp per query.  (50 queries over 1e6 rows: 54 us with a thread each, 10 us
-// now.)
-__global__ void k_query_prep(const float *__restrict__ q, const float *__restrict__ meta, uint32_t nq, uint32_t n,
-                             const float *__restrict__ ts_t, const int32_t *__restrict__ lab_c,
-                             const float *__restrict__ ts_c, QueryDesc *__restrict__ desc) {
-  const uint64_t i = query_of_warp();
-  const uint32_t lane = threadIdx.x & 31;
-  if (i >= nq) return;
-  const float *x = q + i * DIM;
-  float v[4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) v[j] = 32 * j + lane < DIM ? x[32 * j + lane] : 0.f;
-  QueryDesc dsc;
-  resolve_slab(meta + i * 4, n, ts_t, lab_c, ts_c, dsc.order, dsc.s, dsc.e);
-  // |q|^2 in dimension order (every lane the same chain)
-  float s = 0.f;
-#pragma unroll
-  for (int d = 0; d < DIM; ++d) {
-    const float t = __shfl_sync(0xffffffffu, v[d / 32], d % 32);
-    s = fmaf(t, t, s);
-  }
-  dsc.qn = s;
-  if (lane == 0) desc[i] = dsc;
+constexpr uint32_t QP_MANY = 32768;
+template <bool WARP>
+__device__ __forceinline__ uint64_t query_of() {
+  const uint64_t t = (uint64_t)blockIdx.x * QP_THREADS + threadIdx.x;
+  return WARP ? t / 32 : t;
+}
+inline unsigned query_blocks(uint32_t nq) {
+  const uint64_t threads = nq < QP_MANY ? (uint64_t)nq * 32 : nq;
+  return (unsigned)((threads + QP_THREADS - 1) / QP_THREADS);
 }
 
-__global__ void k_count(const float *__restrict__ meta, uint32_t nq, uint32_t n, const float *__restrict__ ts_t,
-                        const int32_t *__restrict__ lab_c, const float *__restrict__ ts_c,
-                        uint32_t *__restrict__ counts) {
-  const uint64_t i = query_of_warp();
+template <bool WARP>
+__global__ void __launch_bounds__(QP_THREADS)
+    k_query_prep(const float *__restrict__ q, const float *__restrict__ meta, uint32_t nq, uint32_t n,
+                 const float *__restrict__ ts_t, const int32_t *__restrict__ lab_c, const float *__restrict__ ts_c,
+                 QueryDesc *__restrict__ desc) {
+  const uint64_t i = query_of<WARP>();
+  if (i >= nq) return;
+  const float *x = q + i * DIM;
+  const uint32_t lane = threadIdx.x & 31;
+  float v[4];
+  if (WARP)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = 32 * j + lane < DIM ? x[32 * j + lane] : 0.f;
+  QueryDesc dsc;
+  resolve_slab<WARP>(meta + i * 4, n, ts_t, lab_c, ts_c, dsc.order, dsc.s, dsc.e);
+  // |q|^2 in dimension order (every lane the same chain)
+  float s = 0.f;
+  if (WARP) {
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+      const float t = __shfl_sync(0xffffffffu, v[d / 32], d % 32);
+      s = fmaf(t, t, s);
+    }
+  } else {
+#pragma unroll 10
+    for (int d = 0; d < DIM; ++d) s = fmaf(x[d], x[d], s);
+  }
+  dsc.qn = s;
+  if (!WARP || lane == 0) desc[i] = dsc;
+}
+
+template <bool WARP>
+__global__ void __launch_bounds__(QP_THREADS)
+    k_count(const float *__restrict__ meta, uint32_t nq, uint32_t n, const float *__restrict__ ts_t,
+            const int32_t *__restrict__ lab_c, const float *__restrict__ ts_c, uint32_t *__restrict__ counts) {
+  const uint64_t i = query_of<WARP>();
   if (i >= nq) return;
   int32_t o;
   uint32_t s, e;
-  resolve_slab(meta + i * 4, n, ts_t, lab_c, ts_c, o, s, e);
-  if ((threadIdx.x & 31) == 0) counts[i] = e - s;
+  resolve_slab<WARP>(meta + i * 4, n, ts_t, lab_c, ts_c, o, s, e);
+  if (!WARP || (threadIdx.x & 31) == 0) counts[i] = e - s;
 }
 
 // --------------------------------------------------------------- merge --
@@ -652,8 +686,8 @@ static int check_query_flag(int flag) {
 
 int count_matches(fknn_index *idx, const float *d_meta, uint32_t nq, uint32_t *d_counts, cudaStream_t st) {
   if (nq == 0) return FKNN_OK;
-  k_count<<<query_blocks(nq), QP_THREADS, 0, st>>>(d_meta, nq, (uint32_t)idx->n, idx->ord[ORDER_TIME].ts,
-                                                   idx->ord[ORDER_CAT].label, idx->ord[ORDER_CAT].ts, d_counts);
+  (nq < QP_MANY ? k_count<true> : k_count<false>)<<<query_blocks(nq), QP_THREADS, 0, st>>>(
+      d_meta, nq, (uint32_t)idx->n, idx->ord[ORDER_TIME].ts, idx->ord[ORDER_CAT].label, idx->ord[ORDER_CAT].ts, d_counts);
   g_launches += 1;
   FKNN_CUDA(cudaGetLastError());
   return FKNN_OK;
@@ -895,8 +929,8 @@ int enqueue_query_prep(fknn_index *idx, const float *d_q, const float *d_meta, u
                        cudaStream_t st) {
   int rc;
   if ((rc = validate_queries(idx, d_q, d_meta, nq, st))) return rc;
-  k_query_prep<<<query_blocks(nq), QP_THREADS, 0, st>>>(d_q, d_meta, nq, (uint32_t)idx->n, idx->ord[ORDER_TIME].ts,
-                                                        idx->ord[ORDER_CAT].label, idx->ord[ORDER_CAT].ts, d_desc);
+  (nq < QP_MANY ? k_query_prep<true> : k_query_prep<false>)<<<query_blocks(nq), QP_THREADS, 0, st>>>(
+      d_q, d_meta, nq, (uint32_t)idx->n, idx->ord[ORDER_TIME].ts, idx->ord[ORDER_CAT].label, idx->ord[ORDER_CAT].ts, d_desc);
   g_launches += 1;
   FKNN_CUDA(cudaGetLastError());
   return FKNN_OK;
@@ -911,8 +945,8 @@ int prepare_queries(fknn_index *idx, const float *d_q, const float *d_meta, uint
   QueryDesc *d_desc;
   if ((rc = ws_get(idx, 2, (size_t)nq * sizeof(QueryDesc), (void **)&d_desc))) return rc;
   if ((rc = validate_queries(idx, d_q, d_meta, nq, st))) return rc;
-  k_query_prep<<<query_blocks(nq), QP_THREADS, 0, st>>>(d_q, d_meta, nq, (uint32_t)n, idx->ord[ORDER_TIME].ts,
-                                                        idx->ord[ORDER_CAT].label, idx->ord[ORDER_CAT].ts, d_desc);
+  (nq < QP_MANY ? k_query_prep<true> : k_query_prep<false>)<<<query_blocks(nq), QP_THREADS, 0, st>>>(
+      d_q, d_meta, nq, (uint32_t)n, idx->ord[ORDER_TIME].ts, idx->ord[ORDER_CAT].label, idx->ord[ORDER_CAT].ts, d_desc);
   g_launches += 1;
   QueryDesc *h_desc;
   float *h_meta;

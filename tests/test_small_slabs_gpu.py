@@ -119,3 +119,21 @@ def test_more_queries_than_32_bit_threads_number():
         assert fknn._lib.load().fknn_count_matches(idx._h, metas.data_ptr(), nq, counts.data_ptr(), None) == 0
     assert bool((counts[:-9] == 300).all())
     assert counts[-9:].tolist() == [100, 100, 100, 0] * 2 + [100]
+
+
+@pytest.mark.parametrize("nq", [32767, 32768, 32769])
+def test_ends_by_warps_and_by_threads(nq):
+    vecs, labels, ts, rng = dataset(9, 40_000)
+    metas = np.zeros((nq, 4), np.float32)
+    metas[:, 0] = rng.integers(0, 4, nq)
+    metas[:, 1] = rng.integers(-1, len(SIZES) + 1, nq)
+    edges = np.array([-np.inf, -0.1, 0, 0.02, 0.5, 0.51, 0.98, 1, 1.5, np.inf], np.float32)
+    metas[:, 2:] = edges[rng.integers(0, 10, (nq, 2))]
+    q = rng.standard_normal((nq, 100), dtype=np.float32)
+    some = rng.integers(0, nq, 200)
+    with fknn.Index(vecs, labels, ts) as idx:
+        np.testing.assert_array_equal(idx.count_matches(metas), oracle.count_matches(labels, ts, metas))
+        ids, dists = idx.search(q, metas, k=20)
+        oids, odists = oracle.exact_knn(vecs, labels, ts, q[some], metas[some], k=20)
+        np.testing.assert_array_equal(ids[some], oids)
+        np.testing.assert_array_equal(dists[some], odists)
