@@ -1403,7 +1403,7 @@ static int search_tc(fknn_index *idx, const float *d_q, const float *d_meta, uin
   }
   if (stats) FKNN_CUDA(cudaEventRecord(ev[2], st));
   if (nbig)
-    if ((rc = launch_exact_scan(idx, S.ovf_list, S.ovf_count, 0, 148 * 2, d_desc, d_q, k, d_ids, d_dists, st))) return rc;
+    if ((rc = launch_exact_scan(idx, S.ovf_list, S.ovf_count, 0, 0, d_desc, d_q, k, d_ids, d_dists, st))) return rc;
   if (nsmall_early && (rc = join_small_scans(idx, st))) return rc;
   FKNN_CUDA(cudaGetLastError());
   if (stats) {
@@ -1525,7 +1525,7 @@ static int search_tc_graph(fknn_index *idx, const float *d_q, const float *d_met
       // disjoint from the merge's)
       FKNN_CUDA(cudaEventRecord(G.fork, st));
       FKNN_CUDA(cudaStreamWaitEvent(G.side, G.fork, 0));
-      if ((r = launch_exact_scan(idx, P.small, P.cnt + DP_NSMALL, 0, 148 * 8, d_desc, d_q, k, d_ids, d_dists,
+      if ((r = launch_exact_scan(idx, P.small, P.cnt + DP_NSMALL, 0, nq / 4, d_desc, d_q, k, d_ids, d_dists,
                                  G.side)))
         return r;
       FKNN_CUDA(cudaEventRecord(G.join, G.side));
@@ -1604,7 +1604,7 @@ static int search_tc_graph(fknn_index *idx, const float *d_q, const float *d_met
                                                                                        nullptr, nullptr);
       g_launches += 2;
       FKNN_CUDA(cudaEventRecordWithFlags(G.ev[2], st, cudaEventRecordExternal));  // an event node of the graph
-      if ((r = launch_exact_scan(idx, S.ovf_list, S.ovf_count, 0, 148 * 2, d_desc, d_q, k, d_ids, d_dists, st))) return r;
+      if ((r = launch_exact_scan(idx, S.ovf_list, S.ovf_count, 0, 0, d_desc, d_q, k, d_ids, d_dists, st))) return r;
       FKNN_CUDA(cudaStreamWaitEvent(st, G.join, 0));
       FKNN_CUDA(cudaEventRecordWithFlags(G.ev[3], st, cudaEventRecordExternal));  // an event node of the graph
       FKNN_CUDA(cudaGetLastError());

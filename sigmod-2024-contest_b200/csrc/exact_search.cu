@@ -334,19 +334,20 @@ __global__ void __launch_bounds__(MG_THREADS)
 // ----------------------------------------------------------- exact scan --
 
 // Bound by latency: a slab of 4,096 rows is 1.6 MB, and one block reads it.  So
-// a thread has 25 loads of a row in flight, eight rows cover the longest slab
-// that is planned for here, and its keys stay in shared memory until the k
-// smallest are selected (a radix select, then every survivor counts its place);
-// longer slabs (queries whose candidates overflowed) select whenever the buffer
-// fills.  16 queries over 1e6 rows, 6 of them here: 235 us with 256
-// threads, ten loads and sorts of 1,024 keys, 45 us now.
-constexpr int ES_THREADS = 512;
-constexpr int ES_CAP = 4096;   // keys in shared memory
-constexpr int ES_KEEP = 1024;  // largest k
-
+// a thread has 25 loads of a row in flight, and the keys stay in shared memory
+// until the k smallest are selected (a radix select, then every survivor counts
+// its place).  A few queries have blocks of 512 threads, whose eight rows cover
+// the longest slab that is planned for here (longer ones, of queries whose
+// candidates overflowed, select whenever the buffer fills); from SCAN_MANY
+// queries on blocks of 256, of which an SM runs twice as many.  Calls of slabs
+// of 2,000 to 4,096 rows, by 512 and by 256 threads: 179 and 208 us (100
+// queries), 199 and 222 (300), 257 and 246 (600), 944 and 767 (4,000); of up to
+// 64 rows 748 and 453 (30,000), where 649 was the time with sorts of 1,024 keys.
+constexpr uint32_t SCAN_MANY = 512;
+template <int NT, int CAP>
 struct ScanSmem {
-  uint64_t buf[ES_CAP];
-  uint64_t sel[ES_KEEP];
+  uint64_t buf[CAP];  // keys
+  uint64_t sel[KMAX_TILE];
   float qv[DIM];
   uint32_t hist[256];
   unsigned long long mn, mx;
@@ -356,7 +357,8 @@ struct ScanSmem {
 };
 
 // The k smallest of the cnt > k distinct keys in buf to sel, in no order.
-__device__ void scan_select(ScanSmem &sm, int cnt, uint32_t k) {
+template <int NT, int CAP>
+__device__ void scan_select(ScanSmem<NT, CAP> &sm, int cnt, uint32_t k) {
   const int tid = threadIdx.x, lane = tid & 31;
   if (tid == 0) {
     sm.mn = ~0ull;
@@ -365,7 +367,7 @@ __device__ void scan_select(ScanSmem &sm, int cnt, uint32_t k) {
   }
   __syncthreads();
   uint64_t mn = ~0ull, mx = 0;
-  for (int i = tid; i < cnt; i += ES_THREADS) {
+  for (int i = tid; i < cnt; i += NT) {
     mn = min(mn, sm.buf[i]);
     mx = max(mx, sm.buf[i]);
   }
@@ -379,9 +381,9 @@ __device__ void scan_select(ScanSmem &sm, int cnt, uint32_t k) {
   uint32_t want = k;
   while (hi > 0) {
     const int w = min(8, hi), shift = hi - w;
-    for (int i = tid; i < 256; i += ES_THREADS) sm.hist[i] = 0;
+    for (int i = tid; i < 256; i += NT) sm.hist[i] = 0;
     __syncthreads();
-    for (int i = tid; i < cnt; i += ES_THREADS) {
+    for (int i = tid; i < cnt; i += NT) {
       const uint64_t u = sm.buf[i];
       if ((u & mask) == prefix) atomicAdd(&sm.hist[(u >> shift) & ((1u << w) - 1)], 1u);
     }
@@ -419,20 +421,21 @@ __device__ void scan_select(ScanSmem &sm, int cnt, uint32_t k) {
     hi = shift;
     if (sm.count == 1) break;
   }
-  for (int i = tid; i < cnt; i += ES_THREADS) {
+  for (int i = tid; i < cnt; i += NT) {
     const uint64_t u = sm.buf[i];
     if ((u & mask) <= prefix) sm.sel[atomicAdd(&sm.kept, 1)] = u;
   }
   __syncthreads();
 }
 
-__global__ void __launch_bounds__(ES_THREADS)
+template <int NT, int CAP>
+__global__ void __launch_bounds__(NT)
     k_exact_scan(const uint32_t *__restrict__ list, const uint32_t *__restrict__ d_count, uint32_t h_count,
                  const QueryDesc *__restrict__ desc, const float *__restrict__ q, const float *__restrict__ blocks_t,
                  const float *__restrict__ blocks_c, const uint32_t *__restrict__ perm_t,
                  const uint32_t *__restrict__ perm_c, uint32_t k, uint32_t *__restrict__ ids,
                  float *__restrict__ dists) {
-  __shared__ ScanSmem sm;
+  __shared__ ScanSmem<NT, CAP> sm;
   const uint32_t count = d_count ? *d_count : h_count;
   const int tid = threadIdx.x;
   for (uint32_t li = blockIdx.x; li < count; li += gridDim.x) {
@@ -440,14 +443,14 @@ __global__ void __launch_bounds__(ES_THREADS)
     const QueryDesc dsc = desc[qi];
     const float *blocks = dsc.order == ORDER_TIME ? blocks_t : blocks_c;
     const uint32_t *perm = dsc.order == ORDER_TIME ? perm_t : perm_c;
-    for (int d = tid; d < DIM; d += ES_THREADS) sm.qv[d] = q[(uint64_t)qi * DIM + d];
+    for (int d = tid; d < DIM; d += NT) sm.qv[d] = q[(uint64_t)qi * DIM + d];
     if (tid == 0) {
       sm.cnt = 0;
       sm.thr = ~0ull;
     }
     __syncthreads();
     int held = 0;  // keys in buf: counted at the step's barrier, for sm.cnt grows again as soon as a warp has passed it
-    for (uint64_t base = dsc.s; base < dsc.e; base += ES_THREADS) {
+    for (uint64_t base = dsc.s; base < dsc.e; base += NT) {
       const uint64_t p = base + tid;
       bool push = false;
       if (p < dsc.e) {
@@ -471,10 +474,10 @@ __global__ void __launch_bounds__(ES_THREADS)
         if (push) sm.buf[atomicAdd(&sm.cnt, 1)] = key;
       }
       held += __syncthreads_count(push);
-      if (held > ES_CAP - ES_THREADS && base + ES_THREADS < dsc.e) {  // (block-uniform)
+      if (held > CAP - NT && base + NT < dsc.e) {  // (block-uniform)
         scan_select(sm, held, k);
         uint64_t mx = 0;
-        for (uint32_t i = tid; i < k; i += ES_THREADS) {
+        for (uint32_t i = tid; i < k; i += NT) {
           sm.buf[i] = sm.sel[i];
           mx = max(mx, sm.sel[i]);
         }
@@ -498,14 +501,14 @@ __global__ void __launch_bounds__(ES_THREADS)
       c = (int)k;
     }
     // a key's place is the number of smaller ones (they are distinct)
-    for (int i = tid; i < c; i += ES_THREADS) {
+    for (int i = tid; i < c; i += NT) {
       const uint64_t e = keys[i];
       uint32_t rank = 0;
       for (int j = 0; j < c; ++j) rank += keys[j] < e ? 1u : 0u;
       ids[(uint64_t)qi * k + rank] = (uint32_t)e;
       if (dists) dists[(uint64_t)qi * k + rank] = sortable_f32((uint32_t)(e >> 32));
     }
-    for (uint32_t j = (uint32_t)c + tid; j < k; j += ES_THREADS) {
+    for (uint32_t j = (uint32_t)c + tid; j < k; j += NT) {
       ids[(uint64_t)qi * k + j] = 0xffffffffu;
       if (dists) dists[(uint64_t)qi * k + j] = INFINITY;
     }
@@ -965,11 +968,16 @@ int prepare_queries(fknn_index *idx, const float *d_q, const float *d_meta, uint
   return FKNN_OK;
 }
 
-int launch_exact_scan(fknn_index *idx, const uint32_t *list, const uint32_t *d_count, uint32_t h_count, unsigned grid,
+// The queries of list, *d_count of them (d_count NULL: h_count); nmax: about how
+// many that may be, 0: as a rule none, and with slabs of any length.
+int launch_exact_scan(fknn_index *idx, const uint32_t *list, const uint32_t *d_count, uint32_t h_count, uint32_t nmax,
                       const QueryDesc *desc, const float *q, uint32_t k, uint32_t *ids, float *dists, cudaStream_t st) {
   const OrderData &OT = idx->ord[ORDER_TIME], &OC = idx->ord[ORDER_CAT];
-  k_exact_scan<<<grid, ES_THREADS, 0, st>>>(list, d_count, h_count, desc, q, OT.blocks, OC.blocks, OT.perm, OC.perm, k,
-                                            ids, dists);
+  const bool many = nmax >= SCAN_MANY;
+  const uint32_t grid = (uint32_t)idx->num_sms * (nmax ? 8 : 2);
+  auto scan = many ? k_exact_scan<256, 2048> : k_exact_scan<512, 4096>;
+  scan<<<d_count ? grid : std::min(h_count, grid), many ? 256 : 512, 0, st>>>(
+      list, d_count, h_count, desc, q, OT.blocks, OC.blocks, OT.perm, OC.perm, k, ids, dists);
   g_launches += 1;
   FKNN_CUDA(cudaGetLastError());
   return FKNN_OK;
@@ -999,8 +1007,7 @@ int launch_small_scans(fknn_index *idx, const QueryDesc *h_desc, const QueryDesc
   FKNN_CUDA(cudaEventRecord(idx->ev_fork, st));
   FKNN_CUDA(cudaStreamWaitEvent(idx->side_stream, idx->ev_fork, 0));
   FKNN_CUDA(cudaMemcpyAsync(d_list, h_list, (size_t)m * 4, cudaMemcpyHostToDevice, idx->side_stream));
-  if ((rc = launch_exact_scan(idx, d_list, nullptr, m, std::min<uint32_t>(m, 148 * 8), d_desc, d_q, k, d_ids,
-                              d_dists, idx->side_stream)))
+  if ((rc = launch_exact_scan(idx, d_list, nullptr, m, m, d_desc, d_q, k, d_ids, d_dists, idx->side_stream)))
     return rc;
   FKNN_CUDA(cudaEventRecord(idx->ev_join, idx->side_stream));
   return FKNN_OK;
@@ -1236,9 +1243,7 @@ int search_exact(fknn_index *idx, const float *d_q, const float *d_meta, uint32_
   }
   if (stats) FKNN_CUDA(cudaEventRecord(ev[2], st));
   if (nbig) {
-    k_exact_scan<<<148 * 2, ES_THREADS, 0, st>>>(ovf_list, ovf_count, 0, d_desc, d_q, OT.blocks, OC.blocks, OT.perm,
-                                                 OC.perm, k, d_ids, d_dists);
-    g_launches += 1;
+    if ((rc = launch_exact_scan(idx, ovf_list, ovf_count, 0, 0, d_desc, d_q, k, d_ids, d_dists, st))) return rc;
   }
   if (nsmall_early && (rc = join_small_scans(idx, st))) return rc;
   FKNN_CUDA(cudaGetLastError());

@@ -422,7 +422,7 @@ int enqueue_query_prep(fknn_index *idx, const float *d_q, const float *d_meta, u
 int check_query_flag_value(int flag);
 int prepare_queries(fknn_index *idx, const float *d_q, const float *d_meta, uint32_t nq, cudaStream_t st,
                     QueryDesc **d_desc, QueryDesc **h_desc, float **h_meta);
-int launch_exact_scan(fknn_index *idx, const uint32_t *list, const uint32_t *d_count, uint32_t h_count, unsigned grid,
+int launch_exact_scan(fknn_index *idx, const uint32_t *list, const uint32_t *d_count, uint32_t h_count, uint32_t nmax,
                       const QueryDesc *desc, const float *q, uint32_t k, uint32_t *ids, float *dists, cudaStream_t st);
 int launch_fill_u32(uint32_t *p, uint32_t n, uint32_t v, cudaStream_t st);
 int launch_small_scans(fknn_index *idx, const QueryDesc *h_desc, const QueryDesc *d_desc, uint32_t nq,

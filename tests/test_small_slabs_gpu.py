@@ -137,3 +137,30 @@ def test_ends_by_warps_and_by_threads(nq):
         oids, odists = oracle.exact_knn(vecs, labels, ts, q[some], metas[some], k=20)
         np.testing.assert_array_equal(ids[some], oids)
         np.testing.assert_array_equal(dists[some], odists)
+
+
+@pytest.mark.parametrize("distinct", [3, 40_000])
+def test_many_slabs_of_every_size(distinct):
+    """As many queries as take blocks of 256 threads and buffers of 2,048 keys."""
+    rng = np.random.default_rng(distinct)
+    sizes = SIZES + [255, 256, 257, 1791, 1792, 1793, 2047, 2048, 2049, 2304]
+    labels = np.repeat(np.arange(len(sizes)), sizes).astype(np.float32)
+    n = labels.shape[0]
+    vecs = rng.standard_normal((distinct, 100), dtype=np.float32)[rng.integers(0, distinct, n)]
+    ts = rng.random(n, dtype=np.float32)
+    q = rng.standard_normal((900, 100), dtype=np.float32)
+    metas = np.zeros((900, 4), np.float32)
+    metas[:, 0] = 1
+    metas[:, 1] = np.arange(900) % len(sizes)
+    with fknn.Index(vecs, labels, ts, build_bf16=True) as idx:
+        for k in (1, 100, 128):
+            oids, odists = oracle.exact_knn(vecs, labels, ts, q, metas, k=k)
+            ids, dists = idx.search(q, metas, k=k)
+            np.testing.assert_array_equal(ids, oids)
+            np.testing.assert_array_equal(dists, odists)
+            # a captured search goes by a share of its queries
+            ids, dists = idx.search(np.tile(q, (4, 1)), np.tile(metas, (4, 1)), k=k, mode=fknn.MODE_BF16_RERANK,
+                                    kprime=200, graph=True)
+            scanned = np.tile(np.array(sizes)[np.arange(900) % len(sizes)] <= 4096, 4)
+            np.testing.assert_array_equal(ids[scanned], np.tile(oids, (4, 1))[scanned])
+            np.testing.assert_array_equal(dists[scanned], np.tile(odists, (4, 1))[scanned])
