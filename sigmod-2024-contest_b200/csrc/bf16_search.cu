@@ -852,6 +852,7 @@ __global__ void __launch_bounds__(B_THREADS, 1) k_screen_tc(ScreenArgs A) {
 constexpr int RR_THREADS = 256;
 constexpr int RR_CAP = 8192;        // screening candidates the large merge holds
 constexpr int RR_CAP_SMALL = 1024;  // ... and the common one (8 blocks per SM)
+constexpr int RR_LARGE_BLOCKS = 3;  // ... of the large one
 constexpr int RR_KMAX = 1024;       // largest k'
 constexpr int RR_ITEMS = 256;       // work items of a tile (the lists' offsets)
 
@@ -863,7 +864,7 @@ struct RerankSmem {
   float qv[DIM];
   uint32_t cnt_prefix[RR_ITEMS + 1];
   uint32_t hist[256], red[4];
-  int total, kept;
+  int total, kept, ties;
 };
 
 struct MergeArgs {
@@ -916,7 +917,7 @@ __device__ void merge_one(const MergeArgs &A, uint32_t b, RerankSmem<CAP> &sm, u
   // candidate counts of the query's items (a tile has at most a few dozen)
   // more items than prefix slots: the exact scan answers the query
   list_offsets(item_slot, tl.item0, nitems, out_cnt, L, BQ, sm.cnt_prefix, &sm.total, RR_ITEMS, RR_CAP + 1);
-  if (tid == 0) sm.kept = 0;
+  if (tid == 0) sm.kept = sm.ties = 0;
   __syncthreads();
   const int M = sm.total;
   if (M > CAP && spill && M <= RR_CAP) {  // the large merge takes it
@@ -951,13 +952,20 @@ __device__ void merge_one(const MergeArgs &A, uint32_t b, RerankSmem<CAP> &sm, u
   for (int i = tid; i < M; i += RR_THREADS) {
     const uint32_t u = f32_sortable(sm.key[i]);
     if (u < kth || M == C) sm.ekey[atomicAdd(&sm.kept, 1)] = sm.val[i];
+    else if (u == kth) atomicAdd(&sm.ties, 1);
   }
   __syncthreads();
   if (M > C) {
     const int below = sm.kept;
+    const bool fit = below + sm.ties == C;  // as a rule the k'-th alone: no walk over all M by its one thread
     const float tie = sortable_f32(kth);
+    __syncthreads();
     for (int i = tid; i < M; i += RR_THREADS)
       if (f32_sortable(sm.key[i]) == kth) {
+        if (fit) {
+          sm.ekey[atomicAdd(&sm.kept, 1)] = sm.val[i];
+          continue;
+        }
         int at = below;
         for (int j = 0; j < M; ++j) at += sm.key[j] == tie && sm.val[j] < sm.val[i] ? 1 : 0;
         if (at < C) sm.ekey[at] = sm.val[i];
@@ -1397,8 +1405,8 @@ static int search_tc(fknn_index *idx, const float *d_q, const float *d_meta, uin
     // queries with more candidates than the common merge holds go to the large one
     k_merge_rerank<RR_CAP_SMALL><<<nbig, RR_THREADS, sizeof(RerankSmem<RR_CAP_SMALL>), st>>>(
         A, nbig, nullptr, nullptr, S.spill, S.spill_count);
-    k_merge_rerank<RR_CAP><<<148 * 2, RR_THREADS, sizeof(RerankSmem<RR_CAP>), st>>>(A, 0, S.spill, S.spill_count,
-                                                                                     nullptr, nullptr);
+    k_merge_rerank<RR_CAP><<<idx->num_sms * RR_LARGE_BLOCKS, RR_THREADS, sizeof(RerankSmem<RR_CAP>), st>>>(
+        A, 0, S.spill, S.spill_count, nullptr, nullptr);
     g_launches += 3;
   }
   if (stats) FKNN_CUDA(cudaEventRecord(ev[2], st));
@@ -1598,10 +1606,11 @@ static int search_tc_graph(fknn_index *idx, const float *d_q, const float *d_met
       A.dists = d_dists;
       A.n_f64 = S.n_f64;
       A.nbig_d = P.cnt + DP_NBIG;
-        k_merge_rerank<RR_CAP_SMALL><<<std::min<uint32_t>(nq, (uint32_t)idx->num_sms * 32), RR_THREADS,
-                                     sizeof(RerankSmem<RR_CAP_SMALL>), st>>>(A, 0, nullptr, nullptr, S.spill, S.spill_count);
-      k_merge_rerank<RR_CAP><<<148 * 2, RR_THREADS, sizeof(RerankSmem<RR_CAP>), st>>>(A, 0, S.spill, S.spill_count,
-                                                                                       nullptr, nullptr);
+      k_merge_rerank<RR_CAP_SMALL><<<std::min<uint32_t>(nq, (uint32_t)idx->num_sms * 32), RR_THREADS,
+                                     sizeof(RerankSmem<RR_CAP_SMALL>), st>>>(A, 0, nullptr, nullptr, S.spill,
+                                                                             S.spill_count);
+      k_merge_rerank<RR_CAP><<<idx->num_sms * RR_LARGE_BLOCKS, RR_THREADS, sizeof(RerankSmem<RR_CAP>), st>>>(
+          A, 0, S.spill, S.spill_count, nullptr, nullptr);
       g_launches += 2;
       FKNN_CUDA(cudaEventRecordWithFlags(G.ev[2], st, cudaEventRecordExternal));  // an event node of the graph
       if ((r = launch_exact_scan(idx, S.ovf_list, S.ovf_count, 0, 0, d_desc, d_q, k, d_ids, d_dists, st))) return r;
