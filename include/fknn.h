@@ -72,9 +72,9 @@ typedef struct fknn_tuning {
                                 than 1,024 queries; another value holds for every call) */
   uint32_t min_chunk_blocks; /* shortest row chunk of a work item, in row blocks (64 rows exact, 128 BF16/FP8) */
   uint32_t bound_refresh;    /* BF16/FP8: 128-row sub-tiles between reloads of the shared per-query bound (0 = at trims) */
-  uint32_t pilot_stride;     /* a pilot pass over every pilot_stride-th row block first seeds the bounds
-                                (0 or 1 = no pilot) with an estimate of the k'-th (exact: of the k-th),
-                                checked by the merge */
+  uint32_t pilot_stride;     /* a pilot pass over every pilot_stride-th row block first seeds the bounds with an
+                                estimate of the k'-th (exact: of the k-th), checked by the merge
+                                (0 or 1: exact no pilot, BF16/FP8 the default stride) */
 } fknn_tuning;
 
 /* fknn_search_opts.flags */

@@ -926,7 +926,7 @@ __device__ void merge_one(const MergeArgs &A, uint32_t b, RerankSmem<CAP> &sm, u
   }
   // a pilot bound that kept fewer than k' rows was set too low: the exact
   // scan answers the query
-  if (M > CAP || (seeded && seeded[qi] && M < (int)kprime)) {
+  if (M > CAP || (seeded[qi] && M < (int)kprime)) {
     if (tid == 0) ovf_list[atomicAdd(ovf_count, 1u)] = qi;
     return;
   }
@@ -1110,9 +1110,16 @@ inline uint32_t target_items(const fknn_index *idx, const fknn_tuning &tune, con
 // Work items a tile may have: what the merge holds of their lists, and the
 // scratch (8 GB).  Behind a seeded bound all of a query's lists together hold
 // 3 k' entries or so, and a query too short to be seeded meets few items.
-inline uint32_t max_items(uint32_t capb, uint32_t pilot_stride, uint64_t per_item, uint64_t tiles) {
-  const uint64_t lists = pilot_stride > 1 ? RR_ITEMS : std::min<uint64_t>(RR_ITEMS, RR_CAP / capb);
-  return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(lists, (8ull << 30) / (per_item * tiles)));
+inline uint32_t max_items(uint64_t per_item, uint64_t tiles) {
+  return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(RR_ITEMS, (8ull << 30) / (per_item * tiles)));
+}
+
+// The pilot's stride.  There is always a pilot: a screen without one pushes
+// rows by the hundred before it has a bound, which costs this epilogue more
+// than the pilot does (1,000 queries over 1e6 rows, k' = 200: screens of 5.7 ms
+// without, 0.7 with it; 20,000 queries 13.9 and 6.0).
+inline uint32_t pilot_stride(const fknn_tuning &tune, const fknn_tuning &dflt) {
+  return tune.pilot_stride > 1 ? tune.pilot_stride : dflt.pilot_stride;
 }
 
 // Entries of a query in an item's result when memory is short: k' and a few
@@ -1195,31 +1202,29 @@ template <class K>
 static void launch_screens(K screen, ScreenArgs X, SeedArgs Z, const TcState &S, uint32_t kprime, uint32_t stride,
                            uint32_t refresh, bool withhold, uint32_t grid, uint32_t nbig_max, size_t smem,
                            cudaStream_t st) {
-  if (stride > 1) {
-    X.T_global = S.T_pilot;
-    X.ovf = S.ovf_pilot;
-    // (the sample of a short slab is up to twice its nominal share)
-    X.kprime = exact_seed_rank(kprime, 2, stride);
-    X.kseed = kprime;
-    X.refresh = 0;
-    X.stride = stride;
-    X.withhold = 0;
-    X.queue = S.queue;
-    screen<<<grid, B_THREADS, smem, st>>>(X);
-    Z.tiles = X.tiles;
-    Z.items = X.items;
-    Z.out = X.out;
-    Z.out_cnt = X.out_cnt;
-    Z.tq = BQ;
-    Z.list_cap = X.ocap;
-    Z.blk_rows = BR;
-    Z.stride = stride;
-    Z.k = kprime;
-    Z.T_global = S.T_global;
-    Z.seeded = S.seeded;
-    launch_screen_seed(Z, nbig_max, SeedBound(), st);
-    g_launches += 1;
-  }
+  X.T_global = S.T_pilot;
+  X.ovf = S.ovf_pilot;
+  // (the sample of a short slab is up to twice its nominal share)
+  X.kprime = exact_seed_rank(kprime, 2, stride);
+  X.kseed = kprime;
+  X.refresh = 0;
+  X.stride = stride;
+  X.withhold = 0;
+  X.queue = S.queue;
+  screen<<<grid, B_THREADS, smem, st>>>(X);
+  Z.tiles = X.tiles;
+  Z.items = X.items;
+  Z.out = X.out;
+  Z.out_cnt = X.out_cnt;
+  Z.tq = BQ;
+  Z.list_cap = X.ocap;
+  Z.blk_rows = BR;
+  Z.stride = stride;
+  Z.k = kprime;
+  Z.T_global = S.T_global;
+  Z.seeded = S.seeded;
+  launch_screen_seed(Z, nbig_max, SeedBound(), st);
+  g_launches += 1;
   X.T_global = S.T_global;
   X.ovf = S.ovf;
   X.kprime = kprime;
@@ -1265,7 +1270,7 @@ static int search_tc(fknn_index *idx, const float *d_q, const float *d_meta, uin
     // results (items x 256 x ocap x 8 B) stay within ~8 GB
     ocap = tight ? tight_cap(kprime, capb) : capb;
     const uint64_t per_item = (uint64_t)BQ * ocap * sizeof(Candidate);
-    shape.max_items_per_tile = tight ? 1u : max_items(capb, tune.pilot_stride, per_item, tiles_est);
+    shape.max_items_per_tile = tight ? 1u : max_items(per_item, tiles_est);
     shape.target_items = tight ? 1u : target_items(idx, tune, DEFAULT_TUNING[mode], nq);
     make_plan(h_desc, h_meta, nq, n, shape, P);
     nitems = (uint32_t)P.items.size();
@@ -1347,7 +1352,7 @@ static int search_tc(fknn_index *idx, const float *d_q, const float *d_meta, uin
                                    (int)sizeof(RerankSmem<RR_CAP>)));
     if (stats) FKNN_CUDA(cudaEventRecord(ev[0], st));
     void *const *blocks = F::kFP8 ? idx->fp8_blocks : idx->bf16_blocks;
-    const uint32_t stride = tune.pilot_stride;
+    const uint32_t stride = pilot_stride(tune, DEFAULT_TUNING[mode]);
     ScreenArgs X;
     X.items = (const WorkItem *)(d_blob + o_items);
     X.tiles = (const Tile *)(d_blob + o_tiles);
@@ -1397,7 +1402,7 @@ static int search_tc(fknn_index *idx, const float *d_q, const float *d_meta, uin
     A.k = k;
     A.kprime = kprime;
     A.capb = ocap;
-    A.seeded = stride > 1 ? S.seeded : nullptr;
+    A.seeded = S.seeded;
     A.ids = d_ids;
     A.dists = d_dists;
     A.n_f64 = S.n_f64;
@@ -1478,7 +1483,7 @@ static int search_tc_graph(fknn_index *idx, const float *d_q, const float *d_met
     shape.target_items = tight ? 1u : target_items(idx, tune, DEFAULT_TUNING[mode], nq);
     z = device_plan_sizes(idx, nq, shape);
     shape.max_items_per_tile =
-        tight ? 1u : max_items(capb, tune.pilot_stride, (uint64_t)BQ * ocap * sizeof(Candidate), z.ntile_max);
+        tight ? 1u : max_items((uint64_t)BQ * ocap * sizeof(Candidate), z.ntile_max);
     void *h;  // the radix sort's histogram slot at its largest: the plan sorts the queries and the work items
     const size_t keys = std::max<size_t>(nq, z.nitems_max);
     rc = ws_get(idx, 15, ((keys + 4095) / 4096) * 256 * sizeof(uint32_t) + 256, &h);
@@ -1492,7 +1497,7 @@ static int search_tc_graph(fknn_index *idx, const float *d_q, const float *d_met
     drop_lists(idx);
   }
   const TcState S(d_state, nq);
-  const uint32_t stride = tune.pilot_stride;
+  const uint32_t stride = pilot_stride(tune, DEFAULT_TUNING[mode]);
   DevPlan P;
   device_plan_layout(P, d_plan, nq, z);
   auto screen = screen_kernel<F>(capb);
@@ -1506,7 +1511,7 @@ static int search_tc_graph(fknn_index *idx, const float *d_q, const float *d_met
   idx->test_withhold = false;
   const std::vector<uint64_t> key = {
       (uint64_t)F::kFP8, nq, k, kprime, capb, ocap, sgrid, shape.target_items, tune.list_slack,
-      tune.items_per_sm, tune.min_chunk_blocks, tune.bound_refresh, tune.pilot_stride, (uint64_t)withhold, (uint64_t)(uintptr_t)d_q, (uint64_t)(uintptr_t)d_meta,
+      tune.items_per_sm, tune.min_chunk_blocks, tune.bound_refresh, stride, (uint64_t)withhold, (uint64_t)(uintptr_t)d_q, (uint64_t)(uintptr_t)d_meta,
       (uint64_t)(uintptr_t)d_ids, (uint64_t)(uintptr_t)d_dists, (uint64_t)(uintptr_t)d_desc,
       (uint64_t)(uintptr_t)d_plan, (uint64_t)(uintptr_t)d_at, (uint64_t)(uintptr_t)d_lqs, (uint64_t)(uintptr_t)d_out,
       (uint64_t)(uintptr_t)d_work,
@@ -1601,7 +1606,7 @@ static int search_tc_graph(fknn_index *idx, const float *d_q, const float *d_met
       A.k = k;
       A.kprime = kprime;
       A.capb = ocap;
-      A.seeded = stride > 1 ? S.seeded : nullptr;
+      A.seeded = S.seeded;
       A.ids = d_ids;
       A.dists = d_dists;
       A.n_f64 = S.n_f64;

@@ -28,7 +28,7 @@ DEFAULT_TABLE = os.path.join(os.path.dirname(os.path.abspath(__file__)), "tuning
 
 SPACE = {
     "items_per_sm": [2, 3, 4, 6, 8],
-    "pilot_stride": [0, 8, 16, 32, 64],
+    "pilot_stride": [8, 16, 32, 64],
     "list_slack": [256, 384, 512],
     "min_chunk_blocks": [4, 8, 16],
     "bound_refresh": [0, 2, 8, 32],
