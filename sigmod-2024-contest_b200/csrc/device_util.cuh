@@ -87,19 +87,6 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity
 
 __device__ __forceinline__ uint32_t ld_volatile_u32(const uint32_t *p) { return *(const volatile uint32_t *)p; }
 
-// distance.h:62-72 normal_l2(base, query): v = x - q; v *= v; r += v, every
-// operation rounded to float, in dimension order, never fused.
-__device__ __forceinline__ float seq_l2_strided(const float *x, int xstride, const float *q) {
-  float r = 0.f;
-#pragma unroll 10
-  for (int d = 0; d < DIM; ++d) {
-    float v = __fsub_rn(x[d * xstride], q[d]);
-    v = __fmul_rn(v, v);
-    r = __fadd_rn(r, v);
-  }
-  return r;
-}
-
 __device__ __forceinline__ uint64_t exact_key(float d, uint32_t id) {
   return ((uint64_t)f32_sortable(d) << 32) | id;
 }
@@ -121,72 +108,6 @@ __device__ void block_bitonic_sort(K *key, int n) {
         }
       }
       __syncthreads();
-    }
-  }
-}
-
-// Key/value variant ordered by (key, val).
-template <typename K, typename V>
-__device__ void block_bitonic_sort_kv(K *key, V *val, int n) {
-  for (int size = 2; size <= n; size <<= 1) {
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (int i = threadIdx.x; i < (n >> 1); i += blockDim.x) {
-        int lo = 2 * stride * (i / stride) + (i % stride);
-        int hi = lo + stride;
-        bool asc = (lo & size) == 0;
-        K a = key[lo], b = key[hi];
-        V va = val[lo], vb = val[hi];
-        bool gt = (a > b) || (a == b && va > vb);
-        if (gt == asc) {
-          key[lo] = b;
-          key[hi] = a;
-          val[lo] = vb;
-          val[hi] = va;
-        }
-      }
-      __syncthreads();
-    }
-  }
-}
-
-// Warp-wide bitonic sort of 32*N (key, val) pairs held N per lane, element
-// e = j*32 + lane in register j, ascending by (key, val).
-template <int N>
-__device__ __forceinline__ void warp_bitonic_sort(float (&key)[N], uint32_t (&val)[N]) {
-  const int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int size = 2; size <= 32 * N; size <<= 1) {
-#pragma unroll
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      if (stride >= 32) {
-        const int rs = stride >> 5;
-#pragma unroll
-        for (int j = 0; j < N; ++j) {
-          const int p = j ^ rs;
-          if (p > j) {
-            const bool asc = (((j << 5) | lane) & size) == 0;
-            const bool gt = key[j] > key[p] || (key[j] == key[p] && val[j] > val[p]);
-            if (gt == asc) {
-              float tk = key[j]; key[j] = key[p]; key[p] = tk;
-              uint32_t tv = val[j]; val[j] = val[p]; val[p] = tv;
-            }
-          }
-        }
-      } else {
-#pragma unroll
-        for (int j = 0; j < N; ++j) {
-          const float ok = __shfl_xor_sync(0xffffffffu, key[j], stride);
-          const uint32_t ov = __shfl_xor_sync(0xffffffffu, val[j], stride);
-          const bool asc = (((j << 5) | lane) & size) == 0;
-          const bool lower = (lane & stride) == 0;
-          const bool other_less = ok < key[j] || (ok == key[j] && ov < val[j]);
-          const bool take_other = (lower == asc) ? other_less : !other_less && !(ok == key[j] && ov == val[j]);
-          if (take_other) {
-            key[j] = ok;
-            val[j] = ov;
-          }
-        }
-      }
     }
   }
 }
@@ -319,7 +240,9 @@ __device__ uint32_t block_kth(const float *key, int n, uint32_t kth, uint32_t *h
   return prefix;
 }
 
-// seq_l2_strided over a 16-byte aligned row, four dimensions per load
+// distance.h:62-72 normal_l2(base, query): v = x - q; v *= v; r += v, every
+// operation rounded to float, in dimension order, never fused.  The row is
+// 16-byte aligned: four dimensions per load.
 __device__ __forceinline__ float seq_l2_row(const float *__restrict__ x, const float *q) {
   const float4 *x4 = reinterpret_cast<const float4 *>(x);
   float r = 0.f;

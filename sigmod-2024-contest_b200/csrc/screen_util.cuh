@@ -12,24 +12,7 @@ namespace fknn {
 
 constexpr int STAGE_ROW = 36;  // floats per lane row of the push staging area
 
-// max of 32 values as a tree of three-input maxima (16 instructions)
-__device__ __forceinline__ float max32(const float *v) {
-  float a[10];
-#pragma unroll
-  for (int k = 0; k < 10; ++k) a[k] = fmax3(v[3 * k], v[3 * k + 1], v[3 * k + 2]);
-  const float b0 = fmax3(a[0], a[1], a[2]), b1 = fmax3(a[3], a[4], a[5]), b2 = fmax3(a[6], a[7], a[8]);
-  const float b3 = fmax3(a[9], v[30], v[31]);
-  return fmax3(b0, b1, fmaxf(b2, b3));
-}
-
-__device__ __forceinline__ float max32(const uint32_t (&r)[32]) {
-  float v[32];
-#pragma unroll
-  for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
-  return max32(v);
-}
-
-// the same with the maxima of the four groups of 8
+// max of 32 values as a tree of three-input maxima, and those of the four groups of 8
 __device__ __forceinline__ float max32(const uint32_t (&r)[32], float (&g)[4]) {
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
