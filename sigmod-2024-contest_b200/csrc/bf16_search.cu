@@ -483,8 +483,8 @@ __device__ __forceinline__ uint32_t pack_query(int r0, int r1, int lane, int col
 }
 
 // Persistent, one CTA per SM, pulling work items (longest first) from a
-// queue: warp 16 copies row blocks in, warp 17 issues MMAs, warps 0-15 are the
-// epilogue.  A tile of more than 128 queries multiplies every row block with
+// queue: warps 0-7 are the epilogue, warp 8 copies row blocks in, warp 9 issues
+// MMAs.  A tile of more than 128 queries multiplies every row block with
 // both halves of its queries, so a block crosses from L2 once for 256 queries.
 // The products go to the two accumulators in turn, and every epilogue warp
 // takes its columns of each into registers and releases it at once: what a
@@ -494,7 +494,7 @@ __device__ __forceinline__ uint32_t pack_query(int r0, int r1, int lane, int col
 // N = 256: an MMA of 128 columns takes 91 cycles here, one of 256 takes 128.
 // Bound by the epilogue's latency: a warp needs about 1,200 cycles a product
 // (the MMAs 896) and 640 more when one of its queries has a candidate; sixteen
-// warps of 64 columns each measured the same.  Screens of a call, pilot
+// epilogue warps of 64 columns each (96 registers a thread) measured the same.  Screens of a call, pilot
 // included, before (tiles of 128 x 128, two CTAs per SM) and now: 50 queries
 // over 1e6 rows 0.92 and 0.17 ms, 4,096 over 2e6 4.35 and 2.04 ms, 100,000 over
 // 4e6 41.1 and 36 to 38 ms.
@@ -663,9 +663,8 @@ __global__ void __launch_bounds__(B_THREADS, 1) k_screen_tc(ScreenArgs A) {
         const uint32_t tb = tmem + ((uint32_t)((warp & 3) * 32) << 16) + ab * BR + c0;
         // A chunk of 32 columns whose maximum reaches the bound holds a
         // candidate, or a row outside the slab that raises it (the appends look
-        // closer).  One chunk in registers at a time: 96 are all a thread has,
-        // and what spills from here comes back from L2 (shared memory takes
-        // the L1's room); the four warps of a scheduler hide the latencies.
+        // closer).  Two chunks are in registers at a time; all four at once
+        // measured the same.
         int cnt = half ? cnt1 : cnt0;
         const float2 qs = sm.qs[L];
         bool any = pilot;
@@ -1101,8 +1100,8 @@ struct TcState {
 
 // Work items of a plan.  Several per SM even out tiles of unequal length; with
 // few queries there are few tiles, cut alike, and every further item only adds
-// its own start, end and lists (50 queries over 1e6 rows: 0.50 ms at one item
-// per SM, 0.60 at three; 4,096 over 2e6: 3.17 and 2.73 ms).
+// its own start, end and lists (100 queries over 1e6 rows: 0.51 ms at one item
+// per SM, 0.63 at four; 5,000 over 1e5 rows 2.27 and 1.89).
 inline uint32_t target_items(const fknn_index *idx, const fknn_tuning &tune, const fknn_tuning &dflt, uint32_t nq) {
   return (uint32_t)idx->num_sms * items_per_sm(tune, dflt, nq);
 }

@@ -12,7 +12,7 @@
 //                     can still reach the running k-th bound are kept in a
 //                     per-(item, query) candidate list; the bound is shared
 //                     across CTAs.  A pilot pass over every pilot_stride-th
-//                     row block seeds the bounds (k_exact_seed).
+//                     row block seeds the bounds (k_screen_seed).
 //   4. k_merge        per query: union of its items' lists, k-th bound, then
 //                     exact re-score of the survivors with the reference's
 //                     sequential arithmetic, (dist, id) order, top-k out.  A
@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(MG_THREADS)
 // its place).  A few queries have blocks of 512 threads, whose eight rows cover
 // the longest slab that is planned for here (longer ones, of queries whose
 // candidates overflowed, select whenever the buffer fills); from SCAN_MANY
-// queries on blocks of 256, of which an SM runs twice as many.  Calls of slabs
+// queries on blocks of 256, of which an SM holds five in place of three.  Calls of slabs
 // of 2,000 to 4,096 rows, by 512 and by 256 threads: 179 and 208 us (100
 // queries), 199 and 222 (300), 257 and 246 (600), 944 and 767 (4,000); of up to
 // 64 rows 748 and 453 (30,000), where 649 was the time with sorts of 1,024 keys.
@@ -463,7 +463,7 @@ __global__ void __launch_bounds__(NT)
 #pragma unroll
           for (int d = 0; d < 25; ++d) v[d] = __ldg(x + (d0 + d) * BLK);
 #pragma unroll
-          for (int d = 0; d < 25; ++d) {  // seq_l2_strided's operations
+          for (int d = 0; d < 25; ++d) {  // seq_l2_row's operations
             float t = __fsub_rn(v[d], sm.qv[d0 + d]);
             t = __fmul_rn(t, t);
             r = __fadd_rn(r, t);
@@ -696,7 +696,7 @@ int count_matches(fknn_index *idx, const float *d_meta, uint32_t nq, uint32_t *d
   return FKNN_OK;
 }
 
-// Groups queries into 64-query tiles whose slabs overlap (same order and
+// Groups queries into tiles (shape.tq of them) whose slabs overlap (same order and
 // predicate class, start bucket, then end), and cuts each tile's union
 // range into row chunks.
 namespace {
@@ -1050,8 +1050,8 @@ int search_exact(fknn_index *idx, const float *d_q, const float *d_meta, uint32_
   shape.min_chunk_blocks = (idx->tuning[FKNN_MODE_EXACT_FP32].min_chunk_blocks + 1) / 2;  // (given in 64-row blocks)
   // Several items per SM even out tiles of unequal length; with few queries
   // there are few tiles, cut alike, and every further item only adds its own
-  // start and end (16 queries over 1e6 rows: 0.82 ms at one item per SM, 1.29
-  // at four; 1e4 queries over 1e5 rows: 3.5 and 3.2 ms).
+  // start and end (100 queries over 1e6 rows: 0.86 ms at one item per SM, 0.99
+  // at five; 1e4 queries over 1e5 rows: 3.5 ms at one, 3.2 at four).
   const uint32_t ips = items_per_sm(idx->tuning[FKNN_MODE_EXACT_FP32], DEFAULT_TUNING[FKNN_MODE_EXACT_FP32], nq);
   Candidate *d_out = nullptr, *d_work = nullptr;
   uint32_t *d_ocnt = nullptr, *d_state, sgrid = 0, nitems = 0;
@@ -1171,13 +1171,12 @@ int search_exact(fknn_index *idx, const float *d_q, const float *d_meta, uint32_
     const uint32_t *big_q = (const uint32_t *)(d_blob + o_big), *big_tile = (const uint32_t *)(d_blob + o_btile),
                    *big_lane = (const uint32_t *)(d_blob + o_blane), *item_slot = (const uint32_t *)(d_blob + o_slot);
     if (pilot) {
-      // Pilot: the same screen over every pstride-th row block.  The r-th
-      // distance of a query's sample seeds its bound: the k-th of all rows
-      // ranks about k / pstride in the sample, and r = 3 k / pstride + 8 lies
-      // above it but for a vanishing fraction of queries, which the merge
-      // finds and the redo pass below screens again without a seed.  The seed
-      // admits about 3 k + 8 pstride rows, a tenth of the pushes that
-      // tracking the k-th from nothing makes.
+      // Pilot: the same screen over every pstride-th row block.  A rank in a
+      // query's sample that lies a little above where the k-th of all its rows
+      // ranks there (exact_seed_rank) seeds its bound; the merge finds the few
+      // queries whose seed is below their k-th all the same, and the redo pass
+      // below screens them again without one.  A seed admits a few times k
+      // rows, a tenth of the pushes that tracking the k-th from nothing makes.
       // (the sample of a short slab is up to twice its nominal share)
       const uint32_t r = exact_seed_rank(k, 2, pstride);
       if ((rc = launch_fill_u32(T_pilot, nq, f32_sortable(INFINITY), st))) return rc;

@@ -61,13 +61,18 @@ __host__ __device__ __forceinline__ float sortable_f32(uint32_t s) {
 }
 __host__ __device__ __forceinline__ uint32_t i32_sortable(int32_t v) { return (uint32_t)v ^ 0x80000000u; }
 
-// Screening error bound.  ds = ||x||^2 + ||q||^2 - 2 q.x, every sum a
-// float FMA chain over 100 terms, differs from the exact real distance by at
-// most gamma_101 (sqrt(xn)+sqrt(qn))^2 + u|ds|, and the reference's
-// sequential float sum (distance.h:62-72) differs from it by at most
-// gamma_102 * d.  With sqrt(xn) <= sqrt(d) + sqrt(qn) both are bounded by a
-// function of ds and qn alone; the constants below carry a factor > 1.5 of
-// slack over gamma_104 = 6.2e-6 (u = 2^-24).
+// Screening error bound of ds = |x|^2 + |q|^2 - 2 q.x against the reference's
+// sequential float sum d (distance.h:62-72), as a function of ds and qn = |q|^2
+// alone (|x| <= sqrt(d) + |q|, so |x| + |q| <= a below).
+//   d itself is within gamma_102 d (6.2e-6) of the real distance: the 1e-5 D.
+//   ds comes from the tensor cores (exact_screen.cu): the fp16 pieces and their
+//   dropped product are within 3 * 2^-22 |q||x|; each of the seven MMA steps at
+//   full size adds 17 terms, and with every term cut at the 24th bit below the
+//   largest they are within 7.1e-6 |q||x|; the norms, rounded once, within 2^-24
+//   of themselves.  Doubled that is below 4e-6 (|x| + |q|)^2, where 2e-5 is
+//   allowed for.  How the tensor cores cut their terms is no documented
+//   property: cut two bits earlier they would still be inside, and measured
+//   against 64 bits the error of ds is at most 3.1e-7 (|x| + |q|)^2.
 __host__ __device__ __forceinline__ float screen_eps(float ds, float qn) {
   float D = fmaxf(ds, 0.f) * 1.0001f + 1e-4f * qn;
   float a = sqrtf(D) + 2.f * sqrtf(qn);
