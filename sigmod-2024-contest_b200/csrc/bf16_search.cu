@@ -311,7 +311,8 @@ struct BScreenSmem {
     float row[B_SLOTS][B_ROW];  // staged chunks
     uint32_t hist[256];         // the histogram of a trim
   } w[B_EPI];
-  float4 q[BQ];      // per query: lowest accumulator value of a candidate, slab (bits), != 0: pilot takes the best of BP
+  float4 q[BQ];      // per query: lowest accumulator value of a candidate, slab (bits), what a pilot keeps: the best of
+                     // every so many rows (BP, 32, 8 or 1)
   float2 qs[BQ];     // |q|^2 (centred for FP8), -2 / lambda
   float thr[BQ];     // current bound T on the k'-th screening distance
   int32_t lq[BQ];
@@ -633,10 +634,21 @@ __global__ void __launch_bounds__(B_THREADS, 1) k_screen_tc(ScreenArgs A) {
         sm.lq[tid] = qi;
         sm.thr[tid] = T;
         sm.qs[tid] = qs;
-        // in the pilot, a slab of many sampled blocks keeps the best of every
-        // BP rows, a shorter one the best of every 32
-        const bool coarse = (e - s) / (BP * A.stride) >= 4 * exact_seed_rank(A.kseed, 1, A.stride);
-        sm.q[tid] = make_float4(acc_bound(T, qs), __uint_as_float(s), __uint_as_float(e), coarse ? 1.f : 0.f);
+        // In the pilot a slab keeps the best of every BP, 32 or 8 of its sampled
+        // rows, or every row, as its length leaves enough of them for the rank:
+        // what has no seed pushes rows by the hundred in the main pass.  (2,000
+        // queries over slabs of 20,000 rows, k' = 400: 3.88 ms with maxima of 32
+        // at least, 0.68 so; 8,000 rows, k' = 200: 1.59 and 0.61.  10,000 queries
+        // over a skewed base of 3e5 rows: screens 2.17 and 1.69 ms, 5.46 and 2.98
+        // at k' = 400.  4,096 over 2e6, few such slabs: 2.11 and 2.15.  Maxima of
+        // 32 from 1.0 or 2.5 to a rank on: 20.1 to 21.3 and 19.8 ms of screens
+        // over 1e6 rows at k' = 400, but 2.24 for the 4,096.)
+        const uint32_t sampled = (e - s) / A.stride, rank = exact_seed_rank(A.kseed, 1, A.stride);
+        sm.q[tid] = make_float4(acc_bound(T, qs), __uint_as_float(s), __uint_as_float(e),
+                                (float)(sampled / BP >= 4 * rank         ? BP
+                                        : sampled / 32 >= rank * 8 / 5   ? 32
+                                        : sampled / 8 >= rank + rank / 5 ? 8
+                                                                         : 1));
       }
       asm volatile("bar.sync 1, %0;" ::"n"(B_EPI * 32) : "memory");
       Candidate *const work = A.work + (uint64_t)blockIdx.x * A.halves * B_LISTS * A.capb;
@@ -668,7 +680,7 @@ __global__ void __launch_bounds__(B_THREADS, 1) k_screen_tc(ScreenArgs A) {
         int cnt = half ? cnt1 : cnt0;
         const float2 qs = sm.qs[L];
         bool any = pilot;
-        const bool fine = pilot && __any_sync(0xffffffffu, q.w == 0.f);
+        const bool fine = pilot && __any_sync(0xffffffffu, q.w <= 32.f);
         float best = -INFINITY;
 #pragma unroll 1
         for (int c = 0; c < BP; c += 64) {
@@ -691,14 +703,20 @@ __global__ void __launch_bounds__(B_THREADS, 1) k_screen_tc(ScreenArgs A) {
           any = true;
           Candidate *const lists = work + (half * B_LISTS + warp * 32) * A.capb;
           const int col0 = c0 + c;
-          if (pilot) {
-            if (q.w == 0.f) {
-              if ((todo & 1u) && col0 >= r0 && col0 + 32 <= r1)
-                lists[lane * A.capb + cnt++] = {fmaf(qs.y, ma, qs.x), p0 + col0};
-              if ((todo & 2u) && col0 + 32 >= r0 && col0 + 64 <= r1)
-                lists[lane * A.capb + cnt++] = {fmaf(qs.y, mb, qs.x), p0 + col0 + 32};
+          if (pilot && q.w > 1.f) {
+            Candidate *const mine = lists + lane * A.capb;
+            if (q.w == 32.f) {
+              if ((todo & 1u) && col0 >= r0 && col0 + 32 <= r1) mine[cnt++] = {fmaf(qs.y, ma, qs.x), p0 + col0};
+              if ((todo & 2u) && col0 + 32 >= r0 && col0 + 64 <= r1) mine[cnt++] = {fmaf(qs.y, mb, qs.x), p0 + col0 + 32};
+            } else if (q.w == 8.f) {
+#pragma unroll
+              for (int j = 0; j < 8; ++j) {
+                const float m = j < 4 ? ga[j] : gb[j - 4];
+                const int c8 = col0 + 8 * j;
+                if (m >= bound && c8 >= r0 && c8 + 8 <= r1) mine[cnt++] = {fmaf(qs.y, m, qs.x), p0 + c8};
+              }
             }
-            continue;
+            todo = 0;
           }
           // One that passes on its own, as in most chunks: it is the maximum,
           // and its lane appends it by itself if it is inside the slab.  The
@@ -754,7 +772,7 @@ __global__ void __launch_bounds__(B_THREADS, 1) k_screen_tc(ScreenArgs A) {
           }
         }
         if (any) {
-          if (pilot && q.w != 0.f && best >= bound && c0 >= r0 && c0 + BP <= r1)
+          if (pilot && q.w == (float)BP && best >= bound && c0 >= r0 && c0 + BP <= r1)
             work[(half * B_LISTS + tid) * A.capb + cnt++] = {fmaf(qs.y, best, qs.x), p0 + c0};
           Candidate *const lists = work + (half * B_LISTS + warp * 32) * A.capb;
           // lists that could overflow next are trimmed (a product adds at most BP)
@@ -1194,9 +1212,10 @@ int build_fp8(fknn_index *idx, cudaStream_t st) {
 }
 
 // The pilot, its seeds and the screen proper.  The pilot keeps the best of
-// every 32 rows of every stride-th row block: as the few rows that matter lie
-// in different groups as a rule, the r-th best of these is little above the
-// r-th of the sample's rows (and never below it), at a 32nd of the entries.
+// every 128, 32 or 8 rows of every stride-th row block: as the few rows that
+// matter lie in different groups as a rule, the r-th best of these is little
+// above the r-th of the sample's rows (and never below it), at a fraction of the
+// entries.  Where even that leaves too few for the rank it keeps every row.
 template <class K>
 static void launch_screens(K screen, ScreenArgs X, SeedArgs Z, const TcState &S, uint32_t kprime, uint32_t stride,
                            uint32_t refresh, bool withhold, uint32_t grid, uint32_t nbig_max, size_t smem,

@@ -136,3 +136,28 @@ def test_captured_plan_of_many_short_categories():
     got, got_d = oracle.exact_knn(vecs, labels, ts, q, metas, k=k)
     np.testing.assert_array_equal(ids, got)
     np.testing.assert_array_equal(dists, got_d)
+
+
+def test_slabs_around_the_pilots_forms():
+    """Slabs whose sample is ranked by rows and by the best of every 8, 32 and
+    128: all are seeded, so none falls to the exact scan, and the answers are
+    the oracle's."""
+    rng = np.random.default_rng(23)
+    sizes = [4100, 4300, 6300, 7000, 10_000, 12_500, 17_600, 26_000, 31_000, 70_000]
+    labels = np.repeat(np.arange(len(sizes)), sizes).astype(np.float32)
+    n, nq = len(labels), 900
+    vecs, q = grid(rng, (n, 100)), grid(rng, (nq, 100))
+    ts = rng.random(n, dtype=np.float32)
+    metas = np.full((nq, 4), -1, np.float32)
+    metas[:, 0] = 1
+    metas[:, 1] = np.arange(nq) % len(sizes)
+    ids, dists = oracle.exact_knn(vecs, labels, ts, q, metas, k=100)
+    with fknn.Index(vecs, labels, ts, build_bf16=True) as idx:
+        for kprime in (128, 400, 1024):
+            for m in (9, nq):
+                for graph in (False, True):
+                    got, d, st = idx.search(q[:m], metas[:m], k=100, mode=fknn.MODE_BF16_RERANK, kprime=kprime, graph=graph,
+                                            return_stats=True)
+                    np.testing.assert_array_equal(got, ids[:m])
+                    np.testing.assert_array_equal(d, dists[:m])
+                    assert st["n_overflow"] <= m // 100, (kprime, m, graph, st)
