@@ -69,7 +69,7 @@ typedef struct fknn_tuning {
   uint32_t list_slack;       /* BF16/FP8: candidate-list room beyond k' between trims, rows (>= 256) */
   uint32_t items_per_sm;     /* contraction work items per SM: load balance against candidate traffic
                                 (the default, 4 exact and 3 BF16/FP8, counts as 1 in calls of fewer
-                                than 1,024 queries; another value holds for every call) */
+                                than 1,024 and 800 queries; another value holds for every call) */
   uint32_t min_chunk_blocks; /* shortest row chunk of a work item, in row blocks (64 rows exact, 128 BF16/FP8) */
   uint32_t bound_refresh;    /* BF16/FP8: 128-row sub-tiles between reloads of the shared per-query bound (0 = at trims) */
   uint32_t pilot_stride;     /* a pilot pass over every pilot_stride-th row block first seeds the bounds with an

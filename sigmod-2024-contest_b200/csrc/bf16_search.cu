@@ -1118,10 +1118,10 @@ struct TcState {
 
 // Work items of a plan.  Several per SM even out tiles of unequal length; with
 // few queries there are few tiles, cut alike, and every further item only adds
-// its own start, end and lists (100 queries over 1e6 rows: 0.51 ms at one item
-// per SM, 0.63 at four; 5,000 over 1e5 rows 2.27 and 1.89).
-inline uint32_t target_items(const fknn_index *idx, const fknn_tuning &tune, const fknn_tuning &dflt, uint32_t nq) {
-  return (uint32_t)idx->num_sms * items_per_sm(tune, dflt, nq);
+// its own start, end and lists (100 queries over 1e6 rows: 0.46 ms at one item
+// per SM, 0.54 at four; 5,000 over 1e5 rows 1.50 and 1.06).
+inline uint32_t target_items(const fknn_index *idx, const fknn_tuning &tune, int mode, uint32_t nq) {
+  return (uint32_t)idx->num_sms * items_per_sm(tune, mode, nq);
 }
 
 // Work items a tile may have: what the merge holds of their lists, and the
@@ -1289,7 +1289,7 @@ static int search_tc(fknn_index *idx, const float *d_q, const float *d_meta, uin
     ocap = tight ? tight_cap(kprime, capb) : capb;
     const uint64_t per_item = (uint64_t)BQ * ocap * sizeof(Candidate);
     shape.max_items_per_tile = tight ? 1u : max_items(per_item, tiles_est);
-    shape.target_items = tight ? 1u : target_items(idx, tune, DEFAULT_TUNING[mode], nq);
+    shape.target_items = tight ? 1u : target_items(idx, tune, mode, nq);
     make_plan(h_desc, h_meta, nq, n, shape, P);
     nitems = (uint32_t)P.items.size();
     for (const Tile &t : P.tiles)
@@ -1498,7 +1498,7 @@ static int search_tc_graph(fknn_index *idx, const float *d_q, const float *d_met
   if ((rc = ws_get(idx, 5, TcState::bytes(nq), (void **)&d_state))) return rc;
   for (int tight = 0;; ++tight) {
     ocap = tight ? tight_cap(kprime, capb) : capb;
-    shape.target_items = tight ? 1u : target_items(idx, tune, DEFAULT_TUNING[mode], nq);
+    shape.target_items = tight ? 1u : target_items(idx, tune, mode, nq);
     z = device_plan_sizes(idx, nq, shape);
     shape.max_items_per_tile =
         tight ? 1u : max_items((uint64_t)BQ * ocap * sizeof(Candidate), z.ntile_max);

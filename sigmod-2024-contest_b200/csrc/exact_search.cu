@@ -1052,7 +1052,7 @@ int search_exact(fknn_index *idx, const float *d_q, const float *d_meta, uint32_
   // there are few tiles, cut alike, and every further item only adds its own
   // start and end (100 queries over 1e6 rows: 0.86 ms at one item per SM, 0.99
   // at five; 1e4 queries over 1e5 rows: 3.5 ms at one, 3.2 at four).
-  const uint32_t ips = items_per_sm(idx->tuning[FKNN_MODE_EXACT_FP32], DEFAULT_TUNING[FKNN_MODE_EXACT_FP32], nq);
+  const uint32_t ips = items_per_sm(idx->tuning[FKNN_MODE_EXACT_FP32], FKNN_MODE_EXACT_FP32, nq);
   Candidate *d_out = nullptr, *d_work = nullptr;
   uint32_t *d_ocnt = nullptr, *d_state, sgrid = 0, nitems = 0;
   unsigned char *d_blob;

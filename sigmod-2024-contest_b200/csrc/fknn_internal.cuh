@@ -260,15 +260,16 @@ struct HostBuf {
 // The tuning an index starts with, by mode (exact, BF16, FP8), and the work
 // items per SM of a call: below ITEMS_MIN_QUERIES queries the default is one
 // (another value is the caller's and holds for every call).  Both sides of the
-// line, one item per SM and several: exact over 1e6 rows 1.49 and 1.48 ms
-// (1,000 queries), 1.74 and 1.82 (1,600), 3.14 and 3.12 (5,000); BF16 1.05 and
-// 1.10, 1.41 and 1.49, 2.71 and 2.84.  Over 1e5 rows exact 0.69 and 0.70, 0.74
-// and 0.75, 1.48 and 1.36; BF16 would take several from 600 queries on (0.69
-// and 0.65 ms, 0.93 and 0.75 at 1,000).
+// lines, one item per SM and several, ms: exact over 1e6 rows 1.29 and 1.38 (800
+// queries), 1.48 and 1.47 (1,000), 1.73 and 1.82 (1,600), 3.15 and 3.14 (5,000),
+// over 1e5 rows 0.54 and 0.62, 0.69 and 0.72, 0.74 and 0.75, 1.49 and 1.35; BF16
+// (k' = 200) over 1e6 rows 0.83 and 0.81 (600), 0.94 and 0.93 (1,000), 2.32 and
+// 2.39 (5,000), over 1e5 rows 0.40 and 0.43, 0.72 and 0.51, 1.50 and 1.06, on a
+// skewed base of 1e5 rows 0.40 and 0.43 (600), 0.50 and 0.46 (800), 0.55 and 0.49.
 constexpr fknn_tuning DEFAULT_TUNING[3] = {{0, 4, 32, 0, 32}, {256, 3, 8, 0, 8}, {256, 3, 8, 0, 8}};
-constexpr uint32_t ITEMS_MIN_QUERIES = 1024;
-inline uint32_t items_per_sm(const fknn_tuning &t, const fknn_tuning &dflt, uint32_t nq) {
-  return nq < ITEMS_MIN_QUERIES && t.items_per_sm == dflt.items_per_sm ? 1u : t.items_per_sm;
+constexpr uint32_t ITEMS_MIN_QUERIES[3] = {1024, 800, 800};
+inline uint32_t items_per_sm(const fknn_tuning &t, int mode, uint32_t nq) {
+  return nq < ITEMS_MIN_QUERIES[mode] && t.items_per_sm == DEFAULT_TUNING[mode].items_per_sm ? 1u : t.items_per_sm;
 }
 
 }  // namespace fknn
